@@ -45,15 +45,16 @@ size_t cholesky_work_bytes(int ld, int precision) {
   return (size_t)(ld / NB) * NB * NB * es + df_work_bytes(ld);
 }
 
-// Factors A in place with the data-flow kernel and leaves the inverted
-// diagonal tiles of the factor at the start of `work` (used by the SPD inverse
-// and the triangular solve of the midpoint scheme).
-int launch_cholesky_ws(void* A, int n, int ld, int precision, int* info, void* work, cudaStream_t st) {
+// Factors A in place with the data-flow kernel; with want_inv the inverted
+// diagonal tiles of the factor are left at the start of `work` (used by the
+// triangular solve of the midpoint scheme).
+int launch_cholesky_ws(void* A, int n, int ld, int precision, int* info, void* work, cudaStream_t st,
+                       bool want_inv) {
   if (ld % NB != 0 || n > ld || n < 0) return PBG_ERR_ARG;
   const size_t es = precision == PBG_PREC_FP64 ? 8 : 4;
   unsigned char* inv_tiles = static_cast<unsigned char*>(work);
   unsigned char* df = inv_tiles + (size_t)(ld / NB) * NB * NB * es;
-  return launch_cholesky_df(A, n, ld, precision, info, inv_tiles, df, st);
+  return launch_cholesky_df(A, n, ld, precision, info, inv_tiles, want_inv, df, st);
 }
 
 // Workspace: the factorisation's (inv(L_kk) tiles, data-flow scratch), then
@@ -69,7 +70,8 @@ int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStre
   unsigned char* w = static_cast<unsigned char*>(work);
   double* inv = reinterpret_cast<double*>(w);
   double* X = reinterpret_cast<double*>(w + spd_x_offset(ld));
-  int rc = launch_cholesky_df(A, n, ld, PBG_PREC_FP64, info, inv, w + (size_t)nt * NB * NB * sizeof(double), st, X);
+  int rc = launch_cholesky_df(A, n, ld, PBG_PREC_FP64, info, inv, true,
+                              w + (size_t)nt * NB * NB * sizeof(double), st, X);
   if (rc != PBG_OK) return rc;
   if ((rc = launch_trtri_diag(inv, X, ld, PBG_PREC_FP64, st))) return rc;
   return launch_lauum_tc(X, ld, 1.0, false, A, PBG_PREC_FP64, st);

@@ -4,33 +4,32 @@
 // Single matrix: one persistent kernel, all CTAs co-resident (cooperative
 // launch), one CTA per SM.  The 64 x 64 tiles of the lower triangle are
 // processed as tasks:
-//   F(k)     diagonal tile k: its last update (column k-1), then the
-//            factorisation by 8-column panels (each 8 x 8 pivot block
-//            factored in registers, rank-8 trailing updates by the other
-//            warps) and the explicit inverse inv(L_kk);
+//   F(k)     diagonal tile k: its last update (column k-1), the factorisation
+//            by 8-column panels, and the solve blocks of L_kk (factor_tile);
 //   S(i, k)  tile (i, k) below the diagonal: its last update, then
-//            L_ik = A_ik inv(L_kk)^T as one tile product;
+//            L_ik = A_ik L_kk^-T by forward substitution with 8 x 8 blocks
+//            (solve_rows);
 //   U(i,j,k) trailing update A_ij -= L_ik L_jk^T (j >= k+2): FP64 DMMA
 //            (mma.sync m8n8k4 f64) in the FP64 path; in the mixed path
 //            3xTF32 split products (hi*hi + hi*lo + lo*hi) on the tcgen05
 //            tensor cores, up to four rows per task, accumulated in TMEM
-//            (tc_tile.cuh).
-// The FP64 path factors and inverts the diagonal tiles in FP64; the mixed
-// path (FP32 matrix) does both in FP32 on the chain CTA (run_chain_f32), or
-// in FP64 rounded to FP32 on store (PBG_PREC_MIXED_FP64_DIAG).
+//            (tc_tile.cuh);
+//   LEAD(k)  row k+2 of panel k: S(k+2, k), U(k+2, k+1, k), U(k+2, k+2, k) as
+//            one task, because the chain waits for them;
+//   I(k)     inv(L_kk), only when the caller wants the inverted diagonal tiles.
+// The FP64 path factors the diagonal tiles in FP64; the mixed path (FP32
+// matrix) in FP32, or in FP64 rounded to FP32 on store
+// (PBG_PREC_MIXED_FP64_DIAG).
 //
 // The critical path of the factorisation is F(0), S(1,0), F(1), S(2,1), ...:
 // block 0 (the chain CTA) runs exactly that sequence and keeps what one step
-// hands to the next in shared memory (L(k, k-1) for the update of F(k) and
-// S(k+1, k); inv(L_kk) for S(k+1, k)), so the chain never waits on a round
+// hands to the next in shared memory (the solve blocks for S(k+1, k);
+// L(k+1, k) for the update of F(k+1)), so the chain never waits on a round
 // trip through L2.  The other CTAs take the remaining tasks in a fixed order
-// from an atomic counter: S(., 0), then for each k the solves S(i, k+1)
-// (i >= k+3) and the updates U(., ., k), the update that gates the next panel
-// first; the last update of the chain's next solve S(k+2, k+1) leads the list
-// for panel k.  With an output X (the SPD inverse) the same list also forms
-// X = inv(L) (XG / XZ tasks).  Every task depends only on chain tasks and on
-// tasks earlier in the list, so with all CTAs resident the lowest unfinished
-// task can always run.
+// from an atomic counter (df_task_list).  With an output X (the SPD inverse)
+// the same list also forms X = inv(L) (XG / XZ tasks).  Every task depends only
+// on chain tasks and on tasks earlier in the list, so with all CTAs resident
+// the lowest unfinished task can always run.
 //
 // Batches of independent matrices: FP64 right-looking tile tasks
 // (chol_batch_kernel<double>); mixed left-looking tasks that accumulate a
@@ -67,6 +66,9 @@ enum : int { TASK_F = 0, TASK_S = 1, TASK_U = 2, TASK_I = 3, TASK_U2 = 4, TASK_U
 // XG / XZ: the tasks that form X = inv(L) in the same list (single-matrix
 // lists of an SPD inverse only; see inverse_update / inverse_finish).
 enum : int { TASK_XG = 7, TASK_XZ = 8 };
+// LEAD(k): the tile row k + 2 of panel k, on which the chain's next step waits
+// (lead_task).
+enum : int { TASK_LEAD = 9 };
 
 struct DFArgs {
   void* A;
@@ -76,7 +78,8 @@ struct DFArgs {
   int* upd;      // nt * nt
   int* fin;      // nt * nt
   int* info;
-  void* invdiag; // nt * 64 * 64 (T): inv(L_kk), row-major tiles
+  void* invdiag; // nt * 64 * 64: inv(L_kk), row-major tiles (I tasks)
+  void* lp;      // nt * 64 * 64: the solve blocks of L_kk (factor_tile)
   unsigned* err;
   long long spin_limit;  // polls before a wait gives up
   void* X;       // or null: X = inv(L) is formed too (off-diagonal tiles of the ld x ld matrix)
@@ -385,69 +388,6 @@ __device__ __forceinline__ void load_and_update(const DFArgs& a, int i, int j, i
   __syncthreads();
 }
 
-// ---------------------------------------------------------------- F(k)
-template <typename T>
-__device__ __forceinline__ T rsqrt_t(T x);
-// 1/sqrt(x) for the FP64 pivots: the PTX rsqrt.approx.ftz.f64 estimate
-// refined by two Newton-Raphson steps y <- y + y (1 - x y^2) / 2, which
-// converge quadratically to full precision (measured <= 1.24 ulp over
-// [1e-30, 1e30] against a long-double reference; the library call measured
-// about 100 cycles more per pivot inside the pivot-block code).  For positive
-// normal x: subnormals are flushed to zero and x <= 0 gives inf or NaN, which
-// the factorisation reports as a non-positive pivot before it is used.
-__device__ __forceinline__ double rsqrt_nr(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
-  return fma(0.5 * y, fma(-x * y, y, 1.0), y);
-}
-template <>
-__device__ __forceinline__ double rsqrt_t<double>(double x) { return rsqrt_nr(x); }
-
-
-// Panel strip row length: 8 values padded so that 16-byte row loads and the
-// tensor-core fragment loads of eight different rows hit distinct banks.
-template <typename T> struct Strip { static constexpr int PB = sizeof(T) == 8 ? 10 : 12; };
-
-// Shared memory of factor_tile besides Lk and X: two panel strips
-// (alternating; reused as scratch by the inversion), the reciprocal pivots.
-template <typename T>
-constexpr int factor_smem_elems() { return 2 * NB * Strip<T>::PB + NB; }
-
-// Rank-8 update acc -= Pr Pc^T of the calling warp's 16 x 32 block on the
-// tensor cores, Pr / Pc rows = the block's rows / columns of the panel strip
-// P (8 values each).  Strip rows below `lo` are read as zero, so columns
-// before the trailing part (and rows above it) are left unchanged.
-__device__ __forceinline__ void strip_update(const double* P, int lo, double acc[16]) {
-  constexpr int PB = Strip<double>::PB;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int m0 = 16 * (w >> 1), n0 = 32 * (w & 1), g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int k0 = 0; k0 < 8; k0 += 4) {
-    double a[2], b[4];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-      const int r = m0 + 8 * mt + g;
-      a[mt] = r >= lo ? -P[r * PB + k0 + t] : 0.0;
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int c = n0 + 8 * nt + g;
-      b[nt] = c >= lo ? P[c * PB + k0 + t] : 0.0;
-    }
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        double& c0 = acc[(mt * 4 + nt) * 2];
-        double& c1 = acc[(mt * 4 + nt) * 2 + 1];
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                     : "+d"(c0), "+d"(c1)
-                     : "d"(a[mt]), "d"(b[nt]));
-      }
-  }
-}
-
 // One warp's output tile D = A B of a small smem product on the tensor cores:
 // A rows with stride lda (k contiguous), B k-major rows with stride ldb, K a
 // multiple of 4: an 8 x 8 FP64 tile (mma m8n8k4), lane holds D[g][2t + h].
@@ -588,245 +528,6 @@ __device__ __forceinline__ void store_inverse(const DFArgs& a, int k, const T* L
   }
 }
 
-// The eight 8 x 8 diagonal blocks of inv(L) (L in Lk, Rinv = 1 / L_jj) into
-// XL[b][i][c] (8 x 8 x 8 doubles): warp b, lane c < 8 solves column c by
-// forward substitution.  The caller orders XL's readers after a CTA barrier.
-__device__ __forceinline__ void leaf_inverses(const double* Lk, const double* Rinv, double* XL) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane < 8) {
-    const double* D = Lk + 8 * warp * LDA + 8 * warp;
-    const double* R = Rinv + 8 * warp;
-    double x[8];
-#pragma unroll
-    for (int ii = 0; ii < 8; ++ii) {
-      double sacc = 0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (q < ii && q >= lane) sacc += D[ii * LDA + q] * x[q];
-      x[ii] = ii < lane ? 0.0 : (ii == lane ? R[ii] : -sacc * R[ii]);
-    }
-#pragma unroll
-    for (int ii = 0; ii < 8; ++ii) XL[warp * 64 + ii * 8 + lane] = x[ii];
-  }
-}
-
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
-// C <- C inv(L)^T for the 64 x 64 tile C (T, [64][LDA] smem) by blocked
-// forward substitution in FP64 on the tensor cores: warp w owns rows
-// 8w .. 8w+7 and, for each 8-column block j,
-//   W_j = (C_j - W_{<j} L_{j,<j}^T) inv(L_jj)^T,
-// where W ([64][LDA] doubles) holds the rows in FP64 (W may alias C when T
-// is double).  L: [64][LDA] doubles, XL: leaf_inverses.  Only warp-level
-// synchronisation: every warp reads its own rows, L and XL.
-template <typename T>
-__device__ __forceinline__ void trsm_rows(const double* L, const double* XL, T* C, double* W) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int r0 = 8 * warp;
-  if constexpr (sizeof(T) != sizeof(double)) {
-#pragma unroll 4
-    for (int e = lane; e < 8 * NB; e += 32) W[(r0 + (e >> 6)) * LDA + (e & 63)] = (double)C[(r0 + (e >> 6)) * LDA + (e & 63)];
-    __syncwarp();
-  }
-  double* Wr = W + r0 * LDA;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int c0 = 8 * j;
-    // the update's operands first, then its 2j products on four accumulators
-    double av[14], bv[14];
-    const double* Lj = L + (c0 + g) * LDA;
-#pragma unroll
-    for (int q = 0; q < 2 * j; ++q) {
-      av[q] = -Wr[g * LDA + 4 * q + t];
-      bv[q] = Lj[4 * q + t];
-    }
-    double d[4][2] = {{Wr[g * LDA + c0 + 2 * t], Wr[g * LDA + c0 + 2 * t + 1]}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-    for (int q = 0; q < 2 * j; ++q) dmma(d[q & 3], av[q], bv[q]);
-    __syncwarp();
-    Wr[g * LDA + c0 + 2 * t] = (d[0][0] + d[1][0]) + (d[2][0] + d[3][0]);
-    Wr[g * LDA + c0 + 2 * t + 1] = (d[0][1] + d[1][1]) + (d[2][1] + d[3][1]);
-    __syncwarp();
-    // times inv(L_jj)^T: B[k][n] = XL[j][n][k]
-    double e0[2] = {0.0, 0.0}, e1[2] = {0.0, 0.0};
-    const double a0 = Wr[g * LDA + c0 + t], a1 = Wr[g * LDA + c0 + 4 + t];
-    const double b0 = XL[j * 64 + g * 8 + t], b1 = XL[j * 64 + g * 8 + 4 + t];
-    dmma(e0, a0, b0);
-    dmma(e1, a1, b1);
-    __syncwarp();
-    Wr[g * LDA + c0 + 2 * t] = e0[0] + e1[0];
-    Wr[g * LDA + c0 + 2 * t + 1] = e0[1] + e1[1];
-    __syncwarp();
-  }
-  if constexpr (sizeof(T) != sizeof(double)) {
-#pragma unroll 4
-    for (int e = lane; e < 8 * NB; e += 32) C[(r0 + (e >> 6)) * LDA + (e & 63)] = (T)W[(r0 + (e >> 6)) * LDA + (e & 63)];
-  }
-}
-
-// Factor the 64 x 64 tile held in acc (already fully updated) in T arithmetic,
-// by eight 8-column panels.  Per panel p (columns c0 = 8p .. c0+7):
-//  1. the owners copy the panel's column strip (rows >= c0) to shared memory;
-//  2. warps 0 and 1 each factor the 8 x 8 diagonal block -- every lane holds
-//     the whole block and factors it in its own registers, so the pivot chain
-//     is rsqrt -> multiply -> FMA with no shuffles -- and then each lane
-//     solves one strip row below it against the block (L_r = A_r L_pp^-T);
-//  3. every owner takes its final strip values back, and the warps whose
-//     16 x 32 block has trailing elements apply the rank-8 update on the
-//     tensor cores (strip_update).
-// Two CTA barriers per panel (the strips alternate between two buffers).
-// Then L_kk (upper triangle zeroed) goes to global memory and to Lk
-// ([64][LDA] smem), and its inverse is formed in X ([64][LDA] smem) and
-// written to the global invdiag array.  Ends with a CTA barrier.
-// T is the arithmetic, S the type of the matrix in global memory (the mixed
-// path factors its FP32 diagonal tiles in FP64 and stores them rounded).
-// Optional early fetch of the chain's next solve input during F(k): at the
-// start of the last panel, if *flag >= target, the tile src is staged into dst
-// ([64][LDA]) with cp.async and *ready is set (read after the tile's final
-// barrier).
-template <typename S>
-struct SolveInput {
-  const int* flag;
-  int target;
-  const S* src;
-  int ld;
-  S* dst;
-  int* ready;
-};
-
-template <typename T, typename S = T, bool INVERSE = true>
-__device__ __forceinline__ void factor_tile(const DFArgs& a, int k, T acc[16], T* fs, T* Lk, T* X,
-                                            const SolveInput<S>* pre = nullptr) {
-  constexpr int PB = Strip<T>::PB;
-  T* Rinv = fs + 2 * NB * PB;  // [64] 1 / L_jj
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
-#pragma unroll 1
-  for (int p = 0; p < 8; ++p) {
-    const int c0 = 8 * p;
-    T* P = fs + (p & 1) * NB * PB;
-    // this panel's columns are the accumulator column pair (c0 - n0) / 8 of
-    // the warps with n0 <= c0 < n0 + 32
-    const bool owner = c0 >= n0 && c0 < n0 + 32;
-    const int pair = (c0 - n0) >> 3;
-    if (owner) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q == pair)
-#pragma unroll
-          for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int r = acc_row(rs), cs = 2 * q + h;
-              if (r >= c0) P[r * PB + acc_col(cs) - c0] = acc[TileMMA<T>::idx(rs, cs)];
-            }
-    }
-    // warp 7 has no trailing update in the last panel: it polls the flag
-    // before the barrier, takes the value after it and stages the tile
-    int pre_v = 0;
-    if (pre && p == 7 && tid == 32 * 7) pre_v = ld_acquire(pre->flag);
-    __syncthreads();
-    if (pre && p == 7 && warp == 7) {
-      const int v = __shfl_sync(0xffffffffu, pre_v, 0);
-      __syncwarp();  // lane 0's acquire orders the other lanes' copies
-      const bool go = v >= pre->target;
-      if (go) {
-        constexpr int per_row = NB * (int)sizeof(S) / 16, elems = 16 / (int)sizeof(S);
-        for (int c = lane; c < NB * per_row; c += 32) {
-          const int r = c / per_row, cc = (c % per_row) * elems;
-          cp_async16(pre->dst + r * LDA + cc, pre->src + (size_t)r * pre->ld + cc);
-        }
-      }
-      if (lane == 0) *pre->ready = go ? 1 : 0;
-    }
-    if (warp < 2) {
-      // the diagonal block, in every lane (upper entries are not used)
-      T l[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) lds_vec(P + (c0 + i) * PB, l[i]);
-      const int r0 = c0 + 8 + 32 * warp + lane;
-      const bool v0 = r0 < NB;
-      T x0[8];
-      if (v0) lds_vec(P + r0 * PB, x0);
-      else
-#pragma unroll
-        for (int c = 0; c < 8; ++c) x0[c] = T(0);
-      // right-looking 8 x 8 Cholesky; a non-positive pivot is recorded and
-      // reported after the block
-      int bad = -1;
-      T rinv[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const T d = l[j][j];
-        if (!(d > T(0)) && bad < 0) bad = j;
-        const T rs = rsqrt_t<T>(d);
-        rinv[j] = rs;
-        l[j][j] = d * rs;
-#pragma unroll
-        for (int i = j + 1; i < 8; ++i) l[i][j] *= rs;
-#pragma unroll
-        for (int i = j + 1; i < 8; ++i)
-#pragma unroll
-          for (int c = j + 1; c <= i; ++c) l[i][c] -= l[i][j] * l[c][j];
-      }
-      // the strip row below the block: x = a L_pp^-T by forward substitution
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        x0[j] *= rinv[j];
-#pragma unroll
-        for (int c = j + 1; c < 8; ++c) x0[c] -= x0[j] * l[c][j];
-      }
-      if (v0)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) P[r0 * PB + c] = x0[c];
-      if (warp == 0 && lane == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) P[(c0 + i) * PB + c] = c <= i ? l[i][c] : T(0);
-          Rinv[c0 + i] = rinv[i];
-        }
-        if (bad >= 0 && k * NB + c0 + bad < a.n) atomicCAS(a.info, 0, k * NB + c0 + bad + 1);
-      }
-    }
-    __syncthreads();
-    // final values of this panel's strip back into the accumulators
-    if (owner) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q == pair)
-#pragma unroll
-          for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int r = acc_row(rs), cs = 2 * q + h;
-              if (r >= c0) acc[TileMMA<T>::idx(rs, cs)] = P[r * PB + acc_col(cs) - c0];
-            }
-    }
-    // trailing elements (c >= c0 + 8, r >= c) exist in this warp's block?
-    const int lo = c0 + 8;
-    if (m0 + 15 >= lo && m0 + 15 >= n0 && n0 + 31 >= lo) strip_update(P, lo, acc);
-    // no barrier here: the next panel writes the other strip buffer, and the
-    // two barriers of that panel separate these reads from its next reuse
-  }
-  S* g = tile<S>(a, k, k);
-#pragma unroll
-  for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-    for (int cs = 0; cs < 8; ++cs) {
-      const int r = acc_row(rs), c = acc_col(cs);
-      const T v = c <= r ? acc[TileMMA<T>::idx(rs, cs)] : T(0);
-      g[(size_t)r * a.ld + c] = (S)v;
-      Lk[r * LDA + c] = v;
-    }
-  __syncthreads();
-  if constexpr (INVERSE) store_inverse<T, S>(a, k, Lk, Rinv, X, fs);
-}
-
 // acc = -(acc + ...) helpers for S: acc = C inv(L_kk)^T with C, X in smem.
 template <typename T>
 __device__ __forceinline__ void solve_by_inverse(const T* C, const T* X, T acc[16]) {
@@ -846,11 +547,784 @@ __device__ __forceinline__ void smem_to_acc(const T* s, T acc[16]) {
 }
 
 template <typename T>
-__device__ __forceinline__ void acc_to_smem(const T acc[16], T* s) {
+__device__ __forceinline__ void acc_to_smem(const T acc[16], T* s, int lds = LDA) {
 #pragma unroll
   for (int rs = 0; rs < 2; ++rs)
 #pragma unroll
-    for (int cs = 0; cs < 8; ++cs) s[acc_row(rs) * LDA + acc_col(cs)] = acc[TileMMA<T>::idx(rs, cs)];
+    for (int cs = 0; cs < 8; ++cs) s[acc_row(rs) * lds + acc_col(cs)] = acc[TileMMA<T>::idx(rs, cs)];
+}
+
+// ---------------------------------------------------------------- F(k)
+// The factorisation's critical path runs through the diagonal tiles: their
+// 64 pivots are one dependent chain.  What a column costs is latency, not
+// work (a 64 x 64 tile is 0.09 MFLOP), so everything here is arranged around
+// the chain: LDL^T pivots (one reciprocal per column; the square roots are
+// taken for all 64 columns at once afterwards), no hand-over between warps
+// inside an 8-column panel, one CTA-level barrier per panel, and the trailing
+// update one panel behind on the other warps.  Measured (order 1856, one B200
+// at 1965 MHz): FP64 F(k) 7.7 us against 11.7 with rsqrt pivots and two
+// barriers per panel (a chain step, F to F, 13.5 us against 19.2); FP32 7.0 us
+// against 9.6 with the explicit inverse that the solves below do without (a
+// step 12.2 us against 15.8).  What is left of F(k) is the panels' hand-overs
+// through shared memory (about 1350 cycles a panel, of which the pivot chain
+// 430 in FP64).
+
+// Rows of a staged tile in the chain's shared memory (LT) and of the 8-wide
+// strips (MS): 16-byte fragment loads of two FP64 rows fall on different banks.
+template <typename T> struct ChainLd;
+template <> struct ChainLd<double> { static constexpr int LT = NB + 8, MS = 10; };
+template <> struct ChainLd<float> { static constexpr int LT = NB + 4, MS = 12; };
+
+// 1 / d and 1 / sqrt(d) of a pivot.  FP64: the PTX approximations refined to
+// full precision -- the reciprocal by one third-order step
+// y <- y + y (e + e^2), e = 1 - d y (from ~2^-20 to ~2^-60), the square root by
+// two Newton-Raphson steps y <- y + y (1 - d y^2) / 2.  FP32: the MUFU
+// estimates (1 ulp; 2^-22).  d <= 0, NaN and subnormal d give values that are
+// reported as a non-positive pivot and not used.
+__device__ __forceinline__ double pivot_rcp(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ float pivot_rcp(float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return y;
+}
+__device__ __forceinline__ double pivot_rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  return fma(0.5 * y, fma(-x * y, y, 1.0), y);
+}
+__device__ __forceinline__ float pivot_rsqrt(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// A pivot below the smallest normal float (FP32), not positive, or NaN.
+__device__ __forceinline__ bool pivot_bad(double d) { return !(d > 0.0); }
+__device__ __forceinline__ bool pivot_bad(float d) { return !(d >= 1.17549435e-38f); }
+
+// Named barriers (0 is __syncthreads); __syncwarp first reconverges a warp
+// after divergent code (the barrier instructions are warp-aligned).
+__device__ __forceinline__ void bar_wait(int id, int count) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// d -= A B^T for 8 x 8 blocks in shared memory, lane (g, t) = (lane / 4,
+// lane % 4) holding d[h] = D[g][2t + h].  FP64: two DMMAs on separate
+// accumulators; the K slots (t, first / second MMA) take columns 2t and 2t + 1,
+// so each operand is one 16-byte load.  FP32: dot products on the FMA pipe.
+// Operands are loaded first (load_a, load_b) so that several blocks' loads,
+// products and stores overlap.
+template <typename T> struct Block;
+template <> struct Block<double> {
+  struct Op { double2 v; };
+  static __device__ __forceinline__ Op load_a(const double* A, int lda) {
+    const int lane = threadIdx.x & 31;
+    return Op{*reinterpret_cast<const double2*>(A + (lane >> 2) * lda + 2 * (lane & 3))};
+  }
+  using OpB = Op;
+  static __device__ __forceinline__ OpB load_b(const double* B, int ldb) { return load_a(B, ldb); }
+  static __device__ __forceinline__ void sub(double (&d)[2], const Op& a, const OpB& b) {
+    double e[2] = {0.0, 0.0};
+    dmma(e, -a.v.y, b.v.y);
+    dmma(d, -a.v.x, b.v.x);
+    d[0] += e[0];
+    d[1] += e[1];
+  }
+};
+template <> struct Block<float> {
+  struct Op { float v[8]; };
+  struct OpB { float v[8], w[8]; };
+  static __device__ __forceinline__ Op load_a(const float* A, int lda) {
+    Op o;
+    lds_vec(A + ((threadIdx.x & 31) >> 2) * lda, o.v);
+    return o;
+  }
+  static __device__ __forceinline__ OpB load_b(const float* B, int ldb) {
+    OpB o;
+    lds_vec(B + 2 * (threadIdx.x & 3) * ldb, o.v);
+    lds_vec(B + (2 * (threadIdx.x & 3) + 1) * ldb, o.w);
+    return o;
+  }
+  static __device__ __forceinline__ void sub(float (&d)[2], const Op& a, const OpB& b) {
+    float e0 = 0.0f, e1 = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      d[0] = fmaf(-a.v[q], b.v[q], d[0]);
+      d[1] = fmaf(-a.v[q], b.w[q], d[1]);
+      e0 = fmaf(-a.v[q + 4], b.v[q + 4], e0);
+      e1 = fmaf(-a.v[q + 4], b.w[q + 4], e1);
+    }
+    d[0] += e0;
+    d[1] += e1;
+  }
+};
+__device__ __forceinline__ void load_pair(const double* p, double (&d)[2]) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  d[0] = v.x;
+  d[1] = v.y;
+}
+__device__ __forceinline__ void load_pair(const float* p, float (&d)[2]) {
+  const float2 v = *reinterpret_cast<const float2*>(p);
+  d[0] = v.x;
+  d[1] = v.y;
+}
+__device__ __forceinline__ void store_pair(double* p, double x, double y) {
+  *reinterpret_cast<double2*>(p) = make_double2(x, y);
+}
+__device__ __forceinline__ void store_pair(float* p, float x, float y) {
+  *reinterpret_cast<float2*>(p) = make_float2(x, y);
+}
+__device__ __forceinline__ void store_row8(double* p, const double (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q < 8; q += 2) *reinterpret_cast<double2*>(p + q) = make_double2(v[q], v[q + 1]);
+}
+__device__ __forceinline__ void store_row8(float* p, const float (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q < 8; q += 4) *reinterpret_cast<float4*>(p + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+}
+
+// The first i + 1 values of a row of eight (and one more when i is even).
+template <typename T>
+__device__ __forceinline__ void load_lower(const T* p, int i, T (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q <= i; q += 2) {
+    T w[2];
+    load_pair(p + q, w);
+    v[q] = w[0];
+    v[q + 1] = w[1];
+  }
+}
+
+// Shared memory of a factorisation besides the tile and the solve blocks: two
+// multiplier strips, the two pivot warps' scratch, 1 / L_jj twice, two words
+// (panels done, first non-positive pivot).
+template <typename T>
+constexpr int factor_scratch_elems() {
+  return 2 * NB * ChainLd<T>::MS + 2 * 40 * ChainLd<T>::MS + 2 * NB + 16 / (int)sizeof(T);
+}
+
+template <typename T>
+struct FactorMem {
+  T* A;   // [64][LT] the tile
+  T* V;   // [64][LT] its solve blocks
+  T* M;   // [2][64][MS] multipliers of a panel
+  T* R;   // [2][40][MS] scratch of the pivot warps
+  T* rs;  // [2][64] 1 / L_jj, a copy for each finishing warp
+  int* w; // [2]
+  __device__ FactorMem(T* tile_, T* blocks, T* scratch) : A(tile_), V(blocks), M(scratch) {
+    R = M + 2 * NB * ChainLd<T>::MS;
+    rs = R + 2 * 40 * ChainLd<T>::MS;
+    w = reinterpret_cast<int*>(rs + 2 * NB);
+  }
+};
+
+// Column-major numbering, from the last column back, of the lower blocks of
+// the trailing triangle: entry u = (block row) << 4 | (block column).
+__constant__ unsigned char c_tri[28] = {0x77, 0x76, 0x66, 0x75, 0x65, 0x55, 0x74, 0x64, 0x54, 0x44,
+                                        0x73, 0x63, 0x53, 0x43, 0x33, 0x72, 0x62, 0x52, 0x42, 0x32,
+                                        0x22, 0x71, 0x61, 0x51, 0x41, 0x31, 0x21, 0x11};
+
+// F's pivots, warps 0 .. 4: the tile A (lower triangle valid with every update
+// applied) by eight 8-column panels, in the LDL^T form: column j of A becomes
+// x_j = L_j sqrt(d_j) (its diagonal entry the pivot d_j); the multipliers
+// m = x / d of a panel go to a strip in M.
+//  - Warps 0 and 1 own the rows from the panel's first one on (one row per
+//    lane): they update the panel's own columns with the previous panel (rank
+//    8, 8 x 8 blocks), both factor the 8 x 8 pivot block in every lane's
+//    registers -- the chain is reciprocal -> multiply-add, 53 cycles a column in
+//    FP64, 25 in FP32 -- and eliminate their rows, the block's own among them,
+//    in the same instruction stream.
+//  - Warps 2 .. 4 apply the previous panel to the columns right of the present
+//    one; they are done before the next panel needs the first of them.
+// One barrier per panel (named barrier 1) separates the panels' reads and
+// writes; f.w[0] counts the panels done for the finishing warps.
+constexpr int FACTOR_TRAIL = 3;  // warps 2 .. 4
+template <typename T>
+__device__ __forceinline__ void factor_panels(const FactorMem<T>& f) {
+  constexpr int LT = ChainLd<T>::LT, MS = ChainLd<T>::MS;
+  using B = Block<T>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  T* A = f.A;
+#pragma unroll 1
+  for (int p = 0; p < 8; ++p) {
+    const int c0 = 8 * p;
+    const T* Mp = f.M + ((p + 1) & 1) * NB * MS;  // the previous panel's multipliers
+    if (warp < 2) {
+      const int s0 = c0 + 32 * warp;  // this warp's rows s0 .. s0 + 31
+      const bool own = s0 + lane < NB;
+      T l[8][8], x[8];
+      if (p == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) load_lower(A + i * LT, i, l[i]);
+        lds_vec(A + (s0 + lane) * LT, x);
+      } else {
+        // the pivot block (block 0) and this warp's four blocks of rows; rows
+        // past the tile repeat the pivot block
+        T* Rw = f.R + warp * 40 * MS;
+        T d[5][2];
+        typename B::Op av[5];
+        const typename B::OpB bv = B::load_b(Mp + c0 * MS, MS);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+          const int r1 = s0 + 8 * (q - 1), r0 = q == 0 || r1 >= NB ? c0 : r1;
+          av[q] = B::load_a(A + r0 * LT + c0 - 8, LT);
+          load_pair(A + (r0 + g) * LT + c0 + 2 * t, d[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q) B::sub(d[q], av[q], bv);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) store_pair(Rw + (8 * q + g) * MS + 2 * t, d[q][0], d[q][1]);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) load_lower(Rw + i * MS, i, l[i]);
+        lds_vec(Rw + (8 + lane) * MS, x);
+      }
+      T m[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const T r = pivot_rcp(l[j][j]);
+        if (j < 7) l[j + 1][j + 1] = fma(-(l[j + 1][j] * l[j + 1][j]), r, l[j + 1][j + 1]);
+        m[j] = x[j] * r;
+#pragma unroll
+        for (int c = j + 1; c < 8; ++c) {
+          const T e = l[c][j] * r;
+          x[c] = fma(-x[j], e, x[c]);
+#pragma unroll
+          for (int i = c; i < 8; ++i)
+            if (i != j + 1) l[i][c] = fma(-l[i][j], e, l[i][c]);
+        }
+      }
+      if (own) {
+        store_row8(A + (s0 + lane) * LT + c0, x);
+        store_row8(f.M + (p & 1) * NB * MS + (s0 + lane) * MS, m);
+      }
+    } else if (p > 0) {
+      // blocks (ri, cj), cj = p + 1 .. 7, ri = cj .. 7, column by column
+      const int n = (7 - p) * (8 - p) / 2;
+      for (int q0 = warp - 2; q0 < n; q0 += 4 * FACTOR_TRAIL) {
+        T d[4][2];
+        typename B::Op av[4];
+        typename B::OpB bv[4];
+        int at[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int q = q0 + u * FACTOR_TRAIL, e = c_tri[q < n ? n - 1 - q : 0], ri = e >> 4, cj = e & 15;
+          at[u] = q < n ? (8 * ri + g) * LT + 8 * cj + 2 * t : -1;
+          av[u] = B::load_a(A + 8 * ri * LT + c0 - 8, LT);
+          bv[u] = B::load_b(Mp + 8 * cj * MS, MS);
+          load_pair(A + (8 * ri + g) * LT + 8 * cj + 2 * t, d[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) B::sub(d[u], av[u], bv[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (at[u] >= 0) store_pair(A + at[u], d[u][0], d[u][1]);
+      }
+    }
+    bar_wait(1, 32 * (2 + FACTOR_TRAIL));
+    if (threadIdx.x == 0) asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(tc::smem_u32(f.w)), "r"(p + 1) : "memory");
+  }
+}
+
+// The pair (row 8j + lane / 4, columns 8q + 2 (lane % 4) ..) of L_kk = x / sqrt(d)
+// into the factor's tile (zero above the diagonal).
+template <typename T, typename S>
+__device__ __forceinline__ void store_factor_pair(const FactorMem<T>& f, const T* rs, S* out, int ld, int j, int q) {
+  constexpr int LT = ChainLd<T>::LT;
+  const int lane = threadIdx.x & 31, r = 8 * j + (lane >> 2), c = 8 * q + 2 * (lane & 3);
+  T v[2] = {T(0), T(0)};
+  if (q <= j) {
+    load_pair(f.A + r * LT + c, v);
+    v[0] = c <= r ? v[0] * rs[c] : T(0);
+    v[1] = c + 1 <= r ? v[1] * rs[c + 1] : T(0);
+  }
+  store_pair(out + (size_t)r * ld + c, (S)v[0], (S)v[1]);
+}
+
+// V_jq = V_jj L_jq for blocks q = q0 .. q0 + N - 1 below `end`.
+template <typename T, typename S, int N>
+__device__ __forceinline__ void solve_blocks(const FactorMem<T>& f, const T* rs, S* V_out, int j, int q0, int end) {
+  constexpr int LT = ChainLd<T>::LT;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const T* Vj = f.V + 8 * j * LT + 8 * j;
+  T d[N][2];
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const int q = min(q0 + u, end - 1);
+    const T* Lb = f.A + 8 * j * LT + 8 * q;  // x; times 1 / sqrt(d) of its columns
+    d[u][0] = d[u][1] = T(0);
+    if constexpr (sizeof(T) == 8) {
+      double v[2];
+      load_pair(Vj + g * LT + 2 * t, v);
+      const double s = rs[8 * q + g];
+      dmma(d[u], v[0], Lb[2 * t * LT + g] * s);
+      dmma(d[u], v[1], Lb[(2 * t + 1) * LT + g] * s);
+    } else {
+      T v[8], s[2];
+      lds_vec(Vj + g * LT, v);
+      load_pair(rs + 8 * q + 2 * t, s);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        T b[2];
+        load_pair(Lb + i * LT + 2 * t, b);
+        d[u][0] = fma(v[i], b[0], d[u][0]);
+        d[u][1] = fma(v[i], b[1], d[u][1]);
+      }
+      d[u][0] *= s[0];
+      d[u][1] *= s[1];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+    if (q0 + u < end) {
+      store_pair(f.V + (8 * j + g) * LT + 8 * (q0 + u) + 2 * t, d[u][0], d[u][1]);
+      if (V_out) store_pair(V_out + (8 * j + g) * NB + 8 * (q0 + u) + 2 * t, (S)d[u][0], (S)d[u][1]);
+    }
+}
+
+// 1 / L_ii of blocks j - 1 and j into rs, block j's first non-positive pivot, and
+// V_jj = inv(L_jj) (lane c < 8: column c by forward substitution on
+// z_i = y_i / L_ii, whose chain is one multiply-add and one product per row).
+// One warp; every second j suffices to fill rs.
+template <typename T, typename S>
+__device__ __forceinline__ void invert_block(const FactorMem<T>& f, T* rs, S* V_out, int j) {
+  constexpr int LT = ChainLd<T>::LT;
+  const int lane = threadIdx.x & 31, c = lane & 7;
+  const T* D = f.A + 8 * j * LT + 8 * j;
+  const int i0 = 8 * ((lane & 8) && j > 0 ? j - 1 : j) + c;
+  const T d = f.A[i0 * LT + i0];
+  const T r = pivot_rsqrt(d);
+  const unsigned bad = __ballot_sync(0xffffffffu, pivot_bad(d)) & 0xffu;
+  if (lane == 0 && bad) atomicMin(f.w + 1, 8 * j + __ffs(bad) - 1);
+  if (lane < 16) rs[i0] = r;
+  T l[8][8], y[8], z[8];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) load_lower(D + i * LT, i - 1, l[i]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const T ri = __shfl_sync(0xffffffffu, r, i);
+    T s = i == c ? T(1) : T(0);
+#pragma unroll
+    for (int q = 0; q < i; ++q) s = fma(-l[i][q], z[q], s);
+    y[i] = s * ri;
+    z[i] = s * (ri * ri);
+  }
+  if (lane < 8)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      f.V[(8 * j + i) * LT + 8 * j + c] = y[i];
+      if (V_out) V_out[(8 * j + i) * NB + 8 * j + c] = (S)y[i];
+    }
+  __syncwarp();
+}
+
+// F(k) of the updated tile f.A, warps 0 .. 6 (warp 7 returns at once): L_kk =
+// x / sqrt(d) to tile (k, k) of the factor (type S, zero above the diagonal),
+// the solve blocks of L_kk to f.V and to V_out (global 64 x 64, type S, or
+// null): with 8 x 8 blocks, V_jj = inv(L_jj) and V_jq = inv(L_jj) L_jq for
+// q < j, so that a row C of the solve C L_kk^-T is
+// W_j = C_j V_jj^T - sum_{q < j} W_q V_jq^T.  (Blocks above the block diagonal
+// are neither written nor read.)  Warps 5 and 6 finish a row of blocks (the
+// square roots, V, the stores) while the panels after it are factored; only
+// the last row is left when the last pivot is done.  A non-positive pivot is
+// recorded in info.  f.w: {0, 64} on entry.  Ends with a barrier of warps
+// 0 .. 6 (named barrier 2).
+template <typename T, typename S>
+__device__ __forceinline__ void factor_tile(const DFArgs& a, int k, const FactorMem<T>& f, S* V_out) {
+  const int warp = threadIdx.x >> 5;
+  if (warp == 7) return;
+  S* out = tile<S>(a, k, k);
+  if (warp < 5) {
+    factor_panels(f);
+  } else {
+    T* rs = f.rs + (warp - 5) * NB;
+    for (int j = warp - 5; j < 8; j += 2) {
+      // bounded like every wait; the panels do not wait on anything else
+      for (long long it = 0; it < a.spin_limit; ++it) {
+        int done;
+        asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(done) : "r"(tc::smem_u32(f.w)) : "memory");
+        if (done > j) break;
+      }
+      __syncwarp();
+      invert_block<T, S>(f, rs, V_out, j);
+      if (j == 7) break;
+      for (int q = 0; q < j; q += 4) solve_blocks<T, S, 4>(f, rs, V_out, j, q, j);
+#pragma unroll 4
+      for (int q = 0; q < 8; ++q) store_factor_pair<T, S>(f, rs, out, a.ld, j, q);
+    }
+  }
+  bar_wait(2, 32 * 7);
+  const T* rs = f.rs + NB;  // warp 6's copy is complete
+  solve_blocks<T, S, 1>(f, rs, V_out, 7, warp, 7);
+  store_factor_pair<T, S>(f, rs, out, a.ld, 7, warp);
+  if (warp == 5) store_factor_pair<T, S>(f, rs, out, a.ld, 7, 7);
+  if (threadIdx.x == 0) {
+    if (f.w[1] < NB && k * NB + f.w[1] < a.n) atomicCAS(a.info, 0, k * NB + f.w[1] + 1);
+    f.w[0] = 0;
+    f.w[1] = NB;
+  }
+  bar_wait(2, 32 * 7);
+}
+
+// ---------------------------------------------------------------- S(i, k)
+// W = C L_kk^-T for a 64 x 64 tile C (smem rows of ldc) with the solve blocks
+// V of L_kk (smem [64][LT], factor_tile), W_j = C_j V_jj^T - sum_q W_q V_jq^T
+// block column by block column.  A warp keeps its rows' accumulators in
+// registers; with the K slots chosen as columns 2t, 2t + 1 the accumulator
+// fragment of W_j is at once the next products' A fragment, so the chain over
+// the eight block columns is one MMA and one add per column, without shuffles
+// or shared memory.  out(row, col, w0, w1) receives the pairs of W
+// (columns col, col + 1).  All warps of the CTA; a warp's rows of C are read
+// before its first out(), which may therefore overwrite them.
+// Against the product with the explicit inverse: half the operations and no
+// inversion before it.  FP64: DMMA, eight rows per warp (bound by the FP64
+// tensor pipe: 576 DMMAs, 2.4k cycles).
+template <typename F>
+__device__ __forceinline__ void solve_rows(const double* C, int ldc, const double* V, F out) {
+  constexpr int LT = ChainLd<double>::LT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double p[8][2], q[8][2], v[8][2];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    double c[2];
+    load_pair(C + (8 * warp + g) * ldc + 8 * j + 2 * t, c);
+    load_pair(V + (8 * j + g) * LT + 8 * j + 2 * t, v[j]);
+    p[j][0] = p[j][1] = q[j][0] = q[j][1] = 0.0;
+    dmma(p[j], c[0], v[j][0]);
+    dmma(q[j], c[1], v[j][1]);
+  }
+  __syncwarp();
+  auto load_column = [&](int j) {  // V_ij, i > j
+#pragma unroll
+    for (int i = 1; i < 8; ++i)
+      if (i > j) load_pair(V + (8 * i + g) * LT + 8 * j + 2 * t, v[i]);
+  };
+  load_column(0);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const double w0 = p[j][0] + q[j][0], w1 = p[j][1] + q[j][1];
+#pragma unroll
+    for (int i = j + 1; i < 8; ++i) {
+      dmma(p[i], -w0, v[i][0]);
+      dmma(q[i], -w1, v[i][1]);
+    }
+    load_column(j + 1);  // ahead of this column's stores
+    out(8 * warp + g, 8 * j + 2 * t, w0, w1);
+  }
+}
+
+// D (16 x 8) += A (16 x 8) B (8 x 8) in TF32; a = {(g, k0), (g + 8, k0),
+// (g, k1), (g + 8, k1)}, b = {k0, k1} of column g, k0 / k1 the lane's K slots.
+__device__ __forceinline__ void tf32_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// hi + lo TF32 halves of x
+__device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
+  hi = to_tf32(x);
+  lo = to_tf32(x - __uint_as_float(hi));
+}
+
+// FP32: 3xTF32 m16n8k8, sixteen rows per warp (warps 0 .. 3), the hi * hi
+// products and the two cross terms on separate accumulators.
+template <typename F>
+__device__ __forceinline__ void solve_rows(const float* C, int ldc, const float* V, F out) {
+  constexpr int LT = ChainLd<float>::LT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if (warp >= 4) return;
+  const int r0 = 16 * warp + g;
+  float p[8][4], q[8][4];
+  auto mul = [&](int i, const float (&w)[4], const float* vb) {  // p[i], q[i] += w V^T (block at vb)
+    unsigned ah[4], al[4], bh[2], bl[2];
+    float v[2];
+    load_pair(vb + g * LT + 2 * t, v);
+    // fragment order: (g, 2t), (g + 8, 2t), (g, 2t + 1), (g + 8, 2t + 1)
+    const float a[4] = {w[0], w[2], w[1], w[3]};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split_tf32(a[e], ah[e], al[e]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) split_tf32(v[e], bh[e], bl[e]);
+    tf32_mma(p[i], ah, bh);
+    tf32_mma(q[i], al, bh);
+    tf32_mma(q[i], ah, bl);
+  };
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float c[2], e[2];
+    load_pair(C + r0 * ldc + 8 * j + 2 * t, c);
+    load_pair(C + (r0 + 8) * ldc + 8 * j + 2 * t, e);
+    const float w[4] = {c[0], c[1], e[0], e[1]};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p[j][u] = q[j][u] = 0.0f;
+    mul(j, w, V + 8 * j * LT + 8 * j);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float w[4], n[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      w[u] = p[j][u] + q[j][u];
+      n[u] = -w[u];
+    }
+#pragma unroll
+    for (int i = j + 1; i < 8; ++i) mul(i, n, V + 8 * i * LT + 8 * j);
+    out(r0, 8 * j + 2 * t, w[0], w[1]);
+    out(r0 + 8, 8 * j + 2 * t, w[2], w[3]);
+  }
+}
+
+// ---------------------------------------------------------------- the chain's SYRK
+// A = N - L L^T on and below the block diagonal (smem tiles, rows of LT): the
+// last update of the next diagonal tile, with the solve's result still in
+// shared memory.  FP64: the 36 lower 8 x 8 blocks, 9 per SM quarter (warps w
+// and w + 4): row 7 - w and row w of blocks.
+__device__ __forceinline__ void syrk_lower(const double* N, const double* L, double* A) {
+  constexpr int LT = ChainLd<double>::LT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  auto row = [&](int i, int j0, int j1) {  // blocks (i, j0 .. j1 - 1)
+    double av[8][2];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) load_pair(L + (8 * i + g) * LT + 8 * k + 2 * t, av[k]);
+#pragma unroll 1
+    for (int j = j0; j < j1; ++j) {
+      double d[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, n[2];
+      load_pair(N + (8 * i + g) * LT + 8 * j + 2 * t, n);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        double b[2];
+        load_pair(L + (8 * j + g) * LT + 8 * k + 2 * t, b);
+        dmma(d[2 * (k & 1)], av[k][0], b[0]);
+        dmma(d[2 * (k & 1) + 1], av[k][1], b[1]);
+      }
+      store_pair(A + (8 * i + g) * LT + 8 * j + 2 * t, n[0] - ((d[0][0] + d[1][0]) + (d[2][0] + d[3][0])),
+                 n[1] - ((d[0][1] + d[1][1]) + (d[2][1] + d[3][1])));
+    }
+  };
+  if (warp < 4) {
+    row(7 - warp, 0, 5);
+  } else {
+    const int w = warp - 4;
+    if (w < 3) row(7 - w, 5, 8 - w);
+    row(w, 0, w + 1);
+  }
+}
+// FP32: the twenty 16 x 8 blocks that meet the lower triangle in 3xTF32, five
+// per SM quarter; the product is accumulated from zero and subtracted once.
+__device__ __forceinline__ void syrk_lower(const float* N, const float* L, float* A) {
+  constexpr int LT = ChainLd<float>::LT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  // block row, first block column, count of warp w
+  constexpr int RB[8] = {3, 3, 2, 2, 0, 1, 3, 1}, J0[8] = {0, 3, 0, 3, 0, 0, 6, 2}, CN[8] = {3, 3, 3, 3, 2, 2, 2, 2};
+  int rb = 0, j0 = 0, cn = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w)
+    if (w == warp) {
+      rb = RB[w];
+      j0 = J0[w];
+      cn = CN[w];
+    }
+  const float* La = L + (16 * rb + g) * LT;
+  float p[3][4], q[3][4];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p[c][u] = q[c][u] = 0.0f;
+#pragma unroll 2
+  for (int k0 = 0; k0 < NB; k0 += 8) {
+    float x[2], y[2];
+    load_pair(La + k0 + 2 * t, x);
+    load_pair(La + 8 * LT + k0 + 2 * t, y);
+    const float av[4] = {x[0], y[0], x[1], y[1]};
+    unsigned ah[4], al[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split_tf32(av[e], ah[e], al[e]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (c < cn) {
+        float v[2];
+        load_pair(L + (8 * (j0 + c) + g) * LT + k0 + 2 * t, v);
+        unsigned bh[2], bl[2];
+        split_tf32(v[0], bh[0], bl[0]);
+        split_tf32(v[1], bh[1], bl[1]);
+        tf32_mma(p[c], ah, bh);
+        tf32_mma(q[c], al, bh);
+        tf32_mma(q[c], ah, bl);
+      }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    if (c < cn) {
+      const int r = 16 * rb + g, col = 8 * (j0 + c) + 2 * t;
+      float n[2], m[2];
+      load_pair(N + r * LT + col, n);
+      load_pair(N + (r + 8) * LT + col, m);
+      store_pair(A + r * LT + col, n[0] - (p[c][0] + q[c][0]), n[1] - (p[c][1] + q[c][1]));
+      store_pair(A + (r + 8) * LT + col, m[0] - (p[c][2] + q[c][2]), m[1] - (p[c][3] + q[c][3]));
+    }
+}
+
+// ---------------------------------------------------------------- the chain CTA
+// Shared memory of the chain CTA: five [64][LT] tiles (the diagonal tile, the
+// solve's input, its result, the next diagonal tile, the solve blocks) and
+// the factor scratch.
+template <typename T>
+constexpr size_t chain_smem_bytes() {
+  return sizeof(T) * (5 * NB * ChainLd<T>::LT + factor_scratch_elems<T>());
+}
+
+// One warp's copy of a 64 x 64 tile into smem rows of LT: asynchronous (the
+// warp waits with cp_async_wait_all), or converted when the matrix is FP32
+// and the chain works in FP64.
+template <typename T, typename S>
+__device__ __forceinline__ void fetch_tile_warp(const S* g, int ld, T* s) {
+  constexpr int LT = ChainLd<T>::LT;
+  const int lane = threadIdx.x & 31;
+  if constexpr (sizeof(T) == sizeof(S)) {
+    constexpr int per_row = NB * (int)sizeof(T) / 16, elems = 16 / (int)sizeof(T);
+#pragma unroll 8
+    for (int c = lane; c < NB * per_row; c += 32)
+      cp_async16(s + (c / per_row) * LT + (c % per_row) * elems, g + (size_t)(c / per_row) * ld + (c % per_row) * elems);
+  } else {
+#pragma unroll 8
+    for (int c = lane; c < NB * NB / 4; c += 32) {
+      const int r = c >> 4, q = 4 * (c & 15);
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(g + (size_t)r * ld + q));
+      store_pair(s + r * LT + q, (T)v.x, (T)v.y);
+      store_pair(s + r * LT + q + 2, (T)v.z, (T)v.w);
+    }
+  }
+}
+
+// A single warp's bounded wait for *flag >= target (the abort polling and the
+// expiry of wait_all) while the other warps of the CTA compute: lane 0 polls
+// with relaxed loads and sleeps in between, because an acquire load per poll
+// invalidates the SM's L1 each time and slowed the other warps' shared-memory
+// accesses several times over.  The flag is then acquired once by every lane,
+// which orders the lane's own later copies.
+__device__ __forceinline__ int ld_relaxed(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool warp_wait_geq(const DFArgs& a, const int* flag, int target) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) {
+    for (long long it = 0; ld_relaxed(flag) < target; ++it) {
+      if ((it & 15) == 15 && ld_relaxed(a.ctl + 1)) {
+        ok = 0;
+        break;
+      }
+      if (it + 1 > a.spin_limit) {
+        atomicExch(a.ctl + 1, 1);
+        atomicAdd(a.ctl + 2, 1);
+        atomicOr(a.err, PBG_DEV_ERR_BARRIER);
+        atomicCAS(a.info, 0, -1);  // -1: the factorisation gave up waiting
+        ok = 0;
+        break;
+      }
+      __nanosleep(it > 256 ? 200 : 40);
+    }
+  }
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  return ok && __all_sync(0xffffffffu, ld_acquire(flag) >= target);
+}
+
+// The chain CTA: F(0), S(1, 0), F(1), S(2, 1), ... in T arithmetic on a matrix
+// of type S.  For each k: F(k) on warps 0 .. 6 (L_kk to the factor, the solve
+// blocks to a.lp for the workers' solves of column k, fin(k, k) = 1), while
+// warp 7 fetches the solve's input A(k+1, k) as soon as its last update is in
+// and the next diagonal tile; S(k+1, k) on all warps, kept in shared memory
+// and published as fin(k+1, k) = 1; the last update of A(k+1, k+1) from the
+// result (syrk_lower).
+template <typename T, typename S>
+__device__ void run_chain(const DFArgs& a, unsigned char* smem, int* s_ok) {
+  constexpr int LT = ChainLd<T>::LT;
+  __shared__ int s_pf;  // the next diagonal tile is in N
+  T* A = reinterpret_cast<T*>(smem);
+  T* C = A + NB * LT;
+  T* L = C + NB * LT;
+  T* N = L + NB * LT;
+  T* V = N + NB * LT;
+  const FactorMem<T> f(A, V, V + NB * LT);
+  const int nt = a.nt, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    *s_ok = 1;
+    f.w[0] = 0;
+    f.w[1] = NB;
+  }
+  if (warp == 7) {
+    fetch_tile_warp<T, S>(tile<S>(a, 0, 0), a.ld, A);
+    cp_async_wait_all();
+  }
+  __syncthreads();
+  for (int k = 0; k < nt; ++k) {
+    TRACE(0, a.ntasks + 2 * k);
+    TRACE(3, a.ntasks + 2 * k);
+    TRACE(1, a.ntasks + 2 * k);
+    if (warp < 7) {
+      CTRACE(k, 0);
+      factor_tile<T, S>(a, k, f, a.lp ? reinterpret_cast<S*>(a.lp) + (size_t)k * NB * NB : nullptr);
+      if (threadIdx.x == 32 * 6) st_release(a.fin + k * nt + k, 1);
+    } else if (k + 1 < nt) {
+      bool ok = warp_wait_geq(a, a.upd + (k + 1) * nt + k, k);
+      int pf = 0;
+      if (ok) {
+        fetch_tile_warp<T, S>(tile<S>(a, k + 1, k), a.ld, C);
+        pf = __all_sync(0xffffffffu, ld_acquire(a.upd + (k + 1) * nt + k + 1) >= k);
+        if (pf) fetch_tile_warp<T, S>(tile<S>(a, k + 1, k + 1), a.ld, N);
+        cp_async_wait_all();
+      }
+      if (lane == 0) {
+        s_pf = pf;
+        if (!ok) *s_ok = 0;
+      }
+    }
+    TRACE(2, a.ntasks + 2 * k);
+    CTRACE(k, 1);
+    __syncthreads();
+    if (!*s_ok || k + 1 == nt) return;
+    TRACE(0, a.ntasks + 2 * k + 1);
+    TRACE(3, a.ntasks + 2 * k + 1);
+    TRACE(1, a.ntasks + 2 * k + 1);
+    CTRACE(k, 2);
+    S* out = tile<S>(a, k + 1, k);
+    solve_rows(C, LT, V, [&](int r, int c, T w0, T w1) {
+      store_pair(L + r * LT + c, w0, w1);
+      store_pair(out + (size_t)r * a.ld + c, (S)w0, (S)w1);
+    });
+    CTRACE(k, 3);
+    if (!s_pf && warp == 7) {
+      const bool ok = warp_wait_geq(a, a.upd + (k + 1) * nt + k + 1, k);
+      if (ok) {
+        fetch_tile_warp<T, S>(tile<S>(a, k + 1, k + 1), a.ld, N);
+        cp_async_wait_all();
+      } else if (lane == 0) {
+        *s_ok = 0;
+      }
+    }
+    __syncthreads();
+    if (!*s_ok) return;
+    CTRACE(k, 4);
+    if (threadIdx.x == 32 * 7) st_release(a.fin + (k + 1) * nt + k, 1);
+    TRACE(2, a.ntasks + 2 * k + 1);
+    syrk_lower(N, L, A);
+    __syncthreads();
+    CTRACE(k, 5);
+  }
 }
 
 // ---------------------------------------------------------------- FP32 chain
@@ -860,17 +1334,11 @@ __device__ __forceinline__ void acc_to_smem(const T acc[16], T* s) {
 // while every step of the panel chain gets shorter (MUFU rsqrt instead of
 // a refined FP64 rsqrt, FP32 FMA latency, no FP64 conversion).
 
-// Named barriers (0 is __syncthreads): arrive does not wait; both order the
-// calling threads' earlier shared-memory accesses before the barrier completes.
-// Whole warps call them; __syncwarp first reconverges a warp after divergent
-// code (the barrier instructions are warp-aligned).
+// Named barrier arrival without waiting (orders the calling threads' earlier
+// shared-memory accesses before the barrier completes; see bar_wait).
 __device__ __forceinline__ void bar_arrive(int id, int count) {
   __syncwarp();
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_wait(int id, int count) {
-  __syncwarp();
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
 // T[r][c] -= sum_q T[r][c0+q] T[c][c0+q] (q = 0..7, in order): the rank-8
@@ -1045,209 +1513,6 @@ __device__ __forceinline__ void factor_task_f32(const DFArgs& a, int k, const fl
   factor_tile_f32(a, k, T, Rinv);
   invert_factor<float>(T, Rinv, X, Tm);
   store_factor_inverse(a, k, T, X);
-}
-
-// Shared memory of the FP32 chain: five [64][LDA] float tiles (the tile
-// being factored, inv(L_kk), the solve's input, the previous solve's
-// result, the prefetched next diagonal tile), the inversion scratch
-// (32 x 36) and 1 / L_jj.
-constexpr size_t chain_f32_smem_bytes() { return sizeof(float) * (5 * NB * LDA + 32 * 36 + NB); }
-
-// The FP32 chain CTA: for k = 0, 1, ...
-//   A_kk after its updates by the workers, minus L(k,k-1) L(k,k-1)^T (3xTF32
-//   on the tensor cores; L(k,k-1) is still in shared memory);
-//   F(k) (factor_tile_f32), inv(L_kk) (FP32, on the FMA pipe) -- L_kk goes to
-//   the factor and inv(L_kk) to invdiag, published as fin(k,k) = 2 for the
-//   workers' solves (no I(k) tasks in this list);
-//   S(k+1,k) = A(k+1,k) inv(L_kk)^T (3xTF32), kept in shared memory for the
-//   next step and published as fin(k+1,k) = 1.
-// The solve's input is fetched during F(k) when its last update is already
-// done, and the next diagonal tile during S(k+1,k) when its worker updates
-// are.
-__device__ void run_chain_f32(const DFArgs& a, unsigned char* smem, int* s_ok) {
-  __shared__ int s_pf[2];  // [0] next diagonal tile fetched, [1] solve input fetched
-  float* T = reinterpret_cast<float*>(smem);
-  float* X = T + NB * LDA;
-  float* Cn = X + NB * LDA;
-  float* Lp = Cn + NB * LDA;
-  float* sA = Lp + NB * LDA;
-  float* Tm = sA + NB * LDA;
-  float* Rinv = Tm + 32 * 36;
-  const int nt = a.nt;
-  bool pf_diag = false;
-  for (int k = 0; k < nt; ++k) {
-    float acc[16];
-    TRACE(0, a.ntasks + 2 * k);
-    TRACE(3, a.ntasks + 2 * k);
-    CTRACE(k, 7);
-    if (k > 0) {
-      if (pf_diag) {
-        cp_async_wait_all();
-        __syncthreads();
-        smem_to_acc(sA, acc);
-      } else {
-        if (!wait_geq(a, a.upd + k * nt + k, k - 1, s_ok)) return;
-        load_acc(tile<float>(a, k, k), a.ld, acc);
-      }
-      TileMMA<float>::sub(Lp, Lp, acc);
-    } else {
-      load_acc(tile<float>(a, 0, 0), a.ld, acc);
-    }
-    acc_to_smem(acc, T);
-    if (threadIdx.x == 0) s_pf[1] = k + 1 < nt && ld_acquire(a.upd + (k + 1) * nt + k) >= k;
-    __syncthreads();
-    // thread 0's acquire and the barrier order the early fetch after the updates
-    const bool have_in = s_pf[1] != 0;
-    if (have_in) stage_async(tile<float>(a, k + 1, k), a.ld, Cn, LDA);
-    TRACE(1, a.ntasks + 2 * k);
-    CTRACE(k, 0);
-    factor_tile_f32(a, k, T, Rinv);
-    CTRACE(k, 1);
-    invert_factor<float>(T, Rinv, X, Tm);
-    CTRACE(k, 2);
-    store_factor_inverse(a, k, T, X);
-    publish(a.fin + k * nt + k, 2);
-    CTRACE(k, 3);
-    TRACE(2, a.ntasks + 2 * k);
-    if (k + 1 == nt) return;
-    TRACE(0, a.ntasks + 2 * k + 1);
-    TRACE(3, a.ntasks + 2 * k + 1);
-    if (!have_in) {
-      if (!wait_geq(a, a.upd + (k + 1) * nt + k, k, s_ok)) return;
-      stage_async(tile<float>(a, k + 1, k), a.ld, Cn, LDA);
-    }
-    if (threadIdx.x == 0) s_pf[0] = ld_acquire(a.upd + (k + 1) * nt + k + 1) >= k;
-    cp_async_wait_all();
-    __syncthreads();
-    pf_diag = s_pf[0] != 0;
-    if (pf_diag) stage_async(tile<float>(a, k + 1, k + 1), a.ld, sA, LDA);
-    TRACE(1, a.ntasks + 2 * k + 1);
-    CTRACE(k, 4);
-    solve_by_inverse(Cn, X, acc);
-    CTRACE(k, 5);
-    acc_to_smem(acc, Lp);
-    __syncthreads();
-    store_tile(Lp, LDA, tile<float>(a, k + 1, k), a.ld);
-    publish(a.fin + (k + 1) * nt + k, 1);
-    CTRACE(k, 6);
-    TRACE(2, a.ntasks + 2 * k + 1);
-  }
-}
-
-// Shared memory of the chain CTA: four T tiles Cp, Cn, X, sA ([64][LDA]
-// each) and the FP64 factor scratch -- in the FP64 path X holds L_kk from F(k)
-// to S(k+1, k); in the mixed path two more FP64 tiles (L_kk, the FP64 rows of
-// the solve) come first.  Every piece is a multiple of 16 bytes, so each
-// starts 16-byte aligned.
-template <typename T>
-constexpr size_t chain_smem_bytes() {
-  return sizeof(T) * 4 * NB * LDA + (sizeof(T) == 8 ? 0 : sizeof(double) * 2 * NB * LDA) +
-         sizeof(double) * factor_smem_elems<double>();
-}
-
-// The chain CTA: F(0), S(1, 0), F(1), S(2, 1), ... with L(k, k-1) and the
-// FP64 L_kk kept in shared memory from one task to the next.  F(k) does not
-// form inv(L_kk) (a worker task I(k) does, for the other solves of column k);
-// S(k+1, k) is a blocked forward substitution against L_kk (trsm_rows).  The
-// last update of S(k+1, k) (with panel k-1) is a worker task that runs during
-// F(k); while S(k+1, k) runs, the next diagonal tile is prefetched into
-// shared memory if its updates by the workers are already complete.
-template <typename T>
-__device__ void run_chain(const DFArgs& a, unsigned char* smem, int* s_ok) {
-  __shared__ int s_pf;
-  T* Cp = reinterpret_cast<T*>(smem);  // L(k, k-1), the previous solve's result
-  T* Cn = Cp + NB * LDA;               // this step's solve input / result L(k+1, k)
-  T* X = Cn + NB * LDA;                // FP64 path: L_kk
-  T* sA = X + NB * LDA;                // prefetched A_kk
-  double* Lk64;  // L_kk in FP64, F(k) to S(k+1, k)
-  double* W64;   // FP64 rows of the solve (the mixed path; the FP64 path solves in Cn)
-  double* fs64;  // factor scratch; its strip area holds the leaf inverses during S
-  if constexpr (sizeof(T) == 8) {
-    Lk64 = reinterpret_cast<double*>(X);
-    W64 = nullptr;
-    fs64 = reinterpret_cast<double*>(sA + NB * LDA);
-  } else {
-    Lk64 = reinterpret_cast<double*>(sA + NB * LDA);
-    W64 = Lk64 + NB * LDA;
-    fs64 = W64 + NB * LDA;
-  }
-  double* Rinv64 = fs64 + 2 * NB * Strip<double>::PB;
-  double* XL = fs64;
-  __shared__ int s_in;  // A(k+1, k) staged into Cn during F(k)
-  const int nt = a.nt;
-  bool pf = false;  // A_kk prefetched into sA
-  for (int k = 0; k < nt; ++k) {
-    T acc[16];
-    const SolveInput<T> pre{a.upd + (k + 1) * nt + k, k, tile<T>(a, k + 1, k), a.ld, Cn, &s_in};
-    const SolveInput<T>* ppre = k + 1 < nt ? &pre : nullptr;
-    // F(k): A_kk after updates 0 .. k-2 (other CTAs), minus L(k,k-1) L(k,k-1)^T
-    TRACE(0, a.ntasks + 2 * k);
-    TRACE(3, a.ntasks + 2 * k);
-    if (k > 0) {
-      if (pf) {
-        cp_async_wait_all();
-        __syncthreads();
-        smem_to_acc(sA, acc);
-      } else {
-        if (!wait_geq(a, a.upd + k * nt + k, k - 1, s_ok)) return;
-        load_acc(tile<T>(a, k, k), a.ld, acc);
-      }
-      TileMMA<T>::sub(Cp, Cp, acc);  // Cp is complete: the last solve ended with a barrier
-    } else {
-      load_acc(tile<T>(a, 0, 0), a.ld, acc);
-    }
-    TRACE(1, a.ntasks + 2 * k);
-    if constexpr (sizeof(T) == 8) {
-      factor_tile<double, double, false>(a, k, acc, fs64, Lk64, nullptr, ppre);
-    } else {
-      double acc64[16];
-#pragma unroll
-      for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-        for (int cs = 0; cs < 8; ++cs)
-          acc64[TileMMA<double>::idx(rs, cs)] = (double)acc[TileMMA<float>::idx(rs, cs)];
-      factor_tile<double, float, false>(a, k, acc64, fs64, Lk64, nullptr, ppre);
-    }
-    publish(a.fin + k * nt + k, 1);
-    TRACE(2, a.ntasks + 2 * k);
-    if (k + 1 == nt) {
-      // the last inverse has no solve task after it: form it here
-      double* X64 = sizeof(T) == 8 ? reinterpret_cast<double*>(Cn) : W64;
-      store_inverse<double, T>(a, k, Lk64, Rinv64, X64, fs64);
-      publish(a.fin + k * nt + k, 2);
-      return;
-    }
-    // S(k+1, k): A(k+1,k) after updates 0 .. k-1 (other CTAs), times inv(L_kk)^T
-    TRACE(0, a.ntasks + 2 * k + 1);
-    TRACE(3, a.ntasks + 2 * k + 1);
-    const bool have_in = s_in != 0;
-    if (have_in) cp_async_wait_all();
-    if (threadIdx.x == 0) s_pf = ld_acquire(a.upd + (k + 1) * nt + k + 1) >= k;
-    leaf_inverses(Lk64, Rinv64, XL);
-    if (k > 0 && !have_in) {
-      if (!wait_geq(a, a.upd + (k + 1) * nt + k, k, s_ok)) return;
-    } else {
-      __syncthreads();
-    }
-    // thread 0's acquire and the barrier order the prefetch after the updates
-    pf = s_pf != 0;
-    if (pf) stage_async(tile<T>(a, k + 1, k + 1), a.ld, sA, LDA);
-    if (!have_in) {
-      load_acc(tile<T>(a, k + 1, k), a.ld, acc);
-      acc_to_smem(acc, Cn);
-    }
-    TRACE(1, a.ntasks + 2 * k + 1);
-    __syncthreads();  // each warp solves rows that other warps stored
-    if constexpr (sizeof(T) == 8) trsm_rows<T>(Lk64, XL, Cn, reinterpret_cast<double*>(Cn));
-    else trsm_rows<T>(Lk64, XL, Cn, W64);
-    __syncthreads();
-    store_tile(Cn, LDA, tile<T>(a, k + 1, k), a.ld);
-    publish(a.fin + (k + 1) * nt + k, 1);
-    TRACE(2, a.ntasks + 2 * k + 1);
-    T* t = Cp;
-    Cp = Cn;
-    Cn = t;
-  }
 }
 
 // U(i, j, k) with every tile moved by 16-byte copies: the target tile is
@@ -1520,6 +1785,78 @@ __device__ void inverse_finish(const DFArgs& a, int i, int j, T* s) {
   store_acc(xtile_out<T>(a, i, j), a.ld, acc);
 }
 
+// acc = A(i, j) with the updates of columns < j (the last one, with column
+// j-1, applied here; the smem tiles are free again on return).
+template <typename T>
+__device__ bool solve_input(const DFArgs& a, int i, int j, T acc[16], T* sA, T* sB, int* s_ok) {
+  const int nt = a.nt;
+  if (j == 0) {
+    load_acc(tile<T>(a, i, 0), a.ld, acc);
+    return true;
+  }
+  const int* fl[3] = {a.fin + i * nt + j - 1, a.fin + j * nt + j - 1, a.upd + i * nt + j};
+  const int tg[3] = {1, 1, j - 1};
+  if (!wait_all(a, fl, tg, 3, s_ok)) return false;
+  load_and_update(a, i, j, j - 1, acc, sA, sB);  // ends with a barrier
+  return true;
+}
+
+// Shared memory of a worker's LEAD task: five tiles.
+template <typename T>
+constexpr size_t lead_smem_bytes() { return sizeof(T) * 5 * NB * ChainLd<T>::LT; }
+
+// LEAD(k), the row i = k + 2 of panel k: S(i, k), then U(i, k+1, k) -- the last
+// update of the chain's next solve input -- and U(i, i, k), with L(i, k) kept
+// in shared memory in between.  Everything that does not need L_kk is done
+// before the wait for it (the last update of A(i, k), the fetch of both
+// targets), so that from F(k) to the chain's input there are one solve, one
+// product and two hand-overs: as separate tasks (solve through an inverse
+// formed by a third task) the chain waited 3 to 16 us for them.
+template <typename T>
+__device__ bool lead_task(const DFArgs& a, int k, T* s, int* s_ok) {
+  constexpr int LT = ChainLd<T>::LT;
+  const int nt = a.nt, i = k + 2;
+  T* Li = s;             // A(i, k), then L(i, k)
+  T* sV = s + NB * LT;   // the solve blocks of L_kk
+  T* sB = sV + NB * LT;  // L(k+1, k)
+  T* sC = sB + NB * LT;  // A(i, k+1)
+  T* sD = sC + NB * LT;  // A(i, i)
+  T acc[16];
+  if (!solve_input<T>(a, i, k, acc, sV, sB, s_ok)) return false;
+  acc_to_smem(acc, Li);
+  if (k > 0) {
+    const int* fl[2] = {a.upd + i * nt + k + 1, a.upd + i * nt + i};
+    const int tg[2] = {k, k};
+    if (!wait_all(a, fl, tg, 2, s_ok)) return false;
+  }
+  stage_async(tile<T>(a, i, k + 1), a.ld, sC, LDA);
+  stage_async(tile<T>(a, i, i), a.ld, sD, LDA);
+  if (!wait_geq(a, a.fin + k * nt + k, 1, s_ok)) return false;
+  stage_async(reinterpret_cast<const T*>(a.lp) + (size_t)k * NB * NB, NB, sV, LT);
+  cp_async_wait_all();
+  __syncthreads();
+  T* out = tile<T>(a, i, k);
+  solve_rows(Li, LDA, sV, [&](int r, int c, T w0, T w1) {
+    store_pair(Li + r * LDA + c, w0, w1);
+    store_pair(out + (size_t)r * a.ld + c, w0, w1);
+  });
+  if (!wait_geq(a, a.fin + (k + 1) * nt + k, 1, s_ok)) return false;
+  stage_async(tile<T>(a, k + 1, k), a.ld, sB, LDA);
+  smem_to_acc(sC, acc);
+  cp_async_wait_all();
+  __syncthreads();
+  TileMMA<T>::sub(Li, sB, acc);
+  store_acc(tile<T>(a, i, k + 1), a.ld, acc);
+  __syncthreads();
+  if (threadIdx.x == 0) st_release(a.upd + i * nt + k + 1, k + 1);
+  if (threadIdx.x == 32) st_release(a.fin + i * nt + k, 1);
+  smem_to_acc(sD, acc);
+  TileMMA<T>::sub(Li, Li, acc);
+  store_acc(tile<T>(a, i, i), a.ld, acc);
+  publish(a.upd + i * nt + i, k + 1);
+  return true;
+}
+
 // The worker CTAs' task loop.  FP32 lists (T = float): every update task
 // (one to four rows) runs on the tcgen05 tensor cores (update_rows_tc, w
 // holds the CTA's TMEM); FP64 lists: DMMA tile products.
@@ -1630,43 +1967,37 @@ __device__ void df_worker_loop(const DFArgs& a, unsigned char* smem, int* s_task
         st_release(a.upd + (i + 1) * nt + j, k + 1);
       }
       TRACE(2, t);
+    } else if (type == TASK_LEAD) {
+      if (!lead_task<T>(a, k, sA, &s_ok)) return;
+      TRACE(2, t);
     } else {
-      // S(i, j), i >= j + 2: the tile after its last update, times inv(L_jj)^T
-      const int col = j;
-      if (col > 0) {
-        const int* fl[3] = {a.fin + i * nt + col - 1, a.fin + col * nt + col - 1, a.upd + i * nt + col};
-        const int tg[3] = {1, 1, col - 1};
-        if (!wait_all(a, fl, tg, 3, &s_ok)) return;
-        load_and_update(a, i, col, col - 1, acc, sA, sB);  // ends with a barrier: smem is free
-      } else {
-        load_acc(tile<T>(a, i, col), a.ld, acc);
-      }
-      if (!wait_geq(a, a.fin + col * nt + col, 2, &s_ok)) return;  // inv(L_col,col) stored
+      // S(i, j), i >= j + 3: the tile after its last update, times L_jj^-T
+      if (!solve_input<T>(a, i, j, acc, sA, sB, &s_ok)) return;
+      if (!wait_geq(a, a.fin + j * nt + j, 1, &s_ok)) return;  // the solve blocks of L_jj are stored
       TRACE(1, t);
-      stage_async(reinterpret_cast<const T*>(a.invdiag) + (size_t)col * NB * NB, NB, sB, LDA);
+      constexpr int LT = ChainLd<T>::LT;
+      stage_async(reinterpret_cast<const T*>(a.lp) + (size_t)j * NB * NB, NB, sB, LT);
       acc_to_smem(acc, sA);
       cp_async_wait_all();
       __syncthreads();
-      solve_by_inverse(sA, sB, acc);
-      store_acc(tile<T>(a, i, col), a.ld, acc);
-      publish(a.fin + i * nt + col, 1);
+      T* out = tile<T>(a, i, j);
+      solve_rows(sA, LDA, sB, [&](int r, int c, T w0, T w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
+      publish(a.fin + i * nt + j, 1);
       TRACE(2, t);
     }
     __syncthreads();
   }
 }
 
-// F32CHAIN (FP32 matrices only): the chain CTA runs the FP32 chain
-// (run_chain_f32) and the task list has no I(k) tasks; otherwise run_chain,
-// whose diagonal tiles are factored in FP64.  The FP32 workers hold TMEM for
-// their tensor-core updates from start to end.
-template <typename T, bool F32CHAIN>
+// A matrix of type T; the chain CTA works in CT (FP64 for a FP32 matrix in
+// PBG_PREC_MIXED_FP64_DIAG).  The FP32 workers hold TMEM for their tensor-core
+// updates from start to end.
+template <typename T, typename CT>
 __global__ void __launch_bounds__(THREADS, 1) chol_df_kernel(DFArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_task, s_ok;
   if (blockIdx.x == 0) {
-    if constexpr (F32CHAIN) run_chain_f32(a, smem, &s_ok);
-    else run_chain<T>(a, smem, &s_ok);
+    run_chain<CT, T>(a, smem, &s_ok);
     return;
   }
   if constexpr (sizeof(T) == 4) {
@@ -1687,8 +2018,9 @@ __global__ void __launch_bounds__(THREADS, 1) chol_df_kernel(DFArgs a) {
 // memory: two tiles (sA, sB) for the updates and solves; F uses two tiles
 // (L_kk, inverse) over the same bytes and the factor scratch after them.
 constexpr size_t batch_smem_bytes() {
-  // an F task's factor scratch, or a paired update's five tiles
-  return std::max(sizeof(double) * (2 * NB * LDA + factor_smem_elems<double>()), 5 * NB * LDA * sizeof(double));
+  // an F task's tile, solve blocks and factor scratch, or a paired update's five tiles
+  return std::max(sizeof(double) * (2 * NB * ChainLd<double>::LT + factor_scratch_elems<double>()),
+                  5 * NB * LDA * sizeof(double));
 }
 
 // The FP64 batched kernel's task loop: DMMA updates in pairs (five tiles
@@ -1699,9 +2031,9 @@ __device__ void batch_worker_loop(const CholRep* __restrict__ reps, const int4* 
   __shared__ int s_task, s_ok;
   T* sA = reinterpret_cast<T*>(smem);
   T* sB = sA + NB * LDA;
-  double* Lk64 = reinterpret_cast<double*>(smem);
-  double* X64 = Lk64 + NB * LDA;
-  double* fs64 = X64 + NB * LDA;
+  constexpr int LT = ChainLd<T>::LT;
+  T* Ft = reinterpret_cast<T*>(smem);  // F: the tile, its solve blocks, the scratch
+  const FactorMem<T> f(Ft, Ft + NB * LT, Ft + 2 * NB * LT);
   while (true) {
     if (threadIdx.x == 0) s_task = ld_acquire(ctl + 1) ? ntasks : atomicAdd(ctl, 1);
     __syncthreads();
@@ -1722,7 +2054,7 @@ __device__ void batch_worker_loop(const CholRep* __restrict__ reps, const int4* 
     a.upd = R.upd;
     a.fin = R.fin;
     a.info = R.info;
-    a.invdiag = R.invdiag;
+    a.lp = R.invdiag;  // the solve blocks take the place of the inverses
     a.err = reinterpret_cast<unsigned*>(ctl + 3);
     a.spin_limit = SPIN_LIMIT;
     const int nt = a.nt;
@@ -1756,15 +2088,21 @@ __device__ void batch_worker_loop(const CholRep* __restrict__ reps, const int4* 
         load_acc(tile<T>(a, i, col), a.ld, acc);
       }
       if (type == TASK_F) {
-        factor_tile<double>(a, col, acc, fs64, Lk64, X64);
+        acc_to_smem(acc, Ft, LT);
+        if (threadIdx.x == 0) {
+          f.w[0] = 0;
+          f.w[1] = NB;
+        }
+        __syncthreads();
+        factor_tile<T, T>(a, col, f, reinterpret_cast<T*>(a.lp) + (size_t)col * NB * NB);
       } else {
         if (!wait_geq(a, a.fin + col * nt + col, 1, &s_ok)) return;
-        stage_async(reinterpret_cast<const T*>(a.invdiag) + (size_t)col * NB * NB, NB, sB, LDA);
+        stage_async(reinterpret_cast<const T*>(a.lp) + (size_t)col * NB * NB, NB, sB, LT);
         acc_to_smem(acc, sA);
         cp_async_wait_all();
         __syncthreads();
-        solve_by_inverse(sA, sB, acc);
-        store_acc(tile<T>(a, i, col), a.ld, acc);
+        T* out = tile<T>(a, i, col);
+        solve_rows(sA, LDA, sB, [&](int r, int c, T w0, T w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
       }
       publish(a.fin + i * nt + col, 1);
     }
@@ -1851,6 +2189,7 @@ __device__ __forceinline__ DFArgs batch_args(const CholRep& R, const int4* tasks
   a.fin = R.fin;
   a.info = R.info;
   a.invdiag = R.invdiag;
+  a.lp = nullptr;
   a.err = reinterpret_cast<unsigned*>(ctl + 3);
   a.spin_limit = SPIN_LIMIT;
   a.X = nullptr;
@@ -2271,10 +2610,47 @@ std::map<int, std::pair<int4*, int>> g_task_tables;
 
 // Task list of the worker CTAs for an nt x nt tile grid (see the file comment).
 // group: updates per task down a column (2; 4 for the FP32 kernel, whose
-// updates run on the tcgen05 tensor cores); inverse: the tasks that form
-// X = inv(L) as well;
-// inv_tasks: the I(k) tasks that invert the diagonal tiles (left out when the
-// chain CTA stores the inverses itself).
+// updates run on the tcgen05 tensor cores); inv_tasks: the I(k) tasks that
+// store inv(L_kk); inverse: the tasks that form X = inv(L) as well (they need
+// the I(k) tasks).
+std::vector<int4> df_task_list(int nt, int group, bool inv_tasks, bool inverse) {
+  // The chain tasks F(k) and S(k+1, k) run on the chain CTA and are left out.
+  std::vector<int4> t;
+  for (int k = 0; k < nt; ++k) {
+    const int q = k - 1;  // the panel whose trailing updates this block holds
+    if (k > 0 && k + 2 < nt) {
+      // the two updates that LEAD(k) waits for
+      t.push_back(make_int4(TASK_U, k + 2, k + 1, q));
+      t.push_back(make_int4(TASK_U, k + 2, k + 2, q));
+    }
+    if (k + 2 < nt) t.push_back(make_int4(TASK_LEAD, 0, 0, k));
+    for (int i = k + 3; i < nt; ++i) t.push_back(make_int4(TASK_S, i, k, k));
+    if (inv_tasks) t.push_back(make_int4(TASK_I, 0, 0, k));
+    // Column k of the update with panel q is fused into F(k), LEAD(k) and the
+    // S(., k); U(k+1, k, q) and U(k+1, k+1, q) belong to LEAD(q).  The plain
+    // updates cover the rest, columns from the left (rows grouped:
+    // U(i, jj, q), U(i+1, jj, q), ... share L(jj, q)).
+    if (k > 0)
+      for (int jj = k + 1; jj < nt; ++jj) {
+        int i = std::max(jj, k + 3);
+        if (group >= 4)
+          for (; i + 3 < nt; i += 4) t.push_back(make_int4(TASK_U4, i, jj, q));
+        if (group >= 3)
+          for (; i + 2 < nt; i += 3) t.push_back(make_int4(TASK_U3, i, jj, q));
+        for (; i + 1 < nt; i += 2) t.push_back(make_int4(TASK_U2, i, jj, q));
+        if (i < nt) t.push_back(make_int4(TASK_U, i, jj, q));
+      }
+    if (inverse) {
+      // X = inv(L): row k finished, then column q's contributions to the rows
+      // below (pairs of rows)
+      for (int j = 0; j < k; ++j) t.push_back(make_int4(TASK_XZ, k, j, 0));
+      for (int j = 0; j <= q; ++j)
+        for (int i = k + 1; i < nt; i += 2) t.push_back(make_int4(TASK_XG, i, j, q));
+    }
+  }
+  return t;
+}
+
 int get_task_table(int nt, int group, bool inv_tasks, bool inverse, const int4** out, int* count) {
   std::lock_guard<std::mutex> lk(g_task_mu);
   const int key = ((nt * 8 + group) * 2 + (inv_tasks ? 1 : 0)) * 2 + (inverse ? 1 : 0);
@@ -2284,37 +2660,7 @@ int get_task_table(int nt, int group, bool inv_tasks, bool inverse, const int4**
     *count = it->second.second;
     return PBG_OK;
   }
-  // The chain tasks F(k) and S(k+1, k) run on the chain CTA and are left out;
-  // so is I(nt-1), which the chain forms after its last factorisation.
-  std::vector<int4> t;
-  if (nt > 1 && inv_tasks) t.push_back(make_int4(TASK_I, 0, 0, 0));
-  for (int i = 2; i < nt; ++i) t.push_back(make_int4(TASK_S, i, 0, 0));
-  for (int k = 0; k + 1 < nt; ++k) {
-    // the last update of the chain's S(k+2, k+1), first: it runs during F(k+1)
-    if (k + 2 < nt) t.push_back(make_int4(TASK_U, k + 2, k + 1, k));
-    if (k + 2 < nt && inv_tasks) t.push_back(make_int4(TASK_I, 0, 0, k + 1));
-    for (int i = k + 3; i < nt; ++i) t.push_back(make_int4(TASK_S, i, k + 1, k + 1));
-    // the rest of column k+1 of the update with panel k is fused into F(k+1)
-    // and the workers' S(., k+1); the plain updates cover columns >= k+2, the
-    // one gating the next panel first
-    // (rows grouped: U(i, jj, k), U(i+1, jj, k) [, U(i+2, jj, k)] share L_jj,k)
-    for (int jj = k + 2; jj < nt; ++jj) {
-      int i = jj;
-      if (group >= 4)
-        for (; i + 3 < nt; i += 4) t.push_back(make_int4(TASK_U4, i, jj, k));
-      if (group >= 3)
-        for (; i + 2 < nt; i += 3) t.push_back(make_int4(TASK_U3, i, jj, k));
-      for (; i + 1 < nt; i += 2) t.push_back(make_int4(TASK_U2, i, jj, k));
-      if (i < nt) t.push_back(make_int4(TASK_U, i, jj, k));
-    }
-    if (inverse) {
-      // X = inv(L): row k+1 finished, then column k's contributions to the
-      // rows below (pairs of rows)
-      for (int j = 0; j <= k; ++j) t.push_back(make_int4(TASK_XZ, k + 1, j, 0));
-      for (int j = 0; j <= k; ++j)
-        for (int i = k + 2; i < nt; i += 2) t.push_back(make_int4(TASK_XG, i, j, k));
-    }
-  }
+  const std::vector<int4> t = df_task_list(nt, group, inv_tasks, inverse);
   int4* d = nullptr;
   if (!t.empty()) {
     if (cudaMalloc(&d, t.size() * sizeof(int4)) != cudaSuccess) {
@@ -2329,22 +2675,21 @@ int get_task_table(int nt, int group, bool inv_tasks, bool inverse, const int4**
   return PBG_OK;
 }
 
-template <typename T, bool F32CHAIN>
+template <typename T, typename CT>
 size_t df_smem_bytes() {
-  // the chain, or a grouped update (the tensor-core operands in FP32, five
-  // tiles in FP64)
-  return std::max(F32CHAIN ? chain_f32_smem_bytes() : chain_smem_bytes<T>(),
-                  sizeof(T) == 4 ? tc_worker_smem_bytes(2) : 5 * NB * LDA * sizeof(T));
+  // the chain, a LEAD task, or a grouped update (the tensor-core operands in
+  // FP32, five tiles in FP64)
+  return std::max({chain_smem_bytes<CT>(), lead_smem_bytes<T>(),
+                   sizeof(T) == 4 ? tc_worker_smem_bytes(2) : 5 * NB * LDA * sizeof(T)});
 }
 
 // tasks_override / spin_limit: only for the wait-expiry self-test.
-// X (or null): also form X = inv(L) (off-diagonal tiles); ints then holds
-// the X flags after the factorisation's.
-template <typename T, bool F32CHAIN = false>
-int launch_df(T* A, int n, int ld, int* info, void* invdiag, int* ints, unsigned* err, cudaStream_t st,
-              const int4* tasks_override = nullptr, int ntasks_override = 0, long long spin_limit = SPIN_LIMIT,
-              T* X = nullptr) {
-  static_assert(!F32CHAIN || sizeof(T) == 4, "the FP32 chain factors FP32 matrices");
+// inv_tasks: inv(L_kk) goes to invdiag.  X (or null): also form X = inv(L)
+// (off-diagonal tiles); ints then holds the X flags after the factorisation's.
+template <typename T, typename CT>
+int launch_df(T* A, int n, int ld, int* info, void* invdiag, bool inv_tasks, int* ints, void* lp, unsigned* err,
+              cudaStream_t st, const int4* tasks_override = nullptr, int ntasks_override = 0,
+              long long spin_limit = SPIN_LIMIT, T* X = nullptr) {
   const int nt = ld / NB;
   const int4* tasks = nullptr;
   int ntasks = 0;
@@ -2352,19 +2697,19 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, int* ints, unsigned
     tasks = tasks_override;
     ntasks = ntasks_override;
   } else {
-    int rc = get_task_table(nt, sizeof(T) == 4 ? 4 : 2, !F32CHAIN, X != nullptr, &tasks, &ntasks);
+    int rc = get_task_table(nt, sizeof(T) == 4 ? 4 : 2, inv_tasks || X, X != nullptr, &tasks, &ntasks);
     if (rc) return rc;
   }
-  const size_t smem = df_smem_bytes<T, F32CHAIN>();
+  const size_t smem = df_smem_bytes<T, CT>();
   static int max_blocks_per_sm = -1;
   static int num_sms = 0;
   if (max_blocks_per_sm < 0) {
-    PBG_CUDA_TRY(cudaFuncSetAttribute(chol_df_kernel<T, F32CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    PBG_CUDA_TRY(cudaFuncSetAttribute(chol_df_kernel<T, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     int dev;
     PBG_CUDA_TRY(cudaGetDevice(&dev));
     PBG_CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-    PBG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_blocks_per_sm, chol_df_kernel<T, F32CHAIN>,
+    PBG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_blocks_per_sm, chol_df_kernel<T, CT>,
                                                                THREADS, smem));
     if (max_blocks_per_sm < 1) {
       pbg_set_error_message("cholesky kernel does not fit on an SM");
@@ -2391,6 +2736,7 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, int* ints, unsigned
   args.xfin = ints + 3 + 3 * nt * nt;
   args.info = info;
   args.invdiag = invdiag;
+  args.lp = lp;
   args.err = err;
   args.spin_limit = spin_limit;
   cudaLaunchConfig_t cfg = {};
@@ -2403,7 +2749,7 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, int* ints, unsigned
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  PBG_CUDA_TRY(cudaLaunchKernelEx(&cfg, chol_df_kernel<T, F32CHAIN>, args));
+  PBG_CUDA_TRY(cudaLaunchKernelEx(&cfg, chol_df_kernel<T, CT>, args));
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
@@ -2412,7 +2758,7 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, int* ints, unsigned
 
 // Self-test of the bounded waits (no counterpart in the reference): factors a
 // 192 x 192 SPD matrix with a task list from which the host drops the update
-// U(2,2,0), so the wait of F(2) for it can never be satisfied.  The wait
+// LEAD(0), so the chain's wait for U(2,1,0) can never be satisfied.  The wait
 // gives up after spin_limit polls; the launch must end with info = -1 and the
 // barrier error bit, the device must stay usable, and a normal
 // factorisation right after must succeed.  Returns PBG_OK when all of that
@@ -2424,12 +2770,12 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
   if (spin_limit < 1 || spin_limit > (1LL << 24)) return PBG_ERR_ARG;
   const int4* full = nullptr;
   int nfull = 0;
-  int rc = get_task_table(nt, 2, true, false, &full, &nfull);
+  int rc = get_task_table(nt, 2, false, false, &full, &nfull);
   if (rc) return rc;
   std::vector<int4> tasks(nfull);
   PBG_CUDA_TRY(cudaMemcpy(tasks.data(), full, nfull * sizeof(int4), cudaMemcpyDeviceToHost));
   const auto dropped = std::remove_if(tasks.begin(), tasks.end(), [](const int4& t) {
-    return (t.x == TASK_U || t.x == TASK_U2) && t.y == 2 && t.z == 2 && t.w == 0;
+    return t.x == TASK_LEAD && t.w == 0;
   });
   if (dropped == tasks.end()) return PBG_ERR_STATE;
   tasks.erase(dropped, tasks.end());
@@ -2438,13 +2784,13 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
     h[(size_t)i * ld + i] = 4.0;
     if (i > 0) h[(size_t)i * ld + i - 1] = h[(size_t)(i - 1) * ld + i] = 1.0;
   }
-  double *A = nullptr, *inv = nullptr;
+  double *A = nullptr, *lp = nullptr;
   int4* dt = nullptr;
   int* ints = nullptr;
   const size_t nints = 3 + 2 * (size_t)nt * nt + 2;
   bool ok = cudaMalloc(&A, h.size() * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&inv, (size_t)nt * NB * NB * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&dt, tasks.size() * sizeof(int4)) == cudaSuccess &&
+            cudaMalloc(&lp, (size_t)nt * NB * NB * sizeof(double)) == cudaSuccess &&
+            cudaMalloc(&dt, std::max<size_t>(tasks.size(), 1) * sizeof(int4)) == cudaSuccess &&
             cudaMalloc(&ints, nints * sizeof(int)) == cudaSuccess;
   int result = PBG_OK;
   if (!ok) {
@@ -2458,7 +2804,7 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
     cudaMemcpy(A, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(dt, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemset(err, 0, sizeof(unsigned));
-    result = launch_df<double>(A, n, ld, info, inv, ints, err, 0, dt, (int)tasks.size(), spin_limit);
+    result = launch_df<double, double>(A, n, ld, info, nullptr, false, ints, lp, err, 0, dt, (int)tasks.size(), spin_limit);
     if (result == PBG_OK && cudaDeviceSynchronize() != cudaSuccess) result = PBG_ERR_CUDA;
     if (result == PBG_OK) {
       cudaMemcpy(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost);
@@ -2471,7 +2817,7 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
       // the context is still usable: the full task list factors the matrix
       cudaMemcpy(A, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
       cudaMemset(err, 0, sizeof(unsigned));
-      result = launch_df<double>(A, n, ld, info, inv, ints, err, 0);
+      result = launch_df<double, double>(A, n, ld, info, nullptr, false, ints, lp, err, 0);
       if (result == PBG_OK && cudaDeviceSynchronize() != cudaSuccess) result = PBG_ERR_CUDA;
       if (result == PBG_OK) {
         cudaMemcpy(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost);
@@ -2480,7 +2826,7 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
     }
   }
   if (A) cudaFree(A);
-  if (inv) cudaFree(inv);
+  if (lp) cudaFree(lp);
   if (dt) cudaFree(dt);
   if (ints) cudaFree(ints);
   if (result != PBG_OK && result != PBG_ERR_CUDA)
@@ -2504,31 +2850,36 @@ extern "C" __attribute__((visibility("default"))) int pbg_chain_trace(long long*
 #endif
 
 // Scratch of one factorisation: task counter, abort flag, per-tile flags,
-// error word.
+// error word; from the next 256-byte boundary the solve blocks.
+static size_t df_flag_bytes(int nt) { return ((3 + 4 * (size_t)nt * nt + 1) * sizeof(int) + 255) / 256 * 256; }
 size_t df_work_bytes(int ld) {
   const int nt = ld / NB;
-  return (3 + 4 * (size_t)nt * nt + 1) * sizeof(int) + 64;
+  return df_flag_bytes(nt) + (size_t)nt * NB * NB * sizeof(double);
 }
 
-// Factors A in place and writes the inverse of every diagonal factor tile to
-// invdiag (nt x 64 x 64 row-major tiles, precision of A; the solves of the
-// factorisation use them, and so do the SPD inverse and the triangular solve
-// of the midpoint scheme).  Both A and invdiag start on 16-byte boundaries.
-int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* invdiag, void* work,
+// Factors A in place; with want_inv (or X) the inverse of every diagonal
+// factor tile goes to invdiag (nt x 64 x 64 row-major tiles, precision of A:
+// the SPD inverse and the triangular solve of the midpoint scheme use them).
+// A, invdiag and work start on 16-byte boundaries.
+int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* invdiag, bool want_inv, void* work,
                        cudaStream_t st, void* X) {
   const int nt = ld / NB;
-  if (reinterpret_cast<uintptr_t>(A) % 16 != 0 || reinterpret_cast<uintptr_t>(invdiag) % 16 != 0) {
+  if (reinterpret_cast<uintptr_t>(A) % 16 != 0 || reinterpret_cast<uintptr_t>(invdiag) % 16 != 0 ||
+      reinterpret_cast<uintptr_t>(work) % 16 != 0) {
     pbg_set_error_message("cholesky: the matrix and its workspace must start on 16-byte boundaries");
     return PBG_ERR_ARG;
   }
   int* ints = static_cast<int*>(work);
   unsigned* err = reinterpret_cast<unsigned*>(ints + 3 + 4 * (size_t)nt * nt);
+  void* lp = static_cast<unsigned char*>(work) + df_flag_bytes(nt);
   if (precision == PBG_PREC_FP64)
-    return launch_df<double>((double*)A, n, ld, info, invdiag, ints, err, st, nullptr, 0, SPIN_LIMIT, (double*)X);
+    return launch_df<double, double>((double*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0,
+                                     SPIN_LIMIT, (double*)X);
   if (precision == PBG_PREC_MIXED_FP64_DIAG)
-    return launch_df<float, false>((float*)A, n, ld, info, invdiag, ints, err, st, nullptr, 0, SPIN_LIMIT,
-                                   (float*)X);
-  return launch_df<float, true>((float*)A, n, ld, info, invdiag, ints, err, st, nullptr, 0, SPIN_LIMIT, (float*)X);
+    return launch_df<float, double>((float*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0,
+                                    SPIN_LIMIT, (float*)X);
+  return launch_df<float, float>((float*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0, SPIN_LIMIT,
+                                 (float*)X);
 }
 
 
@@ -3016,7 +3367,7 @@ int tc_factor_invert(int ld, int* info, void* work, cudaStream_t st) {
     return PBG_ERR_ARG;
   }
   // the factorisation forms X's off-diagonal tiles in the same launch
-  int rc = launch_cholesky_df(w.F, ld, ld, PBG_PREC_MIXED, info, w.invdiag, w.scratch, st, w.X);
+  int rc = launch_cholesky_df(w.F, ld, ld, PBG_PREC_MIXED, info, w.invdiag, true, w.scratch, st, w.X);
   if (rc != PBG_OK) return rc;
   return launch_trtri_diag(w.invdiag, w.X, ld, PBG_PREC_MIXED, st);
 }

@@ -122,16 +122,17 @@ int launch_jo_pair(double ai, double aj, double rx, double ry, double rz, double
 // ---- cholesky.cu ----------------------------------------------------------
 // Sets rows/cols n..ld-1 of an ld x ld matrix to the identity.
 int launch_pad_identity(void* A, int n, int ld, int precision, cudaStream_t st);
-// Workspace: inverted diagonal tiles of the factor followed by the data-flow
-// scratch (see cholesky.cu).
+// Workspace: inverted diagonal tiles of the factor (written with want_inv)
+// followed by the data-flow scratch (see cholesky.cu).
 size_t cholesky_work_bytes(int ld, int precision);
-int launch_cholesky_ws(void* A, int n, int ld, int precision, int* info, void* work, cudaStream_t st);
+int launch_cholesky_ws(void* A, int n, int ld, int precision, int* info, void* work, cudaStream_t st,
+                       bool want_inv = false);
 // cholesky_df.cu
 size_t df_work_bytes(int ld);
 // X (or null): the same launch also forms the off-diagonal tiles of
 // X = inv(L) (ld x ld, lower; launch_trtri_diag copies the diagonal ones from
 // invdiag).
-int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* invdiag, void* work,
+int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* invdiag, bool want_inv, void* work,
                        cudaStream_t st, void* X = nullptr);
 size_t spd_inverse_work_bytes(int ld);
 int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStream_t st);
@@ -162,7 +163,7 @@ int tc_reversed_factor(const float* X, const float* G, int ld, double s, float* 
 // Batched factorisation of many independent matrices (one per replica).
 struct CholRep {
   void* A;        // ld x ld, padded with the identity beyond n
-  void* invdiag;  // nt x 64 x 64: inv(L_kk) tiles
+  void* invdiag;  // nt x 64 x 64: inv(L_kk) tiles (FP32), the solve blocks of L_kk (FP64)
   int* upd;       // nt x nt, zero before the launch
   int* fin;       // nt x nt, zero before the launch
   int* info;      // zero before the launch

@@ -402,7 +402,9 @@ int decompose(pbg_system* s, cudaStream_t st) {
     PBG_CHECK_LAUNCH();
   }
   s->b_holds_lower_D = false;  // the factorisation overwrites it
-  return launch_cholesky_ws(s->B, s->n, s->ld, s->prec, s->dflags + 1, s->chol_work, st);
+  // the midpoint scheme's back substitution needs the inverted diagonal tiles
+  return launch_cholesky_ws(s->B, s->n, s->ld, s->prec, s->dflags + 1, s->chol_work, st,
+                            s->p.propagation_scheme == PBG_SCHEME_MIDPOINT);
 }
 
 static int overlap_check(pbg_system* s, cudaStream_t st, bool* overlap) {
