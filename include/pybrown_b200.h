@@ -104,7 +104,8 @@ PBG_API int pbg_dev_rpy_matrix(const double *pos, const double *radii, int n_bea
 
 /* Smith-Ewald RPY (diff_tensor.c:170-266) from positions. precision:
  * PBG_PREC_FP64 writes doubles to M; PBG_PREC_MIXED writes floats (M is a
- * float*).  Scratch (phase tables) is taken from the stream-ordered pool. */
+ * float*).  No scratch; the lattice weights of a parameter set are kept on the
+ * device after its first use. */
 PBG_API int pbg_dev_smith_matrix(const double *pos, const double *radii, int n_beads, double box_length,
                          double alpha, int m_max, int n_max, double scale, int precision,
                          void *M, int ld, void *stream);
@@ -113,12 +114,12 @@ PBG_API int pbg_dev_smith_matrix(const double *pos, const double *radii, int n_b
  * memory (an application whose own memory manager holds all of it, or a step
  * loop that must not hit the device-wide synchronisation of cudaMalloc/cudaFree).
  * No counterpart in the reference: it is an addition of this library.
- * All scratch lives in one fixed array inside the library (about 4.3 MiB held
+ * The lattice weights live in one fixed array inside the library (9 KiB held
  * by every GPU that loads it, until exit); nothing is allocated.  Limits:
  * at most 4096 real-space images, 2048 reciprocal half-vectors and
- * n_beads * (reciprocal half-vectors) * 16 bytes <= 4 MiB of phase tables
- * (e.g. 4096 beads at ewald_imag = 4); larger inputs (checked before any
- * table is built) return PBG_ERR_ARG.  The lattice tables reach the array as
+ * n_beads * (reciprocal half-vectors) * 16 bytes (8 in the mixed precision)
+ * <= 4 MiB (e.g. 4096 beads at ewald_imag = 4); larger inputs (checked before
+ * any table is built) return PBG_ERR_ARG.  The lattice tables reach the array as
  * kernel launch parameters, so no host buffer is staged and the host does not
  * wait for the stream.  The first call on a device looks up the array's device
  * address (make it before any stream capture).  Every call reuses the same

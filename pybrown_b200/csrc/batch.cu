@@ -11,8 +11,8 @@
 // per-replica descriptors and work lists that the kernels read are rebuilt
 // only when the membership changes, so replicas can join and leave between
 // steps while the others keep their state on the device.  One step is a
-// fixed sequence of launches over all replicas: phase tables and Ewald tiles
-// (one work list), the padded copy into B, one cooperative data-flow Cholesky
+// fixed sequence of launches over all replicas: Ewald tiles (one work list),
+// written to D and to B's lower triangle, one cooperative data-flow Cholesky
 // over every replica's tiles (left-looking on the tcgen05 tensor cores in the
 // mixed precision, right-looking DMMA tile tasks in FP64), then the
 // per-replica vector kernels (replica = blockIdx.y).  Replicas never interact, and each one's arithmetic does not
@@ -57,7 +57,7 @@ struct BatchReplica {
   int N = 0, n = 0, ld = 0, nt = 0;
   double scale = 0;  // kBT 1e19 / eta: D = scale * M (box.py:498)
   double *pos = nullptr, *radii = nullptr, *force = nullptr, *U = nullptr, *xi = nullptr;
-  void *D = nullptr, *B = nullptr, *invdiag = nullptr, *phase = nullptr;
+  void *D = nullptr, *B = nullptr, *invdiag = nullptr;
   bool has_force = false;
   unsigned long long seed = 0, draws = 0;
   // this replica's Cholesky task list on the device (built once, when added)
@@ -171,21 +171,6 @@ __global__ void batch_copy_lower_kernel(const BatchDev* __restrict__ reps) {
     if (row < n && col < n) v = col <= row ? src[t] : (T)0;
     else v = (T)(row == col ? 1 : 0);
     dst[t] = v;
-  }
-}
-
-// The padding rows of B's lower triangle: identity (rows n .. ld-1, columns
-// up to the diagonal).  The rest of the lower triangle comes from the Ewald
-// build; nothing reads B above the diagonal.
-template <typename T>
-__global__ void batch_pad_lower_kernel(const BatchDev* __restrict__ reps) {
-  const BatchDev& r = reps[blockIdx.y];
-  T* dst = static_cast<T*>(r.B);
-  const int n = r.n, ld = r.ld;
-  const long long total = (long long)(ld - n) * ld;
-  for (long long t = threadIdx.x; t < total; t += blockDim.x) {
-    const int row = n + (int)(t / ld), col = (int)(t % ld);
-    if (col <= row) dst[(size_t)row * ld + col] = (T)(row == col ? 1 : 0);
   }
 }
 
@@ -366,7 +351,7 @@ inline size_t elem_size(int precision) { return precision == PBG_PREC_FP64 ? 8 :
 // on that stream (and on every blocking stream) and need no device-wide sync.
 void free_replica(BatchReplica* r) {
   if (!r) return;
-  void* bufs[] = {r->pos, r->radii, r->force, r->U, r->xi, r->D, r->B, r->invdiag, r->phase, r->tasks};
+  void* bufs[] = {r->pos, r->radii, r->force, r->U, r->xi, r->D, r->B, r->invdiag, r->tasks};
   for (void* p : bufs)
     if (p) cudaFreeAsync(p, 0);
   delete r;
@@ -567,7 +552,7 @@ int rebuild(pbg_batch* b, cudaStream_t st) {
     d.check = r->p.check_overlaps;
     d.has_force = r->has_force;
     d.pad = 0;
-    rpy_batch_arg(r->pos, r->radii, r->N, r->p.box_length, smith, b->tables, r->scale, r->D, r->B, r->ld, r->phase,
+    rpy_batch_arg(r->pos, r->radii, r->N, r->p.box_length, smith, b->tables, r->scale, r->D, r->B, r->ld,
                   rpy.data() + q * rpy_batch_arg_bytes());
     CholRep& c = chol[q];
     c.A = r->B;
@@ -762,19 +747,14 @@ PBG_API int pbg_cholesky_task_list(int nt, int precision, int* tasks, int cap, i
   return PBG_OK;
 }
 
-// Device bytes a replica of n_beads takes in a batch of this precision.
+// Device bytes a replica of n_beads takes in a batch of this precision (the
+// Ewald build keeps no per-bead tables, so the lattice does not enter).
 PBG_API long long pbg_batch_footprint(int precision, int hydrodynamics, int ewald_imag, int n_beads) {
+  (void)hydrodynamics;
+  (void)ewald_imag;
   const long long n = 3LL * n_beads, ld = (n + PBG_TILE - 1) / PBG_TILE * PBG_TILE, nt = ld / PBG_TILE;
   const long long es = elem_size(precision);
-  long long n_recip = 0;
-  if (hydrodynamics == PBG_HI_RPY_SMITH)
-    for (int x = -ewald_imag; x <= ewald_imag; ++x)
-      for (int y = -ewald_imag; y <= ewald_imag; ++y)
-        for (int z = -ewald_imag; z <= ewald_imag; ++z)
-          if (std::abs(x) + std::abs(y) + std::abs(z) <= ewald_imag && (x || y || z)) ++n_recip;
-  n_recip /= 2;
-  return 2 * ld * ld * es + nt * PBG_TILE * PBG_TILE * es + (long long)n_beads * n_recip * 2 * es +
-         (4 * ld + 4 * n_beads) * 8 + 2 * nt * nt * 4;
+  return 2 * ld * ld * es + nt * PBG_TILE * PBG_TILE * es + (4 * ld + 4 * n_beads) * 8 + 2 * nt * nt * 4;
 }
 
 PBG_API int pbg_batch_add(pbg_batch* b, const pbg_params* p, const double* pos, const double* radii, int* slot) {
@@ -800,8 +780,6 @@ PBG_API int pbg_batch_add(pbg_batch* b, const pbg_params* p, const double* pos, 
             pool_alloc(&r->force, ld * sizeof(double)) && pool_alloc(&r->U, ld * sizeof(double)) &&
             pool_alloc(&r->xi, ld * sizeof(double)) && pool_alloc(&r->D, ld * ld * es) &&
             pool_alloc(&r->B, ld * ld * es) && pool_alloc(&r->invdiag, (size_t)r->nt * PBG_TILE * PBG_TILE * es);
-  const size_t ph = phase_scratch_bytes(r->N, b->tables, b->precision);
-  if (ok && ph) ok = pool_alloc(&r->phase, ph);
   std::vector<int4> tasks;
   cholesky_replica_tasks(r->nt, b->precision, tasks, r->seg_start);
   if (ok && !tasks.empty()) {
@@ -949,21 +927,17 @@ static int enqueue_begin(pbg_batch* b, double dt, int build_D, int cholesky, boo
   const bool smith = b->hydrodynamics == PBG_HI_RPY_SMITH;
   int rc;
   // a step that builds and factors D has the Ewald build write D's lower
-  // triangle into B as well; only B's padding rows are then set here
-  if (build_D && (rc = launch_rpy_batch(b->precision, smith, b->tables, b->d_rpy, b->d_ework, b->n_ework, R,
+  // triangle (and the padding) into B as well
+  if (build_D && (rc = launch_rpy_batch(b->precision, smith, b->tables, b->d_rpy, b->d_ework, b->n_ework,
                                         cholesky != 0, st)))
     return rc;
   if (cholesky) {
-    if (build_D) {
-      const dim3 g(1, R);
-      if (f64) batch_pad_lower_kernel<double><<<g, 256, 0, st>>>(b->d_reps);
-      else batch_pad_lower_kernel<float><<<g, 256, 0, st>>>(b->d_reps);
-    } else {
+    if (!build_D) {
       const dim3 g(64, R);
       if (f64) batch_copy_lower_kernel<double><<<g, 256, 0, st>>>(b->d_reps);
       else batch_copy_lower_kernel<float><<<g, 256, 0, st>>>(b->d_reps);
+      PBG_CHECK_LAUNCH();
     }
-    PBG_CHECK_LAUNCH();
     PBG_CUDA_TRY(cudaMemsetAsync(b->d_flags, 0, b->flag_ints * sizeof(int), st));
     if ((rc = launch_cholesky_batch(b->precision, b->d_chol, b->d_tasks, b->ntasks, b->d_flags, b->ctas_per_sm, st)))
       return rc;

@@ -114,11 +114,10 @@ int legacy_rpy(double* as, double* pointers, int N, bool smith, double L, double
     if (rc) return rc;
   }
   const size_t n3 = 3 * (size_t)N, npairs = (size_t)N * (N - 1) / 2;
-  DevBuf d_as(st), d_pairs(st), d_pos(st), d_M(st), d_phase(st);
+  DevBuf d_as(st), d_pairs(st), d_pos(st), d_M(st);
   int rc;
   if ((rc = d_as.alloc(N * sizeof(double))) || (rc = d_pairs.alloc(3 * npairs * sizeof(double))) ||
-      (rc = d_pos.alloc(3 * (size_t)N * sizeof(double))) || (rc = d_M.alloc(n3 * n3 * sizeof(double))) ||
-      (rc = d_phase.alloc(pbg::phase_scratch_bytes(N, t, PBG_PREC_FP64))))
+      (rc = d_pos.alloc(3 * (size_t)N * sizeof(double))) || (rc = d_M.alloc(n3 * n3 * sizeof(double))))
     return rc;
   if ((rc = h2d(d_as.p, as, N * sizeof(double), st))) return rc;
   if (npairs && (rc = h2d(d_pairs.p, pointers, 3 * npairs * sizeof(double), st))) return rc;
@@ -129,7 +128,7 @@ int legacy_rpy(double* as, double* pointers, int N, bool smith, double L, double
   pbg::PairSource src{nullptr, npairs ? d_pairs.as<double>() : nullptr, N, L};
   if (!npairs) src.pos = d_pos.as<double>();
   if ((rc = pbg::launch_rpy_tensor(src, d_pos.as<double>(), d_as.as<double>(), smith, t, 1.0, PBG_PREC_FP64,
-                                   d_M.p, (int)n3, d_phase.p, st)))
+                                   d_M.p, (int)n3, st)))
     return rc;
   if ((rc = d2h(M, d_M.p, n3 * n3 * sizeof(double), st))) return rc;
   return sync(st);
@@ -273,7 +272,7 @@ int pbg_dev_rpy_matrix(const double* pos, const double* radii, int n_beads, doub
                        double* M, int ld, void* stream) {
   if (n_beads < 0 || ld < 3 * n_beads) return PBG_ERR_ARG;
   pbg::PairSource src{pos, nullptr, n_beads, box_length};
-  return pbg::launch_rpy_tensor(src, pos, radii, false, nullptr, scale, PBG_PREC_FP64, M, ld, nullptr,
+  return pbg::launch_rpy_tensor(src, pos, radii, false, nullptr, scale, PBG_PREC_FP64, M, ld,
                                 (cudaStream_t)stream);
 }
 
@@ -285,10 +284,8 @@ int pbg_dev_smith_matrix(const double* pos, const double* radii, int n_beads, do
   const pbg::EwaldTables* t = nullptr;
   int rc = pbg::get_ewald_tables(alpha, m_max, n_max, &t);
   if (rc) return rc;
-  DevBuf phase(st);
-  if ((rc = phase.alloc(pbg::phase_scratch_bytes(n_beads, t, precision)))) return rc;
   pbg::PairSource src{pos, nullptr, n_beads, box_length};
-  return pbg::launch_rpy_tensor(src, pos, radii, true, t, scale, precision, M, ld, phase.p, st);
+  return pbg::launch_rpy_tensor(src, pos, radii, true, t, scale, precision, M, ld, st);
 }
 
 int pbg_dev_lubrication_add(const double* pos, const double* radii, int n_beads, double box_length, double cutoff,

@@ -71,17 +71,14 @@ int launch_overlap(const double* pos, const double* radii, int n, double L, doub
                    const int* conn, int* flag, cudaStream_t st);
 
 // ---- ewald.cu -------------------------------------------------------------
-// Reciprocal-space and real-space tables of one (alpha, m_max, n_max) set.
+// Weights and self-block sums of one (alpha, m_max, n_max) set.
 struct EwaldTables {
   double alpha = 0;
   int m_max = -1, n_max = -1;
-  int n_real = 0;      // images with |m|_1 <= m_max (m = 0 included)
-  int n_recip = 0;     // half of the n != 0 vectors with |n|_1 <= n_max
   double self_O[6];    // lattice sums of the self block (a-independent part)
   double self_Q[6];
-  double* d_real = nullptr;   // n_real x 4 doubles: mx, my, mz, 0
-  double* d_recip = nullptr;  // n_recip x 8 doubles: nx, ny, nz, P, R, S, 0, 0
-  float* d_recip_f = nullptr; // same, float
+  double* d_w = nullptr;   // [n_max^2 + 1][4]: the reciprocal weights P, R, S of a vector by |n|^2
+  float* d_w_f = nullptr;  // same, float
 };
 
 // Returns the (cached) tables for a parameter set; they live until exit.
@@ -91,26 +88,23 @@ int get_ewald_tables(double alpha, int m_max, int n_max, const EwaldTables** out
 // of ewald_imag = n.
 long long lattice_points_l1(int m);
 // Host tables of one (alpha, m_max, n_max) set in the layout of EwaldTables
-// (real: 4 doubles per image, recip: 8 doubles per half-vector) and the
-// a-independent self-block lattice sums.  The one builder behind every
-// device copy of the tables.
-void build_lattice_tables(double alpha, int m_max, int n_max, std::vector<double>& real,
-                          std::vector<double>& recip, double self_O[6], double self_Q[6]);
+// (w: 4 doubles per |n|^2, the row of n = 0 zero) and the a-independent
+// self-block lattice sums.  The one builder behind every device copy.
+void build_lattice_tables(double alpha, int m_max, int n_max, std::vector<double>& w, double self_O[6],
+                          double self_Q[6]);
 
 // Writes scale * M for the free-space (smith == false) or Smith-Ewald RPY
 // tensor of positions `pos` into M (row-major, leading dimension ld).
 // precision: PBG_PREC_FP64 (double* M) or PBG_PREC_MIXED (float* M).
-// `phase` is scratch of phase_scratch_bytes(n, tables) bytes (may be null for
-// the free-space tensor).
-size_t phase_scratch_bytes(int n, const EwaldTables* t, int precision);
 // `pos` feeds the reciprocal phases (for pair-vector input pass the
 // reconstructed coordinates of launch_positions_from_pairs).
 // M_lower (optional): a second matrix that receives the same values in the
 // bead tiles on and below the block diagonal (every element of the lower
 // triangle; the rest of it is left as it was).
+// pad: rows and columns 3n .. ld-1 of M (rows of M_lower) are set to the identity.
 int launch_rpy_tensor(const PairSource& src, const double* pos, const double* radii, bool smith,
-                      const EwaldTables* t, double scale, int precision, void* M, int ld,
-                      void* phase, cudaStream_t st, void* M_lower = nullptr);
+                      const EwaldTables* t, double scale, int precision, void* M, int ld, cudaStream_t st,
+                      void* M_lower = nullptr, bool pad = false);
 
 // ---- lubrication.cu -------------------------------------------------------
 int launch_lubrication_add(const PairSource& src, const double* radii, double cutoff,
@@ -184,11 +178,12 @@ int launch_cholesky_batch(int precision, const CholRep* reps, const int4* tasks,
 // a work list of bead tiles (x = replica, y = I, z = J with I >= J).
 size_t rpy_batch_arg_bytes();
 // Fills the argument block of one replica into `dst` (rpy_batch_arg_bytes() bytes);
-// M_lower: the matrix that receives the lower block triangle when a launch asks for it.
+// M_lower: the matrix that receives the lower block triangle when a launch asks
+// for it.  The padding of both is written too.
 void rpy_batch_arg(const double* pos, const double* radii, int n, double L, bool smith, const EwaldTables* t,
-                   double scale, void* M, void* M_lower, int ld, void* phase, void* dst);
+                   double scale, void* M, void* M_lower, int ld, void* dst);
 void rpy_batch_work(int replica, int n, std::vector<int4>& work);
 int launch_rpy_batch(int precision, bool smith, const EwaldTables* t, const void* args, const int4* work,
-                     int nwork, int n_replicas, bool fill_lower, cudaStream_t st);
+                     int nwork, bool fill_lower, cudaStream_t st);
 
 }  // namespace pbg

@@ -1,14 +1,13 @@
 // Allocation-free variant of the Smith-Ewald RPY tensor build.
 //
-// pbg_dev_smith_matrix takes its scratch (the per-bead reciprocal-space phase
-// tables) from the stream-ordered pool and its lattice tables from a cached
-// cudaMalloc.  Some callers cannot allow either: an application whose memory
-// manager has already claimed all device memory, or a step loop that must not
-// run into the implicit device-wide synchronisation of cudaMalloc/cudaFree
-// while other streams are busy.  pbg_dev_smith_matrix_noalloc does the same
-// computation with every byte of scratch in one file-scope device array of
-// fixed size, so it never allocates.  Every GPU that loads the library holds
-// this array until the process exits.
+// pbg_dev_smith_matrix takes its lattice tables from a cached cudaMalloc.  Some
+// callers cannot allow that: an application whose memory manager has already
+// claimed all device memory, or a step loop that must not run into the
+// implicit device-wide synchronisation of cudaMalloc/cudaFree while other
+// streams are busy.  pbg_dev_smith_matrix_noalloc does the same computation
+// with its tables in one file-scope device array of fixed size, so it never
+// allocates.  Every GPU that loads the library holds this array until the
+// process exits.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -21,16 +20,19 @@
 namespace pbg {
 namespace {
 
-// Capacities of the shared scratch array.
-constexpr int NOALLOC_MAX_REAL = 4096;       // real-space images, |m|_1 <= ewald_real
-constexpr int NOALLOC_MAX_RECIP = 2048;      // half of the n != 0 vectors, |n|_1 <= ewald_imag
-constexpr size_t NOALLOC_PHASE_BYTES = 4u << 20;  // n_beads * n_recip * 16 bytes at most
-constexpr size_t NOALLOC_REAL_BYTES = (size_t)NOALLOC_MAX_REAL * 4 * sizeof(double);
-constexpr size_t NOALLOC_RECIP_BYTES = (size_t)NOALLOC_MAX_RECIP * 8 * sizeof(double);
-constexpr size_t NOALLOC_RECIP_F_BYTES = (size_t)NOALLOC_MAX_RECIP * 8 * sizeof(float);
-constexpr size_t NOALLOC_BYTES = NOALLOC_REAL_BYTES + NOALLOC_RECIP_BYTES + NOALLOC_RECIP_F_BYTES + NOALLOC_PHASE_BYTES;
+// Sizes that the call takes: images |m|_1 <= ewald_real, half of the n != 0
+// vectors |n|_1 <= ewald_imag, and n_beads * half-vectors * 16 (FP64) or 8
+// bytes.  (The kernels need no per-bead tables; the last limit is the call's
+// documented one.)
+constexpr int NOALLOC_MAX_REAL = 4096;
+constexpr int NOALLOC_MAX_RECIP = 2048;
+constexpr size_t NOALLOC_PHASE_BYTES = 4u << 20;
+// The weight tables: ewald_imag <= 14 by the second limit, 4 values per |n|^2.
+constexpr int NOALLOC_MAX_IMAG = 14;
+constexpr size_t NOALLOC_W = 4 * (NOALLOC_MAX_IMAG * NOALLOC_MAX_IMAG + 1);
+constexpr size_t NOALLOC_BYTES = NOALLOC_W * (sizeof(double) + sizeof(float));
 
-// Layout: [real images][reciprocal table FP64][reciprocal table FP32][phase tables].
+// Layout: [weights FP64][weights FP32].
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
 // Device address of g_noalloc_scratch, looked up once per device (in host
@@ -119,25 +121,17 @@ extern "C" int pbg_dev_smith_matrix_noalloc(const double* pos, const double* rad
   void* base = nullptr;
   int rc = scratch_address(&base);
   if (rc) return rc;
-  std::vector<double> real, recip;
+  std::vector<double> w;
   EwaldTables t;
-  build_lattice_tables(alpha, m_max, n_max, real, recip, t.self_O, t.self_Q);
+  build_lattice_tables(alpha, m_max, n_max, w, t.self_O, t.self_Q);
   t.alpha = alpha;
   t.m_max = m_max;
   t.n_max = n_max;
-  t.n_real = (int)(real.size() / 4);
-  t.n_recip = (int)(recip.size() / 8);
-  unsigned char* b = static_cast<unsigned char*>(base);
-  t.d_real = reinterpret_cast<double*>(b);
-  t.d_recip = reinterpret_cast<double*>(b + NOALLOC_REAL_BYTES);
-  t.d_recip_f = reinterpret_cast<float*>(b + NOALLOC_REAL_BYTES + NOALLOC_RECIP_BYTES);
-  void* phase = b + NOALLOC_REAL_BYTES + NOALLOC_RECIP_BYTES + NOALLOC_RECIP_F_BYTES;
-  // The tables are rewritten by every call (stream-ordered before the kernels
-  // that read them); the phase tables are fully written by the phase kernel.
-  rc = upload_table(real, t.d_real, nullptr, st);
-  if (rc) return rc;
-  rc = upload_table(recip, t.d_recip, t.d_recip_f, st);
-  if (rc) return rc;
+  t.d_w = static_cast<double*>(base);
+  t.d_w_f = reinterpret_cast<float*>(t.d_w + NOALLOC_W);
+  // The tables are rewritten by every call (stream-ordered before the kernel
+  // that reads them).
+  if ((rc = upload_table(w, t.d_w, t.d_w_f, st))) return rc;
   PairSource src{pos, nullptr, n_beads, box_length};
-  return launch_rpy_tensor(src, pos, radii, true, &t, scale, precision, M, ld, phase, st);
+  return launch_rpy_tensor(src, pos, radii, true, &t, scale, precision, M, ld, st);
 }

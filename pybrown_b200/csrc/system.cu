@@ -137,7 +137,7 @@ void destroy_system(pbg_system* s) {
   free_immobile(s);
   void* ptrs[] = {s->pos,  s->pos_snap, s->radii, s->conn,  s->force, s->D,     s->B,    s->D0,
                   s->Mff,  s->Rff,      s->R,     s->Mff0,  s->Rff0,  s->R0,    s->FX,   s->U,
-                  s->BX,   s->ddet,     s->y,     s->rwork, s->Dy,    s->drift, s->xi,   s->phase,
+                  s->BX,   s->ddet,     s->y,     s->rwork, s->Dy,    s->drift, s->xi,
                   s->chol_work, s->inv_work, s->dflags, s->div, s->sol, s->sol0, s->res, s->corr,
                   s->G,    s->tflags};
   for (void* p : ptrs)
@@ -207,7 +207,6 @@ int create_system(const pbg_params* prm, pbg_system** out) {
   double** vecs[] = {&s->FX, &s->U,  &s->BX,   &s->ddet, &s->y,   &s->rwork, &s->Dy,
                      &s->drift, &s->xi, &s->sol, &s->sol0, &s->res, &s->corr};
   for (double** v : vecs) SYS_ALLOC(*v, ld * sizeof(double));
-  if (s->smith) SYS_ALLOC(s->phase, phase_scratch_bytes(s->N, s->tables, s->prec));
   SYS_ALLOC(s->chol_work, cholesky_work_bytes(s->ld, s->prec));
   SYS_ALLOC(s->dflags, 8 * sizeof(int));
   SYS_ALLOC(s->tflags, (ld / PBG_TILE) * sizeof(int));
@@ -304,23 +303,16 @@ int compute_Dff(pbg_system* s, cudaStream_t st, bool fill_B) {
     // when this step factors D, the build also writes D's lower triangle into
     // B (the factorisation's input), so decompose needs no copy
     void* lower = fill_B ? s->B : nullptr;
-    rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, s->prec, s->D, s->ld, s->phase, st,
-                           lower);
+    rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, s->prec, s->D, s->ld, st, lower, true);
     if (rc) return rc;
-    if ((rc = launch_pad_identity(s->D, s->n, s->ld, s->prec, st))) return rc;
-    if (lower) {
-      if ((rc = launch_pad_identity(s->B, s->n, s->ld, s->prec, st))) return rc;
-      s->b_holds_lower_D = true;
-    }
+    if (lower) s->b_holds_lower_D = true;
     return PBG_OK;
   }
   const double scale = 1e19 / p.viscosity;
   if (s->mlub) {
     // Mff in FP32, Rff = inv(Mff) on the tensor cores (a copy is factored)
-    rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, PBG_PREC_MIXED, s->Mff, s->ld, s->phase,
-                           st);
-    if (rc) return rc;
-    rc = launch_pad_identity(s->Mff, s->n, s->ld, PBG_PREC_MIXED, st);
+    rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, PBG_PREC_MIXED, s->Mff, s->ld, st, nullptr,
+                           true);
     if (rc) return rc;
     const TcInverseWork w = tc_inverse_work(s->inv_work, s->ld);
     PBG_CUDA_TRY(cudaMemcpyAsync(w.F, s->Mff, (size_t)s->ld * s->ld * sizeof(float), cudaMemcpyDeviceToDevice, st));
@@ -328,9 +320,7 @@ int compute_Dff(pbg_system* s, cudaStream_t st, bool fill_B) {
     if ((rc = tc_factor_invert(s->ld, s->dflags + 2, s->inv_work, st))) return rc;
     return tc_lauum(w.X, s->ld, 1.0f, false, (float*)s->Rff, s->dflags + 2, st);
   }
-  rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, PBG_PREC_FP64, s->Mff, s->ld, s->phase, st);
-  if (rc) return rc;
-  rc = launch_pad_identity(s->Mff, s->n, s->ld, PBG_PREC_FP64, st);
+  rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, PBG_PREC_FP64, s->Mff, s->ld, st, nullptr, true);
   if (rc) return rc;
   PBG_CUDA_TRY(cudaMemcpyAsync(s->Rff, s->Mff, (size_t)s->ld * s->ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
   return launch_spd_inverse(s->Rff, s->n, s->ld, s->dflags + 2, s->inv_work, st);

@@ -39,7 +39,6 @@ struct pbg_system {
   double *FX = nullptr, *U = nullptr, *BX = nullptr, *ddet = nullptr, *y = nullptr;
   double *rwork = nullptr, *Dy = nullptr, *drift = nullptr, *xi = nullptr;  // ld each
   double *sol = nullptr, *sol0 = nullptr, *res = nullptr, *corr = nullptr;  // ld each: refined solves (mlub)
-  void* phase = nullptr;       // Ewald phase tables
   void* chol_work = nullptr;   // inverted diagonal tiles of B
   void* inv_work = nullptr;    // SPD inverse workspace (tensor-core inverse workspace if mlub)
   int* dflags = nullptr;       // [0] overlap, [1] cholesky info, [2] Rff info, [3] D info,
