@@ -72,7 +72,27 @@ struct GatherSeg {
   int count, replica;
 };
 
-// What the vector kernels need of one replica.
+// Attempts of one replica that a round evaluates together once its first
+// attempt of the step was rejected (see batch_trmv_kernel).
+constexpr int SPEC = 8;
+
+// An entry of a round's work list: replica q with `attempts` attempts, its first
+// unit of the B xi product and of the overlap test.
+struct RoundEntry {
+  int q, attempts, trmv0, ovl0;
+};
+// Entry counts and units of the two lists (one being worked on, the next one
+// being built), count << 48 | product units << 26 | overlap units, so that one
+// atomic reserves a consistent place in all three; blocks done.
+struct RoundState {
+  unsigned long long packed[2];
+  int done, pad;
+};
+constexpr int TRMV_ROWS = 16;  // rows per unit of the product: two per warp
+constexpr int OVL_BEADS = 8;   // beads per unit of the overlap test: one per warp
+
+// What the vector kernels need of one replica.  U: SPEC + 1 vectors of ld, xi:
+// SPEC vectors of ld.
 struct BatchDev {
   double* pos;
   const double* radii;
@@ -115,7 +135,11 @@ struct pbg_batch {
   int* d_flags = nullptr;  // [4 ctl][per replica: upd nt^2, fin nt^2][R infos]
   size_t flag_ints = 0;
   int* d_info = nullptr;
-  int* d_ovl = nullptr;
+  int* d_ovl = nullptr;                // [cap][SPEC] overlap flags of a round's candidates
+  int* d_rejected = nullptr;           // [cap] outcome of a host-driven attempt
+  int* d_spec = nullptr;               // [cap] attempts of the present round
+  pbg::RoundEntry* d_lists = nullptr;  // [2][cap]
+  pbg::RoundState* d_state = nullptr;
   unsigned char* d_mask = nullptr;
   unsigned long long* d_stream = nullptr;  // [R][2]: seed, draws of each noise stream
   int* h_ovl = nullptr;  // pinned, read after a stream synchronisation
@@ -197,47 +221,174 @@ __global__ void batch_det_move_kernel(const BatchDev* __restrict__ reps) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r.n; i += gridDim.x * blockDim.x) r.pos[i] += r.U[i];
 }
 
-// U = B xi for the masked replicas (box.py:371; B lower triangular).
+// ---- attempt rounds -------------------------------------------------------
+// A replica's stochastic attempts (box.py:219-248) in rounds: xi, U = B xi and
+// the move, the overlap test, the undo of rejected moves and the bookkeeping.
+// The first attempt of a step goes alone; a replica whose attempt was rejected
+// takes its next SPEC attempts in one round: their noise is at known places of
+// its stream, B is read once for all of them, and the first accepted one
+// counts, exactly as if they had been made one after the other (rejected moves
+// are added and taken back in their order, so the positions agree to the last
+// bit; draws and attempts count up to the accepted one).  A round works from a
+// list of the moving replicas, so its cost is that of the replicas in it: one
+// 1865-bead replica of 24 took 112 us for B xi (64 blocks) and 65 us for the
+// overlap test per attempt before, with up to 70 attempts in a step.
+
+// The list entry that unit u belongs to (product units, or overlap units).
+__device__ __forceinline__ RoundEntry find_entry(const RoundEntry* list, int count, int u, bool trmv) {
+  int lo = 0, hi = count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    const int first = trmv ? list[mid].trmv0 : list[mid].ovl0;
+    if (first <= u) lo = mid;
+    else hi = mid - 1;
+  }
+  return list[lo];
+}
+__device__ __forceinline__ int packed_count(unsigned long long v) { return (int)(v >> 48); }
+__device__ __forceinline__ int packed_trmv(unsigned long long v) { return (int)((v >> 26) & 0x3FFFFFu); }
+__device__ __forceinline__ int packed_ovl(unsigned long long v) { return (int)(v & 0x3FFFFFFu); }
+
+// Appends replica q to the list being built.
+__device__ __forceinline__ void append_entry(const BatchDev& r, int q, int attempts, RoundEntry* list,
+                                             unsigned long long* packed) {
+  const unsigned long long tu = (r.n + TRMV_ROWS - 1) / TRMV_ROWS;
+  const unsigned long long ou = r.check ? (unsigned long long)((r.N + OVL_BEADS - 1) / OVL_BEADS) * attempts : 0;
+  const unsigned long long at = atomicAdd(packed, (1ULL << 48) | (tu << 26) | ou);
+  list[packed_count(at)] = RoundEntry{q, attempts, packed_trmv(at), packed_ovl(at)};
+}
+
+// Two rows of B times NA noise vectors (stride ld), in the term order of
+// row_dot (propagate.cuh) for each product.
+template <typename T, int NA>
+__device__ __forceinline__ void row_pair_dots(const T* __restrict__ b0, const T* __restrict__ b1, int j0, int j1,
+                                              const double* __restrict__ xi, int ld, double (&s0)[NA],
+                                              double (&s1)[NA]) {
+  using C = Chunk<T>;
+  constexpr int W = C::W, U = NA == 1 ? 4 : 2;
+  const int lane = threadIdx.x & 31, nchunks = (j1 + W - 1) / W;
+  const typename C::V* v0 = reinterpret_cast<const typename C::V*>(b0);
+  const typename C::V* v1 = reinterpret_cast<const typename C::V*>(b1);
+#pragma unroll
+  for (int a = 0; a < NA; ++a) s0[a] = s1[a] = 0.0;
+  for (int c0 = lane; c0 < nchunks; c0 += 32 * U) {
+    typename C::V p0[U], p1[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + 32 * u < nchunks) {
+        p0[u] = __ldg(v0 + c0 + 32 * u);
+        p1[u] = __ldg(v1 + c0 + 32 * u);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = c0 + 32 * u;
+      if (c >= nchunks) continue;
+      double e0[W], e1[W];
+      C::get(p0[u], e0);
+      C::get(p1[u], e1);
+      // a row's terms beyond its diagonal are left out
+      const int k0 = j0 - c * W, k1 = j1 - c * W;
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        double x[W];
+#pragma unroll
+        for (int q = 0; q < W; q += 2) {
+          const double2 y = *reinterpret_cast<const double2*>(xi + (size_t)a * ld + c * W + q);
+          x[q] = y.x;
+          x[q + 1] = y.y;
+        }
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+          if (q < k0) s0[a] += e0[q] * x[q];
+          if (q < k1) s1[a] += e1[q] * x[q];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < NA; ++a)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s0[a] += __shfl_xor_sync(0xffffffffu, s0[a], o);
+      s1[a] += __shfl_xor_sync(0xffffffffu, s1[a], o);
+    }
+}
+
+// One row's candidates: U[a][row] = the position after attempt a (the attempts
+// before it added and taken back), U[attempts][row] = after all of them were
+// taken back (box.py:366-375; every product and sum rounded on its own).
+template <int NA>
+__device__ __forceinline__ void write_candidates(const BatchDev& r, int row, const double (&s)[NA], int attempts,
+                                                 double s1) {
+  double p = r.pos[row];
+#pragma unroll
+  for (int a = 0; a < NA; ++a)
+    if (a < attempts) {
+      const double m = __dmul_rn(s[a], s1), c = __dadd_rn(p, m);
+      r.U[(size_t)a * r.ld + row] = c;
+      p = __dadd_rn(c, -m);
+    }
+  r.U[(size_t)attempts * r.ld + row] = p;
+}
+
+// U = B xi (box.py:371; B lower triangular) and the candidate positions of the
+// listed replicas' attempts.  Bound by reading B (once for all attempts of a
+// round): two rows per warp share the noise vectors' loads.  rounds: the
+// step's round counter (its parity names the list), null for list 0.
 template <typename T>
-__global__ void batch_trmv_kernel(const BatchDev* __restrict__ reps, const unsigned char* __restrict__ mask) {
-  if (!mask[blockIdx.y]) return;
-  const BatchDev& r = reps[blockIdx.y];
-  const T* B = static_cast<const T*>(r.B);
-  const double* xi = r.xi;
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < r.n; row += gridDim.x * warps) {
-    const double s = row_dot(B + (size_t)row * r.ld, row + 1, [&](int j, double b) { return b * xi[j]; });
-    if (lane == 0) r.U[row] = s;
+__global__ void __launch_bounds__(256) batch_trmv_kernel(const BatchDev* __restrict__ reps,
+                                                         const RoundEntry* __restrict__ lists, int cap,
+                                                         const RoundState* __restrict__ state,
+                                                         const int* __restrict__ rounds, double s1) {
+  const int par = rounds ? *rounds & 1 : 0;
+  const unsigned long long pk = state->packed[par];
+  const RoundEntry* list = lists + (size_t)par * cap;
+  const int count = packed_count(pk), units = packed_trmv(pk), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    const RoundEntry e = find_entry(list, count, u, true);
+    const BatchDev r = reps[e.q];
+    const int row = (u - e.trmv0) * TRMV_ROWS + 2 * warp;
+    if (row >= r.n) continue;
+    const bool two = row + 1 < r.n;
+    const T* b0 = static_cast<const T*>(r.B) + (size_t)row * r.ld;
+    const T* b1 = two ? b0 + r.ld : b0;
+    const int j0 = row + 1, j1 = two ? row + 2 : row + 1;
+    if (e.attempts == 1) {
+      double x0[1], x1[1];
+      row_pair_dots<T, 1>(b0, b1, j0, j1, r.xi, r.ld, x0, x1);
+      if (lane == 0) write_candidates<1>(r, row, x0, 1, s1);
+      if (lane == 1 && two) write_candidates<1>(r, row + 1, x1, 1, s1);
+    } else {
+      double x0[SPEC], x1[SPEC];
+      row_pair_dots<T, SPEC>(b0, b1, j0, j1, r.xi, r.ld, x0, x1);
+      if (lane == 0) write_candidates<SPEC>(r, row, x0, e.attempts, s1);
+      if (lane == 1 && two) write_candidates<SPEC>(r, row + 1, x1, e.attempts, s1);
+    }
   }
 }
 
-// Stochastic step (box.py:366-375): pos += (U sqrt(2 dt)) * mult, for the
-// masked replicas; with `undo`, only those whose overlap flag is set.
-__global__ void batch_move_kernel(const BatchDev* __restrict__ reps, const unsigned char* __restrict__ mask,
-                                  const int* __restrict__ ovl, double s1, double mult, int undo) {
-  if (!mask[blockIdx.y]) return;
-  if (undo && !ovl[blockIdx.y]) return;
-  const BatchDev& r = reps[blockIdx.y];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r.n; i += gridDim.x * blockDim.x)
-    r.pos[i] += (r.U[i] * s1) * mult;
-}
-
-// Overlap test of the masked replicas (bead.c:169-218), no bonded pairs.
-__global__ void batch_overlap_kernel(const BatchDev* __restrict__ reps, const unsigned char* __restrict__ mask,
-                                     int* __restrict__ ovl) {
-  if (!mask[blockIdx.y]) return;
-  const BatchDev& r = reps[blockIdx.y];
-  if (!r.check) return;
-  const long long npairs = (long long)r.N * (r.N - 1) / 2;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npairs;
-       p += (long long)gridDim.x * blockDim.x) {
-    if (ovl[blockIdx.y]) return;
-    int i, j;
-    pair_from_linear(p, i, j);
-    if (pair_overlaps(r.pos, r.radii, i, j, r.L, r.thr)) {
-      atomicOr(ovl + blockIdx.y, 1);
-      return;
-    }
+// Overlap test of every candidate (bead.c:169-218), no bonded pairs: one warp
+// per bead i and attempt over the beads j < i.
+__global__ void __launch_bounds__(256) batch_overlap_kernel(const BatchDev* __restrict__ reps,
+                                                            const RoundEntry* __restrict__ lists, int cap,
+                                                            const RoundState* __restrict__ state,
+                                                            const int* __restrict__ rounds, int* ovl) {
+  const int par = rounds ? *rounds & 1 : 0;
+  const unsigned long long pk = state->packed[par];
+  const RoundEntry* list = lists + (size_t)par * cap;
+  const int count = packed_count(pk), units = packed_ovl(pk), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    const RoundEntry e = find_entry(list, count, u, false);
+    const BatchDev r = reps[e.q];
+    const int blocks = (r.N + OVL_BEADS - 1) / OVL_BEADS, k = u - e.ovl0, a = k / blocks;
+    const int i = (k % blocks) * OVL_BEADS + warp;
+    int* flag = ovl + e.q * SPEC + a;
+    // lane 0's view of the flag for the whole warp
+    if (i >= r.N || __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(flag), 0)) continue;
+    const double* pos = r.U + (size_t)a * r.ld;
+    bool hit = false;
+    for (int j = lane; j < i && !hit; j += 32) hit = pair_overlaps(pos, r.radii, i, j, r.L, r.thr);
+    if (__any_sync(0xffffffffu, hit) && lane == 0) atomicOr(flag, 1);
   }
 }
 
@@ -277,6 +428,18 @@ __device__ __forceinline__ double u53(uint32_t hi, uint32_t lo) {
   return ((double)v + 0.5) * (1.0 / 9007199254740992.0);  // (0, 1)
 }
 
+// Draws 2 pair and 2 pair + 1 of a stream.
+__device__ __forceinline__ void philox_pair(unsigned long long seed, unsigned long long pair, double& x, double& y) {
+  uint32_t c[4] = {(uint32_t)pair, (uint32_t)(pair >> 32), 0u, 0u};
+  philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+  const double u1 = u53(c[0], c[1]), u2 = u53(c[2], c[3]);
+  const double rad = sqrt(-2.0 * log(u1));
+  double sn, cs;
+  sincospi(2.0 * u2, &sn, &cs);
+  x = rad * cs;
+  y = rad * sn;
+}
+
 __global__ void batch_noise_kernel(const BatchDev* __restrict__ reps, const unsigned char* __restrict__ mask,
                                    const unsigned long long* __restrict__ streams) {
   if (!mask[blockIdx.y]) return;
@@ -284,64 +447,130 @@ __global__ void batch_noise_kernel(const BatchDev* __restrict__ reps, const unsi
   const unsigned long long seed = streams[2 * blockIdx.y], base = streams[2 * blockIdx.y + 1] / 2;  // even
   const int pairs = (r.n + 1) / 2;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < pairs; q += gridDim.x * blockDim.x) {
-    const unsigned long long ctr = base + (unsigned long long)q;
-    uint32_t c[4] = {(uint32_t)ctr, (uint32_t)(ctr >> 32), 0u, 0u};
-    philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-    const double u1 = u53(c[0], c[1]), u2 = u53(c[2], c[3]);
-    const double rad = sqrt(-2.0 * log(u1));
-    double sn, cs;
-    sincospi(2.0 * u2, &sn, &cs);
-    r.xi[2 * q] = rad * cs;
-    if (2 * q + 1 < r.n) r.xi[2 * q + 1] = rad * sn;
+    double x, y;
+    philox_pair(seed, base + (unsigned long long)q, x, y);
+    r.xi[2 * q] = x;
+    if (2 * q + 1 < r.n) r.xi[2 * q + 1] = y;
   }
 }
 
-// Start of the attempt rounds of a device step: every replica moves; the
-// attempt counts and the step words are cleared.
-__global__ void batch_round_init_kernel(int R, unsigned char* __restrict__ mask, int* __restrict__ att,
-                                        int* __restrict__ words) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < R; q += gridDim.x * blockDim.x) {
+// The noise of `attempts` attempts from stream position `base` (even): attempt a
+// takes the n draws from base + a (n + (n & 1)) on.
+__device__ __forceinline__ void stream_noise(const BatchDev& r, unsigned long long seed, unsigned long long base,
+                                             int attempts) {
+  const int pairs = (r.n + 1) / 2;
+  for (int t = threadIdx.x; t < attempts * pairs; t += blockDim.x) {
+    const int a = t / pairs, q = t - a * pairs;
+    double x, y;
+    philox_pair(seed, base / 2 + (unsigned long long)t, x, y);
+    double* xi = r.xi + (size_t)a * r.ld;
+    xi[2 * q] = x;
+    if (2 * q + 1 < r.n) xi[2 * q + 1] = y;
+  }
+}
+
+// Start of the attempt rounds of a device step (one block per replica): every
+// replica moves, with one attempt; the attempt counts and the step words are
+// cleared, the first noise drawn.
+__global__ void batch_round_init_kernel(const BatchDev* __restrict__ reps, unsigned char* __restrict__ mask,
+                                        int* __restrict__ att, int* __restrict__ words, int* __restrict__ ovl,
+                                        int* __restrict__ spec, const unsigned long long* __restrict__ streams,
+                                        RoundEntry* lists, RoundState* state) {
+  const int q = blockIdx.x;
+  const BatchDev r = reps[q];
+  if (threadIdx.x < SPEC) ovl[q * SPEC + threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
     mask[q] = 1;
     att[q] = 0;
+    spec[q] = 1;
+    append_entry(r, q, 1, lists, &state->packed[0]);
   }
-  if (blockIdx.x == 0 && threadIdx.x < 4) words[threadIdx.x] = 0;
+  if (q == 0 && threadIdx.x < 4) words[threadIdx.x] = 0;
+  stream_noise(r, streams[2 * q], streams[2 * q + 1], 1);
 }
 
-// End of one round of attempts (one block): each moving replica has taken one
-// more attempt and consumed 3N draws (rounded up to even) of its stream; it
-// stops when its move was accepted (already undone otherwise) or when it has
-// used max_move_attempts (error bit ATTEMPTS, as box.py:248 asserts).
+// End of one round of attempts (one block per replica): the first accepted
+// candidate (or, when all were rejected, the positions after all were taken
+// back) becomes the position; the attempts taken and the draws consumed (3N
+// per attempt, rounded up to even) are counted.  A replica stops when a move
+// was accepted or it has used max_move_attempts (error bit ATTEMPTS, as
+// box.py:248 asserts); otherwise it joins the next round's list and draws the
+// noise of its next attempts.  The last block to finish closes the round:
 // words[0] = whether any replica still moves; inside the step's graph the
 // WHILE node's condition is set to it, and a round cap bounds every launch.
 constexpr int BATCH_ROUND_CAP = 4096;
-__global__ void batch_round_update_kernel(const BatchDev* __restrict__ reps, int R, unsigned char* __restrict__ mask,
-                                          const int* __restrict__ ovl, int* __restrict__ att,
-                                          const int* __restrict__ maxatt, unsigned long long* __restrict__ streams,
-                                          int* __restrict__ words, cudaGraphConditionalHandle handle,
-                                          int use_handle) {
-  int moving = 0;
-  for (int q = threadIdx.x; q < R; q += blockDim.x) {
-    if (!mask[q]) continue;
-    const int n = reps[q].n;
-    const int a = att[q] + 1;
-    att[q] = a;
-    streams[2 * q + 1] += (unsigned long long)(n + (n & 1));
-    if (!ovl[q]) {
-      mask[q] = 0;
-    } else if (a >= maxatt[q]) {
-      mask[q] = 0;
-      atomicOr(words + 1, (int)PBG_DEV_ERR_ATTEMPTS);
-    } else {
-      moving = 1;
+__global__ void __launch_bounds__(512) batch_round_end_kernel(
+    const BatchDev* __restrict__ reps, unsigned char* __restrict__ mask, int* __restrict__ ovl, int* __restrict__ spec,
+    int* __restrict__ att, const int* __restrict__ maxatt, unsigned long long* __restrict__ streams,
+    int* __restrict__ words, RoundEntry* lists, int cap, RoundState* state, cudaGraphConditionalHandle handle,
+    int use_handle) {
+  __shared__ int s_take, s_next;
+  const int q = blockIdx.x, par = words[2] & 1;
+  const BatchDev r = reps[q];
+  const bool moving = mask[q] != 0;
+  __syncthreads();  // thread 0 changes mask[q] below
+  if (moving) {
+    if (threadIdx.x == 0) {
+      const int n = spec[q];
+      int k = 0;
+      while (k < n && ovl[q * SPEC + k]) ++k;
+      for (int a = 0; a < n; ++a) ovl[q * SPEC + a] = 0;
+      s_take = k;  // n: none accepted, U[n] holds the positions after the undo
+      const int used = k < n ? k + 1 : n, total = att[q] + used;
+      att[q] = total;
+      streams[2 * q + 1] += (unsigned long long)used * (unsigned long long)(r.n + (r.n & 1));
+      s_next = 0;
+      if (k < n) {
+        mask[q] = 0;
+      } else if (total >= maxatt[q]) {
+        mask[q] = 0;
+        atomicOr(words + 1, (int)PBG_DEV_ERR_ATTEMPTS);
+      } else {
+        s_next = spec[q] = min(SPEC, maxatt[q] - total);
+        append_entry(r, q, s_next, lists + (size_t)(par ^ 1) * cap, &state->packed[par ^ 1]);
+      }
+    }
+    __syncthreads();
+    const double* src = r.U + (size_t)s_take * r.ld;
+    for (int i = threadIdx.x; i < r.n; i += blockDim.x) r.pos[i] = src[i];
+    if (s_next) stream_noise(r, streams[2 * q], streams[2 * q + 1], s_next);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&state->done, 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      const int any = packed_count(atomicAdd(&state->packed[par ^ 1], 0ULL)) > 0;
+      const int rounds = words[2] + 1;
+      words[2] = rounds;
+      words[0] = any;
+      state->packed[par] = 0;
+      state->done = 0;
+      if (use_handle) cudaGraphSetConditional(handle, (any && rounds % BATCH_ROUND_CAP != 0) ? 1u : 0u);
     }
   }
-  const int any = __syncthreads_or(moving);
-  if (threadIdx.x == 0) {
-    const int rounds = words[2] + 1;
-    words[2] = rounds;
-    words[0] = any;
-    if (use_handle) cudaGraphSetConditional(handle, (any && rounds % BATCH_ROUND_CAP != 0) ? 1u : 0u);
+}
+
+// A host-driven attempt: the masked replicas' list (one attempt each), and its
+// outcome -- the candidate or, on an overlap, the position after the undo.
+__global__ void batch_attempt_list_kernel(const BatchDev* __restrict__ reps, int R,
+                                          const unsigned char* __restrict__ mask, int* __restrict__ ovl,
+                                          RoundEntry* lists, RoundState* state) {
+  for (int q = threadIdx.x; q < R; q += blockDim.x) {
+    ovl[q * SPEC] = 0;
+    if (mask[q]) append_entry(reps[q], q, 1, lists, &state->packed[0]);
   }
+}
+__global__ void batch_attempt_end_kernel(const BatchDev* __restrict__ reps, const unsigned char* __restrict__ mask,
+                                         int* __restrict__ ovl, int* __restrict__ rejected, RoundState* state) {
+  const int q = blockIdx.y;
+  if (q == 0 && blockIdx.x == 0 && threadIdx.x == 0) state->packed[0] = 0;
+  if (!mask[q]) return;
+  const BatchDev& r = reps[q];
+  const int hit = ovl[q * SPEC];
+  if (blockIdx.x == 0 && threadIdx.x == 0) rejected[q] = hit;
+  const double* src = r.U + (hit ? r.ld : 0);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r.n; i += gridDim.x * blockDim.x) r.pos[i] = src[i];
 }
 
 inline size_t elem_size(int precision) { return precision == PBG_PREC_FP64 ? 8 : 4; }
@@ -478,18 +707,26 @@ int rebuild(pbg_batch* b, cudaStream_t st) {
     // arrays: the stream-ordered frees wait for them, the host buffers are
     // released once the stream has drained
     PBG_CUDA_TRY(cudaStreamSynchronize(st));
-    for (void* p : {(void*)b->d_ovl, (void*)b->d_mask, (void*)b->d_stream, (void*)b->d_maxatt})
+    for (void* p : {(void*)b->d_ovl, (void*)b->d_mask, (void*)b->d_stream, (void*)b->d_maxatt, (void*)b->d_rejected,
+                    (void*)b->d_spec, (void*)b->d_lists, (void*)b->d_state})
       if (p) PBG_CUDA_TRY(cudaFreeAsync(p, st));
     b->d_ovl = nullptr;
     b->d_mask = nullptr;
     b->d_stream = nullptr;
     b->d_maxatt = nullptr;
+    b->d_rejected = b->d_spec = nullptr;
+    b->d_lists = nullptr;
+    b->d_state = nullptr;
     if (b->h_ovl) cudaFreeHost(b->h_ovl);
     if (b->h_info) cudaFreeHost(b->h_info);
     if (b->h_step) cudaFreeHost(b->h_step);
     b->h_ovl = b->h_info = b->h_step = nullptr;
     b->cap = std::max<size_t>(2 * R, 16);
-    PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_ovl, b->cap * sizeof(int), st));
+    PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_ovl, b->cap * SPEC * sizeof(int), st));
+    PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_rejected, b->cap * sizeof(int), st));
+    PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_spec, b->cap * sizeof(int), st));
+    PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_lists, 2 * b->cap * sizeof(RoundEntry), st));
+    PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_state, sizeof(RoundState), st));
     PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_mask, b->cap, st));
     PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_stream, 2 * b->cap * sizeof(unsigned long long), st));
     PBG_CUDA_TRY(cudaMallocAsync((void**)&b->d_maxatt, b->cap * sizeof(int), st));
@@ -622,6 +859,8 @@ int rebuild(pbg_batch* b, cudaStream_t st) {
       (rc = ensure(b->d_segs, b->cap_segs, std::max<size_t>(segs.size(), 1) * sizeof(GatherSeg))) ||
       (rc = ensure(b->d_eparts, b->cap_eparts, R * sizeof(int4))))
     return rc;
+  PBG_CUDA_TRY(cudaMemsetAsync(b->d_state, 0, sizeof(RoundState), st));
+  PBG_CUDA_TRY(cudaMemsetAsync(b->d_ovl, 0, b->cap * SPEC * sizeof(int), st));
   // pageable sources: each copy is staged before the call returns
   PBG_CUDA_TRY(cudaMemcpyAsync(b->d_reps, reps.data(), R * sizeof(BatchDev), cudaMemcpyHostToDevice, st));
   PBG_CUDA_TRY(cudaMemcpyAsync(b->d_rpy, rpy.data(), rpy.size(), cudaMemcpyHostToDevice, st));
@@ -718,6 +957,10 @@ PBG_API int pbg_batch_destroy(pbg_batch* b) {
   free_dev(b->d_mask);
   free_dev(b->d_stream);
   free_dev(b->d_maxatt);
+  free_dev(b->d_rejected);
+  free_dev(b->d_spec);
+  free_dev(b->d_lists);
+  free_dev(b->d_state);
   if (b->h_ovl) cudaFreeHost(b->h_ovl);
   if (b->h_info) cudaFreeHost(b->h_info);
   if (b->h_step) cudaFreeHost(b->h_step);
@@ -754,7 +997,7 @@ PBG_API long long pbg_batch_footprint(int precision, int hydrodynamics, int ewal
   (void)ewald_imag;
   const long long n = 3LL * n_beads, ld = (n + PBG_TILE - 1) / PBG_TILE * PBG_TILE, nt = ld / PBG_TILE;
   const long long es = elem_size(precision);
-  return 2 * ld * ld * es + nt * PBG_TILE * PBG_TILE * es + (4 * ld + 4 * n_beads) * 8 + 2 * nt * nt * 4;
+  return 2 * ld * ld * es + nt * PBG_TILE * PBG_TILE * es + ((2 * SPEC + 2) * ld + 4 * n_beads) * 8 + 2 * nt * nt * 4;
 }
 
 PBG_API int pbg_batch_add(pbg_batch* b, const pbg_params* p, const double* pos, const double* radii, int* slot) {
@@ -777,8 +1020,8 @@ PBG_API int pbg_batch_add(pbg_batch* b, const pbg_params* p, const double* pos, 
   const size_t es = elem_size(b->precision), ld = r->ld;
   batch_pool_keep();
   bool ok = pool_alloc(&r->pos, r->n * sizeof(double)) && pool_alloc(&r->radii, r->N * sizeof(double)) &&
-            pool_alloc(&r->force, ld * sizeof(double)) && pool_alloc(&r->U, ld * sizeof(double)) &&
-            pool_alloc(&r->xi, ld * sizeof(double)) && pool_alloc(&r->D, ld * ld * es) &&
+            pool_alloc(&r->force, ld * sizeof(double)) && pool_alloc(&r->U, (SPEC + 1) * ld * sizeof(double)) &&
+            pool_alloc(&r->xi, SPEC * ld * sizeof(double)) && pool_alloc(&r->D, ld * ld * es) &&
             pool_alloc(&r->B, ld * ld * es) && pool_alloc(&r->invdiag, (size_t)r->nt * PBG_TILE * PBG_TILE * es);
   std::vector<int4> tasks;
   cholesky_replica_tasks(r->nt, b->precision, tasks, r->seg_start);
@@ -794,8 +1037,8 @@ PBG_API int pbg_batch_add(pbg_batch* b, const pbg_params* p, const double* pos, 
     return PBG_ERR_NOMEM;
   }
   cudaMemsetAsync(r->force, 0, ld * sizeof(double), 0);
-  cudaMemsetAsync(r->U, 0, ld * sizeof(double), 0);
-  cudaMemsetAsync(r->xi, 0, ld * sizeof(double), 0);
+  cudaMemsetAsync(r->U, 0, (SPEC + 1) * ld * sizeof(double), 0);
+  cudaMemsetAsync(r->xi, 0, SPEC * ld * sizeof(double), 0);
   // ordered on the legacy stream after the allocations; a pageable source is
   // staged before the call returns
   PBG_CUDA_TRY(cudaMemcpyAsync(r->pos, pos, r->n * sizeof(double), cudaMemcpyDefault, 0));
@@ -1036,31 +1279,38 @@ PBG_API int pbg_batch_step_begin(pbg_batch* b, double dt, int build_D, int chole
   return PBG_OK;
 }
 
-// One round of attempts of the replicas still moving (mask): their noise,
-// U = B xi, the move, the overlap test, the undo of the rejected moves and
-// the round's bookkeeping (batch_round_update_kernel).  Six kernels.
-static int enqueue_round(pbg_batch* b, cudaStream_t st, cudaGraphConditionalHandle handle, int use_handle) {
-  const int R = (int)b->active.size();
-  const bool f64 = b->precision == PBG_PREC_FP64;
+// Blocks of the list-driven kernels: four (product) and eight per SM, fewer
+// where the batch has fewer units.
+static int round_blocks(const pbg_batch* b, int per_sm, int unit_rows, int rows) {
+  const long long units = (long long)b->active.size() * ((rows + unit_rows - 1) / unit_rows);
+  return (int)std::max<long long>(1, std::min<long long>(units, 148LL * per_sm));
+}
+
+static int enqueue_moves(pbg_batch* b, const int* rounds, cudaStream_t st) {
   const double s1 = std::sqrt(2 * b->dt);
-  batch_noise_kernel<<<rows_grid(b, 512), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_stream);
+  const int cap = (int)b->cap, blocks = round_blocks(b, 4, TRMV_ROWS, b->max_n);
+  if (b->precision == PBG_PREC_FP64)
+    batch_trmv_kernel<double><<<blocks, 256, 0, st>>>(b->d_reps, b->d_lists, cap, b->d_state, rounds, s1);
+  else
+    batch_trmv_kernel<float><<<blocks, 256, 0, st>>>(b->d_reps, b->d_lists, cap, b->d_state, rounds, s1);
   PBG_CHECK_LAUNCH();
-  if (f64) batch_trmv_kernel<double><<<rows_grid(b, 8), 256, 0, st>>>(b->d_reps, b->d_mask);
-  else batch_trmv_kernel<float><<<rows_grid(b, 8), 256, 0, st>>>(b->d_reps, b->d_mask);
-  PBG_CHECK_LAUNCH();
-  batch_move_kernel<<<rows_grid(b, 256), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl, s1, 1.0, 0);
-  PBG_CHECK_LAUNCH();
-  PBG_CUDA_TRY(cudaMemsetAsync(b->d_ovl, 0, R * sizeof(int), st));
-  batch_overlap_kernel<<<dim3(64, R), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl);
-  PBG_CHECK_LAUNCH();
-  batch_move_kernel<<<rows_grid(b, 256), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl, s1, -1.0, 1);
-  PBG_CHECK_LAUNCH();
-  batch_round_update_kernel<<<1, 1024, 0, st>>>(b->d_reps, R, b->d_mask, b->d_ovl, b->d_att, b->d_maxatt,
-                                                 b->d_stream, b->d_words, handle, use_handle);
+  batch_overlap_kernel<<<round_blocks(b, 8, 1, b->max_n), 256, 0, st>>>(b->d_reps, b->d_lists, cap, b->d_state, rounds,
+                                                                        b->d_ovl);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
-constexpr int ROUND_KERNELS = 6;
+
+// One round of attempts of the replicas still moving: the product and the
+// candidates, the overlap tests, the outcome.  Three kernels.
+static int enqueue_round(pbg_batch* b, cudaStream_t st, cudaGraphConditionalHandle handle, int use_handle) {
+  if (int rc = enqueue_moves(b, b->d_words + 2, st)) return rc;
+  batch_round_end_kernel<<<(int)b->active.size(), 512, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl, b->d_spec, b->d_att,
+                                                                b->d_maxatt, b->d_stream, b->d_words, b->d_lists,
+                                                                (int)b->cap, b->d_state, handle, use_handle);
+  PBG_CHECK_LAUNCH();
+  return PBG_OK;
+}
+constexpr int ROUND_KERNELS = 3;
 
 // The wrap into the box and the step's report (infos, attempts, words) into
 // pinned host memory.
@@ -1074,7 +1324,9 @@ static int enqueue_step_tail(pbg_batch* b, cudaStream_t st) {
 
 static int enqueue_round_init(pbg_batch* b, cudaStream_t st) {
   const int R = (int)b->active.size();
-  batch_round_init_kernel<<<(R + 255) / 256, 256, 0, st>>>(R, b->d_mask, b->d_att, b->d_words);
+  PBG_CUDA_TRY(cudaMemsetAsync(b->d_state, 0, sizeof(RoundState), st));
+  batch_round_init_kernel<<<R, 256, 0, st>>>(b->d_reps, b->d_mask, b->d_att, b->d_words, b->d_ovl, b->d_spec,
+                                             b->d_stream, b->d_lists, b->d_state);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
@@ -1254,19 +1506,13 @@ PBG_API int pbg_batch_step_attempt(pbg_batch* b, const unsigned char* mask, unsi
   int count = 0, rc;
   if ((rc = upload_mask(b, mask, st, &count))) return rc;
   if (!count) return PBG_OK;
-  const bool f64 = b->precision == PBG_PREC_FP64;
-  const double s1 = std::sqrt(2 * b->dt);
-  if (f64) batch_trmv_kernel<double><<<rows_grid(b, 8), 256, 0, st>>>(b->d_reps, b->d_mask);
-  else batch_trmv_kernel<float><<<rows_grid(b, 8), 256, 0, st>>>(b->d_reps, b->d_mask);
+  PBG_CUDA_TRY(cudaMemsetAsync(b->d_state, 0, sizeof(RoundState), st));
+  batch_attempt_list_kernel<<<1, 256, 0, st>>>(b->d_reps, R, b->d_mask, b->d_ovl, b->d_lists, b->d_state);
   PBG_CHECK_LAUNCH();
-  batch_move_kernel<<<rows_grid(b, 256), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl, s1, 1.0, 0);
+  if ((rc = enqueue_moves(b, nullptr, st))) return rc;
+  batch_attempt_end_kernel<<<rows_grid(b, 256), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl, b->d_rejected, b->d_state);
   PBG_CHECK_LAUNCH();
-  PBG_CUDA_TRY(cudaMemsetAsync(b->d_ovl, 0, R * sizeof(int), st));
-  batch_overlap_kernel<<<dim3(64, R), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl);
-  PBG_CHECK_LAUNCH();
-  batch_move_kernel<<<rows_grid(b, 256), 256, 0, st>>>(b->d_reps, b->d_mask, b->d_ovl, s1, -1.0, 1);
-  PBG_CHECK_LAUNCH();
-  PBG_CUDA_TRY(cudaMemcpyAsync(b->h_ovl, b->d_ovl, R * sizeof(int), cudaMemcpyDeviceToHost, st));
+  PBG_CUDA_TRY(cudaMemcpyAsync(b->h_ovl, b->d_rejected, R * sizeof(int), cudaMemcpyDeviceToHost, st));
   PBG_CUDA_TRY(cudaStreamSynchronize(st));
   if (accepted)
     for (int q = 0; q < R; ++q)
