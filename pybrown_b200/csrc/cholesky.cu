@@ -63,18 +63,18 @@ static size_t spd_x_offset(int ld) { return (cholesky_work_bytes(ld, PBG_PREC_FP
 
 size_t spd_inverse_work_bytes(int ld) { return spd_x_offset(ld) + (size_t)ld * ld * sizeof(double); }
 
-// inv(A) = X^T X with X = inv(L): one data-flow launch factors A and forms
-// X's off-diagonal tiles, then X's diagonal tiles and the symmetric product.
-int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStream_t st) {
+// scale inv(A) = scale X^T X with X = inv(L): one data-flow launch factors A and
+// forms X's off-diagonal tiles (its diagonal ones are the inverted diagonal
+// tiles), then the symmetric product.
+int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStream_t st, double scale) {
   const int nt = ld / NB;
   unsigned char* w = static_cast<unsigned char*>(work);
   double* inv = reinterpret_cast<double*>(w);
   double* X = reinterpret_cast<double*>(w + spd_x_offset(ld));
-  int rc = launch_cholesky_df(A, n, ld, PBG_PREC_FP64, info, inv, true,
-                              w + (size_t)nt * NB * NB * sizeof(double), st, X);
+  int rc = launch_cholesky_df(A, n, ld, PBG_PREC_FP64, info, inv, true, w + (size_t)nt * NB * NB * sizeof(double), st,
+                              X);
   if (rc != PBG_OK) return rc;
-  if ((rc = launch_trtri_diag(inv, X, ld, PBG_PREC_FP64, st))) return rc;
-  return launch_lauum_tc(X, ld, 1.0, false, A, PBG_PREC_FP64, st);
+  return launch_lauum(X, inv, ld, scale, A, st);
 }
 
 }  // namespace pbg

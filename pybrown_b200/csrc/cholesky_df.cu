@@ -300,6 +300,34 @@ template <> struct TileMMA<double> {
         }
     }
   }
+  // acc -= A B (AT false) or A^T B (AT true) with B, and A in the second case,
+  // staged as they lie in memory (rows = k): a fragment's four k rows are 8
+  // banks apart and its eight columns 2, so these loads are free of conflicts
+  // where a transposing copy into shared memory meets 8-way ones.
+  template <bool AT>
+  static __device__ __forceinline__ void sub_rows(const double* sA, const double* sB, double acc[16]) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int m0 = 16 * (w >> 1), n0 = 32 * (w & 1), g = lane >> 2, t = lane & 3;
+#pragma unroll 4
+    for (int k0 = 0; k0 < NB; k0 += 4) {
+      double a[2], b[4];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+        a[mt] = AT ? -sA[(k0 + t) * LDA + m0 + 8 * mt + g] : -sA[(m0 + 8 * mt + g) * LDA + k0 + t];
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) b[nt] = sB[(k0 + t) * LDA + n0 + 8 * nt + g];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          double& c0 = acc[(mt * 4 + nt) * 2];
+          double& c1 = acc[(mt * 4 + nt) * 2 + 1];
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                       : "+d"(c0), "+d"(c1)
+                       : "d"(a[mt]), "d"(b[nt]));
+        }
+    }
+  }
 };
 
 
@@ -1730,6 +1758,20 @@ __device__ __forceinline__ void acc_to_smem_transposed(const T acc[16], T* s) {
     for (int cs = 0; cs < 8; ++cs) s[acc_col(cs) * LDA + acc_row(rs)] = acc[TileMMA<T>::idx(rs, cs)];
 }
 
+// acc -= A X for the tile X of the inverse at g: staged as it lies (FP64) or
+// transposed for the TF32 product's fragments (FP32).  stage_x starts the
+// copy (the caller waits with cp_async_wait_all and a barrier).
+template <typename T>
+__device__ __forceinline__ void stage_x(const T* g, int ld, T* s) {
+  if constexpr (sizeof(T) == 8) stage_async(g, ld, s, LDA);
+  else stage_transposed_cg<T>(g, ld, s);
+}
+template <typename T>
+__device__ __forceinline__ void sub_x(const T* sA, const T* sX, T acc[16]) {
+  if constexpr (sizeof(T) == 8) TileMMA<T>::template sub_rows<false>(sA, sX, acc);
+  else TileMMA<T>::sub(sA, sX, acc);
+}
+
 // XG(i, j, k) for rows i .. i+rows-1 (rows <= 2).  Shared memory: three tiles.
 template <typename T>
 __device__ void inverse_update(const DFArgs& a, int i, int rows, int j, int k, T* s) {
@@ -1746,11 +1788,11 @@ __device__ void inverse_update(const DFArgs& a, int i, int rows, int j, int k, T
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc0[e] = acc1[e] = T(0);
   }
-  stage_transposed_cg<T>(xtile<T>(a, k, j), k == j ? NB : a.ld, sB);  // X_kj^T
+  stage_x<T>(xtile<T>(a, k, j), k == j ? NB : a.ld, sB);
   cp_async_wait_all();
   __syncthreads();
-  TileMMA<T>::sub(sA0, sB, acc0);
-  if (rows > 1) TileMMA<T>::sub(sA1, sB, acc1);
+  sub_x<T>(sA0, sB, acc0);
+  if (rows > 1) sub_x<T>(sA1, sB, acc1);
   store_acc(xtile_out<T>(a, i, j), a.ld, acc0);
   if (rows > 1) store_acc(xtile_out<T>(a, i + 1, j), a.ld, acc1);
 }
@@ -1770,16 +1812,17 @@ __device__ void inverse_finish(const DFArgs& a, int i, int j, T* s) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = T(0);
   }
-  stage_transposed_cg<T>(xtile<T>(a, i - 1, j), i - 1 == j ? NB : a.ld, sB);  // X_{i-1,j}^T
+  stage_x<T>(xtile<T>(a, i - 1, j), i - 1 == j ? NB : a.ld, sB);
   cp_async_wait_all();
   __syncthreads();
-  TileMMA<T>::sub(sA, sB, acc);  // V_ij complete
+  sub_x<T>(sA, sB, acc);  // V_ij complete
   __syncthreads();
-  acc_to_smem_transposed(acc, sB);  // V^T
+  if constexpr (sizeof(T) == 8) acc_to_smem(acc, sB);
+  else acc_to_smem_transposed(acc, sB);
   __syncthreads();
 #pragma unroll
   for (int e = 0; e < 16; ++e) acc[e] = T(0);
-  TileMMA<T>::sub(sX, sB, acc);  // -X_ii V
+  sub_x<T>(sX, sB, acc);  // -X_ii V
 #pragma unroll
   for (int e = 0; e < 16; ++e) acc[e] = -acc[e];
   store_acc(xtile_out<T>(a, i, j), a.ld, acc);
@@ -3029,32 +3072,6 @@ constexpr size_t tc_smem_bytes() {
   return 2 * NB * LDA * sizeof(T);
 }
 
-// Transposed staging of a 64 x 64 tile, s[c][r] = g[r][c] (rows of LDA in
-// smem), in two halves so that a thread's 16 global loads are all in flight
-// before the first shared store: load_tile_regs, then store_tile_transposed.
-template <typename T>
-__device__ __forceinline__ void load_tile_regs(const T* __restrict__ g, int ld, T (&v)[TILE_PER_THREAD]) {
-#pragma unroll
-  for (int q = 0; q < TILE_PER_THREAD; ++q) {
-    const int e = threadIdx.x + q * THREADS;
-    v[q] = g[(size_t)(e >> 6) * ld + (e & 63)];
-  }
-}
-template <typename T>
-__device__ __forceinline__ void store_tile_transposed(const T (&v)[TILE_PER_THREAD], T* s) {
-#pragma unroll
-  for (int q = 0; q < TILE_PER_THREAD; ++q) {
-    const int e = threadIdx.x + q * THREADS;
-    s[(e & 63) * LDA + (e >> 6)] = v[q];
-  }
-}
-template <typename T>
-__device__ __forceinline__ void stage_transposed(const T* __restrict__ g, int ld, T* s) {
-  T v[TILE_PER_THREAD];
-  load_tile_regs(g, ld, v);
-  store_tile_transposed(v, s);
-}
-
 // X_kk = inv(L_kk), upper triangle zero (one CTA per diagonal tile).
 template <typename T>
 __global__ void __launch_bounds__(THREADS) trtri_diag_kernel(const T* __restrict__ invdiag, T* X, int ld) {
@@ -3072,47 +3089,52 @@ __global__ void __launch_bounds__(THREADS) trtri_diag_kernel(const T* __restrict
 }
 
 // out_IJ = scale (X^T X)_IJ = scale sum_{k >= I} X_kI^T X_kJ for the lower
-// tile (I, J), written to (I, J) and (J, I); with `reversed` every element
-// (r, c) goes to (ld-1-r, ld-1-c) instead.
-template <typename T>
-__global__ void __launch_bounds__(THREADS) lauum_tc_kernel(const T* __restrict__ X, int ld, int nt, T scale,
-                                                           int reversed, T* __restrict__ out) {
+// tile (I, J), written to (I, J) and (J, I); FP64.  Off-diagonal tiles come from
+// X, the diagonal ones from invdiag.  Bound by the FP64 tensor pipe (2.1 us per
+// 64^3 product and SM): the tiles are used as they lie in memory (sub_rows),
+// two K-steps in flight by cp.async; the CTAs with the longest K range start
+// first.  Order 1536: 118 us with transposing copies through registers, 69 now.
+constexpr size_t lauum_smem_bytes() { return 4 * NB * LDA * sizeof(double); }
+__global__ void __launch_bounds__(THREADS) lauum_kernel(const double* __restrict__ X, const double* __restrict__ invdiag,
+                                                        int ld, int nt, double scale, double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem[];
-  T* sA = reinterpret_cast<T*>(smem);
-  T* sB = sA + NB * LDA;
+  double* st = reinterpret_cast<double*>(smem);  // [2][2][64][LDA]
   const int b = blockIdx.x;
   int I = (int)((sqrt(8.0 * b + 1.0) - 1.0) * 0.5);
   while ((I + 1) * (I + 2) / 2 <= b) ++I;
   while (I * (I + 1) / 2 > b) --I;
   const int J = b - I * (I + 1) / 2;
-  T acc[16];
+  auto fetch = [&](int k, double* s) {
+    auto one = [&](int c, double* d) {
+      if (k == c) stage_async(invdiag + (size_t)k * NB * NB, NB, d, LDA);
+      else stage_async(X + (size_t)k * NB * ld + (size_t)c * NB, ld, d, LDA);
+    };
+    one(I, s);
+    if (J != I) one(J, s + NB * LDA);
+    cp_async_commit();
+  };
+  double acc[16];
 #pragma unroll
-  for (int e = 0; e < 16; ++e) acc[e] = T(0);
-  // the tiles of step k+1 are loaded into registers while step k multiplies
-  T va[TILE_PER_THREAD], vb[TILE_PER_THREAD];
-  load_tile_regs(X + (size_t)I * NB * ld + (size_t)I * NB, ld, va);
-  load_tile_regs(X + (size_t)I * NB * ld + (size_t)J * NB, ld, vb);
+  for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+  fetch(I, st);
   for (int k = I; k < nt; ++k) {
-    store_tile_transposed(va, sA);
-    store_tile_transposed(vb, sB);
-    __syncthreads();
+    double* s = st + ((k - I) & 1) * 2 * NB * LDA;
     if (k + 1 < nt) {
-      load_tile_regs(X + (size_t)(k + 1) * NB * ld + (size_t)I * NB, ld, va);
-      load_tile_regs(X + (size_t)(k + 1) * NB * ld + (size_t)J * NB, ld, vb);
+      fetch(k + 1, st + ((k - I + 1) & 1) * 2 * NB * LDA);
+      cp_async_wait_group<1>();
+    } else {
+      cp_async_wait_group<0>();
     }
-    TileMMA<T>::sub(sA, sB, acc);
+    __syncthreads();
+    TileMMA<double>::sub_rows<true>(s, J != I ? s + NB * LDA : s, acc);
     __syncthreads();
   }
 #pragma unroll
   for (int rs = 0; rs < 2; ++rs)
 #pragma unroll
     for (int cs = 0; cs < 8; ++cs) {
-      const T v = -acc[TileMMA<T>::idx(rs, cs)] * scale;
-      int r = I * NB + acc_row(rs), c = J * NB + acc_col(cs);
-      if (reversed) {
-        r = ld - 1 - r;
-        c = ld - 1 - c;
-      }
+      const double v = -acc[TileMMA<double>::idx(rs, cs)] * scale;
+      const int r = I * NB + acc_row(rs), c = J * NB + acc_col(cs);
       out[(size_t)r * ld + c] = v;
       if (I != J) out[(size_t)c * ld + r] = v;  // a diagonal tile writes each element once
     }
@@ -3303,40 +3325,22 @@ __global__ void __launch_bounds__(THREADS, 1) sym_tc_kernel(const float* __restr
   if (tid < 32) tc::tmem_dealloc(tmem, 64);
 }
 
-// Dynamic shared memory above the 48 KB default (the FP64 tiles), set on the
-// current device before each use.
-template <typename T>
-int set_tc_smem() {
-  constexpr int smem = (int)tc_smem_bytes<T>();
-  PBG_CUDA_TRY(cudaFuncSetAttribute(lauum_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  return PBG_OK;
-}
-
-template <typename T>
-int lauum_tc(const T* X, int ld, T scale, bool reversed, T* out, cudaStream_t st) {
-  const int nt = ld / NB;
-  if (int rc = set_tc_smem<T>()) return rc;
-  lauum_tc_kernel<T><<<nt * (nt + 1) / 2, THREADS, tc_smem_bytes<T>(), st>>>(X, ld, nt, scale, reversed ? 1 : 0,
-                                                                             out);
-  PBG_CHECK_LAUNCH();
-  return PBG_OK;
-}
-
 }  // namespace
 
-int launch_trtri_diag(const void* invdiag, void* X, int ld, int precision, cudaStream_t st) {
+int launch_trtri_diag(const float* invdiag, float* X, int ld, cudaStream_t st) {
   if (ld % NB != 0 || ld <= 0) return PBG_ERR_ARG;
-  const int nt = ld / NB;
-  if (precision == PBG_PREC_FP64) trtri_diag_kernel<double><<<nt, THREADS, 0, st>>>((const double*)invdiag, (double*)X, ld);
-  else trtri_diag_kernel<float><<<nt, THREADS, 0, st>>>((const float*)invdiag, (float*)X, ld);
+  trtri_diag_kernel<float><<<ld / NB, THREADS, 0, st>>>(invdiag, X, ld);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
 
-int launch_lauum_tc(const void* X, int ld, double scale, bool reversed, void* out, int precision, cudaStream_t st) {
+int launch_lauum(const double* X, const double* invdiag, int ld, double scale, double* out, cudaStream_t st) {
   if (ld % NB != 0 || ld <= 0) return PBG_ERR_ARG;
-  if (precision == PBG_PREC_FP64) return lauum_tc<double>((const double*)X, ld, scale, reversed, (double*)out, st);
-  return lauum_tc<float>((const float*)X, ld, (float)scale, reversed, (float*)out, st);
+  const int nt = ld / NB;
+  PBG_CUDA_TRY(cudaFuncSetAttribute(lauum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lauum_smem_bytes()));
+  lauum_kernel<<<nt * (nt + 1) / 2, THREADS, lauum_smem_bytes(), st>>>(X, invdiag, ld, nt, scale, out);
+  PBG_CHECK_LAUNCH();
+  return PBG_OK;
 }
 
 // The data-flow scratch rounded up to 256 bytes, so X and F start aligned
@@ -3369,7 +3373,7 @@ int tc_factor_invert(int ld, int* info, void* work, cudaStream_t st) {
   // the factorisation forms X's off-diagonal tiles in the same launch
   int rc = launch_cholesky_df(w.F, ld, ld, PBG_PREC_MIXED, info, w.invdiag, true, w.scratch, st, w.X);
   if (rc != PBG_OK) return rc;
-  return launch_trtri_diag(w.invdiag, w.X, ld, PBG_PREC_MIXED, st);
+  return launch_trtri_diag(w.invdiag, w.X, ld, st);
 }
 
 int tc_lauum(const float* X, int ld, float scale, bool reversed, float* out, int* info, cudaStream_t st) {

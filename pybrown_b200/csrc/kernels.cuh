@@ -129,12 +129,13 @@ size_t df_work_bytes(int ld);
 int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* invdiag, bool want_inv, void* work,
                        cudaStream_t st, void* X = nullptr);
 size_t spd_inverse_work_bytes(int ld);
-int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStream_t st);
+// A <- scale inv(A).
+int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStream_t st, double scale = 1.0);
 
-// X's diagonal tiles from invdiag, and out = scale X^T X (optionally with
-// every index i -> ld-1-i), on the tensor cores, FP64 or FP32 (cholesky_df.cu).
-int launch_trtri_diag(const void* invdiag, void* X, int ld, int precision, cudaStream_t st);
-int launch_lauum_tc(const void* X, int ld, double scale, bool reversed, void* out, int precision, cudaStream_t st);
+// X's diagonal tiles from invdiag (FP32), and out = scale X^T X with X's
+// off-diagonal tiles in X and its diagonal ones in invdiag (cholesky_df.cu).
+int launch_trtri_diag(const float* invdiag, float* X, int ld, cudaStream_t st);
+int launch_lauum(const double* X, const double* invdiag, int ld, double scale, double* out, cudaStream_t st);
 // SPD inverse of the mixed lubricated path (FP32).  The caller puts the
 // matrix (order ld, padded) in F; tc_factor_invert factors it in place
 // (F = G, lower) and forms X = inv(G); tc_lauum writes scale X^T X on the

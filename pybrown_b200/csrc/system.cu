@@ -34,15 +34,6 @@ __global__ void copy_lower_pad_kernel(const T* __restrict__ src, T* __restrict__
   }
 }
 
-__global__ void scale_matrix_kernel(double* __restrict__ A, int n, int ld, double s) {
-  const long long total = (long long)n * ld;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(t % ld);
-    if (c < n) A[t] = s * A[t];
-  }
-}
-
 template <typename T>
 __global__ void cast_matrix_kernel(const double* __restrict__ src, T* __restrict__ dst, long long total) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -320,9 +311,9 @@ int compute_Dff(pbg_system* s, cudaStream_t st, bool fill_B) {
     if ((rc = tc_factor_invert(s->ld, s->dflags + 2, s->inv_work, st))) return rc;
     return tc_lauum(w.X, s->ld, 1.0f, false, (float*)s->Rff, s->dflags + 2, st);
   }
-  rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, PBG_PREC_FP64, s->Mff, s->ld, st, nullptr, true);
+  // the factorisation reads the lower triangle only: the build writes it to Rff as well
+  rc = launch_rpy_tensor(src, s->pos, s->radii, smith, s->tables, scale, PBG_PREC_FP64, s->Mff, s->ld, st, s->Rff, true);
   if (rc) return rc;
-  PBG_CUDA_TRY(cudaMemcpyAsync(s->Rff, s->Mff, (size_t)s->ld * s->ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
   return launch_spd_inverse(s->Rff, s->n, s->ld, s->dflags + 2, s->inv_work, st);
 }
 
@@ -359,11 +350,7 @@ int compute_Dtot(pbg_system* s, cudaStream_t st) {
                                   p.viscosity / 1e19, s->R, s->ld, st);
   if (rc) return rc;
   PBG_CUDA_TRY(cudaMemcpyAsync(s->D, s->R, bytes, cudaMemcpyDeviceToDevice, st));
-  rc = launch_spd_inverse((double*)s->D, s->n, s->ld, s->dflags + 3, s->inv_work, st);
-  if (rc) return rc;
-  scale_matrix_kernel<<<grid_for((long long)s->n * s->ld), 256, 0, st>>>((double*)s->D, s->n, s->ld, p.kBT);
-  PBG_CHECK_LAUNCH();
-  return PBG_OK;
+  return launch_spd_inverse((double*)s->D, s->n, s->ld, s->dflags + 3, s->inv_work, st, p.kBT);
 }
 
 // box.py:546-556: B = chol(D), lower.
