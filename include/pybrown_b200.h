@@ -143,9 +143,9 @@ PBG_API int pbg_dev_check_overlaps(const double *pos, const double *radii, int n
 
 /* In-place lower Cholesky factor of an SPD matrix of order n (row-major,
  * leading dimension ld >= round_up(n, 64), rows/cols n..ld-1 are used as
- * padding).  precision selects FP64, the mixed FP32 path (float*; FP32
- * diagonal tiles, 3xTF32 trailing updates on the tcgen05 tensor cores) or
- * PBG_PREC_MIXED_FP64_DIAG.  Replaces np.linalg.cholesky (box.py:554).
+ * padding).  precision selects FP64, the mixed FP32 path (float*; diagonal
+ * tiles factored in FP64 and rounded on store, 3xTF32 trailing updates on the
+ * tcgen05 tensor cores) or PBG_PREC_MIXED_FP64_DIAG.  Replaces np.linalg.cholesky (box.py:554).
  * info_dev (int, device) receives 0 or 1 + the index of the first
  * non-positive pivot. */
 PBG_API int pbg_dev_cholesky(void *A, int n, int ld, int precision, int *info_dev, void *stream);
@@ -164,9 +164,8 @@ PBG_API int pbg_dev_spd_inverse(double *A, int n, int ld, int *info_dev, void *s
 
 #define PBG_PREC_FP64 0
 #define PBG_PREC_MIXED 1
-/* pbg_dev_cholesky only: an FP32 matrix (as PBG_PREC_MIXED) whose 64 x 64
- * diagonal tiles are factored and inverted in FP64 instead of FP32 (the
- * factorisation the lubricated mixed path uses for its resistance matrices). */
+/* pbg_dev_cholesky only: as PBG_PREC_MIXED, with every positive pivot accepted
+ * (PBG_PREC_MIXED reports one below the smallest normal float as non-positive). */
 #define PBG_PREC_MIXED_FP64_DIAG 2
 
 #define PBG_SCHEME_ERMAK 0

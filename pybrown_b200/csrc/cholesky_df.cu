@@ -17,9 +17,8 @@
 //   LEAD(k)  row k+2 of panel k: S(k+2, k), U(k+2, k+1, k), U(k+2, k+2, k) as
 //            one task, because the chain waits for them;
 //   I(k)     inv(L_kk), only when the caller wants the inverted diagonal tiles.
-// The FP64 path factors the diagonal tiles in FP64; the mixed path (FP32
-// matrix) in FP32, or in FP64 rounded to FP32 on store
-// (PBG_PREC_MIXED_FP64_DIAG).
+// The diagonal tiles are factored in FP64 in every path, in the mixed path (FP32
+// matrix) rounded to FP32 on store.
 //
 // The critical path of the factorisation is F(0), S(1,0), F(1), S(2,1), ...:
 // block 0 (the chain CTA) runs exactly that sequence and keeps what one step
@@ -85,6 +84,7 @@ struct DFArgs {
   void* X;       // or null: X = inv(L) is formed too (off-diagonal tiles of the ld x ld matrix)
   int* xupd;     // nt * nt: terms applied to X's tile (i, j)
   int* xfin;     // nt * nt: X's tile (i, j) final
+  double min_pivot = 0.0;  // a pivot below it counts as non-positive
 };
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -120,7 +120,7 @@ __device__ long long g_ll_prof[1024 * 16];
 #define LLPROF(slot, v) \
   if (threadIdx.x == 0 && blockIdx.x < 1024) g_ll_prof[blockIdx.x * 16 + (slot)] += (v)
 #define LLCLK() clock64()
-// Finer timeline of the FP32 chain: 8 stamps per panel k.
+// Finer timeline of the chain: 8 stamps per panel k.
 __device__ long long g_chain_trace[8 * 1024];
 #define CTRACE(k, slot) \
   if (threadIdx.x == 0 && (k) < 1024) g_chain_trace[8 * (k) + (slot)] = gtimer()
@@ -438,7 +438,7 @@ struct WarpTile64 {
   static constexpr int NQ = 2;
 };
 
-// The FP32 counterpart on the FMA pipe (the FP32 chain inverts its diagonal
+// The FP32 counterpart on the FMA pipe (the mixed batch inverts its diagonal
 // tiles in FP32): lane (g, t) forms D[g][2t], D[g][2t + 1] as K-term dot
 // products in ascending k.
 struct WarpTile32 {
@@ -586,39 +586,40 @@ __device__ __forceinline__ void acc_to_smem(const T acc[16], T* s, int lds = LDA
 // The factorisation's critical path runs through the diagonal tiles: their
 // 64 pivots are one dependent chain.  What a column costs is latency, not
 // work (a 64 x 64 tile is 0.09 MFLOP), so everything here is arranged around
-// the chain: LDL^T pivots (one reciprocal per column; the square roots are
-// taken for all 64 columns at once afterwards), no hand-over between warps
-// inside an 8-column panel, one CTA-level barrier per panel, and the trailing
-// update one panel behind on the other warps.  Measured (order 1856, one B200
-// at 1965 MHz): FP64 F(k) 7.7 us against 11.7 with rsqrt pivots and two
-// barriers per panel (a chain step, F to F, 13.5 us against 19.2); FP32 7.0 us
-// against 9.6 with the explicit inverse that the solves below do without (a
-// step 12.2 us against 15.8).  What is left of F(k) is the panels' hand-overs
-// through shared memory (about 1350 cycles a panel, of which the pivot chain
-// 430 in FP64).
+// the chain.  The tile is factored as LDL^T (one reciprocal per column; the
+// square roots are taken off the chain) in FP64 on 8 x 8 blocks, which live in
+// registers as MMA accumulator fragments, lane (g, t) = (lane / 4, lane % 4)
+// holding the pair (row g, columns 2t and 2t + 1): with the K slots of the FP64
+// m8n8k4 product chosen as columns 2t, 2t + 1 such a fragment is at once an A
+// operand and (transposed) a B operand.  One warp takes the whole pivot chain
+// from block to block: pivot block -> its factor and the inverse U of its unit
+// triangle -> the next block row's X = S U^T (two MMAs) -> the next pivot block
+// D - X M^T (two MMAs).  Everything else is done by the other warps while the
+// next block is factored.
+// Measured (order 1024, one B200 at 1965 MHz): F(k) 5.0 us, of which 3.4 the
+// chain warp on its own (420 ns a block: 190 ns its eight reciprocal steps, the rest the
+// hand-over of D, U and X through shared memory and registers), against 7.7 us
+// (FP64) and 7.0 (FP32) with rows in lanes and one barrier of five warps per
+// block; a chain step, F to F, 10.4 us against 13.5 and 12.2.  An FP32 variant
+// would save reciprocal latency but pay for its products on the FMA pipe, so
+// FP32 matrices are factored in FP64 too and rounded once on store.
 
-// Rows of a staged tile in the chain's shared memory (LT) and of the 8-wide
-// strips (MS): 16-byte fragment loads of two FP64 rows fall on different banks.
+// Rows of a staged 64 x 64 tile in the chain's and the solves' shared memory:
+// 16-byte fragment loads of two FP64 rows fall on different banks.
 template <typename T> struct ChainLd;
-template <> struct ChainLd<double> { static constexpr int LT = NB + 8, MS = 10; };
-template <> struct ChainLd<float> { static constexpr int LT = NB + 4, MS = 12; };
+template <> struct ChainLd<double> { static constexpr int LT = NB + 8; };
+template <> struct ChainLd<float> { static constexpr int LT = NB + 4; };
 
-// 1 / d and 1 / sqrt(d) of a pivot.  FP64: the PTX approximations refined to
-// full precision -- the reciprocal by one third-order step
+// 1 / d and 1 / sqrt(d) of a pivot: the PTX approximations refined to full
+// precision -- the reciprocal by one third-order step
 // y <- y + y (e + e^2), e = 1 - d y (from ~2^-20 to ~2^-60), the square root by
-// two Newton-Raphson steps y <- y + y (1 - d y^2) / 2.  FP32: the MUFU
-// estimates (1 ulp; 2^-22).  d <= 0, NaN and subnormal d give values that are
-// reported as a non-positive pivot and not used.
+// two Newton-Raphson steps y <- y + y (1 - d y^2) / 2.  d <= 0, NaN and
+// subnormal d give values that are reported as a non-positive pivot and not used.
 __device__ __forceinline__ double pivot_rcp(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d, y, 1.0);
   return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ float pivot_rcp(float d) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-  return y;
 }
 __device__ __forceinline__ double pivot_rsqrt(double x) {
   double y;
@@ -626,20 +627,18 @@ __device__ __forceinline__ double pivot_rsqrt(double x) {
   y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
   return fma(0.5 * y, fma(-x * y, y, 1.0), y);
 }
-__device__ __forceinline__ float pivot_rsqrt(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// A pivot below the smallest normal float (FP32), not positive, or NaN.
-__device__ __forceinline__ bool pivot_bad(double d) { return !(d > 0.0); }
-__device__ __forceinline__ bool pivot_bad(float d) { return !(d >= 1.17549435e-38f); }
 
 // Named barriers (0 is __syncthreads); __syncwarp first reconverges a warp
-// after divergent code (the barrier instructions are warp-aligned).
+// after divergent code (the barrier instructions are warp-aligned).  bar_arrive
+// does not wait; both order the calling warp's earlier shared-memory accesses
+// before the barrier completes.
 __device__ __forceinline__ void bar_wait(int id, int count) {
   __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int count) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
@@ -647,57 +646,18 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
 }
-
-// d -= A B^T for 8 x 8 blocks in shared memory, lane (g, t) = (lane / 4,
-// lane % 4) holding d[h] = D[g][2t + h].  FP64: two DMMAs on separate
-// accumulators; the K slots (t, first / second MMA) take columns 2t and 2t + 1,
-// so each operand is one 16-byte load.  FP32: dot products on the FMA pipe.
-// Operands are loaded first (load_a, load_b) so that several blocks' loads,
-// products and stores overlap.
-template <typename T> struct Block;
-template <> struct Block<double> {
-  struct Op { double2 v; };
-  static __device__ __forceinline__ Op load_a(const double* A, int lda) {
-    const int lane = threadIdx.x & 31;
-    return Op{*reinterpret_cast<const double2*>(A + (lane >> 2) * lda + 2 * (lane & 3))};
-  }
-  using OpB = Op;
-  static __device__ __forceinline__ OpB load_b(const double* B, int ldb) { return load_a(B, ldb); }
-  static __device__ __forceinline__ void sub(double (&d)[2], const Op& a, const OpB& b) {
-    double e[2] = {0.0, 0.0};
-    dmma(e, -a.v.y, b.v.y);
-    dmma(d, -a.v.x, b.v.x);
-    d[0] += e[0];
-    d[1] += e[1];
-  }
-};
-template <> struct Block<float> {
-  struct Op { float v[8]; };
-  struct OpB { float v[8], w[8]; };
-  static __device__ __forceinline__ Op load_a(const float* A, int lda) {
-    Op o;
-    lds_vec(A + ((threadIdx.x & 31) >> 2) * lda, o.v);
-    return o;
-  }
-  static __device__ __forceinline__ OpB load_b(const float* B, int ldb) {
-    OpB o;
-    lds_vec(B + 2 * (threadIdx.x & 3) * ldb, o.v);
-    lds_vec(B + (2 * (threadIdx.x & 3) + 1) * ldb, o.w);
-    return o;
-  }
-  static __device__ __forceinline__ void sub(float (&d)[2], const Op& a, const OpB& b) {
-    float e0 = 0.0f, e1 = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      d[0] = fmaf(-a.v[q], b.v[q], d[0]);
-      d[1] = fmaf(-a.v[q], b.w[q], d[1]);
-      e0 = fmaf(-a.v[q + 4], b.v[q + 4], e0);
-      e1 = fmaf(-a.v[q + 4], b.w[q + 4], e1);
-    }
-    d[0] += e0;
-    d[1] += e1;
-  }
-};
+// d += A B^T and d -= A B^T for 8 x 8 fragments, two MMAs on separate accumulators
+__device__ __forceinline__ void block_mul(double (&d)[2], const double (&a)[2], const double (&b)[2]) {
+  double e[2] = {0.0, 0.0};
+  dmma(e, a[1], b[1]);
+  dmma(d, a[0], b[0]);
+  d[0] += e[0];
+  d[1] += e[1];
+}
+__device__ __forceinline__ void block_sub(double (&d)[2], const double (&a)[2], const double (&b)[2]) {
+  const double n[2] = {-a[0], -a[1]};
+  block_mul(d, n, b);
+}
 __device__ __forceinline__ void load_pair(const double* p, double (&d)[2]) {
   const double2 v = *reinterpret_cast<const double2*>(p);
   d[0] = v.x;
@@ -714,342 +674,393 @@ __device__ __forceinline__ void store_pair(double* p, double x, double y) {
 __device__ __forceinline__ void store_pair(float* p, float x, float y) {
   *reinterpret_cast<float2*>(p) = make_float2(x, y);
 }
-__device__ __forceinline__ void store_row8(double* p, const double (&v)[8]) {
-#pragma unroll
-  for (int q = 0; q < 8; q += 2) *reinterpret_cast<double2*>(p + q) = make_double2(v[q], v[q + 1]);
-}
-__device__ __forceinline__ void store_row8(float* p, const float (&v)[8]) {
-#pragma unroll
-  for (int q = 0; q < 8; q += 4) *reinterpret_cast<float4*>(p + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-}
 
-// The first i + 1 values of a row of eight (and one more when i is even).
-template <typename T>
-__device__ __forceinline__ void load_lower(const T* p, int i, T (&v)[8]) {
-#pragma unroll
-  for (int q = 0; q <= i; q += 2) {
-    T w[2];
-    load_pair(p + q, w);
-    v[q] = w[0];
-    v[q + 1] = w[1];
-  }
-}
+// Shared memory of a factorisation besides the tile and the solve blocks, in
+// doubles: a panel's multiplier blocks twice, the inverses and pivots of eight
+// panels, one word (the first non-positive pivot).
+constexpr int RELEASE_WARP = 7;
+constexpr int FETCH_WARP = 4;  // on the chain's SM quarter: takes no part in F(k)
+constexpr int FRAG_LD = 10;  // rows of an 8 x 8 block read by rows and by columns
+constexpr int FACTOR_SCRATCH = 2 * 8 * 64 + 8 * 8 * FRAG_LD + 16 * FRAG_LD + 2 * NB + 2;
 
-// Shared memory of a factorisation besides the tile and the solve blocks: two
-// multiplier strips, the two pivot warps' scratch, 1 / L_jj twice, two words
-// (panels done, first non-positive pivot).
-template <typename T>
-constexpr int factor_scratch_elems() {
-  return 2 * NB * ChainLd<T>::MS + 2 * 40 * ChainLd<T>::MS + 2 * NB + 16 / (int)sizeof(T);
-}
-
-template <typename T>
+// Its parts as shared-memory addresses (a pointer's state space would be lost in
+// the struct, and generic accesses cost the chain half as much again).
 struct FactorMem {
-  T* A;   // [64][LT] the tile
-  T* V;   // [64][LT] its solve blocks
-  T* M;   // [2][64][MS] multipliers of a panel
-  T* R;   // [2][40][MS] scratch of the pivot warps
-  T* rs;  // [2][64] 1 / L_jj, a copy for each finishing warp
-  int* w; // [2]
-  __device__ FactorMem(T* tile_, T* blocks, T* scratch) : A(tile_), V(blocks), M(scratch) {
-    R = M + 2 * NB * ChainLd<T>::MS;
-    rs = R + 2 * 40 * ChainLd<T>::MS;
-    w = reinterpret_cast<int*>(rs + 2 * NB);
+  uint32_t A;    // [64][LT] the tile, then x = L sqrt(d) column by column
+  uint32_t V;    // [64][LT] its solve blocks
+  uint32_t M;    // [2][8 block rows][64] a panel's multipliers x / d, fragment order
+  uint32_t U;    // [8 panels][8][FRAG_LD] inverse of a pivot block's unit triangle, by columns
+  uint32_t D;    // [16][FRAG_LD] the chain's pivot block and the identity
+  uint32_t d;    // [64] pivots
+  uint32_t r;    // [64] 1 / d
+  int* bad;      // the first non-positive pivot (64: none)
+  __device__ FactorMem(const double* tile_, const double* blocks, double* scratch)
+      : A(tc::smem_u32(tile_)), V(tc::smem_u32(blocks)), M(tc::smem_u32(scratch)) {
+    U = M + 8 * (2 * 8 * 64);
+    D = U + 8 * (8 * 8 * FRAG_LD);
+    d = D + 8 * (16 * FRAG_LD);
+    r = d + 8 * NB;
+    bad = reinterpret_cast<int*>(scratch + FACTOR_SCRATCH - 2);
   }
 };
+// A pair (16 bytes, aligned) and one double at element `i` of an array there.
+__device__ __forceinline__ void lds_pair(uint32_t base, int i, double (&v)[2]) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(base + 8 * i));
+}
+__device__ __forceinline__ double lds_one(uint32_t base, int i) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(base + 8 * i));
+  return v;
+}
+__device__ __forceinline__ void sts_pair(uint32_t base, int i, double x, double y) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(base + 8 * i), "d"(x), "d"(y) : "memory");
+}
 
-// Column-major numbering, from the last column back, of the lower blocks of
-// the trailing triangle: entry u = (block row) << 4 | (block column).
-__constant__ unsigned char c_tri[28] = {0x77, 0x76, 0x66, 0x75, 0x65, 0x55, 0x74, 0x64, 0x54, 0x44,
-                                        0x73, 0x63, 0x53, 0x43, 0x33, 0x72, 0x62, 0x52, 0x42, 0x32,
-                                        0x22, 0x71, 0x61, 0x51, 0x41, 0x31, 0x21, 0x11};
+// Roles of the warps (FETCH_WARP takes no part; it shares the SM quarter with the
+// chain, which any other role there slows by a fifth).  Panel p = columns 8p .. 8p + 7,
+// block (r, c) = rows 8r .., columns 8c ...
+//  - Warp 0, the chain: the pivot blocks and X of the block row below.
+//  - Warp 3, the lead: block row p + 2, whose blocks (p + 2, p + 1) and
+//    (p + 2, p + 2) the chain needs a panel later.
+//  - Warps 1, 2, 5, 6: X of the other block rows and the update of the
+//    trailing blocks with it.
+//  - Warp 7: what leaves the tile, behind the others.
+// Named barriers: 1 panel p is stored (the chain arrives and goes on), 3 the
+// chain's next blocks (the lead arrives), 4 all X of the panel (the lead arrives).
+// A barrier cannot be entered twice by one side before the other has left it, and
+// the two halves of M cannot be overtaken: the chain stores panel p after barrier
+// 3 of panel p - 1, which the lead reaches after barrier 1 of panel p - 1, that is
+// when all helpers have done panel p - 2.  U, d, r and X keep a place per panel, so warp 7
+// follows the count f.bad[1] of panels (panel p stored, and all of panel p - 1)
+// at its own pace.
+__device__ __forceinline__ void panels_done(const FactorMem& f, int n) {
+  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(tc::smem_u32(f.bad) + 4), "r"(n) : "memory");
+}
 
-// F's pivots, warps 0 .. 4: the tile A (lower triangle valid with every update
-// applied) by eight 8-column panels, in the LDL^T form: column j of A becomes
-// x_j = L_j sqrt(d_j) (its diagonal entry the pivot d_j); the multipliers
-// m = x / d of a panel go to a strip in M.
-//  - Warps 0 and 1 own the rows from the panel's first one on (one row per
-//    lane): they update the panel's own columns with the previous panel (rank
-//    8, 8 x 8 blocks), both factor the 8 x 8 pivot block in every lane's
-//    registers -- the chain is reciprocal -> multiply-add, 53 cycles a column in
-//    FP64, 25 in FP32 -- and eliminate their rows, the block's own among them,
-//    in the same instruction stream.
-//  - Warps 2 .. 4 apply the previous panel to the columns right of the present
-//    one; they are done before the next panel needs the first of them.
-// One barrier per panel (named barrier 1) separates the panels' reads and
-// writes; f.w[0] counts the panels done for the finishing warps.
-constexpr int FACTOR_TRAIL = 3;  // warps 2 .. 4
-template <typename T>
-__device__ __forceinline__ void factor_panels(const FactorMem<T>& f) {
-  constexpr int LT = ChainLd<T>::LT, MS = ChainLd<T>::MS;
-  using B = Block<T>;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  T* A = f.A;
+// The inverse of pivot block p's unit triangle as a fragment.
+__device__ __forceinline__ void load_inverse(const FactorMem& f, int p, double (&u)[2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  u[0] = lds_one(f.U, (8 * p + 2 * t) * FRAG_LD + g);
+  u[1] = lds_one(f.U, (8 * p + 2 * t + 1) * FRAG_LD + g);
+}
+
+// Block (q, q) of the tile from its lower triangle.
+__device__ __forceinline__ void load_symmetric(uint32_t A, int q, double (&v)[2]) {
+  constexpr int LT = ChainLd<double>::LT;
+  const int lane = threadIdx.x & 31, g = lane >> 2, c = 2 * (lane & 3);
+  v[0] = lds_one(A, (8 * q + max(g, c)) * LT + 8 * q + min(g, c));
+  v[1] = lds_one(A, (8 * q + max(g, c + 1)) * LT + 8 * q + min(g, c + 1));
+}
+
+// The chain.  Every lane factors the pivot block in its own registers (l, lower):
+// reciprocal -> multiply-add per column, without a hand-over.  In the same
+// instruction stream lanes 0 .. 7 eliminate the block's rows (x = L sqrt(d)) and
+// lanes 8 .. 15 the rows of the identity, which become the columns of U = inv(unit
+// triangle).
+__device__ __forceinline__ void factor_chain(const FactorMem& f) {
+  constexpr int LT = ChainLd<double>::LT;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double a[2], s[2] = {0, 0}, next[2] = {0, 0};
+  load_symmetric(f.A, 0, a);
+  sts_pair(f.D, (8 + g) * FRAG_LD + 2 * t, g == 2 * t ? 1.0 : 0.0, g == 2 * t + 1 ? 1.0 : 0.0);
 #pragma unroll 1
   for (int p = 0; p < 8; ++p) {
-    const int c0 = 8 * p;
-    const T* Mp = f.M + ((p + 1) & 1) * NB * MS;  // the previous panel's multipliers
-    if (warp < 2) {
-      const int s0 = c0 + 32 * warp;  // this warp's rows s0 .. s0 + 31
-      const bool own = s0 + lane < NB;
-      T l[8][8], x[8];
-      if (p == 0) {
+    sts_pair(f.D, g * FRAG_LD + 2 * t, a[0], a[1]);
+    const double d0 = __shfl_sync(0xffffffffu, a[0], 0);
+    __syncwarp();
+    double l[8][8], x[8], d[8], r[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) load_lower(A + i * LT, i, l[i]);
-        lds_vec(A + (s0 + lane) * LT, x);
-      } else {
-        // the pivot block (block 0) and this warp's four blocks of rows; rows
-        // past the tile repeat the pivot block
-        T* Rw = f.R + warp * 40 * MS;
-        T d[5][2];
-        typename B::Op av[5];
-        const typename B::OpB bv = B::load_b(Mp + c0 * MS, MS);
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int q = 0; q < 5; ++q) {
-          const int r1 = s0 + 8 * (q - 1), r0 = q == 0 || r1 >= NB ? c0 : r1;
-          av[q] = B::load_a(A + r0 * LT + c0 - 8, LT);
-          load_pair(A + (r0 + g) * LT + c0 + 2 * t, d[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < 5; ++q) B::sub(d[q], av[q], bv);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) store_pair(Rw + (8 * q + g) * MS + 2 * t, d[q][0], d[q][1]);
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) load_lower(Rw + i * MS, i, l[i]);
-        lds_vec(Rw + (8 + lane) * MS, x);
+      for (int c = 0; c <= i; c += 2) {
+        double v[2];
+        lds_pair(f.D, i * FRAG_LD + c, v);
+        l[i][c] = v[0];
+        l[i][c + 1] = v[1];
       }
-      T m[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const T r = pivot_rcp(l[j][j]);
-        if (j < 7) l[j + 1][j + 1] = fma(-(l[j + 1][j] * l[j + 1][j]), r, l[j + 1][j + 1]);
-        m[j] = x[j] * r;
+    for (int c = 0; c < 8; c += 2) {
+      double v[2];
+      lds_pair(f.D, (lane & 15) * FRAG_LD + c, v);
+      x[c] = v[0];
+      x[c + 1] = v[1];
+    }
+    // lanes 16 .. 31 repeat lanes 0 .. 15, stores included: nothing here branches
+    const uint32_t row = lane & 8 ? f.U + 8 * ((8 * p + (lane & 7)) * FRAG_LD) : f.A + 8 * ((8 * p + (lane & 7)) * LT + 8 * p);
 #pragma unroll
-        for (int c = j + 1; c < 8; ++c) {
-          const T e = l[c][j] * r;
-          x[c] = fma(-x[j], e, x[c]);
+    for (int j = 0; j < 8; ++j) {
+      d[j] = j == 0 ? d0 : l[j][j];
+      r[j] = pivot_rcp(d[j]);
+      if (j < 7) l[j + 1][j + 1] = fma(-(l[j + 1][j] * l[j + 1][j]), r[j], l[j + 1][j + 1]);
 #pragma unroll
-          for (int i = c; i < 8; ++i)
-            if (i != j + 1) l[i][c] = fma(-l[i][j], e, l[i][c]);
-        }
+      for (int c = j + 1; c < 8; ++c) {
+        const double e = l[c][j] * r[j];
+        x[c] = fma(-x[j], e, x[c]);
+#pragma unroll
+        for (int i = c; i < 8; ++i)
+          if (i != j + 1) l[i][c] = fma(-l[i][j], e, l[i][c]);
       }
-      if (own) {
-        store_row8(A + (s0 + lane) * LT + c0, x);
-        store_row8(f.M + (p & 1) * NB * MS + (s0 + lane) * MS, m);
+      if ((j & 1) == 0) sts_pair(row, j, x[j], x[j + 1]);  // final
+      if (j == 4 && p < 7) {
+        if (p > 0) bar_wait(3, 64);
+        lds_pair(f.A, (8 * (p + 1) + g) * LT + 8 * p + 2 * t, s);
+        load_symmetric(f.A, p + 1, next);
       }
-    } else if (p > 0) {
-      // blocks (ri, cj), cj = p + 1 .. 7, ri = cj .. 7, column by column
-      const int n = (7 - p) * (8 - p) / 2;
-      for (int q0 = warp - 2; q0 < n; q0 += 4 * FACTOR_TRAIL) {
-        T d[4][2];
-        typename B::Op av[4];
-        typename B::OpB bv[4];
+    }
+    __syncwarp();
+    if (p < 7) {
+      double u[2], rp[2], y[2] = {0, 0}, m[2];
+      load_inverse(f, p, u);
+#pragma unroll
+      for (int c = 0; c < 8; c += 2) sts_pair(f.r, 8 * p + c, r[c], r[c + 1]);
+      __syncwarp();
+      lds_pair(f.r, 8 * p + 2 * t, rp);
+      block_mul(y, s, u);
+      m[0] = y[0] * rp[0];
+      m[1] = y[1] * rp[1];
+      a[0] = next[0];
+      a[1] = next[1];
+      block_sub(a, y, m);
+      sts_pair(f.A, (8 * (p + 1) + g) * LT + 8 * p + 2 * t, y[0], y[1]);
+      sts_pair(f.M, ((p & 1) * 8 + p + 1) * 64 + 2 * lane, m[0], m[1]);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) sts_pair(f.d, 8 * p + c, d[c], d[c + 1]);
+    if (p < 6) {
+      bar_arrive(1, 192);
+    } else {
+      __syncwarp();
+      if (lane == 0) panels_done(f, p + 1);
+    }
+  }
+}
+
+// The first helper: block row p + 2 and its blocks that the chain waits for.
+__device__ __forceinline__ void factor_lead(const FactorMem& f) {
+  constexpr int LT = ChainLd<double>::LT;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+  for (int p = 0; p < 6; ++p) {
+    const int at = (8 * (p + 2) + g) * LT + 8 * p + 2 * t;
+    const uint32_t M = f.M + 8 * (((p & 1) * 8 + p) * 64 + 2 * lane);
+    double u[2], r[2], s[2], b[2], c0[2], c1[2], x[2] = {0, 0}, m[2];
+    bar_wait(1, 192);
+    lds_pair(f.A, at, s);
+    load_inverse(f, p, u);
+    lds_pair(f.r, 8 * p + 2 * t, r);
+    lds_pair(M, 64, b);
+    lds_pair(f.A, at + 8, c0);
+    lds_pair(f.A, at + 16, c1);
+    block_mul(x, s, u);
+    m[0] = x[0] * r[0];
+    m[1] = x[1] * r[1];
+    block_sub(c0, x, b);
+    block_sub(c1, x, m);
+    sts_pair(f.A, at + 8, c0[0], c0[1]);
+    sts_pair(f.A, at + 16, c1[0], c1[1]);
+    sts_pair(f.A, at, x[0], x[1]);
+    sts_pair(M, 2 * 64, m[0], m[1]);
+    bar_arrive(3, 64);
+    if (p < 5) bar_arrive(4, 160);
+    if (lane == 0) panels_done(f, p + 1);
+  }
+}
+
+// The other helpers (h = 1 .. 4): block rows p + 7, 6, 3 and 4, 5.  One copy of each
+// loop body: the code of the warps that run at once has to stay in the
+// instruction cache (a chain step loses a third with four streams of 16 KB).
+__device__ __forceinline__ void factor_help(const FactorMem& f, int h) {
+  constexpr int LT = ChainLd<double>::LT;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int k1 = h == 1 ? 7 : h == 2 ? 6 : h == 3 ? 4 : 5, k0 = h == 3 ? 3 : k1;
+#pragma unroll 1
+  for (int p = 0; p < 6; ++p) {
+    const uint32_t M = f.M + 8 * ((p & 1) * 8 * 64 + 2 * lane);
+    const int last = min(p + k1, 7);
+    bar_wait(1, 192);
+    if (p == 5) break;
+    double u[2], r[2];
+    load_inverse(f, p, u);
+    lds_pair(f.r, 8 * p + 2 * t, r);
+    // X of the block rows, with the multipliers
+#pragma unroll 1
+    for (int row = p + k0; row <= last; ++row) {
+      const int at = (8 * row + g) * LT + 8 * p + 2 * t;
+      double s[2], x[2] = {0, 0};
+      lds_pair(f.A, at, s);
+      block_mul(x, s, u);
+      sts_pair(f.A, at, x[0], x[1]);
+      sts_pair(M, row * 64, x[0] * r[0], x[1] * r[1]);
+    }
+    bar_wait(4, 160);
+    // blocks (row, p + 1 .. row) less X M^T, four at a time (past the end the last
+    // one again, without a branch)
+#pragma unroll 1
+    for (int row = p + k0; row <= last; ++row) {
+      const int base = (8 * row + g) * LT + 2 * t;
+      double x[2];
+      lds_pair(f.A, base + 8 * p, x);
+#pragma unroll 1
+      for (int col = p + 1; col <= row; col += 4) {
+        double c[4][2], b[4][2];
         int at[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int q = q0 + u * FACTOR_TRAIL, e = c_tri[q < n ? n - 1 - q : 0], ri = e >> 4, cj = e & 15;
-          at[u] = q < n ? (8 * ri + g) * LT + 8 * cj + 2 * t : -1;
-          av[u] = B::load_a(A + 8 * ri * LT + c0 - 8, LT);
-          bv[u] = B::load_b(Mp + 8 * cj * MS, MS);
-          load_pair(A + (8 * ri + g) * LT + 8 * cj + 2 * t, d[u]);
+        for (int i = 0; i < 4; ++i) {
+          const int q = min(col + i, row);
+          at[i] = base + 8 * q;
+          lds_pair(M, q * 64, b[i]);
+          lds_pair(f.A, at[i], c[i]);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) B::sub(d[u], av[u], bv[u]);
+        for (int i = 0; i < 4; ++i) block_sub(c[i], x, b[i]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (at[u] >= 0) store_pair(A + at[u], d[u][0], d[u][1]);
+        for (int i = 0; i < 4; ++i) sts_pair(f.A, at[i], c[i][0], c[i][1]);
       }
     }
-    bar_wait(1, 32 * (2 + FACTOR_TRAIL));
-    if (threadIdx.x == 0) asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(tc::smem_u32(f.w)), "r"(p + 1) : "memory");
   }
 }
 
-// The pair (row 8j + lane / 4, columns 8q + 2 (lane % 4) ..) of L_kk = x / sqrt(d)
-// into the factor's tile (zero above the diagonal).
-template <typename T, typename S>
-__device__ __forceinline__ void store_factor_pair(const FactorMem<T>& f, const T* rs, S* out, int ld, int j, int q) {
-  constexpr int LT = ChainLd<T>::LT;
-  const int lane = threadIdx.x & 31, r = 8 * j + (lane >> 2), c = 8 * q + 2 * (lane & 3);
-  T v[2] = {T(0), T(0)};
-  if (q <= j) {
-    load_pair(f.A + r * LT + c, v);
-    v[0] = c <= r ? v[0] * rs[c] : T(0);
-    v[1] = c + 1 <= r ? v[1] * rs[c + 1] : T(0);
-  }
-  store_pair(out + (size_t)r * ld + c, (S)v[0], (S)v[1]);
-}
-
-// V_jq = V_jj L_jq for blocks q = q0 .. q0 + N - 1 below `end`.
-template <typename T, typename S, int N>
-__device__ __forceinline__ void solve_blocks(const FactorMem<T>& f, const T* rs, S* V_out, int j, int q0, int end) {
-  constexpr int LT = ChainLd<T>::LT;
+// Warp 7: the zeros above the block diagonal, then panel by panel the pivots'
+// square roots, the first non-positive pivot, V_pp = inv(L_pp) = diag(1 / sqrt(d)) U
+// and L_pp, and, a panel later, the block column below L_pp, to the factor and to
+// the solve blocks.
+template <typename S>
+__device__ __forceinline__ void factor_finish(const FactorMem& f, S* out, int ld, S* V_out, double min_pivot,
+                                              long long spin_limit) {
+  constexpr int LT = ChainLd<double>::LT;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const T* Vj = f.V + 8 * j * LT + 8 * j;
-  T d[N][2];
-#pragma unroll
-  for (int u = 0; u < N; ++u) {
-    const int q = min(q0 + u, end - 1);
-    const T* Lb = f.A + 8 * j * LT + 8 * q;  // x; times 1 / sqrt(d) of its columns
-    d[u][0] = d[u][1] = T(0);
-    if constexpr (sizeof(T) == 8) {
-      double v[2];
-      load_pair(Vj + g * LT + 2 * t, v);
-      const double s = rs[8 * q + g];
-      dmma(d[u], v[0], Lb[2 * t * LT + g] * s);
-      dmma(d[u], v[1], Lb[(2 * t + 1) * LT + g] * s);
-    } else {
-      T v[8], s[2];
-      lds_vec(Vj + g * LT, v);
-      load_pair(rs + 8 * q + 2 * t, s);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        T b[2];
-        load_pair(Lb + i * LT + 2 * t, b);
-        d[u][0] = fma(v[i], b[0], d[u][0]);
-        d[u][1] = fma(v[i], b[1], d[u][1]);
+  S* o = out + (size_t)g * ld + 2 * t;
+#pragma unroll 1
+  for (int p = 1; p < 8; ++p)
+#pragma unroll 1
+    for (int i = 0; i < p; ++i) store_pair(o + (size_t)8 * i * ld + 8 * p, S(0), S(0));
+  double q0 = 0, q1 = 0;  // 1 / sqrt(d) of the previous panel's columns 2t, 2t + 1
+#pragma unroll 1
+  for (int p = 0; p < 8; ++p) {
+    // bounded like every wait; the other warps do not wait on anything else
+    for (long long it = 0; it < spin_limit; ++it) {
+      int done;
+      asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(done) : "r"(tc::smem_u32(f.bad) + 4) : "memory");
+      if (done > p) break;
+    }
+    __syncwarp();
+    const int c = 8 * p + 2 * t;
+    const double d = lds_one(f.d, 8 * p + g);
+    double u[2], x[2];
+    load_inverse(f, p, u);
+    lds_pair(f.A, (8 * p + g) * LT + c, x);
+    // the column of the panel before
+#pragma unroll 1
+    for (int i = p > 0 ? p : 8; i < 8; i += 2) {
+      double y[2], z[2];
+      const int r0 = 8 * i + g, r1 = 8 * min(i + 1, 7) + g;
+      lds_pair(f.A, r0 * LT + c - 8, y);
+      lds_pair(f.A, r1 * LT + c - 8, z);
+      y[0] *= q0;
+      y[1] *= q1;
+      z[0] *= q0;
+      z[1] *= q1;
+      sts_pair(f.V, r0 * LT + c - 8, y[0], y[1]);
+      sts_pair(f.V, r1 * LT + c - 8, z[0], z[1]);
+      store_pair(out + (size_t)r0 * ld + c - 8, (S)y[0], (S)y[1]);
+      store_pair(out + (size_t)r1 * ld + c - 8, (S)z[0], (S)z[1]);
+      if (V_out) {
+        store_pair(V_out + r0 * NB + c - 8, (S)y[0], (S)y[1]);
+        store_pair(V_out + r1 * NB + c - 8, (S)z[0], (S)z[1]);
       }
-      d[u][0] *= s[0];
-      d[u][1] *= s[1];
     }
+    const unsigned bad = __ballot_sync(0xffffffffu, !(d > 0.0 && d >= min_pivot));
+    const double rg = pivot_rsqrt(d);
+    q0 = __shfl_sync(0xffffffffu, rg, 8 * t);
+    q1 = __shfl_sync(0xffffffffu, rg, 8 * t + 4);
+    sts_pair(f.V, (8 * p + g) * LT + c, rg * u[0], rg * u[1]);
+    if (V_out) store_pair(V_out + (8 * p + g) * NB + c, (S)(rg * u[0]), (S)(rg * u[1]));
+    store_pair(o + (size_t)8 * p * ld + 8 * p, (S)(2 * t <= g ? x[0] * q0 : 0.0), (S)(2 * t + 1 <= g ? x[1] * q1 : 0.0));
+    if (lane == 0 && bad) *f.bad = min(*f.bad, 8 * p + ((__ffs(bad) - 1) >> 2));
   }
-#pragma unroll
-  for (int u = 0; u < N; ++u)
-    if (q0 + u < end) {
-      store_pair(f.V + (8 * j + g) * LT + 8 * (q0 + u) + 2 * t, d[u][0], d[u][1]);
-      if (V_out) store_pair(V_out + (8 * j + g) * NB + 8 * (q0 + u) + 2 * t, (S)d[u][0], (S)d[u][1]);
-    }
 }
 
-// 1 / L_ii of blocks j - 1 and j into rs, block j's first non-positive pivot, and
-// V_jj = inv(L_jj) (lane c < 8: column c by forward substitution on
-// z_i = y_i / L_ii, whose chain is one multiply-add and one product per row).
-// One warp; every second j suffices to fill rs.
-template <typename T, typename S>
-__device__ __forceinline__ void invert_block(const FactorMem<T>& f, T* rs, S* V_out, int j) {
-  constexpr int LT = ChainLd<T>::LT;
-  const int lane = threadIdx.x & 31, c = lane & 7;
-  const T* D = f.A + 8 * j * LT + 8 * j;
-  const int i0 = 8 * ((lane & 8) && j > 0 ? j - 1 : j) + c;
-  const T d = f.A[i0 * LT + i0];
-  const T r = pivot_rsqrt(d);
-  const unsigned bad = __ballot_sync(0xffffffffu, pivot_bad(d)) & 0xffu;
-  if (lane == 0 && bad) atomicMin(f.w + 1, 8 * j + __ffs(bad) - 1);
-  if (lane < 16) rs[i0] = r;
-  T l[8][8], y[8], z[8];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) load_lower(D + i * LT, i - 1, l[i]);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const T ri = __shfl_sync(0xffffffffu, r, i);
-    T s = i == c ? T(1) : T(0);
-#pragma unroll
-    for (int q = 0; q < i; ++q) s = fma(-l[i][q], z[q], s);
-    y[i] = s * ri;
-    z[i] = s * (ri * ri);
-  }
-  if (lane < 8)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      f.V[(8 * j + i) * LT + 8 * j + c] = y[i];
-      if (V_out) V_out[(8 * j + i) * NB + 8 * j + c] = (S)y[i];
-    }
-  __syncwarp();
-}
-
-// F(k) of the updated tile f.A, warps 0 .. 6 (warp 7 returns at once): L_kk =
-// x / sqrt(d) to tile (k, k) of the factor (type S, zero above the diagonal),
+// F(k) of the updated tile f.A (its lower triangle), warps 0 .. 6 (warp 7 returns
+// at once): L_kk to tile (k, k) of the factor (type S, zero above the diagonal),
 // the solve blocks of L_kk to f.V and to V_out (global 64 x 64, type S, or
-// null): with 8 x 8 blocks, V_jj = inv(L_jj) and V_jq = inv(L_jj) L_jq for
-// q < j, so that a row C of the solve C L_kk^-T is
-// W_j = C_j V_jj^T - sum_{q < j} W_q V_jq^T.  (Blocks above the block diagonal
-// are neither written nor read.)  Warps 5 and 6 finish a row of blocks (the
-// square roots, V, the stores) while the panels after it are factored; only
-// the last row is left when the last pivot is done.  A non-positive pivot is
-// recorded in info.  f.w: {0, 64} on entry.  Ends with a barrier of warps
-// 0 .. 6 (named barrier 2).
-template <typename T, typename S>
-__device__ __forceinline__ void factor_tile(const DFArgs& a, int k, const FactorMem<T>& f, S* V_out) {
+// null): with 8 x 8 blocks, V_jj = inv(L_jj) on the block diagonal and L_jq
+// below it.  (Blocks above the block diagonal are neither written nor read.)
+// A non-positive pivot is recorded in info.  f.bad: {64, 0} on entry; on
+// return, after the caller's next CTA barrier, {64, 8}.  Ends with a barrier of warps 0 .. 6
+// (named barrier 2).
+template <typename S>
+__device__ __forceinline__ void factor_tile(const DFArgs& a, int k, const FactorMem& f, S* V_out) {
   const int warp = threadIdx.x >> 5;
-  if (warp == 7) return;
-  S* out = tile<S>(a, k, k);
-  if (warp < 5) {
-    factor_panels(f);
-  } else {
-    T* rs = f.rs + (warp - 5) * NB;
-    for (int j = warp - 5; j < 8; j += 2) {
-      // bounded like every wait; the panels do not wait on anything else
-      for (long long it = 0; it < a.spin_limit; ++it) {
-        int done;
-        asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(done) : "r"(tc::smem_u32(f.w)) : "memory");
-        if (done > j) break;
-      }
-      __syncwarp();
-      invert_block<T, S>(f, rs, V_out, j);
-      if (j == 7) break;
-      for (int q = 0; q < j; q += 4) solve_blocks<T, S, 4>(f, rs, V_out, j, q, j);
-#pragma unroll 4
-      for (int q = 0; q < 8; ++q) store_factor_pair<T, S>(f, rs, out, a.ld, j, q);
-    }
-  }
+  if (warp == FETCH_WARP) return;
+  if (warp == 0) factor_chain(f);
+  else if (warp == 7) factor_finish<S>(f, tile<S>(a, k, k), a.ld, V_out, a.min_pivot, a.spin_limit);
+  else if (warp == 3) factor_lead(f);
+  else factor_help(f, warp < 3 ? warp : warp - 2);
   bar_wait(2, 32 * 7);
-  const T* rs = f.rs + NB;  // warp 6's copy is complete
-  solve_blocks<T, S, 1>(f, rs, V_out, 7, warp, 7);
-  store_factor_pair<T, S>(f, rs, out, a.ld, 7, warp);
-  if (warp == 5) store_factor_pair<T, S>(f, rs, out, a.ld, 7, 7);
   if (threadIdx.x == 0) {
-    if (f.w[1] < NB && k * NB + f.w[1] < a.n) atomicCAS(a.info, 0, k * NB + f.w[1] + 1);
-    f.w[0] = 0;
-    f.w[1] = NB;
+    if (f.bad[0] < NB && k * NB + f.bad[0] < a.n) atomicCAS(a.info, 0, k * NB + f.bad[0] + 1);
+    f.bad[0] = NB;
   }
-  bar_wait(2, 32 * 7);
 }
 
 // ---------------------------------------------------------------- S(i, k)
 // W = C L_kk^-T for a 64 x 64 tile C (smem rows of ldc) with the solve blocks
-// V of L_kk (smem [64][LT], factor_tile), W_j = C_j V_jj^T - sum_q W_q V_jq^T
+// of L_kk (smem [64][LT], factor_tile), W_j = (C_j - sum_{q < j} W_q L_jq^T) V_jj^T
 // block column by block column.  A warp keeps its rows' accumulators in
-// registers; with the K slots chosen as columns 2t, 2t + 1 the accumulator
-// fragment of W_j is at once the next products' A fragment, so the chain over
-// the eight block columns is one MMA and one add per column, without shuffles
+// registers; with the K slots chosen as columns 2t, 2t + 1 an accumulator
+// fragment is at once the next products' A fragment, so the chain over
+// the eight block columns is two MMAs and two adds per column, without shuffles
 // or shared memory.  out(row, col, w0, w1) receives the pairs of W
-// (columns col, col + 1).  All warps of the CTA; a warp's rows of C are read
-// before its first out(), which may therefore overwrite them.
+// (columns col, col + 1).  G groups of eight rows per warp, so warps 0 .. 8 / G - 1;
+// a warp's rows of C are read before its first out(), which may therefore
+// overwrite them.
 // Against the product with the explicit inverse: half the operations and no
 // inversion before it.  FP64: DMMA, eight rows per warp (bound by the FP64
-// tensor pipe: 576 DMMAs, 2.4k cycles).
-template <typename F>
-__device__ __forceinline__ void solve_rows(const double* C, int ldc, const double* V, F out) {
+// tensor pipe: 576 DMMAs, 2.4k cycles, with one warp of sixteen rows per SM quarter as
+// with two of eight).
+template <int G, typename S, typename F>
+__device__ __forceinline__ void solve_rows(const S* C, int ldc, const double* V, F out) {
   constexpr int LT = ChainLd<double>::LT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  double p[8][2], q[8][2], v[8][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, r0 = 8 * G * warp + g;
+  double p[G][8][2], q[G][8][2], v[8][2];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    double c[2];
-    load_pair(C + (8 * warp + g) * ldc + 8 * j + 2 * t, c);
-    load_pair(V + (8 * j + g) * LT + 8 * j + 2 * t, v[j]);
-    p[j][0] = p[j][1] = q[j][0] = q[j][1] = 0.0;
-    dmma(p[j], c[0], v[j][0]);
-    dmma(q[j], c[1], v[j][1]);
-  }
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      S c[2];
+      load_pair(C + (r0 + 8 * i) * ldc + 8 * j + 2 * t, c);
+      p[i][j][0] = c[0];
+      p[i][j][1] = c[1];
+      q[i][j][0] = q[i][j][1] = 0.0;
+    }
   __syncwarp();
-  auto load_column = [&](int j) {  // V_ij, i > j
+  auto load_column = [&](int j) {  // V_jj, L_ij
 #pragma unroll
-    for (int i = 1; i < 8; ++i)
-      if (i > j) load_pair(V + (8 * i + g) * LT + 8 * j + 2 * t, v[i]);
+    for (int i = 0; i < 8; ++i)
+      if (i >= j) load_pair(V + (8 * i + g) * LT + 8 * j + 2 * t, v[i]);
   };
   load_column(0);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const double w0 = p[j][0] + q[j][0], w1 = p[j][1] + q[j][1];
+    double w[G][2];
 #pragma unroll
-    for (int i = j + 1; i < 8; ++i) {
-      dmma(p[i], -w0, v[i][0]);
-      dmma(q[i], -w1, v[i][1]);
+    for (int i = 0; i < G; ++i) {
+      double d[2] = {0.0, 0.0}, e[2] = {0.0, 0.0};
+      dmma(d, p[i][j][0] + q[i][j][0], v[j][0]);
+      dmma(e, p[i][j][1] + q[i][j][1], v[j][1]);
+      w[i][0] = d[0] + e[0];
+      w[i][1] = d[1] + e[1];
     }
+#pragma unroll
+    for (int k = j + 1; k < 8; ++k)
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        dmma(p[i][k], -w[i][0], v[k][0]);
+        dmma(q[i][k], -w[i][1], v[k][1]);
+      }
     load_column(j + 1);  // ahead of this column's stores
-    out(8 * warp + g, 8 * j + 2 * t, w0, w1);
+#pragma unroll
+    for (int i = 0; i < G; ++i) out(r0 + 8 * i, 8 * j + 2 * t, w[i][0], w[i][1]);
   }
 }
 
@@ -1069,172 +1080,117 @@ __device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) 
 // FP32: 3xTF32 m16n8k8, sixteen rows per warp (warps 0 .. 3), the hi * hi
 // products and the two cross terms on separate accumulators.
 template <typename F>
-__device__ __forceinline__ void solve_rows(const float* C, int ldc, const float* V, F out) {
+__device__ __forceinline__ void solve_rows_f32(const float* C, int ldc, const float* V, F out) {
   constexpr int LT = ChainLd<float>::LT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   if (warp >= 4) return;
   const int r0 = 16 * warp + g;
   float p[8][4], q[8][4];
-  auto mul = [&](int i, const float (&w)[4], const float* vb) {  // p[i], q[i] += w V^T (block at vb)
-    unsigned ah[4], al[4], bh[2], bl[2];
+  auto mul = [&](float (&p)[4], float (&q)[4], const unsigned (&ah)[4], const unsigned (&al)[4], const float* vb) {
+    unsigned bh[2], bl[2];
     float v[2];
     load_pair(vb + g * LT + 2 * t, v);
-    // fragment order: (g, 2t), (g + 8, 2t), (g, 2t + 1), (g + 8, 2t + 1)
-    const float a[4] = {w[0], w[2], w[1], w[3]};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) split_tf32(a[e], ah[e], al[e]);
 #pragma unroll
     for (int e = 0; e < 2; ++e) split_tf32(v[e], bh[e], bl[e]);
-    tf32_mma(p[i], ah, bh);
-    tf32_mma(q[i], al, bh);
-    tf32_mma(q[i], ah, bl);
+    tf32_mma(p, ah, bh);
+    tf32_mma(q, al, bh);
+    tf32_mma(q, ah, bl);
   };
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     float c[2], e[2];
     load_pair(C + r0 * ldc + 8 * j + 2 * t, c);
     load_pair(C + (r0 + 8) * ldc + 8 * j + 2 * t, e);
-    const float w[4] = {c[0], c[1], e[0], e[1]};
+    p[j][0] = c[0];
+    p[j][1] = c[1];
+    p[j][2] = e[0];
+    p[j][3] = e[1];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) p[j][u] = q[j][u] = 0.0f;
-    mul(j, w, V + 8 * j * LT + 8 * j);
+    for (int u = 0; u < 4; ++u) q[j][u] = 0.0f;
   }
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    float w[4], n[4];
+    // fragment order: (g, 2t), (g + 8, 2t), (g, 2t + 1), (g + 8, 2t + 1)
+    constexpr int at[4] = {0, 2, 1, 3};
+    unsigned ah[4], al[4];
+    float w[4], d[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      w[u] = p[j][u] + q[j][u];
-      n[u] = -w[u];
-    }
+    for (int u = 0; u < 4; ++u) split_tf32(p[j][at[u]] + q[j][at[u]], ah[u], al[u]);
+    mul(d, e, ah, al, V + 8 * j * LT + 8 * j);
 #pragma unroll
-    for (int i = j + 1; i < 8; ++i) mul(i, n, V + 8 * i * LT + 8 * j);
+    for (int u = 0; u < 4; ++u) w[u] = d[u] + e[u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) split_tf32(-w[at[u]], ah[u], al[u]);
+#pragma unroll
+    for (int i = j + 1; i < 8; ++i) mul(p[i], q[i], ah, al, V + 8 * i * LT + 8 * j);
     out(r0, 8 * j + 2 * t, w[0], w[1]);
     out(r0 + 8, 8 * j + 2 * t, w[2], w[3]);
   }
 }
 
-// ---------------------------------------------------------------- the chain's SYRK
-// A = N - L L^T on and below the block diagonal (smem tiles, rows of LT): the
-// last update of the next diagonal tile, with the solve's result still in
-// shared memory.  FP64: the 36 lower 8 x 8 blocks, 9 per SM quarter (warps w
-// and w + 4): row 7 - w and row w of blocks.
-__device__ __forceinline__ void syrk_lower(const double* N, const double* L, double* A) {
-  constexpr int LT = ChainLd<double>::LT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  auto row = [&](int i, int j0, int j1) {  // blocks (i, j0 .. j1 - 1)
-    double av[8][2];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) load_pair(L + (8 * i + g) * LT + 8 * k + 2 * t, av[k]);
-#pragma unroll 1
-    for (int j = j0; j < j1; ++j) {
-      double d[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, n[2];
-      load_pair(N + (8 * i + g) * LT + 8 * j + 2 * t, n);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        double b[2];
-        load_pair(L + (8 * j + g) * LT + 8 * k + 2 * t, b);
-        dmma(d[2 * (k & 1)], av[k][0], b[0]);
-        dmma(d[2 * (k & 1) + 1], av[k][1], b[1]);
-      }
-      store_pair(A + (8 * i + g) * LT + 8 * j + 2 * t, n[0] - ((d[0][0] + d[1][0]) + (d[2][0] + d[3][0])),
-                 n[1] - ((d[0][1] + d[1][1]) + (d[2][1] + d[3][1])));
-    }
-  };
-  if (warp < 4) {
-    row(7 - warp, 0, 5);
-  } else {
-    const int w = warp - 4;
-    if (w < 3) row(7 - w, 5, 8 - w);
-    row(w, 0, w + 1);
-  }
+template <typename T, typename F>
+__device__ __forceinline__ void solve_rows_t(const T* C, int ldc, const T* V, F out) {
+  if constexpr (sizeof(T) == 8) solve_rows<1>(C, ldc, V, out);
+  else solve_rows_f32(C, ldc, V, out);
 }
-// FP32: the twenty 16 x 8 blocks that meet the lower triangle in 3xTF32, five
-// per SM quarter; the product is accumulated from zero and subtracted once.
-__device__ __forceinline__ void syrk_lower(const float* N, const float* L, float* A) {
-  constexpr int LT = ChainLd<float>::LT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  // block row, first block column, count of warp w
-  constexpr int RB[8] = {3, 3, 2, 2, 0, 1, 3, 1}, J0[8] = {0, 3, 0, 3, 0, 0, 6, 2}, CN[8] = {3, 3, 3, 3, 2, 2, 2, 2};
-  int rb = 0, j0 = 0, cn = 0;
+
+// ---------------------------------------------------------------- the chain's SYRK
+// A = N - L L^T on and below the block diagonal (A, L: smem rows of
+// ChainLd<double>::LT): the last update of the next diagonal tile, with the
+// solve's result still in shared memory.  N (its rows of ChainLd<S>::LT) is not
+// read before ready() returns, so that its way here overlaps with the products.
+// The 36 lower 8 x 8 blocks, nine on each of warps 0 .. 3: rows 7 - w and w of
+// blocks (bound by the FP64 tensor pipe, 2.4k cycles).
+template <typename S, typename R>
+__device__ __forceinline__ void syrk_lower(const S* N, const double* L, double* A, R ready) {
+  constexpr int LT = ChainLd<double>::LT, LS = ChainLd<S>::LT;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int bi[9], bj[9];
+  double d[9][2], e[9][2];
 #pragma unroll
-  for (int w = 0; w < 8; ++w)
-    if (w == warp) {
-      rb = RB[w];
-      j0 = J0[w];
-      cn = CN[w];
-    }
-  const float* La = L + (16 * rb + g) * LT;
-  float p[3][4], q[3][4];
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int u = 0; u < 4; ++u) p[c][u] = q[c][u] = 0.0f;
-#pragma unroll 2
-  for (int k0 = 0; k0 < NB; k0 += 8) {
-    float x[2], y[2];
-    load_pair(La + k0 + 2 * t, x);
-    load_pair(La + 8 * LT + k0 + 2 * t, y);
-    const float av[4] = {x[0], y[0], x[1], y[1]};
-    unsigned ah[4], al[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) split_tf32(av[e], ah[e], al[e]);
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      if (c < cn) {
-        float v[2];
-        load_pair(L + (8 * (j0 + c) + g) * LT + k0 + 2 * t, v);
-        unsigned bh[2], bl[2];
-        split_tf32(v[0], bh[0], bl[0]);
-        split_tf32(v[1], bh[1], bl[1]);
-        tf32_mma(p[c], ah, bh);
-        tf32_mma(q[c], al, bh);
-        tf32_mma(q[c], ah, bl);
-      }
+  for (int b = 0; b < 9; ++b) {
+    const bool low = b < 8 - w;
+    bi[b] = 8 * (low ? 7 - w : w);
+    bj[b] = 8 * (low ? b : b - (8 - w));
+    d[b][0] = d[b][1] = e[b][0] = e[b][1] = 0.0;
   }
+#pragma unroll 1
+  for (int k = 0; k < NB; k += 8)
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
-    if (c < cn) {
-      const int r = 16 * rb + g, col = 8 * (j0 + c) + 2 * t;
-      float n[2], m[2];
-      load_pair(N + r * LT + col, n);
-      load_pair(N + (r + 8) * LT + col, m);
-      store_pair(A + r * LT + col, n[0] - (p[c][0] + q[c][0]), n[1] - (p[c][1] + q[c][1]));
-      store_pair(A + (r + 8) * LT + col, m[0] - (p[c][2] + q[c][2]), m[1] - (p[c][3] + q[c][3]));
+    for (int b = 0; b < 9; ++b) {
+      double x[2], y[2];
+      load_pair(L + (bi[b] + g) * LT + k + 2 * t, x);
+      load_pair(L + (bj[b] + g) * LT + k + 2 * t, y);
+      dmma(d[b], x[0], y[0]);
+      dmma(e[b], x[1], y[1]);
     }
+  ready();
+#pragma unroll
+  for (int b = 0; b < 9; ++b) {
+    S v[2];
+    load_pair(N + (bi[b] + g) * LS + bj[b] + 2 * t, v);
+    store_pair(A + (bi[b] + g) * LT + bj[b] + 2 * t, (double)v[0] - (d[b][0] + e[b][0]), (double)v[1] - (d[b][1] + e[b][1]));
+  }
 }
 
 // ---------------------------------------------------------------- the chain CTA
-// Shared memory of the chain CTA: five [64][LT] tiles (the diagonal tile, the
-// solve's input, its result, the next diagonal tile, the solve blocks) and
-// the factor scratch.
-template <typename T>
+// Shared memory of the chain CTA: three FP64 tiles (the diagonal tile, the
+// solve's result, the solve blocks), two of the matrix's type (the solve's
+// input, the next diagonal tile), and the factor scratch.
+template <typename S>
 constexpr size_t chain_smem_bytes() {
-  return sizeof(T) * (5 * NB * ChainLd<T>::LT + factor_scratch_elems<T>());
+  return sizeof(double) * (3 * NB * ChainLd<double>::LT + FACTOR_SCRATCH) + 2 * sizeof(S) * NB * ChainLd<S>::LT;
 }
 
-// One warp's copy of a 64 x 64 tile into smem rows of LT: asynchronous (the
-// warp waits with cp_async_wait_all), or converted when the matrix is FP32
-// and the chain works in FP64.
-template <typename T, typename S>
-__device__ __forceinline__ void fetch_tile_warp(const S* g, int ld, T* s) {
-  constexpr int LT = ChainLd<T>::LT;
-  const int lane = threadIdx.x & 31;
-  if constexpr (sizeof(T) == sizeof(S)) {
-    constexpr int per_row = NB * (int)sizeof(T) / 16, elems = 16 / (int)sizeof(T);
+// One warp's asynchronous copy of a 64 x 64 tile into smem rows of LT (the
+// warp waits with cp_async_wait_all).
+template <typename S>
+__device__ __forceinline__ void fetch_tile_warp(const S* g, int ld, S* s) {
+  constexpr int LT = ChainLd<S>::LT, per_row = NB * (int)sizeof(S) / 16, elems = 16 / (int)sizeof(S);
 #pragma unroll 8
-    for (int c = lane; c < NB * per_row; c += 32)
-      cp_async16(s + (c / per_row) * LT + (c % per_row) * elems, g + (size_t)(c / per_row) * ld + (c % per_row) * elems);
-  } else {
-#pragma unroll 8
-    for (int c = lane; c < NB * NB / 4; c += 32) {
-      const int r = c >> 4, q = 4 * (c & 15);
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(g + (size_t)r * ld + q));
-      store_pair(s + r * LT + q, (T)v.x, (T)v.y);
-      store_pair(s + r * LT + q + 2, (T)v.z, (T)v.w);
-    }
-  }
+  for (int c = threadIdx.x & 31; c < NB * per_row; c += 32)
+    cp_async16(s + (c / per_row) * LT + (c % per_row) * elems, g + (size_t)(c / per_row) * ld + (c % per_row) * elems);
 }
 
 // A single warp's bounded wait for *flag >= target (the abort polling and the
@@ -1271,103 +1227,93 @@ __device__ __forceinline__ bool warp_wait_geq(const DFArgs& a, const int* flag, 
   return ok && __all_sync(0xffffffffu, ld_acquire(flag) >= target);
 }
 
-// The chain CTA: F(0), S(1, 0), F(1), S(2, 1), ... in T arithmetic on a matrix
-// of type S.  For each k: F(k) on warps 0 .. 6 (L_kk to the factor, the solve
+// The chain CTA: F(0), S(1, 0), F(1), S(2, 1), ... in FP64 on a matrix of
+// type S.  For each k: F(k) on seven warps (L_kk to the factor, the solve
 // blocks to a.lp for the workers' solves of column k, fin(k, k) = 1), while
-// warp 7 fetches the solve's input A(k+1, k) as soon as its last update is in
-// and the next diagonal tile; S(k+1, k) on all warps, kept in shared memory
-// and published as fin(k+1, k) = 1; the last update of A(k+1, k+1) from the
-// result (syrk_lower).
-template <typename T, typename S>
+// FETCH_WARP copies the solve's input A(k+1, k) as soon as its last update is
+// in; S(k+1, k) on warps 0 .. 3 (one per SM quarter fills its FP64 tensor pipe),
+// kept in shared memory and published as fin(k+1, k) = 1; the last update of
+// A(k+1, k+1) from the result (syrk_lower, the same warps), whose tile FETCH_WARP
+// copies meanwhile.  The flags are published by RELEASE_WARP, which has nothing else to
+// do then: a release costs its warp 0.7 us.
+template <typename S>
 __device__ void run_chain(const DFArgs& a, unsigned char* smem, int* s_ok) {
-  constexpr int LT = ChainLd<T>::LT;
-  __shared__ int s_pf;  // the next diagonal tile is in N
-  T* A = reinterpret_cast<T*>(smem);
-  T* C = A + NB * LT;
-  T* L = C + NB * LT;
-  T* N = L + NB * LT;
-  T* V = N + NB * LT;
-  const FactorMem<T> f(A, V, V + NB * LT);
+  constexpr int LT = ChainLd<double>::LT, LS = ChainLd<S>::LT;
+  double* A = reinterpret_cast<double*>(smem);
+  double* L = A + NB * LT;
+  double* V = L + NB * LT;
+  const FactorMem f(A, V, V + NB * LT);
+  S* C = reinterpret_cast<S*>(V + NB * LT + FACTOR_SCRATCH);
+  S* N = C + NB * LS;
   const int nt = a.nt, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     *s_ok = 1;
-    f.w[0] = 0;
-    f.w[1] = NB;
+    f.bad[0] = NB;
+    f.bad[1] = 0;
   }
-  if (warp == 7) {
-    fetch_tile_warp<T, S>(tile<S>(a, 0, 0), a.ld, A);
-    cp_async_wait_all();
-  }
+  for (int e = threadIdx.x; e < NB * NB; e += THREADS)
+    A[(e >> 6) * LT + (e & 63)] = (double)ldcg(tile<S>(a, 0, 0) + (size_t)(e >> 6) * a.ld + (e & 63));
   __syncthreads();
   for (int k = 0; k < nt; ++k) {
     TRACE(0, a.ntasks + 2 * k);
     TRACE(3, a.ntasks + 2 * k);
     TRACE(1, a.ntasks + 2 * k);
-    if (warp < 7) {
+    const int* next = a.upd + (k + 1) * nt + k + 1;
+    if (warp != FETCH_WARP) {
       CTRACE(k, 0);
-      factor_tile<T, S>(a, k, f, a.lp ? reinterpret_cast<S*>(a.lp) + (size_t)k * NB * NB : nullptr);
-      if (threadIdx.x == 32 * 6) st_release(a.fin + k * nt + k, 1);
+      factor_tile<S>(a, k, f, a.lp ? reinterpret_cast<S*>(a.lp) + (size_t)k * NB * NB : nullptr);
     } else if (k + 1 < nt) {
-      bool ok = warp_wait_geq(a, a.upd + (k + 1) * nt + k, k);
-      int pf = 0;
+      const bool ok = warp_wait_geq(a, a.upd + (k + 1) * nt + k, k);
       if (ok) {
-        fetch_tile_warp<T, S>(tile<S>(a, k + 1, k), a.ld, C);
-        pf = __all_sync(0xffffffffu, ld_acquire(a.upd + (k + 1) * nt + k + 1) >= k);
-        if (pf) fetch_tile_warp<T, S>(tile<S>(a, k + 1, k + 1), a.ld, N);
-        cp_async_wait_all();
-      }
-      if (lane == 0) {
-        s_pf = pf;
-        if (!ok) *s_ok = 0;
-      }
-    }
-    TRACE(2, a.ntasks + 2 * k);
-    CTRACE(k, 1);
-    __syncthreads();
-    if (!*s_ok || k + 1 == nt) return;
-    TRACE(0, a.ntasks + 2 * k + 1);
-    TRACE(3, a.ntasks + 2 * k + 1);
-    TRACE(1, a.ntasks + 2 * k + 1);
-    CTRACE(k, 2);
-    S* out = tile<S>(a, k + 1, k);
-    solve_rows(C, LT, V, [&](int r, int c, T w0, T w1) {
-      store_pair(L + r * LT + c, w0, w1);
-      store_pair(out + (size_t)r * a.ld + c, (S)w0, (S)w1);
-    });
-    CTRACE(k, 3);
-    if (!s_pf && warp == 7) {
-      const bool ok = warp_wait_geq(a, a.upd + (k + 1) * nt + k + 1, k);
-      if (ok) {
-        fetch_tile_warp<T, S>(tile<S>(a, k + 1, k + 1), a.ld, N);
+        fetch_tile_warp(tile<S>(a, k + 1, k), a.ld, C);
         cp_async_wait_all();
       } else if (lane == 0) {
         *s_ok = 0;
       }
     }
+    TRACE(2, a.ntasks + 2 * k);
+    CTRACE(k, 1);
     __syncthreads();
-    if (!*s_ok) return;
-    CTRACE(k, 4);
-    if (threadIdx.x == 32 * 7) st_release(a.fin + (k + 1) * nt + k, 1);
-    TRACE(2, a.ntasks + 2 * k + 1);
-    syrk_lower(N, L, A);
+    if (threadIdx.x == 32 * RELEASE_WARP) st_release(a.fin + k * nt + k, 1);
+    if (!*s_ok || k + 1 == nt) return;
+    TRACE(0, a.ntasks + 2 * k + 1);
+    TRACE(3, a.ntasks + 2 * k + 1);
+    TRACE(1, a.ntasks + 2 * k + 1);
+    CTRACE(k, 2);
+    if (warp < 4) {
+      S* out = tile<S>(a, k + 1, k);
+      solve_rows<2>(C, LS, V, [&](int r, int c, double w0, double w1) {
+        store_pair(L + r * LT + c, w0, w1);
+        store_pair(out + (size_t)r * a.ld + c, (S)w0, (S)w1);
+      });
+      CTRACE(k, 3);
+      bar_wait(5, 160);
+      CTRACE(k, 4);
+      TRACE(2, a.ntasks + 2 * k + 1);
+      syrk_lower(N, L, A, [] { bar_wait(6, 160); });
+    } else if (warp == RELEASE_WARP) {
+      bar_wait(5, 160);
+      if (lane == 0) st_release(a.fin + (k + 1) * nt + k, 1);
+    } else if (warp == FETCH_WARP) {
+      if (lane == 0) f.bad[1] = 0;
+      if (warp_wait_geq(a, next, k)) {
+        fetch_tile_warp(tile<S>(a, k + 1, k + 1), a.ld, N);
+        cp_async_wait_all();
+      } else if (lane == 0) {
+        *s_ok = 0;
+      }
+      bar_arrive(6, 160);
+    }
     __syncthreads();
     CTRACE(k, 5);
+    if (!*s_ok) return;
   }
 }
 
-// ---------------------------------------------------------------- FP32 chain
-// The mixed path's chain CTA factors, inverts and solves in FP32: the
-// diagonal tiles of a well-conditioned FP32 matrix lose nothing to FP32
-// pivots that FP32 storage and the 3xTF32 updates have not already cost,
-// while every step of the panel chain gets shorter (MUFU rsqrt instead of
-// a refined FP64 rsqrt, FP32 FMA latency, no FP64 conversion).
-
-// Named barrier arrival without waiting (orders the calling threads' earlier
-// shared-memory accesses before the barrier completes; see bar_wait).
-__device__ __forceinline__ void bar_arrive(int id, int count) {
-  __syncwarp();
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
+// ---------------------------------------------------------------- FP32 diagonal tiles
+// The mixed batch factors, inverts and solves its diagonal tiles in FP32: the
+// tiles of a well-conditioned FP32 matrix lose nothing to FP32
+// pivots that FP32 storage and the 3xTF32 updates have not already cost.
 
 // T[r][c] -= sum_q T[r][c0+q] T[c][c0+q] (q = 0..7, in order): the rank-8
 // update of one trailing element with the factored panel c0..c0+7.
@@ -1388,7 +1334,7 @@ __device__ __forceinline__ void panel_update(float* T, int r, int c, int c0) {
   T[r * LDA + c] = v;
 }
 
-// F(k) of the FP32 chain on the tile T (smem [64][LDA]: lower triangle valid
+// F(k) of the mixed batch on the tile T (smem [64][LDA]: lower triangle valid
 // with every update applied; the caller's writes end with a CTA barrier).
 // Eight 8-column panels.  Warp 0 factors panel p -- the 8 x 8 pivot block in
 // every lane's registers (the pivot chain is rsqrt -> multiply -> FMA) and
@@ -1529,7 +1475,7 @@ __device__ __forceinline__ void store_factor_inverse(const DFArgs& a, int k, con
 constexpr size_t factor_task_f32_smem_bytes() { return sizeof(float) * (2 * NB * LDA + 32 * 36 + NB); }
 
 // F(k) as a list task of the batched mixed factorisation: the updated tile
-// (acc) factored and inverted in FP32 exactly as the FP32 chain does, L_kk
+// (acc) factored and inverted in FP32, L_kk
 // and inv(L_kk) stored; the caller publishes.  smem is free on entry.
 __device__ __forceinline__ void factor_task_f32(const DFArgs& a, int k, const float acc[16], unsigned char* smem) {
   float* T = reinterpret_cast<float*>(smem);
@@ -1879,10 +1825,13 @@ __device__ bool lead_task(const DFArgs& a, int k, T* s, int* s_ok) {
   cp_async_wait_all();
   __syncthreads();
   T* out = tile<T>(a, i, k);
-  solve_rows(Li, LDA, sV, [&](int r, int c, T w0, T w1) {
+  solve_rows_t<T>(Li, LDA, sV, [&](int r, int c, T w0, T w1) {
     store_pair(Li + r * LDA + c, w0, w1);
     store_pair(out + (size_t)r * a.ld + c, w0, w1);
   });
+  // at once: the updates of row k + 2 that the next LEAD starts from wait for it
+  __syncthreads();
+  if (threadIdx.x == 32) st_release(a.fin + i * nt + k, 1);
   if (!wait_geq(a, a.fin + (k + 1) * nt + k, 1, s_ok)) return false;
   stage_async(tile<T>(a, k + 1, k), a.ld, sB, LDA);
   smem_to_acc(sC, acc);
@@ -1892,7 +1841,6 @@ __device__ bool lead_task(const DFArgs& a, int k, T* s, int* s_ok) {
   store_acc(tile<T>(a, i, k + 1), a.ld, acc);
   __syncthreads();
   if (threadIdx.x == 0) st_release(a.upd + i * nt + k + 1, k + 1);
-  if (threadIdx.x == 32) st_release(a.fin + i * nt + k, 1);
   smem_to_acc(sD, acc);
   TileMMA<T>::sub(Li, Li, acc);
   store_acc(tile<T>(a, i, i), a.ld, acc);
@@ -2024,7 +1972,7 @@ __device__ void df_worker_loop(const DFArgs& a, unsigned char* smem, int* s_task
       cp_async_wait_all();
       __syncthreads();
       T* out = tile<T>(a, i, j);
-      solve_rows(sA, LDA, sB, [&](int r, int c, T w0, T w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
+      solve_rows_t<T>(sA, LDA, sB, [&](int r, int c, T w0, T w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
       publish(a.fin + i * nt + j, 1);
       TRACE(2, t);
     }
@@ -2032,15 +1980,14 @@ __device__ void df_worker_loop(const DFArgs& a, unsigned char* smem, int* s_task
   }
 }
 
-// A matrix of type T; the chain CTA works in CT (FP64 for a FP32 matrix in
-// PBG_PREC_MIXED_FP64_DIAG).  The FP32 workers hold TMEM for their tensor-core
+// A matrix of type T; the chain CTA works in FP64.  The FP32 workers hold TMEM for their tensor-core
 // updates from start to end.
-template <typename T, typename CT>
+template <typename T>
 __global__ void __launch_bounds__(THREADS, 1) chol_df_kernel(DFArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_task, s_ok;
   if (blockIdx.x == 0) {
-    run_chain<CT, T>(a, smem, &s_ok);
+    run_chain<T>(a, smem, &s_ok);
     return;
   }
   if constexpr (sizeof(T) == 4) {
@@ -2062,7 +2009,7 @@ __global__ void __launch_bounds__(THREADS, 1) chol_df_kernel(DFArgs a) {
 // (L_kk, inverse) over the same bytes and the factor scratch after them.
 constexpr size_t batch_smem_bytes() {
   // an F task's tile, solve blocks and factor scratch, or a paired update's five tiles
-  return std::max(sizeof(double) * (2 * NB * ChainLd<double>::LT + factor_scratch_elems<double>()),
+  return std::max(sizeof(double) * (2 * NB * ChainLd<double>::LT + FACTOR_SCRATCH),
                   5 * NB * LDA * sizeof(double));
 }
 
@@ -2076,7 +2023,7 @@ __device__ void batch_worker_loop(const CholRep* __restrict__ reps, const int4* 
   T* sB = sA + NB * LDA;
   constexpr int LT = ChainLd<T>::LT;
   T* Ft = reinterpret_cast<T*>(smem);  // F: the tile, its solve blocks, the scratch
-  const FactorMem<T> f(Ft, Ft + NB * LT, Ft + 2 * NB * LT);
+  const FactorMem f(Ft, Ft + NB * LT, Ft + 2 * NB * LT);
   while (true) {
     if (threadIdx.x == 0) s_task = ld_acquire(ctl + 1) ? ntasks : atomicAdd(ctl, 1);
     __syncthreads();
@@ -2133,11 +2080,11 @@ __device__ void batch_worker_loop(const CholRep* __restrict__ reps, const int4* 
       if (type == TASK_F) {
         acc_to_smem(acc, Ft, LT);
         if (threadIdx.x == 0) {
-          f.w[0] = 0;
-          f.w[1] = NB;
+          f.bad[0] = NB;
+          f.bad[1] = 0;
         }
         __syncthreads();
-        factor_tile<T, T>(a, col, f, reinterpret_cast<T*>(a.lp) + (size_t)col * NB * NB);
+        factor_tile<T>(a, col, f, reinterpret_cast<T*>(a.lp) + (size_t)col * NB * NB);
       } else {
         if (!wait_geq(a, a.fin + col * nt + col, 1, &s_ok)) return;
         stage_async(reinterpret_cast<const T*>(a.lp) + (size_t)col * NB * NB, NB, sB, LT);
@@ -2145,7 +2092,7 @@ __device__ void batch_worker_loop(const CholRep* __restrict__ reps, const int4* 
         cp_async_wait_all();
         __syncthreads();
         T* out = tile<T>(a, i, col);
-        solve_rows(sA, LDA, sB, [&](int r, int c, T w0, T w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
+        solve_rows_t<T>(sA, LDA, sB, [&](int r, int c, T w0, T w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
       }
       publish(a.fin + i * nt + col, 1);
     }
@@ -2172,8 +2119,7 @@ __global__ void __launch_bounds__(THREADS, 1) chol_batch_kernel(const CholRep* _
 // shared memory and three MMAs per K-step add A_hi B_hi + A_hi B_lo + A_lo
 // B_hi to the accumulator, while the tiles of k + 1 and k + 2 are on their
 // way (cp.async into two raw FP32 stages).  Then, by the task's kind:
-//   LL_DIAG (i = j): F(j) -- L_jj and inv(L_jj) in FP32, as the FP32 chain
-//     forms them -- published at once, then S(j + 1, j) = U inv(L_jj)^T with
+//   LL_DIAG (i = j): F(j) -- L_jj and inv(L_jj) in FP32 -- published at once, then S(j + 1, j) = U inv(L_jj)^T with
 //     the inverse still in shared memory;
 //   LL_UPDATE (i > j): U written over A's tiles, upd[r] = j + 1;
 //   LL_SOLVE (i > j, a later segment): S(i, j), S(i + 1, j) from the stored
@@ -2718,21 +2664,21 @@ int get_task_table(int nt, int group, bool inv_tasks, bool inverse, const int4**
   return PBG_OK;
 }
 
-template <typename T, typename CT>
+template <typename T>
 size_t df_smem_bytes() {
   // the chain, a LEAD task, or a grouped update (the tensor-core operands in
   // FP32, five tiles in FP64)
-  return std::max({chain_smem_bytes<CT>(), lead_smem_bytes<T>(),
+  return std::max({chain_smem_bytes<T>(), lead_smem_bytes<T>(),
                    sizeof(T) == 4 ? tc_worker_smem_bytes(2) : 5 * NB * LDA * sizeof(T)});
 }
 
 // tasks_override / spin_limit: only for the wait-expiry self-test.
 // inv_tasks: inv(L_kk) goes to invdiag.  X (or null): also form X = inv(L)
 // (off-diagonal tiles); ints then holds the X flags after the factorisation's.
-template <typename T, typename CT>
+template <typename T>
 int launch_df(T* A, int n, int ld, int* info, void* invdiag, bool inv_tasks, int* ints, void* lp, unsigned* err,
               cudaStream_t st, const int4* tasks_override = nullptr, int ntasks_override = 0,
-              long long spin_limit = SPIN_LIMIT, T* X = nullptr) {
+              long long spin_limit = SPIN_LIMIT, T* X = nullptr, double min_pivot = 0.0) {
   const int nt = ld / NB;
   const int4* tasks = nullptr;
   int ntasks = 0;
@@ -2743,16 +2689,16 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, bool inv_tasks, int
     int rc = get_task_table(nt, sizeof(T) == 4 ? 4 : 2, inv_tasks || X, X != nullptr, &tasks, &ntasks);
     if (rc) return rc;
   }
-  const size_t smem = df_smem_bytes<T, CT>();
+  const size_t smem = df_smem_bytes<T>();
   static int max_blocks_per_sm = -1;
   static int num_sms = 0;
   if (max_blocks_per_sm < 0) {
-    PBG_CUDA_TRY(cudaFuncSetAttribute(chol_df_kernel<T, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    PBG_CUDA_TRY(cudaFuncSetAttribute(chol_df_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     int dev;
     PBG_CUDA_TRY(cudaGetDevice(&dev));
     PBG_CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-    PBG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_blocks_per_sm, chol_df_kernel<T, CT>,
+    PBG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_blocks_per_sm, chol_df_kernel<T>,
                                                                THREADS, smem));
     if (max_blocks_per_sm < 1) {
       pbg_set_error_message("cholesky kernel does not fit on an SM");
@@ -2782,6 +2728,7 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, bool inv_tasks, int
   args.lp = lp;
   args.err = err;
   args.spin_limit = spin_limit;
+  args.min_pivot = min_pivot;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(THREADS);
@@ -2792,7 +2739,7 @@ int launch_df(T* A, int n, int ld, int* info, void* invdiag, bool inv_tasks, int
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  PBG_CUDA_TRY(cudaLaunchKernelEx(&cfg, chol_df_kernel<T, CT>, args));
+  PBG_CUDA_TRY(cudaLaunchKernelEx(&cfg, chol_df_kernel<T>, args));
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
@@ -2847,7 +2794,7 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
     cudaMemcpy(A, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(dt, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemset(err, 0, sizeof(unsigned));
-    result = launch_df<double, double>(A, n, ld, info, nullptr, false, ints, lp, err, 0, dt, (int)tasks.size(), spin_limit);
+    result = launch_df<double>(A, n, ld, info, nullptr, false, ints, lp, err, 0, dt, (int)tasks.size(), spin_limit);
     if (result == PBG_OK && cudaDeviceSynchronize() != cudaSuccess) result = PBG_ERR_CUDA;
     if (result == PBG_OK) {
       cudaMemcpy(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost);
@@ -2860,7 +2807,7 @@ extern "C" __attribute__((visibility("default"))) int pbg_selftest_wait_expiry(l
       // the context is still usable: the full task list factors the matrix
       cudaMemcpy(A, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
       cudaMemset(err, 0, sizeof(unsigned));
-      result = launch_df<double, double>(A, n, ld, info, nullptr, false, ints, lp, err, 0);
+      result = launch_df<double>(A, n, ld, info, nullptr, false, ints, lp, err, 0);
       if (result == PBG_OK && cudaDeviceSynchronize() != cudaSuccess) result = PBG_ERR_CUDA;
       if (result == PBG_OK) {
         cudaMemcpy(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost);
@@ -2916,13 +2863,11 @@ int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* i
   unsigned* err = reinterpret_cast<unsigned*>(ints + 3 + 4 * (size_t)nt * nt);
   void* lp = static_cast<unsigned char*>(work) + df_flag_bytes(nt);
   if (precision == PBG_PREC_FP64)
-    return launch_df<double, double>((double*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0,
+    return launch_df<double>((double*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0,
                                      SPIN_LIMIT, (double*)X);
-  if (precision == PBG_PREC_MIXED_FP64_DIAG)
-    return launch_df<float, double>((float*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0,
-                                    SPIN_LIMIT, (float*)X);
-  return launch_df<float, float>((float*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0, SPIN_LIMIT,
-                                 (float*)X);
+  // PBG_PREC_MIXED reports a pivot below the smallest normal float as non-positive
+  return launch_df<float>((float*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0, SPIN_LIMIT, (float*)X,
+                          precision == PBG_PREC_MIXED_FP64_DIAG ? 0.0 : 1.17549435e-38);
 }
 
 
