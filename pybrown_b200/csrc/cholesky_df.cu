@@ -14,7 +14,7 @@
 //            3xTF32 split products (hi*hi + hi*lo + lo*hi) on the tcgen05
 //            tensor cores, up to four rows per task, accumulated in TMEM
 //            (tc_tile.cuh);
-//   LEAD(k)  row k+2 of panel k: S(k+2, k), U(k+2, k+1, k), U(k+2, k+2, k) as
+//   LEAD(k, h) half h of row k+2 of panel k: S(k+2, k), U(k+2, k+1, k) as
 //            one task, because the chain waits for them;
 //   I(k)     inv(L_kk), only when the caller wants the inverted diagonal tiles.
 // The diagonal tiles are factored in FP64 in every path, in the mixed path (FP32
@@ -65,8 +65,8 @@ enum : int { TASK_F = 0, TASK_S = 1, TASK_U = 2, TASK_I = 3, TASK_U2 = 4, TASK_U
 // XG / XZ: the tasks that form X = inv(L) in the same list (single-matrix
 // lists of an SPD inverse only; see inverse_update / inverse_finish).
 enum : int { TASK_XG = 7, TASK_XZ = 8 };
-// LEAD(k): the tile row k + 2 of panel k, on which the chain's next step waits
-// (lead_task).
+// LEAD(k, h): half of the tile row k + 2 of panel k, on which the chain's next
+// step waits (lead_task).
 enum : int { TASK_LEAD = 9 };
 
 struct DFArgs {
@@ -600,7 +600,7 @@ __device__ __forceinline__ void acc_to_smem(const T acc[16], T* s, int lds = LDA
 // chain warp on its own (420 ns a block: 190 ns its eight reciprocal steps, the rest the
 // hand-over of D, U and X through shared memory and registers), against 7.7 us
 // (FP64) and 7.0 (FP32) with rows in lanes and one barrier of five warps per
-// block; a chain step, F to F, 10.4 us against 13.5 and 12.2.  An FP32 variant
+// block; a chain step, F to F, 9.7 us against 13.5 and 12.2.  An FP32 variant
 // would save reciprocal latency but pay for its products on the FMA pipe, so
 // FP32 matrices are factored in FP64 too and rounded once on store.
 
@@ -1129,6 +1129,12 @@ __device__ __forceinline__ void solve_rows_f32(const float* C, int ldc, const fl
   }
 }
 
+// 32 rows (rows of LDA) by the first four warps.
+template <typename T, typename F>
+__device__ __forceinline__ void solve_half(const T* C, const T* V, F out) {
+  if constexpr (sizeof(T) == 8) solve_rows<1>(C, LDA, V, out);
+  else if (threadIdx.x < 64) solve_rows_f32(C, LDA, V, out);
+}
 template <typename T, typename F>
 __device__ __forceinline__ void solve_rows_t(const T* C, int ldc, const T* V, F out) {
   if constexpr (sizeof(T) == 8) solve_rows<1>(C, ldc, V, out);
@@ -1790,61 +1796,142 @@ __device__ bool solve_input(const DFArgs& a, int i, int j, T acc[16], T* sA, T* 
   return true;
 }
 
-// Shared memory of a worker's LEAD task: five tiles.
-template <typename T>
-constexpr size_t lead_smem_bytes() { return sizeof(T) * 5 * NB * ChainLd<T>::LT; }
-
-// LEAD(k), the row i = k + 2 of panel k: S(i, k), then U(i, k+1, k) -- the last
-// update of the chain's next solve input -- and U(i, i, k), with L(i, k) kept
-// in shared memory in between.  Everything that does not need L_kk is done
-// before the wait for it (the last update of A(i, k), the fetch of both
-// targets), so that from F(k) to the chain's input there are one solve, one
-// product and two hand-overs: as separate tasks (solve through an inverse
-// formed by a third task) the chain waited 3 to 16 us for them.
-template <typename T>
-__device__ bool lead_task(const DFArgs& a, int k, T* s, int* s_ok) {
-  constexpr int LT = ChainLd<T>::LT;
-  const int nt = a.nt, i = k + 2;
-  T* Li = s;             // A(i, k), then L(i, k)
-  T* sV = s + NB * LT;   // the solve blocks of L_kk
-  T* sB = sV + NB * LT;  // L(k+1, k)
-  T* sC = sB + NB * LT;  // A(i, k+1)
-  T* sD = sC + NB * LT;  // A(i, i)
-  T acc[16];
-  if (!solve_input<T>(a, i, k, acc, sV, sB, s_ok)) return false;
-  acc_to_smem(acc, Li);
-  if (k > 0) {
-    const int* fl[2] = {a.upd + i * nt + k + 1, a.upd + i * nt + i};
-    const int tg[2] = {k, k};
-    if (!wait_all(a, fl, tg, 2, s_ok)) return false;
+// A B^T of a LEAD task: A 32 rows, B 64 rows (smem rows of LDA), 64 deep.  Warp w
+// owns rows 16 (w / 4) .. and columns 16 (w % 4) .. of the 32 x 64 product;
+// element 4 mt + 2 nt + h of `d` is row 8 mt + lane / 4, column 8 nt + 2 (lane % 4)
+// + h of them (half_at).
+__device__ __forceinline__ int half_row(int mt) { return 16 * (threadIdx.x >> 7) + 8 * mt + ((threadIdx.x & 31) >> 2); }
+__device__ __forceinline__ int half_col(int nt) { return 16 * ((threadIdx.x >> 5) & 3) + 8 * nt + 2 * (threadIdx.x & 3); }
+__device__ __forceinline__ void half_product(const double* sA, const double* sB, double (&d)[8]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const double* A = sA + (16 * (w >> 2) + g) * LDA + t;
+  const double* B = sB + (16 * (w & 3) + g) * LDA + t;
+  double c[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, e[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+#pragma unroll 4
+  for (int k0 = 0; k0 < NB; k0 += 8)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      dmma(c[q], A[8 * (q >> 1) * LDA + k0], B[8 * (q & 1) * LDA + k0]);
+      dmma(e[q], A[8 * (q >> 1) * LDA + k0 + 4], B[8 * (q & 1) * LDA + k0 + 4]);
+    }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    d[2 * q] = c[q][0] + e[q][0];
+    d[2 * q + 1] = c[q][1] + e[q][1];
   }
-  stage_async(tile<T>(a, i, k + 1), a.ld, sC, LDA);
-  stage_async(tile<T>(a, i, i), a.ld, sD, LDA);
+}
+__device__ __forceinline__ void half_product(const float* sA, const float* sB, float (&d)[8]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const float* A = sA + (16 * (w >> 2) + g) * LDA + t;
+  const float* B = sB + (16 * (w & 3) + g) * LDA + t;
+  float c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, e[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll 2
+  for (int k0 = 0; k0 < NB; k0 += 8) {
+    unsigned ah[4], al[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) split_tf32(A[8 * (q & 1) * LDA + k0 + 4 * (q >> 1)], ah[q], al[q]);
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      unsigned bh[2], bl[2];
+      split_tf32(B[8 * n * LDA + k0], bh[0], bl[0]);
+      split_tf32(B[8 * n * LDA + k0 + 4], bh[1], bl[1]);
+      tf32_mma(c[n], ah, bh);
+      tf32_mma(e[n], al, bh);
+      tf32_mma(e[n], ah, bl);
+    }
+  }
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) d[4 * mt + 2 * n + h] = c[n][2 * mt + h] + e[n][2 * mt + h];
+}
+// 32 rows of a tile, as stage_async.
+template <typename T>
+__device__ __forceinline__ void stage_half(const T* g, int ld, T* s) {
+  constexpr int per_row = NB * (int)sizeof(T) / 16, elems = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int q = 0; q < 32 * per_row / THREADS; ++q) {
+    const int t = threadIdx.x + q * THREADS, r = t / per_row, c = (t % per_row) * elems;
+    cp_async16(s + r * LDA + c, g + (size_t)r * ld + c);
+  }
+}
+// The second of two halves to arrive sets the flag: its counter's
+// acquire-release and the flag's release order both halves' stores before it.
+__device__ __forceinline__ void publish_half(int* counter, int* flag, int value) {
+  int old;
+  asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+  if (old == 1) st_release(flag, value);
+}
+
+// Shared memory of a worker's LEAD task: two tiles and two halves.
+template <typename T>
+constexpr size_t lead_smem_bytes() { return sizeof(T) * (NB * ChainLd<T>::LT + 2 * NB * LDA); }
+
+// LEAD(k, h), rows 32 h .. 32 h + 31 of the tile row i = k + 2 of panel k: S(i, k),
+// then U(i, k+1, k) -- the last update of the chain's next solve input -- with
+// the rows of L(i, k) kept in shared memory in between.  Everything that does
+// not need L_kk is done before the wait for it (the last update of A(i, k), the
+// fetch of the target), so that from F(k) to the chain's input there are one
+// solve, one product and two hand-overs.  The row is two tasks because both are
+// bound by one SM's FP64 tensor pipe (a 64-row solve 1.6 us, a 64-row product
+// 2.1 us): at order 1000 in FP64 the chain no longer waits, 174 us against 188.  The counters of the two
+// halves are the flags of tile (k, k + 2), which is above the diagonal.
+template <typename T>
+__device__ bool lead_task(const DFArgs& a, int k, int h, T* s, int* s_ok) {
+  constexpr int LT = ChainLd<T>::LT;
+  const int nt = a.nt, i = k + 2, ld = a.ld;
+  T* Li = s;                 // rows of A(i, k), then of L(i, k)
+  T* sC = Li + 32 * LDA;     // rows of A(i, k+1)
+  T* sB = sC + 32 * LDA;     // L(k, k-1), then L(k+1, k)
+  T* sV = sB + NB * LDA;     // the solve blocks of L_kk
+  auto rows = [&](int j) { return tile<T>(a, i, j) + (size_t)32 * h * ld; };
+  T d[8];
+  if (k > 0) {
+    const int* fl[4] = {a.fin + i * nt + k - 1, a.fin + k * nt + k - 1, a.upd + i * nt + k, a.upd + i * nt + k + 1};
+    const int tg[4] = {1, 1, k - 1, k};
+    if (!wait_all(a, fl, tg, 3, s_ok)) return false;
+    stage_half(rows(k), ld, Li);
+    stage_half(rows(k - 1), ld, sC);
+    stage_async(tile<T>(a, k, k - 1), ld, sB, LDA);
+    cp_async_wait_all();
+    __syncthreads();
+    half_product(sC, sB, d);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) Li[half_row(q >> 2) * LDA + half_col((q >> 1) & 1) + (q & 1)] -= d[q];
+    if (!wait_geq(a, fl[3], tg[3], s_ok)) return false;  // (its barrier: sC is read)
+  } else {
+    stage_half(rows(0), ld, Li);
+  }
+  stage_half(rows(k + 1), ld, sC);
   if (!wait_geq(a, a.fin + k * nt + k, 1, s_ok)) return false;
   stage_async(reinterpret_cast<const T*>(a.lp) + (size_t)k * NB * NB, NB, sV, LT);
   cp_async_wait_all();
   __syncthreads();
-  T* out = tile<T>(a, i, k);
-  solve_rows_t<T>(Li, LDA, sV, [&](int r, int c, T w0, T w1) {
-    store_pair(Li + r * LDA + c, w0, w1);
-    store_pair(out + (size_t)r * a.ld + c, w0, w1);
-  });
-  // at once: the updates of row k + 2 that the next LEAD starts from wait for it
+  T* out = rows(k);
+  if (threadIdx.x < 128)  // 32 rows: warps 0 .. 3 (FP64), 0 and 1 of them in FP32
+    solve_half<T>(Li, sV, [&](int r, int c, T w0, T w1) {
+      store_pair(Li + r * LDA + c, w0, w1);
+      store_pair(out + (size_t)r * ld + c, w0, w1);
+    });
   __syncthreads();
-  if (threadIdx.x == 32) st_release(a.fin + i * nt + k, 1);
+  // at once: the updates of row k + 2 that the next LEAD starts from wait for it
+  int* counter = a.fin + k * nt + i;
+  if (threadIdx.x == 32) publish_half(counter, a.fin + i * nt + k, 1);
   if (!wait_geq(a, a.fin + (k + 1) * nt + k, 1, s_ok)) return false;
-  stage_async(tile<T>(a, k + 1, k), a.ld, sB, LDA);
-  smem_to_acc(sC, acc);
+  stage_async(tile<T>(a, k + 1, k), ld, sB, LDA);
   cp_async_wait_all();
   __syncthreads();
-  TileMMA<T>::sub(Li, sB, acc);
-  store_acc(tile<T>(a, i, k + 1), a.ld, acc);
+  half_product(Li, sB, d);
+  T* o = rows(k + 1);
+#pragma unroll
+  for (int q = 0; q < 8; q += 2) {
+    const int r = half_row(q >> 2), c = half_col((q >> 1) & 1);
+    store_pair(o + (size_t)r * ld + c, sC[r * LDA + c] - d[q], sC[r * LDA + c + 1] - d[q + 1]);
+  }
   __syncthreads();
-  if (threadIdx.x == 0) st_release(a.upd + i * nt + k + 1, k + 1);
-  smem_to_acc(sD, acc);
-  TileMMA<T>::sub(Li, Li, acc);
-  store_acc(tile<T>(a, i, i), a.ld, acc);
-  publish(a.upd + i * nt + i, k + 1);
+  if (threadIdx.x == 0) publish_half(a.upd + k * nt + i, a.upd + i * nt + k + 1, k + 1);
   return true;
 }
 
@@ -1959,7 +2046,7 @@ __device__ void df_worker_loop(const DFArgs& a, unsigned char* smem, int* s_task
       }
       TRACE(2, t);
     } else if (type == TASK_LEAD) {
-      if (!lead_task<T>(a, k, sA, &s_ok)) return;
+      if (!lead_task<T>(a, k, i, sA, &s_ok)) return;
       TRACE(2, t);
     } else {
       // S(i, j), i >= j + 3: the tile after its last update, times L_jj^-T
@@ -2612,11 +2699,15 @@ std::vector<int4> df_task_list(int nt, int group, bool inv_tasks, bool inverse) 
       t.push_back(make_int4(TASK_U, k + 2, k + 1, q));
       t.push_back(make_int4(TASK_U, k + 2, k + 2, q));
     }
-    if (k + 2 < nt) t.push_back(make_int4(TASK_LEAD, 0, 0, k));
+    if (k + 2 < nt) {
+      t.push_back(make_int4(TASK_LEAD, 0, 0, k));
+      t.push_back(make_int4(TASK_LEAD, 1, 0, k));
+      t.push_back(make_int4(TASK_U, k + 2, k + 2, k));  // the chain's next diagonal tile
+    }
     for (int i = k + 3; i < nt; ++i) t.push_back(make_int4(TASK_S, i, k, k));
     if (inv_tasks) t.push_back(make_int4(TASK_I, 0, 0, k));
     // Column k of the update with panel q is fused into F(k), LEAD(k) and the
-    // S(., k); U(k+1, k, q) and U(k+1, k+1, q) belong to LEAD(q).  The plain
+    // S(., k); U(k+1, k, q) belongs to LEAD(q) and U(k+1, k+1, q) follows it.  The plain
     // updates cover the rest, columns from the left (rows grouped:
     // U(i, jj, q), U(i+1, jj, q), ... share L(jj, q)).
     if (k > 0)
