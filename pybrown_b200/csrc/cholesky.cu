@@ -74,7 +74,24 @@ int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStre
   int rc = launch_cholesky_df(A, n, ld, PBG_PREC_FP64, info, inv, true, w + (size_t)nt * NB * NB * sizeof(double), st,
                               X);
   if (rc != PBG_OK) return rc;
-  return launch_lauum(X, inv, ld, scale, A, st);
+  return launch_lauum(X, inv, ld, scale, false, A, st);
+}
+
+int launch_spd_inverse_reversed(double* G, int ld, int* info, void* work, cudaStream_t st, double scale, double* out) {
+  const int nt = ld / NB;
+  unsigned char* w = static_cast<unsigned char*>(work);
+  double* inv = reinterpret_cast<double*>(w);
+  double* X = reinterpret_cast<double*>(w + spd_x_offset(ld));
+  int rc = launch_cholesky_df(G, ld, ld, PBG_PREC_FP64, info, inv, true, w + (size_t)nt * NB * NB * sizeof(double), st,
+                              X);
+  if (rc != PBG_OK) return rc;
+  return launch_lauum(X, inv, ld, scale, true, out, st);
+}
+
+int launch_reversed_factor(double* G, int ld, double s, const void* work, double* invdiag, cudaStream_t st) {
+  const unsigned char* w = static_cast<const unsigned char*>(work);
+  return launch_reversed_factor_tiles<double>(reinterpret_cast<const double*>(w + spd_x_offset(ld)),
+                                              reinterpret_cast<const double*>(w), G, ld, s, G, invdiag, st);
 }
 
 }  // namespace pbg

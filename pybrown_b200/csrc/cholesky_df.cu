@@ -3125,14 +3125,16 @@ __global__ void __launch_bounds__(THREADS) trtri_diag_kernel(const T* __restrict
 }
 
 // out_IJ = scale (X^T X)_IJ = scale sum_{k >= I} X_kI^T X_kJ for the lower
-// tile (I, J), written to (I, J) and (J, I); FP64.  Off-diagonal tiles come from
+// tile (I, J), written to (I, J) and (J, I), with `reversed` every element (r, c) to
+// (ld-1-r, ld-1-c); FP64.  Off-diagonal tiles come from
 // X, the diagonal ones from invdiag.  Bound by the FP64 tensor pipe (2.1 us per
 // 64^3 product and SM): the tiles are used as they lie in memory (sub_rows),
 // two K-steps in flight by cp.async; the CTAs with the longest K range start
 // first.  Order 1536: 118 us with transposing copies through registers, 69 now.
 constexpr size_t lauum_smem_bytes() { return 4 * NB * LDA * sizeof(double); }
 __global__ void __launch_bounds__(THREADS) lauum_kernel(const double* __restrict__ X, const double* __restrict__ invdiag,
-                                                        int ld, int nt, double scale, double* __restrict__ out) {
+                                                        int ld, int nt, double scale, int reversed,
+                                                        double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem[];
   double* st = reinterpret_cast<double*>(smem);  // [2][2][64][LDA]
   const int b = blockIdx.x;
@@ -3170,7 +3172,11 @@ __global__ void __launch_bounds__(THREADS) lauum_kernel(const double* __restrict
 #pragma unroll
     for (int cs = 0; cs < 8; ++cs) {
       const double v = -acc[TileMMA<double>::idx(rs, cs)] * scale;
-      const int r = I * NB + acc_row(rs), c = J * NB + acc_col(cs);
+      int r = I * NB + acc_row(rs), c = J * NB + acc_col(cs);
+      if (reversed) {
+        r = ld - 1 - r;
+        c = ld - 1 - c;
+      }
       out[(size_t)r * ld + c] = v;
       if (I != J) out[(size_t)c * ld + r] = v;  // a diagonal tile writes each element once
     }
@@ -3179,12 +3185,17 @@ __global__ void __launch_bounds__(THREADS) lauum_kernel(const double* __restrict
 // B[i][j] = scale X[ld-1-j][ld-1-i] for the lower triangle of B (32 x 32
 // tiles through smem; tiles above the diagonal are not written).
 template <typename T>
-__global__ void reversed_transpose_kernel(const T* __restrict__ X, int ld, T scale, T* __restrict__ B) {
+__global__ void reversed_transpose_kernel(const T* __restrict__ X, const T* __restrict__ Xdiag, int ld, T scale,
+                                          T* __restrict__ B) {
   __shared__ T t[32][33];
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bj > bi) return;
   const int x0r = ld - 32 * (bj + 1), x0c = ld - 32 * (bi + 1);
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) t[r][threadIdx.x] = X[(size_t)(x0r + r) * ld + x0c + threadIdx.x];
+  // a block within a diagonal tile of X
+  const bool diag = Xdiag && x0r / NB == x0c / NB;
+  const T* src = diag ? Xdiag + (size_t)(x0r / NB) * NB * NB + (x0r % NB) * NB + x0c % NB : X + (size_t)x0r * ld + x0c;
+  const size_t lds = diag ? NB : ld;
+  for (int r = threadIdx.y; r < 32; r += blockDim.y) t[r][threadIdx.x] = src[r * lds + threadIdx.x];
   __syncthreads();
   for (int rr = threadIdx.y; rr < 32; rr += blockDim.y)
     B[(size_t)(bi * 32 + rr) * ld + bj * 32 + threadIdx.x] = scale * t[31 - threadIdx.x][31 - rr];
@@ -3370,11 +3381,13 @@ int launch_trtri_diag(const float* invdiag, float* X, int ld, cudaStream_t st) {
   return PBG_OK;
 }
 
-int launch_lauum(const double* X, const double* invdiag, int ld, double scale, double* out, cudaStream_t st) {
+int launch_lauum(const double* X, const double* invdiag, int ld, double scale, bool reversed, double* out,
+                 cudaStream_t st) {
   if (ld % NB != 0 || ld <= 0) return PBG_ERR_ARG;
   const int nt = ld / NB;
   PBG_CUDA_TRY(cudaFuncSetAttribute(lauum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lauum_smem_bytes()));
-  lauum_kernel<<<nt * (nt + 1) / 2, THREADS, lauum_smem_bytes(), st>>>(X, invdiag, ld, nt, scale, out);
+  lauum_kernel<<<nt * (nt + 1) / 2, THREADS, lauum_smem_bytes(), st>>>(X, invdiag, ld, nt, scale, reversed ? 1 : 0,
+                                                                    out);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
@@ -3422,14 +3435,22 @@ int tc_lauum(const float* X, int ld, float scale, bool reversed, float* out, int
   return PBG_OK;
 }
 
-int tc_reversed_factor(const float* X, const float* G, int ld, double s, float* B, float* invdiag,
-                       cudaStream_t st) {
-  const int nt = ld / NB;
-  reversed_transpose_kernel<float><<<dim3(ld / 32, ld / 32), dim3(32, 8), 0, st>>>(X, ld, (float)s, B);
+template <typename T>
+int launch_reversed_factor_tiles(const T* X, const T* Xdiag, const T* G, int ld, double s, T* B, T* invdiag,
+                                 cudaStream_t st) {
+  // first what reads G, which B may overwrite
+  b_invdiag_kernel<T><<<ld / NB, THREADS, 0, st>>>(G, ld, ld / NB, (T)(1.0 / s), invdiag);
   PBG_CHECK_LAUNCH();
-  b_invdiag_kernel<float><<<nt, THREADS, 0, st>>>(G, ld, nt, (float)(1.0 / s), invdiag);
+  reversed_transpose_kernel<T><<<dim3(ld / 32, ld / 32), dim3(32, 8), 0, st>>>(X, Xdiag, ld, (T)s, B);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
+}
+template int launch_reversed_factor_tiles<double>(const double*, const double*, const double*, int, double, double*,
+                                                  double*, cudaStream_t);
+
+int tc_reversed_factor(const float* X, const float* G, int ld, double s, float* B, float* invdiag,
+                       cudaStream_t st) {
+  return launch_reversed_factor_tiles<float>(X, nullptr, G, ld, s, B, invdiag, st);
 }
 
 }  // namespace pbg

@@ -135,7 +135,19 @@ int launch_spd_inverse(double* A, int n, int ld, int* info, void* work, cudaStre
 // X's diagonal tiles from invdiag (FP32), and out = scale X^T X with X's
 // off-diagonal tiles in X and its diagonal ones in invdiag (cholesky_df.cu).
 int launch_trtri_diag(const float* invdiag, float* X, int ld, cudaStream_t st);
-int launch_lauum(const double* X, const double* invdiag, int ld, double scale, double* out, cudaStream_t st);
+int launch_lauum(const double* X, const double* invdiag, int ld, double scale, bool reversed, double* out,
+                 cudaStream_t st);
+// out = scale J inv(G) J of the padded matrix G (order ld; J reverses the indices).
+// G and out may be the same; else G holds its factor afterwards, and
+// launch_reversed_factor turns it into the factor s J G^{-T} J of out / scale * s^2
+// and writes the inverses of that factor's diagonal tiles.
+int launch_spd_inverse_reversed(double* G, int ld, int* info, void* work, cudaStream_t st, double scale, double* out);
+int launch_reversed_factor(double* G, int ld, double s, const void* work, double* invdiag, cudaStream_t st);
+// The second with G, inv(G) (X, its diagonal tiles in Xdiag when that is not null)
+// and B apart; B may be G.
+template <typename T>
+int launch_reversed_factor_tiles(const T* X, const T* Xdiag, const T* G, int ld, double s, T* B, T* invdiag,
+                                 cudaStream_t st);
 // SPD inverse of the mixed lubricated path (FP32).  The caller puts the
 // matrix (order ld, padded) in F; tc_factor_invert factors it in place
 // (F = G, lower) and forms X = inv(G); tc_lauum writes scale X^T X on the

@@ -62,13 +62,16 @@ __global__ void widen_matrix_kernel(const float* __restrict__ src, double* __res
     dst[t] = (double)src[t];
 }
 
-// F = J R J rounded to FP32, J the reversal of all ld indices (the identity
-// padding moves to the leading rows and columns).
-__global__ void reverse_narrow_kernel(const double* __restrict__ R, int ld, float* __restrict__ F) {
+// F = J R J, tiles on and below the diagonal, J the reversal of all ld indices (the
+// identity padding moves to the leading rows and columns).
+template <typename T>
+__global__ void reverse_kernel(const double* __restrict__ R, int ld, T* __restrict__ F) {
   const long long total = (long long)ld * ld;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x)
-    F[t] = (float)R[total - 1 - t];
+       t += (long long)gridDim.x * blockDim.x) {
+    const int r = (int)(t / ld), c = (int)(t - (long long)r * ld);
+    if (c >> 6 <= r >> 6) F[t] = (T)R[total - 1 - t];
+  }
 }
 
 // res = b - R x in FP64 (one warp per row: 16-byte loads, four in flight per
@@ -323,15 +326,18 @@ int compute_Dff(pbg_system* s, cudaStream_t st, bool fill_B) {
 static int factor_reversed_R(pbg_system* s, int* info, cudaStream_t st) {
   const TcInverseWork w = tc_inverse_work(s->inv_work, s->ld);
   const long long total = (long long)s->ld * s->ld;
-  reverse_narrow_kernel<<<grid_for(total), 256, 0, st>>>(s->R, s->ld, w.F);
+  reverse_kernel<float><<<grid_for(total), 256, 0, st>>>(s->R, s->ld, w.F);
   PBG_CHECK_LAUNCH();
   int rc = tc_factor_invert(s->ld, info, s->inv_work, st);
   s->work_holds_R = rc == PBG_OK;
   return rc;
 }
 
-// box.py:533-541: R = C eta / 1e19 + Rff ; D = kBT inv(R).
-int compute_Dtot(pbg_system* s, cudaStream_t st) {
+// box.py:533-541: R = C eta / 1e19 + Rff ; D = kBT inv(R), through G =
+// chol(J R J) with J the reversal of the indices, so that chol(D) = sqrt(kBT) J
+// G^{-T} J can be read off inv(G) afterwards.  factor_B: the step takes chol(D) next
+// (decompose); FP64 then keeps G and inv(G) for it, G in B.
+int compute_Dtot(pbg_system* s, cudaStream_t st, bool factor_B) {
   const pbg_params& p = s->p;
   if (s->mlub) {
     const long long total = (long long)s->ld * s->ld;
@@ -349,8 +355,13 @@ int compute_Dtot(pbg_system* s, cudaStream_t st) {
   int rc = launch_lubrication_add(pair_source(s), s->radii, p.lubrication_cutoff, p.cichocki_correction,
                                   p.viscosity / 1e19, s->R, s->ld, st);
   if (rc) return rc;
-  PBG_CUDA_TRY(cudaMemcpyAsync(s->D, s->R, bytes, cudaMemcpyDeviceToDevice, st));
-  return launch_spd_inverse((double*)s->D, s->n, s->ld, s->dflags + 3, s->inv_work, st, p.kBT);
+  const long long total = (long long)s->ld * s->ld;
+  double* G = (double*)(factor_B ? s->B : s->D);
+  reverse_kernel<double><<<grid_for(total), 256, 0, st>>>(s->R, s->ld, G);
+  PBG_CHECK_LAUNCH();
+  rc = launch_spd_inverse_reversed(G, s->ld, s->dflags + 3, s->inv_work, st, p.kBT, (double*)s->D);
+  s->b_holds_G = factor_B && rc == PBG_OK;
+  return rc;
 }
 
 // box.py:546-556: B = chol(D), lower.
@@ -369,6 +380,10 @@ int decompose(pbg_system* s, cudaStream_t st) {
       s->g_valid = true;
     }
     return PBG_OK;
+  }
+  if (s->b_holds_G) {
+    s->b_holds_G = false;
+    return launch_reversed_factor((double*)s->B, s->ld, std::sqrt(s->p.kBT), s->inv_work, (double*)s->chol_work, st);
   }
   if (!s->b_holds_lower_D) {
     const long long total = (long long)s->ld * s->ld;
@@ -508,7 +523,7 @@ static int divergence_step(pbg_system* s, cudaStream_t st) {
     add_scalar_kernel<<<1, 32, 0, st>>>(s->pos, m, eps);
     PBG_CHECK_LAUNCH();
     if (s->build_Dff && (rc = compute_Dff(s, st, false))) return rc;
-    if (s->build_Dnf && (rc = compute_Dtot(s, st))) return rc;
+    if (s->build_Dnf && (rc = compute_Dtot(s, st, false))) return rc;
     add_row_kernel<<<(n + 255) / 256, 256, 0, st>>>((const double*)s->D, m, n, ld, s->div);
     PBG_CHECK_LAUNCH();
     add_scalar_kernel<<<1, 32, 0, st>>>(s->pos, m, -eps);
@@ -536,7 +551,7 @@ int step_begin(pbg_system* s, double dt, int build_Dff, int build_Dnf, int chol,
   int rc;
   if (s->p.hydrodynamics != PBG_HI_NONE) {
     if (build_Dff && (rc = compute_Dff(s, st, chol && !s->lub))) return rc;
-    if (s->lub && build_Dnf && (rc = compute_Dtot(s, st))) return rc;
+    if (s->lub && build_Dnf && (rc = compute_Dtot(s, st, chol != 0))) return rc;
     if (chol && (rc = decompose(s, st))) return rc;
   }
   // box.py:186: forces at the step-start positions, after the matrices.
@@ -578,7 +593,7 @@ static int midpoint_rebuild(pbg_system* s, cudaStream_t st) {
   }
   if (s->lub) {
     if (s->build_Dnf) {
-      if ((rc = compute_Dtot(s, st))) return rc;
+      if ((rc = compute_Dtot(s, st, false))) return rc;
     } else {
       PBG_CUDA_TRY(cudaMemcpyAsync(s->R, s->R0, bytes64, cudaMemcpyDeviceToDevice, st));
       if (s->build_Dff) {

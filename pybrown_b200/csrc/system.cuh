@@ -30,6 +30,7 @@ struct pbg_system {
   int* conn = nullptr;         // N x N bond matrix or null
   double* force = nullptr;     // ld (3N used)
   bool force_zero = true;        // the external force is known to be zero (pbg_set_force from host or NULL)
+  bool b_holds_G = false;  // this step's D build left chol(J R J) in B and its inverse in inv_work
   bool b_holds_lower_D = false;  // this step's D build also wrote B's lower triangle (and padding)
   void* D = nullptr;           // ld x ld, prec
   void* B = nullptr;           // ld x ld, prec, lower factor
@@ -89,7 +90,7 @@ void destroy_system(pbg_system* s);
 int system_set_state(pbg_system* s, const double* pos, const double* radii, const int* conn, cudaStream_t st);
 int build_nohi(pbg_system* s, cudaStream_t st);
 int compute_Dff(pbg_system* s, cudaStream_t st, bool fill_B);
-int compute_Dtot(pbg_system* s, cudaStream_t st);
+int compute_Dtot(pbg_system* s, cudaStream_t st, bool factor_B);
 int decompose(pbg_system* s, cudaStream_t st);
 int step_begin(pbg_system* s, double dt, int build_Dff, int build_Dnf, int chol, cudaStream_t st);
 int set_divergence(pbg_system* s, bool on);
