@@ -258,19 +258,23 @@ __device__ __forceinline__ void append_entry(const BatchDev& r, int q, int attem
   list[packed_count(at)] = RoundEntry{q, attempts, packed_trmv(at), packed_ovl(at)};
 }
 
-// Two rows of B times NA noise vectors (stride ld), in the term order of
-// row_dot (propagate.cuh) for each product.
-template <typename T, int NA>
+__device__ __forceinline__ double warp_sum(double s) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// Two rows of B times a noise vector, in the term order of row_dot
+// (propagate.cuh) for each.
+template <typename T>
 __device__ __forceinline__ void row_pair_dots(const T* __restrict__ b0, const T* __restrict__ b1, int j0, int j1,
-                                              const double* __restrict__ xi, int ld, double (&s0)[NA],
-                                              double (&s1)[NA]) {
+                                              const double* __restrict__ xi, double& s0, double& s1) {
   using C = Chunk<T>;
-  constexpr int W = C::W, U = NA == 1 ? 4 : 2;
+  constexpr int W = C::W, U = 4;
   const int lane = threadIdx.x & 31, nchunks = (j1 + W - 1) / W;
   const typename C::V* v0 = reinterpret_cast<const typename C::V*>(b0);
   const typename C::V* v1 = reinterpret_cast<const typename C::V*>(b1);
-#pragma unroll
-  for (int a = 0; a < NA; ++a) s0[a] = s1[a] = 0.0;
+  s0 = s1 = 0.0;
   for (int c0 = lane; c0 < nchunks; c0 += 32 * U) {
     typename C::V p0[U], p1[U];
 #pragma unroll
@@ -283,35 +287,113 @@ __device__ __forceinline__ void row_pair_dots(const T* __restrict__ b0, const T*
     for (int u = 0; u < U; ++u) {
       const int c = c0 + 32 * u;
       if (c >= nchunks) continue;
-      double e0[W], e1[W];
+      double e0[W], e1[W], x[W];
       C::get(p0[u], e0);
       C::get(p1[u], e1);
+#pragma unroll
+      for (int q = 0; q < W; q += 2) {
+        const double2 y = *reinterpret_cast<const double2*>(xi + c * W + q);
+        x[q] = y.x;
+        x[q + 1] = y.y;
+      }
       // a row's terms beyond its diagonal are left out
       const int k0 = j0 - c * W, k1 = j1 - c * W;
 #pragma unroll
-      for (int a = 0; a < NA; ++a) {
-        double x[W];
-#pragma unroll
-        for (int q = 0; q < W; q += 2) {
-          const double2 y = *reinterpret_cast<const double2*>(xi + (size_t)a * ld + c * W + q);
-          x[q] = y.x;
-          x[q + 1] = y.y;
-        }
-#pragma unroll
-        for (int q = 0; q < W; ++q) {
-          if (q < k0) s0[a] += e0[q] * x[q];
-          if (q < k1) s1[a] += e1[q] * x[q];
-        }
+      for (int q = 0; q < W; ++q) {
+        if (q < k0) s0 += e0[q] * x[q];
+        if (q < k1) s1 += e1[q] * x[q];
       }
     }
   }
-#pragma unroll
-  for (int a = 0; a < NA; ++a)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s0[a] += __shfl_xor_sync(0xffffffffu, s0[a], o);
-      s1[a] += __shfl_xor_sync(0xffffffffu, s1[a], o);
+  s0 = warp_sum(s0);
+  s1 = warp_sum(s1);
+}
+
+// The same for SPEC noise vectors (stride ld) by the whole CTA, rows row0 + 2 w and
+// + 1 on warp w: the noise passes through shared memory, TRMV_COLS columns at
+// a time, one block ahead, instead of every warp reading 64 bytes of it per
+// element of B through L1: a round of 23 replicas with up to 5600
+// unknowns 505 -> 189 us, one of 250 replicas 788 -> 316 us.
+constexpr int TRMV_COLS = 256;
+template <typename T>
+__device__ __forceinline__ void row_pair_dots_staged(const BatchDev& r, int row0, double (*xs)[SPEC * TRMV_COLS],
+                                                     double (&s0)[SPEC], double (&s1)[SPEC]) {
+  using C = Chunk<T>;
+  using V = typename C::V;
+  constexpr int W = C::W, U = TRMV_COLS / W / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ra = min(row0 + 2 * warp, r.n - 1), rb = min(row0 + 2 * warp + 1, r.n - 1);
+  const int j0 = ra + 1, j1 = rb + 1, nchunks = (j1 + W - 1) / W;
+  const V* v0 = reinterpret_cast<const V*>(static_cast<const T*>(r.B) + (size_t)ra * r.ld);
+  const V* v1 = reinterpret_cast<const V*>(static_cast<const T*>(r.B) + (size_t)rb * r.ld);
+  const int nb = (min(row0 + TRMV_ROWS, r.n) + TRMV_COLS - 1) / TRMV_COLS;
+  auto stage = [&](int k) {  // the pairs of a chunk 32 places apart: no bank conflicts below
+    for (int i = threadIdx.x; i < SPEC * TRMV_COLS / 2; i += 256) {
+      const int a = i / (TRMV_COLS / 2), q = i % (TRMV_COLS / 2), c = 2 * q / W, h = q % (W / 2);
+      const int col = k * TRMV_COLS + 2 * q;
+      if (col < r.ld) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(&xs[k & 1][a * TRMV_COLS + 2 * ((c / 32 * (W / 2) + h) * 32 + c % 32)]);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(r.xi + (size_t)a * r.ld + col) : "memory");
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  V p0[U], p1[U];
+  auto load = [&](int k, V (&x)[U], V (&y)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = k * (TRMV_COLS / W) + lane + 32 * u;
+      if (c < nchunks) {
+        x[u] = __ldg(v0 + c);
+        y[u] = __ldg(v1 + c);
+      }
+    }
+  };
+#pragma unroll
+  for (int a = 0; a < SPEC; ++a) s0[a] = s1[a] = 0.0;
+  stage(0);
+  for (int k = 0; k < nb; ++k) {
+    load(k, p0, p1);
+    if (k + 1 < nb) {
+      stage(k + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = k * (TRMV_COLS / W) + lane + 32 * u;
+      if (c < nchunks) {
+        double e0[W], e1[W];
+        C::get(p0[u], e0);
+        C::get(p1[u], e1);
+        const int k0 = j0 - c * W, k1 = j1 - c * W;
+#pragma unroll
+        for (int a = 0; a < SPEC; ++a) {
+          double x[W];
+#pragma unroll
+          for (int h = 0; h < W / 2; ++h) {
+            const double2 y = *reinterpret_cast<const double2*>(
+                &xs[k & 1][a * TRMV_COLS + 2 * ((u * (W / 2) + h) * 32 + lane)]);
+            x[2 * h] = y.x;
+            x[2 * h + 1] = y.y;
+          }
+#pragma unroll
+          for (int q = 0; q < W; ++q) {
+            if (q < k0) s0[a] += e0[q] * x[q];
+            if (q < k1) s1[a] += e1[q] * x[q];
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int a = 0; a < SPEC; ++a) {
+    s0[a] = warp_sum(s0[a]);
+    s1[a] = warp_sum(s1[a]);
+  }
 }
 
 // One row's candidates: U[a][row] = the position after attempt a (the attempts
@@ -336,10 +418,11 @@ __device__ __forceinline__ void write_candidates(const BatchDev& r, int row, con
 // round): two rows per warp share the noise vectors' loads.  rounds: the
 // step's round counter (its parity names the list), null for list 0.
 template <typename T>
-__global__ void __launch_bounds__(256) batch_trmv_kernel(const BatchDev* __restrict__ reps,
+__global__ void __launch_bounds__(256, 2) batch_trmv_kernel(const BatchDev* __restrict__ reps,
                                                          const RoundEntry* __restrict__ lists, int cap,
                                                          const RoundState* __restrict__ state,
                                                          const int* __restrict__ rounds, double s1) {
+  __shared__ __align__(16) double xs[2][SPEC * TRMV_COLS];
   const int par = rounds ? *rounds & 1 : 0;
   const unsigned long long pk = state->packed[par];
   const RoundEntry* list = lists + (size_t)par * cap;
@@ -348,20 +431,18 @@ __global__ void __launch_bounds__(256) batch_trmv_kernel(const BatchDev* __restr
     const RoundEntry e = find_entry(list, count, u, true);
     const BatchDev r = reps[e.q];
     const int row = (u - e.trmv0) * TRMV_ROWS + 2 * warp;
-    if (row >= r.n) continue;
     const bool two = row + 1 < r.n;
-    const T* b0 = static_cast<const T*>(r.B) + (size_t)row * r.ld;
-    const T* b1 = two ? b0 + r.ld : b0;
-    const int j0 = row + 1, j1 = two ? row + 2 : row + 1;
     if (e.attempts == 1) {
+      if (row >= r.n) continue;
+      const T* b0 = static_cast<const T*>(r.B) + (size_t)row * r.ld;
       double x0[1], x1[1];
-      row_pair_dots<T, 1>(b0, b1, j0, j1, r.xi, r.ld, x0, x1);
+      row_pair_dots<T>(b0, two ? b0 + r.ld : b0, row + 1, two ? row + 2 : row + 1, r.xi, x0[0], x1[0]);
       if (lane == 0) write_candidates<1>(r, row, x0, 1, s1);
       if (lane == 1 && two) write_candidates<1>(r, row + 1, x1, 1, s1);
     } else {
       double x0[SPEC], x1[SPEC];
-      row_pair_dots<T, SPEC>(b0, b1, j0, j1, r.xi, r.ld, x0, x1);
-      if (lane == 0) write_candidates<SPEC>(r, row, x0, e.attempts, s1);
+      row_pair_dots_staged<T>(r, row - 2 * warp, xs, x0, x1);
+      if (lane == 0 && row < r.n) write_candidates<SPEC>(r, row, x0, e.attempts, s1);
       if (lane == 1 && two) write_candidates<SPEC>(r, row + 1, x1, e.attempts, s1);
     }
   }
