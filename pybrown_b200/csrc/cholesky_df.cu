@@ -331,11 +331,7 @@ template <> struct TileMMA<double> {
 };
 
 
-__device__ __forceinline__ unsigned to_tf32(float x) {
-  unsigned r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
+using tc::split_tf32;
 
 template <> struct TileMMA<float> {
   // mma.m16n8k8 tf32: 1 m-tile of 16 x 4 n-tiles of 8, 4 accumulators each.
@@ -359,17 +355,15 @@ template <> struct TileMMA<float> {
         const float v[4] = {sA[(m0 + g) * LDA + k0 + t], sA[(m0 + g + 8) * LDA + k0 + t],
                             sA[(m0 + g) * LDA + k0 + t + 4], sA[(m0 + g + 8) * LDA + k0 + t + 4]};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          ah[q] = to_tf32(v[q]);
-          al[q] = to_tf32(v[q] - __uint_as_float(ah[q]));
-        }
+        for (int q = 0; q < 4; ++q) split_tf32(v[q], ah[q], al[q]);
       }
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
         const float v0 = sB[(n0 + 8 * nt + g) * LDA + k0 + t];
         const float v1 = sB[(n0 + 8 * nt + g) * LDA + k0 + t + 4];
-        const unsigned bh0 = to_tf32(v0), bh1 = to_tf32(v1);
-        const unsigned bl0 = to_tf32(v0 - __uint_as_float(bh0)), bl1 = to_tf32(v1 - __uint_as_float(bh1));
+        unsigned bh0, bh1, bl0, bl1;
+        split_tf32(v0, bh0, bl0);
+        split_tf32(v1, bh1, bl1);
         float* c = prod + 4 * nt;
 #define PBG_TF32_MMA(A0, A1, A2, A3, B0, B1)                                                        \
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, " \
@@ -1071,12 +1065,6 @@ __device__ __forceinline__ void tf32_mma(float (&c)[4], const unsigned (&a)[4], 
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// hi + lo TF32 halves of x
-__device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
-  hi = to_tf32(x);
-  lo = to_tf32(x - __uint_as_float(hi));
-}
-
 // FP32: 3xTF32 m16n8k8, sixteen rows per warp (warps 0 .. 3), the hi * hi
 // products and the two cross terms on separate accumulators.
 template <typename F>
@@ -2204,8 +2192,8 @@ __global__ void __launch_bounds__(THREADS, 1) chol_batch_kernel(const CholRep* _
 // as one M = 128, N = 64, K = 64 j product accumulated in TMEM: for each k
 // the tiles L_ik, L_{i+1,k}, L_jk are split into TF32 hi / lo halves in
 // shared memory and three MMAs per K-step add A_hi B_hi + A_hi B_lo + A_lo
-// B_hi to the accumulator, while the tiles of k + 1 and k + 2 are on their
-// way (cp.async into two raw FP32 stages).  Then, by the task's kind:
+// B_hi to the accumulator, while the tiles of k + 1 are split into a second
+// operand buffer.  Then, by the task's kind:
 //   LL_DIAG (i = j): F(j) -- L_jj and inv(L_jj) in FP32 -- published at once, then S(j + 1, j) = U inv(L_jj)^T with
 //     the inverse still in shared memory;
 //   LL_UPDATE (i > j): U written over A's tiles, upd[r] = j + 1;
@@ -2220,18 +2208,16 @@ __global__ void __launch_bounds__(THREADS, 1) chol_batch_kernel(const CholRep* _
 constexpr uint32_t LL_A_BYTES = tc::operand_bytes(128);
 constexpr uint32_t LL_B_BYTES = tc::operand_bytes(64);
 constexpr uint32_t LL_OPERAND_BYTES = 2 * LL_A_BYTES + 2 * LL_B_BYTES;
-// The operands (from the 1024-byte aligned start of dynamic shared memory),
-// two raw FP32 stages of a K-step's tiles, then the worker's words
-// (LLShared).  After the last product the operand bytes hold P ([128][LDA]
-// floats from 0), the U tiles ([64][LDA] at LL_U0 and LL_U1) and the factor
-// scratch (from 0).
+// Two operand buffers from the 1024-byte aligned start of dynamic shared memory,
+// then the worker's words (LLShared).  After the last product the first buffer's
+// bytes hold P ([128][LDA] floats from 0), the U tiles ([64][LDA] at LL_U0 and
+// LL_U1) and the factor scratch (from 0).
 struct LLShared {
-  uint64_t mbar, conv;
+  uint64_t mbar[2], conv[2];
   uint32_t tmem;
   int task, ok, seen[3];
 };
-constexpr uint32_t LL_RAW_BYTES = 3 * NB * NB * sizeof(float);  // one raw stage: L_ik, L_{i+1,k}, L_jk
-constexpr uint32_t LL_SHARED_OFFSET = LL_OPERAND_BYTES + 2 * LL_RAW_BYTES;
+constexpr uint32_t LL_SHARED_OFFSET = 2 * LL_OPERAND_BYTES;
 constexpr size_t ll_smem_bytes() { return LL_SHARED_OFFSET + sizeof(LLShared); }
 static_assert(ll_smem_bytes() <= 227 * 1024, "the worker does not fit an SM");
 // task kinds of the left-looking list
@@ -2244,12 +2230,12 @@ static_assert(sizeof(float) * 128 * LDA <= LL_U0, "P overlaps U0");
 static_assert(LL_U1 + sizeof(float) * NB * LDA <= LL_OPERAND_BYTES, "U1 lies outside the operand bytes");
 
 struct LLWorker {
-  uint64_t* mbar;       // completion of the products of one K-step
-  uint64_t* conv;       // every thread's operands of a K-step written (THREADS arrivals)
-  uint32_t tmem;        // TMEM base: the 128 x 64 FP32 accumulator
-  uint32_t phase;
-  uint32_t conv_phase;  // thread 0's
-  unsigned char* base;  // 1024-byte aligned operand area
+  uint64_t* mbar;       // [2] completion of the products of one K-step, per operand buffer
+  uint64_t* conv;       // [2] every thread's operands of a K-step written (THREADS arrivals)
+  uint32_t tmem;        // TMEM base: two 128 x 128 FP32 accumulators (hi hi | cross terms)
+  uint32_t phase;       // bit b: the parity of mbar[b]
+  uint32_t conv_phase;  // thread 0's, of conv
+  unsigned char* base;  // 1024-byte aligned operand buffers
 };
 
 __device__ __forceinline__ DFArgs batch_args(const CholRep& R, const int4* tasks, int ntasks, int* ctl) {
@@ -2338,23 +2324,6 @@ __device__ __forceinline__ void cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// The tiles of K-step k (L_ik, L_{i+1,k}, L_jk) into a raw stage, one group.
-__device__ __forceinline__ void ll_fetch_step(const DFArgs& a, int i, bool two, int j, int k, float* raw) {
-  ll_fetch_tile(tile<float>(a, i, k), a.ld, raw);
-  if (two) ll_fetch_tile(tile<float>(a, i + 1, k), a.ld, raw + NB * NB);
-  ll_fetch_tile(tile<float>(a, j, k), a.ld, raw + 2 * NB * NB);
-  cp_async_commit();
-}
-
-// This thread's share of a raw stage tile, back into registers.
-__device__ __forceinline__ void ll_share_from_raw(const float* raw, tc::TileShare<THREADS>& s) {
-#pragma unroll
-  for (int e = 0; e < tc::TileShare<THREADS>::PER; ++e) {
-    const int q = threadIdx.x + e * THREADS, r = q >> 4, c = q & 15;
-    s.v[e] = *reinterpret_cast<const float4*>(raw + r * NB + 4 * c);
-  }
-}
-
 // Per-thread bounded wait until base[rows[q]] >= target for q = 0, 1, 2,
 // with the counts observed so far kept in the thread's registers (seen): a
 // wait that an earlier observation satisfies costs nothing, and the thread's
@@ -2391,119 +2360,119 @@ __device__ __forceinline__ void ll_arrive(uint64_t* m) {
 }
 
 // P = sum_{k < j} [L_ik; L_{i+1,k}] L_jk^T into shared memory ([128][LDA]
-// floats at the operand area's start), for j > 0.  The tiles of K-step k + 2
-// are fetched (cp.async, two raw stages) while the products of k run.  No
-// CTA barrier inside the K loop: every thread fetches and converts only its
-// own chunks (so the raw stages need no hand-over), waits for the previous
-// products on their mbarrier before overwriting the operands, and arrives on
-// the conversion mbarrier; thread 0 waits for all arrivals and issues the
-// MMAs.  Returns false (after a CTA barrier) if the run was aborted, with no
-// products of this CTA left in flight.
-__device__ bool ll_products(const DFArgs& a, int i, int j, LLWorker& w) {
+// floats at the operand area's start), for j > 0, and A's tiles (i, j), (i + 1, j)
+// into As.  Two operand buffers: the tiles of K-step k are split into one
+// while the products of k - 1 run from the other, and a tile's registers take
+// its successor (loaded straight from L2) as soon as it is split.  The first version had one
+// buffer, and two raw stages in shared memory for the tiles on their way: split
+// and products alternated, and every tile crossed shared memory twice more
+// (3000 cycles a K-step of the 256-replica batch, 1730 now).  No
+// CTA barrier inside the K loop: every thread loads and splits only its
+// own chunks, waits for the products of k - 2 on their mbarrier before overwriting
+// their operands, and arrives on the buffer's conversion mbarrier; thread 0 waits for
+// all arrivals and issues the MMAs.  Returns false (after a CTA barrier) if the
+// run was aborted, with no products of this CTA left in flight.
+__device__ bool ll_products(const DFArgs& a, int i, int j, LLWorker& w, tc::TileShare<THREADS> (&As)[2]) {
   const int tid = threadIdx.x;
   const bool two = i + 1 < a.nt;
-  unsigned char* Ahi = w.base;
-  unsigned char* Alo = Ahi + LL_A_BYTES;
-  unsigned char* Bhi = Alo + LL_A_BYTES;
-  unsigned char* Blo = Bhi + LL_B_BYTES;
-  float* raw[2] = {reinterpret_cast<float*>(w.base + LL_OPERAND_BYTES),
-                   reinterpret_cast<float*>(w.base + LL_OPERAND_BYTES + LL_RAW_BYTES)};
   const int rows[3] = {i, two ? i + 1 : i, j};
   int seen[3] = {0, 0, 0};
   if (!two) {
-    // rows 64 .. 127 of both A halves stay zero for the whole task: bytes
+    // rows 64 .. 127 of the A halves stay zero for the whole task: bytes
     // 8192 .. 16383 of each of the two K blocks (16384 bytes each)
-    for (int e = tid; e < 4 * 512; e += THREADS) {
+    for (int e = tid; e < 8 * 512; e += THREADS) {
       const int part = e >> 9, off = (e & 511) * 16;
-      unsigned char* p = (part & 1 ? Alo : Ahi) + (part >> 1) * 16384 + 8192 + off;
+      unsigned char* p = w.base + (part >> 2) * LL_OPERAND_BYTES + (part & 1) * LL_A_BYTES + ((part >> 1) & 1) * 16384 +
+                         8192 + off;
       *reinterpret_cast<uint4*>(p) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
+  tc::TileShare<THREADS> sB;
   long long c0 = LLCLK();
   bool ok = ll_thread_wait_rows(a, a.fin, rows, 1, seen);
-  if (ok) ll_fetch_step(a, i, two, j, 0, raw[0]);
-  else cp_async_commit();
-  if (j > 1) {
-    ok = ok && ll_thread_wait_rows(a, a.fin, rows, 2, seen);
-    if (ok) ll_fetch_step(a, i, two, j, 1, raw[1]);
-    else cp_async_commit();
+  if (ok) {
+    tc::load_share(tile<float>(a, i, 0), a.ld, As[0]);
+    if (two) tc::load_share(tile<float>(a, i + 1, 0), a.ld, As[1]);
+    tc::load_share(tile<float>(a, j, 0), a.ld, sB);
   }
   LLPROF(2, LLCLK() - c0);
-  // the products accumulate in TMEM for LL_CHUNK K-steps at a time; each
-  // chunk's sum is then added in FP32 to racc (this thread's row m, columns
-  // 32 g .. 32 g + 31), so no accumulation runs longer than K = 64 LL_CHUNK
-  // in the tensor cores
+  // the products accumulate in TMEM for LL_CHUNK K-steps at a time, the chunks in
+  // two accumulators in turn; each chunk's sum is added in FP32 to racc (this
+  // thread's row m, columns 32 g .. 32 g + 31) while the next one runs, so no
+  // accumulation runs longer than K = 64 LL_CHUNK in the tensor cores
   const int warp = tid >> 5, lane = tid & 31, q = warp & 3, g = warp >> 2;
   const int m = 32 * q + lane;
   const uint32_t tacc = w.tmem + ((uint32_t)(32 * q) << 16) + 32 * g;
   float racc[32];
 #pragma unroll
   for (int u = 0; u < 32; ++u) racc[u] = 0.0f;
-  for (int k = 0; k < j; ++k) {
-    float* st = raw[k & 1];
-    c0 = LLCLK();
-    if (k + 1 < j) cp_async_wait_group<1>();
-    else cp_async_wait_group<0>();
-    if (k > 0) {  // the products of k - 1 have read the operands
-      if (!tc::mbar_wait(w.mbar, w.phase, a.spin_limit)) ok = false;
-      w.phase ^= 1;
-      tc::fence_after_sync();
-      if (k % LL_CHUNK == 0) {
-        // a chunk is complete: fold it into racc before the next product
-        // starts the accumulator from zero (ordered by the conversion mbarrier)
-        float v[32];
-        tc::tmem_ld32(tacc, v);
+  auto fold = [&](int chunk) {
+    float v[32], x[32];
+    tc::tmem_ld32(tacc + 128 * (chunk & 1), v);
+    tc::tmem_ld32(tacc + 128 * (chunk & 1) + 64, x);
 #pragma unroll
-        for (int u = 0; u < 32; ++u) racc[u] += v[u];
+    for (int u = 0; u < 32; ++u) racc[u] += v[u] + x[u];
+  };
+  auto finished = [&](int k) {  // waits for the products of K-step k
+    const int b = k & 1;
+    if (!tc::mbar_wait(w.mbar + b, (w.phase >> b) & 1u, a.spin_limit)) ok = false;
+    w.phase ^= 1u << b;
+  };
+  for (int k = 0; k < j; ++k) {
+    const int b = k & 1;
+    unsigned char* Ahi = w.base + b * LL_OPERAND_BYTES;
+    unsigned char* Alo = Ahi + LL_A_BYTES;
+    unsigned char* B = Alo + LL_A_BYTES;
+    c0 = LLCLK();
+    if (k >= 2) {  // the products of k - 2 have read this buffer
+      finished(k - 2);
+      tc::fence_after_sync();
+      if (k > LL_CHUNK && k % LL_CHUNK == 1) {
+        // ... and were the last of a chunk; its accumulator is started again
+        // LL_CHUNK - 1 steps from here (ordered by the conversion mbarriers)
+        fold(k / LL_CHUNK - 1);
         tc::fence_before_sync();
       }
     }
     const long long c1 = LLCLK();
     LLPROF(3, c1 - c0);
-    {
-      tc::TileShare<THREADS> s;
-      ll_share_from_raw(st, s);
-      tc::store_share_split<THREADS>(s, 128, 0, Ahi, Alo);
-      if (two) {
-        ll_share_from_raw(st + NB * NB, s);
-        tc::store_share_split<THREADS>(s, 128, 64, Ahi, Alo);
-      }
-      ll_share_from_raw(st + 2 * NB * NB, s);
-      tc::store_share_split<THREADS>(s, 64, 0, Bhi, Blo);
+    // the next step's tiles (or A's), where their rows are known to be final
+    const bool last = k + 1 == j;
+    const bool ready = __all_sync(0xffffffffu, ok && (last || min(seen[0], min(seen[1], seen[2])) >= k + 2));
+    const int next = last ? j : k + 1;
+    tc::store_share_split<THREADS>(As[0], 128, 0, Ahi, Alo);
+    if (ready) tc::load_share(tile<float>(a, i, next), a.ld, As[0]);
+    if (two) {
+      tc::store_share_split<THREADS>(As[1], 128, 64, Ahi, Alo);
+      if (ready) tc::load_share(tile<float>(a, i + 1, next), a.ld, As[1]);
     }
+    tc::store_share_split<THREADS>(sB, 128, 0, B, B + 64 * 128);  // lo 64 rows below hi
+    if (ready && !last) tc::load_share(tile<float>(a, j, next), a.ld, sB);
     tc::fence_proxy_smem();
-    ll_arrive(w.conv);
+    ll_arrive(w.conv + b);
     if (tid == 0) {
-      if (!tc::mbar_wait(w.conv, w.conv_phase, a.spin_limit)) ok = false;  // every thread's operands written
-      w.conv_phase ^= 1;
+      if (!tc::mbar_wait(w.conv + b, (w.conv_phase >> b) & 1u, a.spin_limit)) ok = false;  // all operands written
+      w.conv_phase ^= 1u << b;
       tc::fence_after_sync();
-      tc::issue_product(w.tmem, tc::smem_u32(Ahi), tc::smem_u32(Alo), tc::smem_u32(Bhi), tc::smem_u32(Blo),
-                        k % LL_CHUNK != 0 ? 1u : 0u);
-      tc::mma_commit(w.mbar);
+      tc::issue_product_wide(w.tmem + 128 * ((k / LL_CHUNK) & 1), tc::smem_u32(Ahi), tc::smem_u32(Alo), tc::smem_u32(B),
+                             k % LL_CHUNK != 0 ? 1u : 0u);
+      tc::mma_commit(w.mbar + b);
     }
     c0 = LLCLK();
     LLPROF(4, c0 - c1);
-    if (k + 1 == j) {
-      // both raw stages are consumed: A's tiles (i, j), (i + 1, j) for the
-      // difference U = A - P come in while the last products run, each
-      // thread's chunks where ll_difference reads them
-      float* As = raw[0];
-      for (int e = tid; e < (two ? 128 : 64) * 16; e += THREADS) {
-        const int row = e >> 4, c4 = e & 15;
-        cp_async16(As + row * NB + 4 * c4, tile<float>(a, i + (row >> 6), j) + (size_t)(row & 63) * a.ld + 4 * c4);
+    if (!ready) {
+      ok = ok && (last || ll_thread_wait_rows(a, a.fin, rows, k + 2, seen));
+      if (ok) {
+        tc::load_share(tile<float>(a, i, next), a.ld, As[0]);
+        if (two) tc::load_share(tile<float>(a, i + 1, next), a.ld, As[1]);
+        if (!last) tc::load_share(tile<float>(a, j, next), a.ld, sB);
       }
-      cp_async_commit();
-    }
-    if (k + 2 < j) {
-      ok = ok && ll_thread_wait_rows(a, a.fin, rows, k + 3, seen);
-      if (ok) ll_fetch_step(a, i, two, j, k + 2, st);
-      else cp_async_commit();
       LLPROF(2, LLCLK() - c0);
     }
   }
   c0 = LLCLK();
-  if (!tc::mbar_wait(w.mbar, w.phase, a.spin_limit)) ok = false;
-  w.phase ^= 1;
+  if (j > 1) finished(j - 2);
+  finished(j - 1);
   ok = __syncthreads_and(ok) != 0;
   LLPROF(3, LLCLK() - c0);
   if (!ok) {
@@ -2515,13 +2484,10 @@ __device__ bool ll_products(const DFArgs& a, int i, int j, LLWorker& w) {
     return false;
   }
   tc::fence_after_sync();
-  // P = racc + the last chunk from TMEM, into shared memory, row m = TMEM lane
-  {
-    float v[32];
-    tc::tmem_ld32(tacc, v);
-#pragma unroll
-    for (int u = 0; u < 32; ++u) racc[u] += v[u];
-  }
+  // P = racc + the chunks still in TMEM, into shared memory, row m = TMEM lane
+  const int chunk = (j - 1) / LL_CHUNK;
+  if (chunk > 0 && (j - 1) % LL_CHUNK == 0) fold(chunk - 1);
+  fold(chunk);
   if (two || q < 2) {  // warp-uniform
     float* dst = reinterpret_cast<float*>(w.base) + (size_t)m * LDA + 32 * g;
 #pragma unroll
@@ -2534,26 +2500,31 @@ __device__ bool ll_products(const DFArgs& a, int i, int j, LLWorker& w) {
   return true;
 }
 
-// U = A - P for rows i (and i + 1) of column j, a row of 64 per 16 threads;
-// A from its prefetched copy As (row-major [128][64], j > 0) or from global
-// memory (j = 0, no P); into the [64][LDA] tiles U0 / U1 in shared memory,
+// U = A - P for rows i (and i + 1) of column j; A's tiles in As (this thread's
+// chunks), no P for j = 0; into the [64][LDA] tiles U0 / U1 in shared memory,
 // or in place into A when to_global.
 __device__ __forceinline__ void ll_difference(const DFArgs& a, int i, int j, bool two, const float* Ps,
-                                              const float* As, float* U0, float* U1, bool to_global) {
-  if (j > 0) cp_async_wait_group<0>();  // this thread's chunks of A, fetched during the last products
-  for (int e = threadIdx.x; e < (two ? 128 : 64) * 16; e += THREADS) {
-    const int row = e >> 4, c4 = e & 15;
-    float4* gp = reinterpret_cast<float4*>(tile<float>(a, i + (row >> 6), j) + (size_t)(row & 63) * a.ld) + c4;
-    float4 cv = j > 0 ? *reinterpret_cast<const float4*>(As + row * NB + 4 * c4) : __ldcg(gp);
-    if (j > 0) {
-      const float4 pv = *reinterpret_cast<const float4*>(Ps + (size_t)row * LDA + 4 * c4);
-      cv.x -= pv.x;
-      cv.y -= pv.y;
-      cv.z -= pv.z;
-      cv.w -= pv.w;
+                                              const tc::TileShare<THREADS> (&As)[2], float* U0, float* U1,
+                                              bool to_global) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (h == 1 && !two) break;
+    float* gp = tile<float>(a, i + h, j);
+    float* U = h == 0 ? U0 : U1;
+#pragma unroll
+    for (int e = 0; e < tc::TileShare<THREADS>::PER; ++e) {
+      const int t = threadIdx.x + e * THREADS, r = t >> 4, c = 4 * (t & 15);
+      float4 cv = As[h].v[e];
+      if (j > 0) {
+        const float4 pv = *reinterpret_cast<const float4*>(Ps + (size_t)(64 * h + r) * LDA + c);
+        cv.x -= pv.x;
+        cv.y -= pv.y;
+        cv.z -= pv.z;
+        cv.w -= pv.w;
+      }
+      if (to_global) *reinterpret_cast<float4*>(gp + (size_t)r * a.ld + c) = cv;
+      else *reinterpret_cast<float4*>(U + r * LDA + c) = cv;
     }
-    if (to_global) *gp = cv;
-    else *reinterpret_cast<float4*>((row < 64 ? U0 : U1) + (row & 63) * LDA + 4 * c4) = cv;
   }
 }
 
@@ -2571,10 +2542,15 @@ __device__ bool ll_task(const DFArgs& a, int kind, int i, int j, LLWorker& w, in
   LLPROF(0, 1);
   LLPROF(1, j);
   if (kind != LL_SOLVE) {
-    if (j > 0 && !ll_products(a, i, j, w)) return false;
+    tc::TileShare<THREADS> As[2];
+    if (j > 0) {
+      if (!ll_products(a, i, j, w, As)) return false;
+    } else {
+      tc::load_share(tile<float>(a, i, 0), a.ld, As[0]);
+      if (two) tc::load_share(tile<float>(a, i + 1, 0), a.ld, As[1]);
+    }
     c0 = LLCLK();
-    ll_difference(a, i, j, two, Ps, reinterpret_cast<const float*>(w.base + LL_OPERAND_BYTES), U0, U1,
-                  kind == LL_UPDATE);
+    ll_difference(a, i, j, two, Ps, As, U0, U1, kind == LL_UPDATE);
     __syncthreads();
     LLPROF(5, LLCLK() - c0);
     c0 = LLCLK();
@@ -2627,7 +2603,7 @@ __device__ bool ll_task(const DFArgs& a, int kind, int i, int j, LLWorker& w, in
   return true;
 }
 
-// One CTA per SM (192 KB of shared memory, 64 TMEM columns), all co-resident
+// One CTA per SM (192 KB of shared memory, 256 TMEM columns), all co-resident
 // (cooperative launch).
 __global__ void __launch_bounds__(THREADS, 1) chol_batch_ll_kernel(const CholRep* __restrict__ reps,
                                                                    const int4* __restrict__ tasks, int ntasks,
@@ -2647,17 +2623,19 @@ __global__ void __launch_bounds__(THREADS, 1) chol_batch_ll_kernel(const CholRep
   }
   LLShared* sh = reinterpret_cast<LLShared*>(smem + LL_SHARED_OFFSET);
   if (threadIdx.x == 0) {
-    tc::mbar_init(&sh->mbar, 1);
-    tc::mbar_init(&sh->conv, THREADS);
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init(&sh->mbar[b], 1);
+      tc::mbar_init(&sh->conv[b], THREADS);
+    }
     sh->ok = 1;
   }
-  if (threadIdx.x < 32) tc::tmem_alloc(&sh->tmem, 64);
+  if (threadIdx.x < 32) tc::tmem_alloc(&sh->tmem, 256);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   LLWorker w;
-  w.mbar = &sh->mbar;
-  w.conv = &sh->conv;
+  w.mbar = sh->mbar;
+  w.conv = sh->conv;
   w.tmem = sh->tmem;
   w.phase = 0;
   w.conv_phase = 0;
@@ -2678,7 +2656,7 @@ __global__ void __launch_bounds__(THREADS, 1) chol_batch_ll_kernel(const CholRep
   LLPROF(10, LLCLK() - k0);
   tc::fence_before_sync();
   __syncthreads();
-  if (threadIdx.x < 32) tc::tmem_dealloc(w.tmem, 64);
+  if (threadIdx.x < 32) tc::tmem_dealloc(w.tmem, 256);
 }
 
 std::mutex g_task_mu;
@@ -3229,6 +3207,7 @@ __global__ void b_invdiag_kernel(const T* __restrict__ G, int ld, int nt, T inv_
 // Each element is written once: (r, c) and, off the diagonal tiles, (c, r);
 // with `reversed`, (ld-1-r, ld-1-c) instead.
 constexpr int SYM_CHUNK = 4;
+constexpr uint32_t LL_RAW_BYTES = 3 * NB * NB * sizeof(float);  // one raw stage: X_kI, X_{k,I+1}, X_kJ
 constexpr uint32_t SYM_SHARED_OFFSET = LL_OPERAND_BYTES + 2 * LL_RAW_BYTES;
 constexpr size_t sym_smem_bytes() { return SYM_SHARED_OFFSET + 16; }  // mbarrier, TMEM address
 static_assert(sym_smem_bytes() <= 227 * 1024, "the symmetric product does not fit an SM");

@@ -2,7 +2,7 @@
 //
 // P = A B^T for 64 x 64 FP32 tiles: A is one or two stacked row tiles (an
 // M = 128 operand), B one tile (N = 64), K = 64.  Each FP32 operand is split
-// as x = hi + lo with hi = rna_tf32(x) and lo = rna_tf32(x - hi), and
+// as x = hi + lo (split_tf32), and
 //   P = A_hi B_hi + A_hi B_lo + A_lo B_hi
 // accumulates in FP32 in tensor memory (TMEM), from zero.  The operands are
 // written by the CTA's threads into shared memory in the canonical K-major
@@ -27,10 +27,16 @@ constexpr int TILE = 64;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ uint32_t rna_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
+// x = hi + lo with both halves rounded to TF32 (11-bit significands), without the
+// conversion unit, whose 16 results per clock and SM bound the split (24 K
+// conversions per K-step of 128 + 64 rows: 1540 of 1840 cycles).  hi: round to
+// nearest on the bits, ties away.  lo = x - hi is exact, then rounded by
+// Veltkamp's splitting.  An infinity stays one; a NaN stays one in lo, whatever
+// the bits of hi become.
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  const float l = __fsub_rn(x, __uint_as_float(hi)), c = __fmul_rn(l, 8193.0f);
+  lo = __float_as_uint(__fsub_rn(c, __fsub_rn(c, l)));
 }
 
 // ---------------------------------------------------------------- mbarrier
@@ -171,10 +177,7 @@ __device__ __forceinline__ void store_share_split(const TileShare<NTHREADS>& s, 
     const float x[4] = {s.v[e].x, s.v[e].y, s.v[e].z, s.v[e].w};
     uint32_t h[4], l[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      h[u] = rna_tf32(x[u]);
-      l[u] = rna_tf32(x[u] - __uint_as_float(h[u]));
-    }
+    for (int u = 0; u < 4; ++u) split_tf32(x[u], h[u], l[u]);
     *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
   }
@@ -186,10 +189,7 @@ __device__ __forceinline__ void store_split_chunk(float4 x4, uint32_t off, unsig
   const float x[4] = {x4.x, x4.y, x4.z, x4.w};
   uint32_t h[4], l[4];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    h[u] = rna_tf32(x[u]);
-    l[u] = rna_tf32(x[u] - __uint_as_float(h[u]));
-  }
+  for (int u = 0; u < 4; ++u) split_tf32(x[u], h[u], l[u]);
   *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
@@ -222,6 +222,21 @@ __device__ __forceinline__ void issue_product(uint32_t d_tmem, uint32_t a_hi, ui
     mma_tf32(d_tmem, sw128_desc(a_hi + ka), sw128_desc(b_hi + kb), idesc, s > 0 ? 1u : accumulate);
     mma_tf32(d_tmem, sw128_desc(a_hi + ka), sw128_desc(b_lo + kb), idesc, 1u);
     mma_tf32(d_tmem, sw128_desc(a_lo + ka), sw128_desc(b_hi + kb), idesc, 1u);
+  }
+}
+
+// The same with B's halves as one 128-row operand (hi in rows 0 .. 63, lo in rows
+// 64 .. 127) and 128 accumulator columns: hi hi in the first 64, the two cross
+// terms in the others.  Two thirds of the instructions, and A_hi and B_hi are read from
+// shared memory once less.
+__device__ __forceinline__ void issue_product_wide(uint32_t d_tmem, uint32_t a_hi, uint32_t a_lo, uint32_t b,
+                                                   uint32_t accumulate) {
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const uint32_t k = (uint32_t)((s >> 2) * 128 * 128 + (s & 3) * 32);  // 128 rows per K block
+    const uint64_t bd = sw128_desc(b + k);
+    mma_tf32(d_tmem, sw128_desc(a_hi + k), bd, idesc_tf32(128, 128), s > 0 ? 1u : accumulate);
+    mma_tf32(d_tmem + 64, sw128_desc(a_lo + k), bd, idesc_tf32(128, 64), 1u);
   }
 }
 
