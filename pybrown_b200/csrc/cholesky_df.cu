@@ -227,24 +227,6 @@ __device__ __forceinline__ void copy_async(const T* g, T* s, int count) {
   for (int t = threadIdx.x; t < count / elems; t += THREADS) cp_async16(s + t * elems, g + t * elems);
 }
 
-// 16-byte shared-memory loads of N consecutive T (p 16-byte aligned).
-template <int N>
-__device__ __forceinline__ void lds_vec(const float* p, float (&v)[N]) {
-#pragma unroll
-  for (int q = 0; q < N; q += 4) {
-    const float4 x = *reinterpret_cast<const float4*>(p + q);
-    v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
-  }
-}
-template <int N>
-__device__ __forceinline__ void lds_vec(const double* p, double (&v)[N]) {
-#pragma unroll
-  for (int q = 0; q < N; q += 2) {
-    const double2 x = *reinterpret_cast<const double2*>(p + q);
-    v[q] = x.x; v[q + 1] = x.y;
-  }
-}
-
 // Row-major copy of a 64 x 64 smem tile (rows of `lds`) to global, 16 bytes per store.
 template <typename T>
 __device__ __forceinline__ void store_tile(const T* s, int lds, T* g, int ld) {
@@ -432,36 +414,6 @@ struct WarpTile64 {
   static constexpr int NQ = 2;
 };
 
-// The FP32 counterpart on the FMA pipe (the mixed batch inverts its diagonal
-// tiles in FP32): lane (g, t) forms D[g][2t], D[g][2t + 1] as K-term dot
-// products in ascending k.
-struct WarpTile32 {
-  static constexpr int TM = 8;
-  static __device__ __forceinline__ void mma(const float* A, int lda, const float* B, int ldb, int K, float d[4]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    float d0 = 0.0f, d1 = 0.0f;
-#pragma unroll 8
-    for (int k0 = 0; k0 < K; k0 += 4) {
-      const float4 a4 = *reinterpret_cast<const float4*>(A + g * lda + k0);
-      const float av[4] = {a4.x, a4.y, a4.z, a4.w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 b = *reinterpret_cast<const float2*>(B + (k0 + q) * ldb + 2 * t);
-        d0 = fmaf(av[q], b.x, d0);
-        d1 = fmaf(av[q], b.y, d1);
-      }
-    }
-    d[0] = d0;
-    d[1] = d1;
-  }
-  static __device__ __forceinline__ int row(int q) { return (threadIdx.x & 31) >> 2; }
-  static __device__ __forceinline__ int col(int q) { return 2 * (threadIdx.x & 3) + (q & 1); }
-  static constexpr int NQ = 2;
-};
-
-template <typename T> struct WarpTileOf;
-template <> struct WarpTileOf<double> { using type = WarpTile64; };
-template <> struct WarpTileOf<float> { using type = WarpTile32; };
 
 // Inverse of the lower-triangular L_kk (in Lk, [64][LDA], zero above the
 // diagonal) into X ([64][LDA]), with Rinv[j] = 1 / L_jj and scratch Tm
@@ -473,7 +425,7 @@ template <> struct WarpTileOf<float> { using type = WarpTile32; };
 // thread at s = 8, by warp tensor-core tiles at s = 16 and 32.
 template <typename T>
 __device__ __forceinline__ void invert_factor(const T* Lk, const T* Rinv, T* X, T* Tm) {
-  using WT = typename WarpTileOf<T>::type;
+  using WT = WarpTile64;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (lane < 8) {
     const T* D = Lk + 8 * warp * LDA + 8 * warp;
@@ -548,16 +500,6 @@ __device__ __forceinline__ void store_inverse(const DFArgs& a, int k, const T* L
   } else {
     for (int t = threadIdx.x; t < NB * NB; t += THREADS) inv[t] = (S)X[(t >> 6) * LDA + (t & 63)];
   }
-}
-
-// acc = -(acc + ...) helpers for S: acc = C inv(L_kk)^T with C, X in smem.
-template <typename T>
-__device__ __forceinline__ void solve_by_inverse(const T* C, const T* X, T acc[16]) {
-#pragma unroll
-  for (int e = 0; e < 16; ++e) acc[e] = T(0);
-  TileMMA<T>::sub(C, X, acc);  // acc = -C X^T
-#pragma unroll
-  for (int e = 0; e < 16; ++e) acc[e] = -acc[e];
 }
 
 template <typename T>
@@ -1068,11 +1010,9 @@ __device__ __forceinline__ void tf32_mma(float (&c)[4], const unsigned (&a)[4], 
 // FP32: 3xTF32 m16n8k8, sixteen rows per warp (warps 0 .. 3), the hi * hi
 // products and the two cross terms on separate accumulators.
 template <typename F>
-__device__ __forceinline__ void solve_rows_f32(const float* C, int ldc, const float* V, F out) {
+__device__ __forceinline__ void solve_rows_f32(const float* C, int ldc, const float* V, int warp, F out) {
   constexpr int LT = ChainLd<float>::LT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  if (warp >= 4) return;
-  const int r0 = 16 * warp + g;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, r0 = 16 * warp + g;
   float p[8][4], q[8][4];
   auto mul = [&](float (&p)[4], float (&q)[4], const unsigned (&ah)[4], const unsigned (&al)[4], const float* vb) {
     unsigned bh[2], bl[2];
@@ -1121,12 +1061,12 @@ __device__ __forceinline__ void solve_rows_f32(const float* C, int ldc, const fl
 template <typename T, typename F>
 __device__ __forceinline__ void solve_half(const T* C, const T* V, F out) {
   if constexpr (sizeof(T) == 8) solve_rows<1>(C, LDA, V, out);
-  else if (threadIdx.x < 64) solve_rows_f32(C, LDA, V, out);
+  else if (threadIdx.x < 64) solve_rows_f32(C, LDA, V, threadIdx.x >> 5, out);
 }
 template <typename T, typename F>
 __device__ __forceinline__ void solve_rows_t(const T* C, int ldc, const T* V, F out) {
   if constexpr (sizeof(T) == 8) solve_rows<1>(C, ldc, V, out);
-  else solve_rows_f32(C, ldc, V, out);
+  else if (threadIdx.x < 128) solve_rows_f32(C, ldc, V, threadIdx.x >> 5, out);
 }
 
 // ---------------------------------------------------------------- the chain's SYRK
@@ -1302,185 +1242,6 @@ __device__ void run_chain(const DFArgs& a, unsigned char* smem, int* s_ok) {
     CTRACE(k, 5);
     if (!*s_ok) return;
   }
-}
-
-// ---------------------------------------------------------------- FP32 diagonal tiles
-// The mixed batch factors, inverts and solves its diagonal tiles in FP32: the
-// tiles of a well-conditioned FP32 matrix lose nothing to FP32
-// pivots that FP32 storage and the 3xTF32 updates have not already cost.
-
-// T[r][c] -= sum_q T[r][c0+q] T[c][c0+q] (q = 0..7, in order): the rank-8
-// update of one trailing element with the factored panel c0..c0+7.
-__device__ __forceinline__ void panel_update(float* T, int r, int c, int c0) {
-  const float4 a0 = *reinterpret_cast<const float4*>(T + r * LDA + c0);
-  const float4 a1 = *reinterpret_cast<const float4*>(T + r * LDA + c0 + 4);
-  const float4 b0 = *reinterpret_cast<const float4*>(T + c * LDA + c0);
-  const float4 b1 = *reinterpret_cast<const float4*>(T + c * LDA + c0 + 4);
-  float v = T[r * LDA + c];
-  v = fmaf(-a0.x, b0.x, v);
-  v = fmaf(-a0.y, b0.y, v);
-  v = fmaf(-a0.z, b0.z, v);
-  v = fmaf(-a0.w, b0.w, v);
-  v = fmaf(-a1.x, b1.x, v);
-  v = fmaf(-a1.y, b1.y, v);
-  v = fmaf(-a1.z, b1.z, v);
-  v = fmaf(-a1.w, b1.w, v);
-  T[r * LDA + c] = v;
-}
-
-// F(k) of the mixed batch on the tile T (smem [64][LDA]: lower triangle valid
-// with every update applied; the caller's writes end with a CTA barrier).
-// Eight 8-column panels.  Warp 0 factors panel p -- the 8 x 8 pivot block in
-// every lane's registers (the pivot chain is rsqrt -> multiply -> FMA) and
-// the strip rows below it (L_r = A_r L_pp^-T, one row per lane) -- while
-// warps 1-7 apply the rank-8 update of panel p-1 to the trailing lower
-// triangle: first the eight columns of panel p+1 (look-ahead), then the
-// rest.  Named barrier 1: panel p factored (warp 0 arrives, warps 1-7
-// wait); named barrier 2: panel p+1's columns updated (warps 1-7 arrive,
-// warp 0 waits).  The update of panel p's columns (c0..c0+7) by warps 1-7 and
-// warp 0's work on them never overlap, nor do the look-ahead and the rest.
-// Returns after a CTA barrier with L_kk in T's lower triangle (the upper one
-// as it was) and Rinv[j] = 1 / L_jj.  A non-positive (or NaN) pivot is
-// recorded in info.
-__device__ __forceinline__ void factor_tile_f32(const DFArgs& a, int k, float* T, float* Rinv) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) {
-#pragma unroll 1
-    for (int p = 0; p < 8; ++p) {
-      const int c0 = 8 * p;
-      if (p > 0) bar_wait(2, THREADS);
-      float l[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) lds_vec(T + (c0 + i) * LDA + c0, l[i]);
-      int bad = -1;
-      float rinv[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float d = l[j][j];
-        // a pivot below the smallest normal float (or NaN) is reported like a
-        // non-positive one; the MUFU estimate (rel. error < 2^-22) is FP32 accurate
-        if (!(d >= 1.17549435e-38f) && bad < 0) bad = j;
-        float rs;
-        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(d));
-        rinv[j] = rs;
-        l[j][j] = d * rs;
-#pragma unroll
-        for (int i = j + 1; i < 8; ++i) l[i][j] *= rs;
-#pragma unroll
-        for (int i = j + 1; i < 8; ++i)
-#pragma unroll
-          for (int c = j + 1; c <= i; ++c) l[i][c] = fmaf(-l[i][j], l[c][j], l[i][c]);
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = c0 + 8 + lane + 32 * h;
-        if (r < NB) {
-          float x[8];
-          lds_vec(T + r * LDA + c0, x);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            x[j] *= rinv[j];
-#pragma unroll
-            for (int c = j + 1; c < 8; ++c) x[c] = fmaf(-x[j], l[c][j], x[c]);
-          }
-          *reinterpret_cast<float4*>(T + r * LDA + c0) = make_float4(x[0], x[1], x[2], x[3]);
-          *reinterpret_cast<float4*>(T + r * LDA + c0 + 4) = make_float4(x[4], x[5], x[6], x[7]);
-        }
-      }
-      if (lane < 8) {  // lane i writes row c0 + i of the pivot block (zero above the diagonal) and 1 / L_ii
-        float row[8], rv = 0.0f;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) row[c] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (i == lane) {
-#pragma unroll
-            for (int c = 0; c <= i; ++c) row[c] = l[i][c];
-            rv = rinv[i];
-          }
-        *reinterpret_cast<float4*>(T + (c0 + lane) * LDA + c0) = make_float4(row[0], row[1], row[2], row[3]);
-        *reinterpret_cast<float4*>(T + (c0 + lane) * LDA + c0 + 4) = make_float4(row[4], row[5], row[6], row[7]);
-        Rinv[c0 + lane] = rv;
-      }
-      if (lane == 0 && bad >= 0 && k * NB + c0 + bad < a.n) atomicCAS(a.info, 0, k * NB + c0 + bad + 1);
-      bar_arrive(1, THREADS);
-    }
-  } else {
-    const int t = threadIdx.x - 32, nthr = THREADS - 32;
-#pragma unroll 1
-    for (int p = 0; p < 8; ++p) {
-      const int c0 = 8 * p;
-      bar_wait(1, THREADS);
-      if (p == 7) break;
-      // look-ahead: the columns c0+8 .. c0+15 of panel p+1, rows below them
-      for (int e = t; e < (NB - c0 - 8) * 8; e += nthr) {
-        const int r = c0 + 8 + (e >> 3), c = c0 + 8 + (e & 7);
-        if (c <= r) panel_update(T, r, c, c0);
-      }
-      bar_arrive(2, THREADS);
-      // the rest of the trailing triangle, columns >= c0 + 16 and rows >= the
-      // column: thread t takes columns c0 + 16 + (t & 15) + 16 m of the rows
-      // c0 + 16 + (t >> 4) + 14 q (no integer division); each row's panel
-      // values are loaded once
-      const int cl = t & 15;
-      for (int r = c0 + 16 + (t >> 4); r < NB; r += nthr / 16) {
-        const float4 a0 = *reinterpret_cast<const float4*>(T + r * LDA + c0);
-        const float4 a1 = *reinterpret_cast<const float4*>(T + r * LDA + c0 + 4);
-        for (int c = c0 + 16 + cl; c <= r; c += 16) {
-          const float4 b0 = *reinterpret_cast<const float4*>(T + c * LDA + c0);
-          const float4 b1 = *reinterpret_cast<const float4*>(T + c * LDA + c0 + 4);
-          float v = T[r * LDA + c];
-          v = fmaf(-a0.x, b0.x, v);
-          v = fmaf(-a0.y, b0.y, v);
-          v = fmaf(-a0.z, b0.z, v);
-          v = fmaf(-a0.w, b0.w, v);
-          v = fmaf(-a1.x, b1.x, v);
-          v = fmaf(-a1.y, b1.y, v);
-          v = fmaf(-a1.z, b1.z, v);
-          v = fmaf(-a1.w, b1.w, v);
-          T[r * LDA + c] = v;
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// L_kk from T (zero above the diagonal) into tile (k, k) of the factor and
-// inv(L_kk) from X into invdiag, 16 bytes per store.
-__device__ __forceinline__ void store_factor_inverse(const DFArgs& a, int k, const float* T, const float* X) {
-  float* g = tile<float>(a, k, k);
-  float* inv = reinterpret_cast<float*>(a.invdiag) + (size_t)k * NB * NB;
-#pragma unroll
-  for (int q = 0; q < NB * NB / 4 / THREADS; ++q) {
-    const int e = threadIdx.x + q * THREADS, r = e >> 4, c = (e & 15) * 4;
-    float4 v = *reinterpret_cast<const float4*>(T + r * LDA + c);
-    if (c + 1 > r) v.y = 0.0f;
-    if (c + 2 > r) v.z = 0.0f;
-    if (c + 3 > r) v.w = 0.0f;
-    if (c > r) v.x = 0.0f;
-    *reinterpret_cast<float4*>(g + (size_t)r * a.ld + c) = v;
-    *reinterpret_cast<float4*>(inv + r * NB + c) = *reinterpret_cast<const float4*>(X + r * LDA + c);
-  }
-}
-
-// Shared memory of an FP32 factor task: the tile, its inverse, the inversion
-// scratch (32 x 36) and 1 / L_jj.
-constexpr size_t factor_task_f32_smem_bytes() { return sizeof(float) * (2 * NB * LDA + 32 * 36 + NB); }
-
-// F(k) as a list task of the batched mixed factorisation: the updated tile
-// (acc) factored and inverted in FP32, L_kk
-// and inv(L_kk) stored; the caller publishes.  smem is free on entry.
-__device__ __forceinline__ void factor_task_f32(const DFArgs& a, int k, const float acc[16], unsigned char* smem) {
-  float* T = reinterpret_cast<float*>(smem);
-  float* X = T + NB * LDA;
-  float* Tm = X + NB * LDA;
-  float* Rinv = Tm + 32 * 36;
-  acc_to_smem(acc, T);
-  __syncthreads();
-  factor_tile_f32(a, k, T, Rinv);
-  invert_factor<float>(T, Rinv, X, Tm);
-  store_factor_inverse(a, k, T, X);
 }
 
 // U(i, j, k) with every tile moved by 16-byte copies: the target tile is
@@ -2194,8 +1955,8 @@ __global__ void __launch_bounds__(THREADS, 1) chol_batch_kernel(const CholRep* _
 // shared memory and three MMAs per K-step add A_hi B_hi + A_hi B_lo + A_lo
 // B_hi to the accumulator, while the tiles of k + 1 are split into a second
 // operand buffer.  Then, by the task's kind:
-//   LL_DIAG (i = j): F(j) -- L_jj and inv(L_jj) in FP32 -- published at once, then S(j + 1, j) = U inv(L_jj)^T with
-//     the inverse still in shared memory;
+//   LL_DIAG (i = j): F(j) (factor_tile, FP64 rounded on store), published at once,
+//     then S(j + 1, j) with the solve blocks still in shared memory;
 //   LL_UPDATE (i > j): U written over A's tiles, upd[r] = j + 1;
 //   LL_SOLVE (i > j, a later segment): S(i, j), S(i + 1, j) from the stored
 //     U once F(j) is published.
@@ -2225,7 +1986,9 @@ enum : int { LL_DIAG = 0, LL_UPDATE = 1, LL_SOLVE = 2 };
 // K-steps (of 64) accumulated in TMEM before the sum is added in FP32
 constexpr int LL_CHUNK = 4;
 constexpr uint32_t LL_U0 = 40960, LL_U1 = 61440;
-static_assert(factor_task_f32_smem_bytes() <= LL_U0, "the factor scratch overlaps U0");
+// F(j)'s tile, solve blocks and scratch take the second buffer's bytes
+constexpr uint32_t LL_FACTOR_BYTES = sizeof(double) * (2 * NB * ChainLd<double>::LT + FACTOR_SCRATCH);
+static_assert(LL_FACTOR_BYTES <= LL_OPERAND_BYTES, "the factor does not fit an operand buffer");
 static_assert(sizeof(float) * 128 * LDA <= LL_U0, "P overlaps U0");
 static_assert(LL_U1 + sizeof(float) * NB * LDA <= LL_OPERAND_BYTES, "U1 lies outside the operand bytes");
 
@@ -2250,8 +2013,9 @@ __device__ __forceinline__ DFArgs batch_args(const CholRep& R, const int4* tasks
   a.upd = R.upd;
   a.fin = R.fin;
   a.info = R.info;
-  a.invdiag = R.invdiag;
-  a.lp = nullptr;
+  a.invdiag = nullptr;
+  a.lp = R.invdiag;  // the solve blocks take the place of the inverses
+  a.min_pivot = 1.17549435e-38;  // a smaller pivot is reported as non-positive
   a.err = reinterpret_cast<unsigned*>(ctl + 3);
   a.spin_limit = SPIN_LIMIT;
   a.X = nullptr;
@@ -2555,17 +2319,26 @@ __device__ bool ll_task(const DFArgs& a, int kind, int i, int j, LLWorker& w, in
     LLPROF(5, LLCLK() - c0);
     c0 = LLCLK();
   }
-  float acc[16];
   if (kind == LL_DIAG) {
-    // F(j) over P's bytes (no longer read), then S(j + 1, j) with inv(L_jj)
-    // where factor_task_f32 left it
+    // F(j) in FP64, as the single-matrix chain does it, in the second buffer's bytes,
+    // then S(j + 1, j) with the solve blocks still in shared memory
     LLPROF(11, 1);
-    smem_to_acc(U0, acc);
-    factor_task_f32(a, j, acc, w.base);
+    constexpr int LT = ChainLd<double>::LT;
+    double* F = reinterpret_cast<double*>(w.base + LL_OPERAND_BYTES);
+    double* V = F + NB * LT;
+    const FactorMem f(F, V, V + NB * LT);
+    for (int e = tid; e < NB * NB; e += THREADS) F[(e >> 6) * LT + (e & 63)] = U0[(e >> 6) * LDA + (e & 63)];
+    if (tid == 0) {
+      f.bad[0] = NB;
+      f.bad[1] = 0;
+    }
+    __syncthreads();
+    factor_tile<float>(a, j, f, reinterpret_cast<float*>(a.lp) + (size_t)j * NB * NB);
     publish(a.fin + j, j + 1);
     if (two) {
-      solve_by_inverse(U1, reinterpret_cast<const float*>(w.base) + NB * LDA, acc);
-      store_acc(tile<float>(a, j + 1, j), a.ld, acc);
+      float* out = tile<float>(a, j + 1, j);
+      solve_rows<1>(U1, LDA, V,
+                    [&](int r, int c, double w0, double w1) { store_pair(out + (size_t)r * a.ld + c, (float)w0, (float)w1); });
       publish(a.fin + j + 1, j + 1);
     }
     LLPROF(6, LLCLK() - c0);
@@ -2580,17 +2353,18 @@ __device__ bool ll_task(const DFArgs& a, int kind, int i, int j, LLWorker& w, in
     if (!ll_wait_rows(a, a.fin, rows, 4u, j + 1, seen, s_ok)) return false;             // F(j)
     LLPROF(7, LLCLK() - c0);
     c0 = LLCLK();
-    float* Xs = reinterpret_cast<float*>(w.base);
-    stage_async(reinterpret_cast<const float*>(a.invdiag) + (size_t)j * NB * NB, NB, Xs, LDA);
+    float* Vs = reinterpret_cast<float*>(w.base);
+    stage_async(reinterpret_cast<const float*>(a.lp) + (size_t)j * NB * NB, NB, Vs, ChainLd<float>::LT);
     stage_async(tile<float>(a, i, j), a.ld, U0, LDA);
     if (two) stage_async(tile<float>(a, i + 1, j), a.ld, U1, LDA);
     cp_async_wait_all();
     __syncthreads();
-    solve_by_inverse(U0, Xs, acc);
-    store_acc(tile<float>(a, i, j), a.ld, acc);
-    if (two) {
-      solve_by_inverse(U1, Xs, acc);
-      store_acc(tile<float>(a, i + 1, j), a.ld, acc);
+    // a tile on four warps each
+    const int h = tid >> 7;
+    if (h == 0 || two) {
+      float* out = tile<float>(a, i + h, j);
+      solve_rows_f32(h ? U1 : U0, LDA, Vs, (tid >> 5) & 3,
+                     [&](int r, int c, float w0, float w1) { store_pair(out + (size_t)r * a.ld + c, w0, w1); });
     }
     __syncthreads();
     if (tid == 0) {
