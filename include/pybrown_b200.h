@@ -392,7 +392,7 @@ PBG_API int pbg_batch_check_factor(pbg_batch *b, int slot, int *info, void *stre
 
 /* Schedule of the batched factorisation (no counterpart in the reference).
  * merge_order: how the replicas' task segments are interleaved in the one
- * task list; ctas_per_sm: resident CTAs per SM of the persistent kernel
+ * task list (the first three: spread evenly over the longest replica's); ctas_per_sm: resident CTAs per SM of the persistent kernel
  * (0 = as many as fit; a larger count is cut to what fits).  No choice
  * changes any result bit.  The mixed batch factors left-looking (tasks per
  * column: the diagonal pair and the updates, then the solves), the FP64 batch
