@@ -16,14 +16,24 @@ namespace pbg {
 
 namespace {
 
-// y_i = sum_j fl(c * A_ij) x_j  (box.py:356: dt / kBT * D @ F).
+// pos_i += (v s1) s2, every product and the sum rounded on its own: the evaluation
+// order of box.py:356,371 (X = M @ v * sqrt(2 dt) * mult) and Bead.translate
+// (bead.py:92-101; all beads mobile).
+__device__ __forceinline__ void apply_move(const Move& mv, int i, double v) {
+  if (mv.pos) mv.pos[i] = __dadd_rn(mv.pos[i], __dmul_rn(__dmul_rn(v, mv.s1), mv.s2));
+}
+
+// y_i = sum_j fl(c * A_ij) x_j  (box.py:356: dt / kBT * D @ F), and the move by it.
 template <typename T>
 __global__ void gemv_scaled_kernel(const T* __restrict__ A, int ld, int n, const double* __restrict__ x,
-                                   double c, double* __restrict__ y) {
+                                   double c, double* __restrict__ y, Move mv) {
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= n) return;
   const double s = row_dot(A + (size_t)row * ld, n, [&](int j, double a) { return (c * a) * x[j]; });
-  if (lane == 0) y[row] = s;
+  if (lane == 0) {
+    y[row] = s;
+    apply_move(mv, row, s);
+  }
 }
 
 // y_i = sum_j fl(c * (A_ij - A0_ij)) x_j  (box.py:306: m dt/(2 kBT) (D - D0) @ F).
@@ -38,22 +48,24 @@ __global__ void gemv_diff_kernel(const T* __restrict__ A, const T* __restrict__ 
   if (lane == 0) y[row] = s;
 }
 
-// y_i = sum_{j <= i} B_ij x_j  (box.py:371: B @ N with B lower triangular).
+// y_i = sum_{j <= i} B_ij x_j  (box.py:371: B @ N with B lower triangular), and
+// the move by it: one launch where the product, its scaling and the
+// translation were three (2.5 us each in a step of 64 beads).
 template <typename T>
 __global__ void trmv_lower_kernel(const T* __restrict__ B, int ld, int n, const double* __restrict__ x,
-                                  double* __restrict__ y) {
+                                  double* __restrict__ y, Move mv) {
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= n) return;
   const double s = row_dot(B + (size_t)row * ld, row + 1, [&](int j, double b) { return b * x[j]; });
-  if (lane == 0) y[row] = s;
+  if (lane == 0) {
+    y[row] = s;
+    apply_move(mv, row, s);
+  }
 }
 
-// out = (in * s1) * s2, the evaluation order of box.py:356,371
-// (X = M @ v * sqrt(2 dt) * mult).
-__global__ void scale2_kernel(const double* __restrict__ in, double s1, double s2, int n,
-                              double* __restrict__ out) {
+__global__ void move_kernel(Move mv, const double* __restrict__ v, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = (in[i] * s1) * s2;
+  if (i < n) apply_move(mv, i, v[i]);
 }
 
 // pos += v (Bead.translate, bead.py:92-101; all beads mobile).
@@ -210,11 +222,11 @@ inline int vec_grid(int n) { return (n + 255) / 256; }
 }  // namespace
 
 int launch_gemv_scaled(const void* A, int ld, int n, int precision, const double* x, double c,
-                       double* y, cudaStream_t st) {
+                       double* y, cudaStream_t st, const Move& mv) {
   if (precision == PBG_PREC_FP64)
-    gemv_scaled_kernel<double><<<rows_grid(n), 256, 0, st>>>((const double*)A, ld, n, x, c, y);
+    gemv_scaled_kernel<double><<<rows_grid(n), 256, 0, st>>>((const double*)A, ld, n, x, c, y, mv);
   else
-    gemv_scaled_kernel<float><<<rows_grid(n), 256, 0, st>>>((const float*)A, ld, n, x, c, y);
+    gemv_scaled_kernel<float><<<rows_grid(n), 256, 0, st>>>((const float*)A, ld, n, x, c, y, mv);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
@@ -230,17 +242,17 @@ int launch_gemv_diff(const void* A, const void* A0, int ld, int n, int precision
 }
 
 int launch_trmv_lower(const void* B, int ld, int n, int precision, const double* x, double* y,
-                      cudaStream_t st) {
+                      cudaStream_t st, const Move& mv) {
   if (precision == PBG_PREC_FP64)
-    trmv_lower_kernel<double><<<rows_grid(n), 256, 0, st>>>((const double*)B, ld, n, x, y);
+    trmv_lower_kernel<double><<<rows_grid(n), 256, 0, st>>>((const double*)B, ld, n, x, y, mv);
   else
-    trmv_lower_kernel<float><<<rows_grid(n), 256, 0, st>>>((const float*)B, ld, n, x, y);
+    trmv_lower_kernel<float><<<rows_grid(n), 256, 0, st>>>((const float*)B, ld, n, x, y, mv);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }
 
-int launch_scale2(const double* in, double s1, double s2, int n, double* out, cudaStream_t st) {
-  scale2_kernel<<<vec_grid(n), 256, 0, st>>>(in, s1, s2, n, out);
+int launch_move(const Move& mv, const double* v, int n, cudaStream_t st) {
+  move_kernel<<<vec_grid(n), 256, 0, st>>>(mv, v, n);
   PBG_CHECK_LAUNCH();
   return PBG_OK;
 }

@@ -59,13 +59,18 @@ __device__ __forceinline__ double row_dot(const T* __restrict__ a, int jend, F t
   return s;
 }
 
+// A move by a vector: pos += (v s1) s2 (pos null: none).
+struct Move {
+  double* pos = nullptr;
+  double s1 = 1.0, s2 = 1.0;
+};
 int launch_gemv_scaled(const void* A, int ld, int n, int precision, const double* x, double c,
-                       double* y, cudaStream_t st);
+                       double* y, cudaStream_t st, const Move& mv = Move());
 int launch_gemv_diff(const void* A, const void* A0, int ld, int n, int precision, const double* x,
                      double c, double* y, cudaStream_t st);
 int launch_trmv_lower(const void* B, int ld, int n, int precision, const double* x, double* y,
-                      cudaStream_t st);
-int launch_scale2(const double* in, double s1, double s2, int n, double* out, cudaStream_t st);
+                      cudaStream_t st, const Move& mv = Move());
+int launch_move(const Move& mv, const double* v, int n, cudaStream_t st);
 int launch_translate(double* pos, const double* v, int n, bool negate, cudaStream_t st);
 int launch_wrap(double* pos, int n3, double L, cudaStream_t st);
 int launch_drift_combine(const double* Dy, const double* Bxi, const double* ddet, double c2, int n,

@@ -131,7 +131,7 @@ void destroy_system(pbg_system* s) {
   free_immobile(s);
   void* ptrs[] = {s->pos,  s->pos_snap, s->radii, s->conn,  s->force, s->D,     s->B,    s->D0,
                   s->Mff,  s->Rff,      s->R,     s->Mff0,  s->Rff0,  s->R0,    s->FX,   s->U,
-                  s->BX,   s->ddet,     s->y,     s->rwork, s->Dy,    s->drift, s->xi,
+                  s->ddet, s->y,     s->rwork, s->Dy,    s->drift, s->xi,
                   s->chol_work, s->inv_work, s->dflags, s->div, s->sol, s->sol0, s->res, s->corr,
                   s->G,    s->tflags};
   for (void* p : ptrs)
@@ -198,7 +198,7 @@ int create_system(const pbg_params* prm, pbg_system** out) {
     SYS_ALLOC(s->inv_work, s->mlub ? tc_inverse_work_bytes(s->ld) : spd_inverse_work_bytes(s->ld));
     if (s->mlub && p.propagation_scheme == PBG_SCHEME_MIDPOINT) SYS_ALLOC(s->G, mat * sizeof(float));
   }
-  double** vecs[] = {&s->FX, &s->U,  &s->BX,   &s->ddet, &s->y,   &s->rwork, &s->Dy,
+  double** vecs[] = {&s->FX, &s->U,  &s->ddet, &s->y,   &s->rwork, &s->Dy,
                      &s->drift, &s->xi, &s->sol, &s->sol0, &s->res, &s->corr};
   for (double** v : vecs) SYS_ALLOC(*v, ld * sizeof(double));
   SYS_ALLOC(s->chol_work, cholesky_work_bytes(s->ld, s->prec));
@@ -434,23 +434,17 @@ static int deterministic_step(pbg_system* s, const void* D, double mult, cudaStr
     // (dt/kBT) D F = dt R^{-1} F, by the refined solve
     int rc = refined_solve(s, D, s->R, step_force(s), s->sol, st);
     if (rc) return rc;
-    if ((rc = launch_scale2(s->sol, s->dt, mult, s->n, s->FX, st))) return rc;
-    return launch_translate(s->pos, s->FX, s->n, false, st);
+    return launch_move(Move{s->pos, s->dt, mult}, s->sol, s->n, st);
   }
   // F = 0: every term of ((dt/kBT) D F) mult is +-0 and pos + (+-0) = pos
   if (!s->ff && s->force_zero) return PBG_OK;
-  int rc = launch_gemv_scaled(D, s->ld, s->n, s->prec, step_force(s), s->dt / s->p.kBT, s->FX, st);
-  if (rc) return rc;
-  rc = launch_scale2(s->FX, 1.0, mult, s->n, s->FX, st);
-  if (rc) return rc;
-  return launch_translate(s->pos, s->FX, s->n, false, st);
+  return launch_gemv_scaled(D, s->ld, s->n, s->prec, step_force(s), s->dt / s->p.kBT, s->FX, st,
+                            Move{s->pos, 1.0, mult});
 }
 
 // Stochastic step (box.py:366-375) from U = B @ xi: pos += (U sqrt(2 dt)) * mult.
 static int stochastic_step(pbg_system* s, double mult, cudaStream_t st) {
-  int rc = launch_scale2(s->U, std::sqrt(2 * s->dt), mult, s->n, s->BX, st);
-  if (rc) return rc;
-  return launch_translate(s->pos, s->BX, s->n, false, st);
+  return launch_move(Move{s->pos, std::sqrt(2 * s->dt), mult}, s->U, s->n, st);
 }
 
 // ---- divergence of the lubricated D (box.py:560-610) ----------------------
@@ -638,11 +632,13 @@ int step_attempt(pbg_system* s, const double* xi, int* accepted, cudaStream_t st
   const int n = s->n;
   int rc;
   PBG_CUDA_TRY(cudaMemcpyAsync(s->xi, xi, n * sizeof(double), cudaMemcpyDefault, st));
-  if ((rc = launch_trmv_lower(s->B, s->ld, n, s->prec, s->xi, s->U, st))) return rc;
+  // U = B xi and the first move of the attempt
+  const double first = s->p.propagation_scheme == PBG_SCHEME_ERMAK ? 1.0 : 1.0 / s->p.m_midpoint;
+  if ((rc = launch_trmv_lower(s->B, s->ld, n, s->prec, s->xi, s->U, st, Move{s->pos, std::sqrt(2 * s->dt), first})))
+    return rc;
   bool overlap = false;
   if (s->p.propagation_scheme == PBG_SCHEME_ERMAK) {
     // box.py:219-248
-    if ((rc = stochastic_step(s, 1.0, st))) return rc;
     if ((rc = overlap_check(s, st, &overlap))) return rc;
     if (overlap) {
       if ((rc = stochastic_step(s, -1.0, st))) return rc;
@@ -654,7 +650,6 @@ int step_attempt(pbg_system* s, const double* xi, int* accepted, cudaStream_t st
   }
   // Midpoint (box.py:272-347).
   const double m = s->p.m_midpoint;
-  if ((rc = stochastic_step(s, 1.0 / m, st))) return rc;
   if ((rc = overlap_check(s, st, &overlap))) return rc;
   if (overlap) {
     if ((rc = stochastic_step(s, -1.0 / m, st))) return rc;
@@ -795,7 +790,7 @@ __global__ void run_gather_kernel(const RunDev* __restrict__ r, int n, double* _
 }
 
 // The undo of a rejected move, pos += (U sqrt(2 dt)) * (-1): the arithmetic of
-// the host-driven undo (scale2 with mult = -1, then translate), each product
+// the host-driven undo (launch_move with mult = -1), each product
 // and sum rounded on its own (no contraction into an FMA).
 __global__ void run_undo_kernel(double* __restrict__ pos, const double* __restrict__ U, double s1, int n,
                                 const int* __restrict__ overlap) {
@@ -827,15 +822,14 @@ __global__ void run_round_update_kernel(RunDev* r, int n, int max_att, const int
 
 }  // namespace
 
-// One round of attempts (six kernels and the overlap flag's reset).
+// One round of attempts (five kernels and the overlap flag's reset).
 static int enqueue_run_round(pbg_system* s, cudaStream_t st, cudaGraphConditionalHandle handle, int use_handle) {
   const int n = s->n;
   RunDev* r = static_cast<RunDev*>(s->d_run);
   run_gather_kernel<<<(n + 255) / 256, 256, 0, st>>>(r, n, s->xi);
   PBG_CHECK_LAUNCH();
-  int rc = launch_trmv_lower(s->B, s->ld, n, s->prec, s->xi, s->U, st);
+  int rc = launch_trmv_lower(s->B, s->ld, n, s->prec, s->xi, s->U, st, Move{s->pos, std::sqrt(2 * s->dt), 1.0});
   if (rc) return rc;
-  if ((rc = stochastic_step(s, 1.0, st))) return rc;
   if ((rc = launch_overlap(s->pos, s->radii, s->N, s->p.box_length, s->p.overlap_treshold, s->conn, s->dflags,
                            st)))
     return rc;

@@ -37,7 +37,7 @@ struct pbg_system {
   void* D0 = nullptr;          // midpoint: step-start D
   double *Mff = nullptr, *Rff = nullptr, *R = nullptr;     // lubrication modes (Mff, Rff FP32 if mlub)
   double *Mff0 = nullptr, *Rff0 = nullptr, *R0 = nullptr;  // midpoint copies
-  double *FX = nullptr, *U = nullptr, *BX = nullptr, *ddet = nullptr, *y = nullptr;
+  double *FX = nullptr, *U = nullptr, *ddet = nullptr, *y = nullptr;
   double *rwork = nullptr, *Dy = nullptr, *drift = nullptr, *xi = nullptr;  // ld each
   double *sol = nullptr, *sol0 = nullptr, *res = nullptr, *corr = nullptr;  // ld each: refined solves (mlub)
   void* chol_work = nullptr;   // inverted diagonal tiles of B
