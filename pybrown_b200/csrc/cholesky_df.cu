@@ -532,7 +532,7 @@ __device__ __forceinline__ void acc_to_smem(const T acc[16], T* s, int lds = LDA
 // triangle -> the next block row's X = S U^T (two MMAs) -> the next pivot block
 // D - X M^T (two MMAs).  Everything else is done by the other warps while the
 // next block is factored.
-// Measured (order 1024, one B200 at 1965 MHz): F(k) 5.0 us, of which 3.4 the
+// Measured (order 1000, one B200 at 1965 MHz): F(k) 5.0 us, of which 3.4 the
 // chain warp on its own (420 ns a block: 190 ns its eight reciprocal steps, the rest the
 // hand-over of D, U and X through shared memory and registers), against 7.7 us
 // (FP64) and 7.0 (FP32) with rows in lanes and one barrier of five warps per
@@ -916,14 +916,14 @@ __device__ __forceinline__ void factor_finish(const FactorMem& f, S* out, int ld
   }
 }
 
-// F(k) of the updated tile f.A (its lower triangle), warps 0 .. 6 (warp 7 returns
-// at once): L_kk to tile (k, k) of the factor (type S, zero above the diagonal),
+// F(k) of the updated tile f.A (its lower triangle) by all warps but FETCH_WARP
+// (which returns at once): L_kk to tile (k, k) of the factor (type S, zero above the diagonal),
 // the solve blocks of L_kk to f.V and to V_out (global 64 x 64, type S, or
 // null): with 8 x 8 blocks, V_jj = inv(L_jj) on the block diagonal and L_jq
 // below it.  (Blocks above the block diagonal are neither written nor read.)
 // A non-positive pivot is recorded in info.  f.bad: {64, 0} on entry; on
-// return, after the caller's next CTA barrier, {64, 8}.  Ends with a barrier of warps 0 .. 6
-// (named barrier 2).
+// return, after the caller's next CTA barrier, {64, 8}.  Ends with a barrier of the
+// seven warps (named barrier 2).
 template <typename S>
 __device__ __forceinline__ void factor_tile(const DFArgs& a, int k, const FactorMem& f, S* V_out) {
   const int warp = threadIdx.x >> 5;

@@ -170,7 +170,7 @@ int tc_reversed_factor(const float* X, const float* G, int ld, double s, float* 
 // Batched factorisation of many independent matrices (one per replica).
 struct CholRep {
   void* A;        // ld x ld, padded with the identity beyond n
-  void* invdiag;  // nt x 64 x 64: inv(L_kk) tiles (FP32), the solve blocks of L_kk (FP64)
+  void* invdiag;  // nt x 64 x 64: the solve blocks of L_kk
   int* upd;       // nt x nt, zero before the launch
   int* fin;       // nt x nt, zero before the launch
   int* info;      // zero before the launch
