@@ -722,7 +722,8 @@ __device__ __forceinline__ void factor_chain(const FactorMem& f) {
       x[c + 1] = v[1];
     }
     // lanes 16 .. 31 repeat lanes 0 .. 15, stores included: nothing here branches
-    const uint32_t row = lane & 8 ? f.U + 8 * ((8 * p + (lane & 7)) * FRAG_LD) : f.A + 8 * ((8 * p + (lane & 7)) * LT + 8 * p);
+    const uint32_t row =
+        lane & 8 ? f.U + 8 * ((8 * p + (lane & 7)) * FRAG_LD) : f.A + 8 * ((8 * p + (lane & 7)) * LT + 8 * p);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       d[j] = j == 0 ? d0 : l[j][j];
