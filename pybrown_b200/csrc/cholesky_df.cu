@@ -668,9 +668,10 @@ __device__ __forceinline__ void sts_pair(uint32_t base, int i, double x, double 
 // 3 of panel p - 1, which the lead reaches after barrier 1 of panel p - 1, that is
 // when all helpers have done panel p - 2.  U, d, r and X keep a place per panel, so warp 7
 // follows the count f.bad[1] of panels (panel p stored, and all of panel p - 1)
-// at its own pace.
+// at its own pace.  The count is published as a maximum: the lead stores its last one
+// (6) after the barrier 3 that lets the chain go on to 7 and 8, in either order.
 __device__ __forceinline__ void panels_done(const FactorMem& f, int n) {
-  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(tc::smem_u32(f.bad) + 4), "r"(n) : "memory");
+  asm volatile("red.release.cta.shared::cta.max.s32 [%0], %1;" ::"r"(tc::smem_u32(f.bad) + 4), "r"(n) : "memory");
 }
 
 // The inverse of pivot block p's unit triangle as a fragment.
