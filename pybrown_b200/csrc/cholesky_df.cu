@@ -134,6 +134,14 @@ __device__ long long g_chain_trace[8 * 1024];
 __device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ float ldcg(const float* p) { return __ldcg(p); }
 
+// A bounded wait ran out: every CTA gives up, and the caller learns of it.
+__device__ __forceinline__ void wait_expired(const DFArgs& a) {
+  atomicExch(a.ctl + 1, 1);
+  atomicAdd(a.ctl + 2, 1);
+  atomicOr(a.err, PBG_DEV_ERR_BARRIER);
+  atomicCAS(a.info, 0, -1);  // -1: the factorisation gave up waiting
+}
+
 // Warp 0 waits until every flags[q] >= targets[q] (count <= 9, bounded);
 // returns false if the run was aborted.  Lane q polls flag q, so one round
 // costs one L2 round trip whatever the count.  The acquire loads followed by
@@ -164,12 +172,7 @@ __device__ bool wait_all(const DFArgs& a, const int* const* flags, const int* ta
         }
       }
       if (it + 1 > a.spin_limit) {
-        if (lane == 0) {
-          atomicExch(a.ctl + 1, 1);
-          atomicAdd(a.ctl + 2, 1);
-          atomicOr(a.err, PBG_DEV_ERR_BARRIER);
-          atomicCAS(a.info, 0, -1);  // -1: the factorisation gave up waiting
-        }
+        if (lane == 0) wait_expired(a);
         ok = 0;
         break;
       }
@@ -863,8 +866,10 @@ __device__ __forceinline__ void factor_help(const FactorMem& f, int h) {
 // and L_pp, and, a panel later, the block column below L_pp, to the factor and to
 // the solve blocks.
 template <typename S>
-__device__ __forceinline__ void factor_finish(const FactorMem& f, S* out, int ld, S* V_out, double min_pivot,
-                                              long long spin_limit) {
+__device__ __forceinline__ void factor_finish(const DFArgs& a, int k, const FactorMem& f, S* V_out) {
+  S* out = tile<S>(a, k, k);
+  const int ld = a.ld;
+  const double min_pivot = a.min_pivot;
   constexpr int LT = ChainLd<double>::LT;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   S* o = out + (size_t)g * ld + 2 * t;
@@ -875,13 +880,15 @@ __device__ __forceinline__ void factor_finish(const FactorMem& f, S* out, int ld
   double q0 = 0, q1 = 0;  // 1 / sqrt(d) of the previous panel's columns 2t, 2t + 1
 #pragma unroll 1
   for (int p = 0; p < 8; ++p) {
-    // bounded like every wait; the other warps do not wait on anything else
-    for (long long it = 0; it < spin_limit; ++it) {
-      int done;
+    // bounded and reported like every wait, but not by the caller's limit: it depends
+    // on no other CTA, and the panels take what they take
+    int done = 0;
+    for (long long it = 0; done <= p && it < SPIN_LIMIT; ++it)
       asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(done) : "r"(tc::smem_u32(f.bad) + 4) : "memory");
-      if (done > p) break;
+    if (!__all_sync(0xffffffffu, done > p)) {
+      if (lane == 0) wait_expired(a);
+      return;
     }
-    __syncwarp();
     const int c = 8 * p + 2 * t;
     const double d = lds_one(f.d, 8 * p + g);
     double u[2], x[2];
@@ -931,7 +938,7 @@ __device__ __forceinline__ void factor_tile(const DFArgs& a, int k, const Factor
   const int warp = threadIdx.x >> 5;
   if (warp == FETCH_WARP) return;
   if (warp == 0) factor_chain(f);
-  else if (warp == 7) factor_finish<S>(f, tile<S>(a, k, k), a.ld, V_out, a.min_pivot, a.spin_limit);
+  else if (warp == 7) factor_finish<S>(a, k, f, V_out);
   else if (warp == 3) factor_lead(f);
   else factor_help(f, warp < 3 ? warp : warp - 2);
   bar_wait(2, 32 * 7);
@@ -1149,10 +1156,7 @@ __device__ __forceinline__ bool warp_wait_geq(const DFArgs& a, const int* flag, 
         break;
       }
       if (it + 1 > a.spin_limit) {
-        atomicExch(a.ctl + 1, 1);
-        atomicAdd(a.ctl + 2, 1);
-        atomicOr(a.err, PBG_DEV_ERR_BARRIER);
-        atomicCAS(a.info, 0, -1);  // -1: the factorisation gave up waiting
+        wait_expired(a);
         ok = 0;
         break;
       }
@@ -2056,12 +2060,7 @@ __device__ bool ll_wait_rows(const DFArgs& a, const int* base, const int (&rows)
         }
       }
       if (it + 1 > a.spin_limit) {
-        if (lane == 0) {
-          atomicExch(a.ctl + 1, 1);
-          atomicAdd(a.ctl + 2, 1);
-          atomicOr(a.err, PBG_DEV_ERR_BARRIER);
-          atomicCAS(a.info, 0, -1);
-        }
+        if (lane == 0) wait_expired(a);
         ok = false;
         break;
       }
@@ -2108,10 +2107,7 @@ __device__ bool ll_thread_wait_rows(const DFArgs& a, const int* base, const int 
       if ((it & 63) == 63) {
         if (ld_acquire(a.ctl + 1)) return false;
         if (it > a.spin_limit) {
-          atomicExch(a.ctl + 1, 1);
-          atomicAdd(a.ctl + 2, 1);
-          atomicOr(a.err, PBG_DEV_ERR_BARRIER);
-          atomicCAS(a.info, 0, -1);
+          wait_expired(a);
           return false;
         }
         __nanosleep(64);
