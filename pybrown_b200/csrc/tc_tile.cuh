@@ -64,13 +64,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* m, uint32_t parity, long lon
 
 // ---------------------------------------------------------------- TMEM
 // Warp-wide (all 32 lanes of one warp): allocate `cols` columns (a power of
-// two >= 32) and write the TMEM address to *dst (shared memory).
+// two >= 32) and write the TMEM address to *dst (shared memory).  These and
+// tmem_ld32 are `.sync.aligned`: the warp has to be converged, also after a
+// branch of one thread or a per-thread wait, hence the __syncwarp in each.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t cols) {
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(cols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -81,6 +85,7 @@ __device__ __forceinline__ void fence_proxy_smem() { asm volatile("fence.proxy.a
 // 32 lanes x 32 columns of FP32 from TMEM (lane quarter of the calling warp).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
