@@ -565,23 +565,23 @@ __device__ __forceinline__ void rpy_tile_body(const RpyArgs& a, int I, int J, vo
         k.cQ = (T)((ai * ai + aj * aj) * a.cQ0);
         const T sx = (T)(rx * a.invL), sy = (T)(ry * a.invL), sz = (T)(rz * a.invL);
         Block6<T> rest;
-        T blk[6];
+        double blk[6];
         if constexpr (sizeof(T) == 8) {
           Block6<T> main;
           pair_sums<SMALL>(k, s_ph[ti], s_ph[TB + tj], s_w, a, sx, sy, sz, main, rest, rest);
 #pragma unroll
           for (int c = 0; c < 6; ++c) blk[c] = main.c[c] + (c < 3 ? rest.c[c] + (main.d + rest.d) : rest.c[c]);
         } else {
+          // FP32 sums, added and scaled in FP64 and rounded once
           ImageSum im;
           pair_sums<SMALL>(k, s_ph[ti], s_ph[TB + tj], s_w, a, sx, sy, sz, im, im, rest);
-          const T d = im.d + (im.r[6] + rest.d);
+          const double d = (double)(im.d + (im.r[6] + rest.d));
 #pragma unroll
           for (int c = 0; c < 6; ++c) {
-            const T o = im.c[c] + (im.r[c] + rest.c[c]);
+            const double o = (double)(im.c[c] + (im.r[c] + rest.c[c]));
             blk[c] = c < 3 ? o + d : o;
           }
         }
-        const T scale = (T)a.scale;
         const double d2 = rx * rx + ry * ry + rz * rz;
         if (d2 < (ai + aj) * (ai + aj)) {
           // Overlap fix (diff_tensor.c:614-643): swap far-field RPY for the
@@ -598,10 +598,10 @@ __device__ __forceinline__ void rpy_tile_body(const RpyArgs& a, int I, int J, vo
           far[4] = f1 * f3 * rx * rz;
           far[5] = f1 * f3 * ry * rz;
 #pragma unroll
-          for (int c = 0; c < 6; ++c) v[c] = (T)(((double)blk[c] + (near[c] - far[c])) * a.scale);
+          for (int c = 0; c < 6; ++c) v[c] = (T)((blk[c] + (near[c] - far[c])) * a.scale);
         } else {
 #pragma unroll
-          for (int c = 0; c < 6; ++c) v[c] = blk[c] * scale;
+          for (int c = 0; c < 6; ++c) v[c] = (T)(blk[c] * a.scale);
         }
       } else {
         double blk[6];
