@@ -164,9 +164,9 @@ template <typename T>
 struct Block6 {
   T c[6] = {0, 0, 0, 0, 0, 0}, d = 0;
 };
-// FP32: the sum of the images, with its rounding errors carried along (r): a plain sum's error
-// grows with the images (|m|_1 <= 8 at alpha = 0.05: 3.0e-6 of the value, 2e-7
-// compensated).
+// FP32: the sum of the images, with its rounding errors carried along (r): a plain
+// sum's error grows with the images (|m|_1 <= 8 at alpha = 0.05: 3.0e-6 of the
+// value, 2e-7 compensated).
 struct ImageSum {
   float c[6] = {0, 0, 0, 0, 0, 0}, d = 0, r[7] = {0, 0, 0, 0, 0, 0, 0};
 };
@@ -213,7 +213,8 @@ __device__ __forceinline__ void add_image(const PairConst<double>& k, double x, 
 }
 // exp(-alpha^2 (s + m)^2), m = -2 .. 2.  FP32: one MUFU exponential each.  FP64:
 // three exponentials, E(m) = E(0) exp(-2 alpha^2 s m) exp(-alpha^2 m^2) (the products
-// taken in an order that cannot overflow for alpha <= 16, |s| <= 1/2).
+// taken in an order that cannot overflow for 2 alpha^2 |s| <= 700: every minimum-image
+// vector for alpha <= 16; pair_sums takes the other pairs to real_sum).
 __device__ __forceinline__ void gauss_axis(const PairConst<float>& k, float s, float (&e)[5]) {
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
@@ -234,9 +235,9 @@ __device__ __forceinline__ void gauss_axis(const PairConst<double>& k, double s,
 // The images |m|_1 <= m_max <= 2 (25 at most), the nearest one (m = 0) first.
 // FP64: it is returned apart from the others, which are summed among themselves.
 // FP32: one compensated sum (main and rest are the same: the largest term comes
-// first, as add_compensated wants it); unrolled, the per-axis values in registers.  FP64: the loops stay
-// rolled (an image is about 100 instructions) with the axis values selected by
-// the uniform loop counters; images +-m_z run side by side.
+// first, as add_compensated wants it); unrolled, the per-axis values in registers.
+// FP64: the loops stay rolled (an image is about 100 instructions) with the axis
+// values selected by the uniform loop counters; images +-m_z run side by side.
 template <typename T, typename A>
 __device__ __forceinline__ void real_sum_small(const PairConst<T>& k, T sx, T sy, T sz, int m_max, A& main, A& rest) {
   T ex[5], ey[5], ez[5];
@@ -484,7 +485,11 @@ __device__ __forceinline__ void pair_sums(const PairConst<T>& k, const V2* pi, c
                                           const RpyArgs& a, T sx, T sy, T sz, A& main, A& images, Block6<T>& recip) {
   if constexpr (SMALL) {
     recip_sum_small<T>(k, pi, pj, w, a.n_max, recip);
-    real_sum_small<T>(k, sx, sy, sz, a.m_max, main, images);
+    // pair vectors of a caller can lie any number of boxes away (see gauss_axis)
+    if (sizeof(T) == 8 && 2.0 * k.alpha2 * fmax(fmax(fabs(sx), fabs(sy)), fabs(sz)) > 700.0)
+      real_sum<T>(k, sx, sy, sz, a.m_max, main, images);
+    else
+      real_sum_small<T>(k, sx, sy, sz, a.m_max, main, images);
   } else {
     recip_sum<T>(k, pi, pj, w, a.n_max, recip);
     real_sum<T>(k, sx, sy, sz, a.m_max, main, images);

@@ -48,8 +48,9 @@ def test_powers_of_two_scale_exactly():
 def test_scaled_once():
     """1 + 2^-24 rounds to 1 in FP32 (a tie), so a scale taken in FP32 leaves every
     element as it is; the FP64 product of a float of mantissa m in (1, 2) moves
-    by m / 2 > 1/2 of its spacing, to the next float."""
+    by m / 2 > 1/2 of its spacing, to the next float: all pair elements off their
+    blocks' diagonals (two thirds) and about half of the others."""
     pos, radii = _config()
     one = _tensor(pos, radii, 2e4, 1, 1.0)
     two = _tensor(pos, radii, 2e4, 1, 1.0 + 2.0 ** -24)
-    assert rel_err(two, one) <= 1.2e-7 and np.count_nonzero(two != one) > 0
+    assert rel_err(two, one) <= 1.2e-7 and np.count_nonzero(two != one) > 0.6 * one.size
