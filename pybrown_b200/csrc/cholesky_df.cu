@@ -551,14 +551,14 @@ template <> struct ChainLd<float> { static constexpr int LT = NB + 4; };
 
 // 1 / d and 1 / sqrt(d) of a pivot: the PTX approximations refined to full
 // precision -- the reciprocal by one third-order step
-// y <- y + y (e + e^2), e = 1 - d y (from ~2^-20 to ~2^-60), the square root by
+// y <- y + y g, g = e + e^2, e = 1 - d y (from ~2^-20 to ~2^-60; y and g are kept
+// apart, see factor_chain), the square root by
 // two Newton-Raphson steps y <- y + y (1 - d y^2) / 2.  d <= 0, NaN and
 // subnormal d give values that are reported as a non-positive pivot and not used.
-__device__ __forceinline__ double pivot_rcp(double d) {
-  double y;
+__device__ __forceinline__ void pivot_rcp(double d, double& y, double& g) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d, y, 1.0);
-  return fma(y, fma(e, e, e), y);
+  g = fma(e, e, e);
 }
 __device__ __forceinline__ double pivot_rsqrt(double x) {
   double y;
@@ -731,11 +731,19 @@ __device__ __forceinline__ void factor_chain(const FactorMem& f) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       d[j] = j == 0 ? d0 : l[j][j];
-      r[j] = pivot_rcp(d[j]);
-      if (j < 7) l[j + 1][j + 1] = fma(-(l[j + 1][j] * l[j + 1][j]), r[j], l[j + 1][j + 1]);
+      double y, gy, m = 0.0;
+      pivot_rcp(d[j], y, gy);
+      r[j] = fma(y, gy, y);
+      if (j < 7) {
+        // the next pivot less l (l / d), with l / d refined beside 1 / d: l^2 would
+        // leave the FP64 range for matrices of 1e-154 or 1e154, at no gain
+        const double u = l[j + 1][j] * y;
+        m = fma(u, gy, u);
+        l[j + 1][j + 1] = fma(-l[j + 1][j], m, l[j + 1][j + 1]);
+      }
 #pragma unroll
       for (int c = j + 1; c < 8; ++c) {
-        const double e = l[c][j] * r[j];
+        const double e = c == j + 1 ? m : l[c][j] * r[j];
         x[c] = fma(-x[j], e, x[c]);
 #pragma unroll
         for (int i = c; i < 8; ++i)
