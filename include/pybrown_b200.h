@@ -165,7 +165,8 @@ PBG_API int pbg_dev_spd_inverse(double *A, int n, int ld, int *info_dev, void *s
 #define PBG_PREC_FP64 0
 #define PBG_PREC_MIXED 1
 /* pbg_dev_cholesky only: as PBG_PREC_MIXED, with every positive pivot accepted
- * (PBG_PREC_MIXED reports one below the smallest normal float as non-positive). */
+ * (PBG_PREC_MIXED reports one below the smallest normal float as non-positive;
+ * PBG_PREC_FP64 one outside 2^-1022 .. 2^1022). */
 #define PBG_PREC_MIXED_FP64_DIAG 2
 
 #define PBG_SCHEME_ERMAK 0

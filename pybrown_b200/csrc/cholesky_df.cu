@@ -69,6 +69,10 @@ enum : int { TASK_XG = 7, TASK_XZ = 8 };
 // step waits (lead_task).
 enum : int { TASK_LEAD = 9 };
 
+// Pivots that a tile's factorisation takes: 1 / d of others is flushed to zero or
+// infinite (pivot_rcp).  They are reported as non-positive.
+constexpr double MIN_PIVOT = 2.2250738585072014e-308, MAX_PIVOT = 4.49423283715579e307;  // 2^-1022, 2^1022
+
 struct DFArgs {
   void* A;
   int ld, n, nt, ntasks;
@@ -84,7 +88,7 @@ struct DFArgs {
   void* X;       // or null: X = inv(L) is formed too (off-diagonal tiles of the ld x ld matrix)
   int* xupd;     // nt * nt: terms applied to X's tile (i, j)
   int* xfin;     // nt * nt: X's tile (i, j) final
-  double min_pivot = 0.0;  // a pivot below it counts as non-positive
+  double min_pivot = MIN_PIVOT;  // a pivot below it counts as non-positive
 };
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -553,8 +557,8 @@ template <> struct ChainLd<float> { static constexpr int LT = NB + 4; };
 // precision -- the reciprocal by one third-order step
 // y <- y + y g, g = e + e^2, e = 1 - d y (from ~2^-20 to ~2^-60; y and g are kept
 // apart, see factor_chain), the square root by
-// two Newton-Raphson steps y <- y + y (1 - d y^2) / 2.  d <= 0, NaN and
-// subnormal d give values that are reported as a non-positive pivot and not used.
+// two Newton-Raphson steps y <- y + y (1 - d y^2) / 2.  d <= 0, NaN and d outside
+// MIN_PIVOT .. MAX_PIVOT give values that factor_finish reports.
 __device__ __forceinline__ void pivot_rcp(double d, double& y, double& g) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d, y, 1.0);
@@ -922,7 +926,7 @@ __device__ __forceinline__ void factor_finish(const DFArgs& a, int k, const Fact
         store_pair(V_out + r1 * NB + c - 8, (S)z[0], (S)z[1]);
       }
     }
-    const unsigned bad = __ballot_sync(0xffffffffu, !(d > 0.0 && d >= min_pivot));
+    const unsigned bad = __ballot_sync(0xffffffffu, !(d >= min_pivot && d <= MAX_PIVOT));
     const double rg = pivot_rsqrt(d);
     q0 = __shfl_sync(0xffffffffu, rg, 8 * t);
     q1 = __shfl_sync(0xffffffffu, rg, 8 * t + 4);
@@ -2527,7 +2531,7 @@ size_t df_smem_bytes() {
 template <typename T>
 int launch_df(T* A, int n, int ld, int* info, void* invdiag, bool inv_tasks, int* ints, void* lp, unsigned* err,
               cudaStream_t st, const int4* tasks_override = nullptr, int ntasks_override = 0,
-              long long spin_limit = SPIN_LIMIT, T* X = nullptr, double min_pivot = 0.0) {
+              long long spin_limit = SPIN_LIMIT, T* X = nullptr, double min_pivot = MIN_PIVOT) {
   const int nt = ld / NB;
   const int4* tasks = nullptr;
   int ntasks = 0;
@@ -2716,7 +2720,7 @@ int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* i
                                      SPIN_LIMIT, (double*)X);
   // PBG_PREC_MIXED reports a pivot below the smallest normal float as non-positive
   return launch_df<float>((float*)A, n, ld, info, invdiag, want_inv, ints, lp, err, st, nullptr, 0, SPIN_LIMIT, (float*)X,
-                          precision == PBG_PREC_MIXED_FP64_DIAG ? 0.0 : 1.17549435e-38);
+                          precision == PBG_PREC_MIXED_FP64_DIAG ? MIN_PIVOT : 1.17549435e-38);
 }
 
 
