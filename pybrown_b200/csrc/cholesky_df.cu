@@ -1065,7 +1065,7 @@ __device__ __forceinline__ void solve_rows_f32(const float* C, int ldc, const fl
     unsigned ah[4], al[4];
     float w[4], d[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int u = 0; u < 4; ++u) split_tf32(p[j][at[u]] + q[j][at[u]], ah[u], al[u]);
+    for (int u = 0; u < 4; ++u) tc::split_tf32_any(p[j][at[u]] + q[j][at[u]], ah[u], al[u]);
     mul(d, e, ah, al, V + 8 * j * LT + 8 * j);
 #pragma unroll
     for (int u = 0; u < 4; ++u) w[u] = d[u] + e[u];

@@ -31,12 +31,25 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // conversion unit, whose 16 results per clock and SM bound the split (24 K
 // conversions per K-step of 128 + 64 rows: 1540 of 1840 cycles).  hi: round to
 // nearest on the bits, ties away.  lo = x - hi is exact, then rounded by
-// Veltkamp's splitting.  An infinity stays one; a NaN stays one in lo, whatever
-// the bits of hi become.
+// Veltkamp's splitting.  For |x| < 2^126: beyond it the splitting's product
+// overflows and lo is NaN (split_tf32_any takes every finite x).  The operands are
+// elements of a factor of an FP32 matrix, below 2^64, or of its inverse.  x infinite or
+// NaN: lo is NaN.
 __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
   hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
   const float l = __fsub_rn(x, __uint_as_float(hi)), c = __fmul_rn(l, 8193.0f);
   lo = __float_as_uint(__fsub_rn(c, __fsub_rn(c, l)));
+}
+
+// The same for any finite x (matrix elements), on the conversion unit.
+__device__ __forceinline__ uint32_t rna_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void split_tf32_any(float x, uint32_t& hi, uint32_t& lo) {
+  hi = rna_tf32(x);
+  lo = rna_tf32(x - __uint_as_float(hi));
 }
 
 // ---------------------------------------------------------------- mbarrier
