@@ -364,13 +364,22 @@ int compute_Dtot(pbg_system* s, cudaStream_t st, bool factor_B) {
   return rc;
 }
 
+// B comes from another factorisation of this step, which reports for it: the info word
+// that a factorisation of D or R on its own left in an earlier step no longer holds.
+static int clear_info(pbg_system* s, int word, cudaStream_t st) {
+  PBG_CUDA_TRY(cudaMemsetAsync(s->dflags + word, 0, sizeof(int), st));
+  return PBG_OK;
+}
+
 // box.py:546-556: B = chol(D), lower.
 int decompose(pbg_system* s, cudaStream_t st) {
   if (s->p.hydrodynamics == PBG_HI_NONE) return PBG_OK;
   if (s->mlub) {
     // chol(kBT inv(R)) = sqrt(kBT) J G^{-T} J: read off X = inv(G), no second factorisation
     int rc;
-    if (!s->work_holds_R && (rc = factor_reversed_R(s, s->dflags + 1, st))) return rc;
+    if (s->work_holds_R) rc = clear_info(s, 1, st);
+    else rc = factor_reversed_R(s, s->dflags + 1, st);
+    if (rc) return rc;
     const TcInverseWork w = tc_inverse_work(s->inv_work, s->ld);
     if ((rc = tc_reversed_factor(w.X, w.F, s->ld, std::sqrt(s->p.kBT), (float*)s->B, (float*)s->chol_work, st)))
       return rc;
@@ -383,6 +392,8 @@ int decompose(pbg_system* s, cudaStream_t st) {
   }
   if (s->b_holds_G) {
     s->b_holds_G = false;
+    int rc = clear_info(s, 1, st);
+    if (rc) return rc;
     return launch_reversed_factor((double*)s->B, s->ld, std::sqrt(s->p.kBT), s->inv_work, (double*)s->chol_work, st);
   }
   if (!s->b_holds_lower_D) {
