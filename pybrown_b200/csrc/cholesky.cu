@@ -92,6 +92,13 @@ int launch_spd_inverse_reversed(double* G, int ld, int* info, void* work, cudaSt
   return launch_lauum(X, inv, ld, scale, true, out, st);
 }
 
+int launch_first_pivot(const double* R, int n, int ld, int* info, void* work, cudaStream_t st) {
+  unsigned char* w = static_cast<unsigned char*>(work);
+  double* A = reinterpret_cast<double*>(w + spd_x_offset(ld));
+  PBG_CUDA_TRY(cudaMemcpyAsync(A, R, (size_t)ld * ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  return launch_cholesky_ws(A, n, ld, PBG_PREC_FP64, info, work, st);
+}
+
 int launch_reversed_factor(double* G, int ld, double s, const void* work, double* invdiag, cudaStream_t st) {
   const unsigned char* w = static_cast<const unsigned char*>(work);
   return launch_reversed_factor_tiles<double>(reinterpret_cast<const double*>(w + spd_x_offset(ld)),

@@ -143,7 +143,10 @@ int launch_lauum(const double* X, const double* invdiag, int ld, double scale, b
 // and writes the inverses of that factor's diagonal tiles.
 int launch_spd_inverse_reversed(double* G, int ld, int* info, void* work, cudaStream_t st, double scale, double* out);
 int launch_reversed_factor(double* G, int ld, double s, const void* work, double* invdiag, cudaStream_t st);
-// The second with G, inv(G) (X, its diagonal tiles in Xdiag when that is not null)
+// info = the first non-positive pivot of R in its own order (1-based, 0: none); R is kept
+// (its copy is factored in the workspace of an SPD inverse).
+int launch_first_pivot(const double* R, int n, int ld, int* info, void* work, cudaStream_t st);
+// launch_reversed_factor with G, inv(G) (X, its diagonal tiles in Xdiag when that is not null)
 // and B apart; B may be G.
 template <typename T>
 int launch_reversed_factor_tiles(const T* X, const T* Xdiag, const T* G, int ld, double s, T* B, T* invdiag,

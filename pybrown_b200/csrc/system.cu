@@ -361,6 +361,7 @@ int compute_Dtot(pbg_system* s, cudaStream_t st, bool factor_B) {
   PBG_CHECK_LAUNCH();
   rc = launch_spd_inverse_reversed(G, s->ld, s->dflags + 3, s->inv_work, st, p.kBT, (double*)s->D);
   s->b_holds_G = factor_B && rc == PBG_OK;
+  s->reversed_R = s->R;
   return rc;
 }
 
@@ -368,6 +369,21 @@ int compute_Dtot(pbg_system* s, cudaStream_t st, bool factor_B) {
 // that a factorisation of D or R on its own left in an earlier step no longer holds.
 static int clear_info(pbg_system* s, int word, cudaStream_t st) {
   PBG_CUDA_TRY(cudaMemsetAsync(s->dflags + word, 0, sizeof(int), st));
+  return PBG_OK;
+}
+
+// A refused factorisation of J R J counts its pivots from the end of R and of its padding;
+// the step reports the first non-positive one in R's own order, as the inverse of R
+// would (or, where rounding lets that order pass, the place of the one found).
+static int report_first_pivot(pbg_system* s, cudaStream_t st) {
+  const int found = s->ld + 1 - s->hflags[3];
+  int rc = launch_first_pivot(s->reversed_R, s->n, s->ld, s->dflags + 3, s->inv_work, st);
+  if (rc) return rc;
+  PBG_CUDA_TRY(cudaMemcpyAsync(s->hflags + 3, s->dflags + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
+  PBG_CUDA_TRY(cudaStreamSynchronize(st));
+  if (s->hflags[3]) return PBG_OK;
+  s->hflags[3] = found;
+  PBG_CUDA_TRY(cudaMemcpyAsync(s->dflags + 3, s->hflags + 3, sizeof(int), cudaMemcpyHostToDevice, st));
   return PBG_OK;
 }
 
@@ -737,6 +753,8 @@ int step_end(pbg_system* s, cudaStream_t st, double* pos_out) {
   PBG_CUDA_TRY(cudaMemcpyAsync(s->hflags, s->dflags, 5 * sizeof(int), cudaMemcpyDeviceToHost, st));
   PBG_CUDA_TRY(cudaStreamSynchronize(st));
   if (pos_out) std::memcpy(pos_out, s->hpos, pos_bytes);
+  if (s->reversed_R && s->hflags[3] > 0 && (rc = report_first_pivot(s, st))) return rc;
+  s->reversed_R = nullptr;
   if (s->hflags[4] < 0) {
     PBG_CUDA_TRY(cudaMemsetAsync(s->dflags + 4, 0, sizeof(int), st));
     pbg_set_error_message("a device-wide wait in the back substitution gave up");

@@ -31,6 +31,7 @@ struct pbg_system {
   double* force = nullptr;     // ld (3N used)
   bool force_zero = true;        // the external force is known to be zero (pbg_set_force from host or NULL)
   bool b_holds_G = false;  // this step's D build left chol(J R J) in B and its inverse in inv_work
+  const double* reversed_R = nullptr;  // the R whose reversed factorisation this step's dflags[3] is of (FP64)
   bool b_holds_lower_D = false;  // this step's D build also wrote B's lower triangle (and padding)
   void* D = nullptr;           // ld x ld, prec
   void* B = nullptr;           // ld x ld, prec, lower factor
