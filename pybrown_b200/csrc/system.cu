@@ -356,6 +356,9 @@ int compute_Dtot(pbg_system* s, cudaStream_t st, bool factor_B) {
                                   p.viscosity / 1e19, s->R, s->ld, st);
   if (rc) return rc;
   const long long total = (long long)s->ld * s->ld;
+  // sqrt(kBT) J G^{-T} J is the factor for kBT > 0; otherwise decompose factors D itself,
+  // and refuses it as numpy's does
+  factor_B = factor_B && p.kBT > 0 && std::isfinite(p.kBT);
   double* G = (double*)(factor_B ? s->B : s->D);
   reverse_kernel<double><<<grid_for(total), 256, 0, st>>>(s->R, s->ld, G);
   PBG_CHECK_LAUNCH();
