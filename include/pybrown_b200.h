@@ -393,9 +393,9 @@ PBG_API int pbg_batch_check_factor(pbg_batch *b, int slot, int *info, void *stre
 
 /* Schedule of the batched factorisation (no counterpart in the reference).
  * merge_order: how the replicas' task segments are interleaved in the one
- * task list (the first three: spread evenly over the longest replica's); ctas_per_sm: resident CTAs per SM of the persistent kernel
- * (0 = as many as fit; a larger count is cut to what fits).  No choice
- * changes any result bit.  The mixed batch factors left-looking (tasks per
+ * task list (the first three: spread evenly over the longest replica's);
+ * ctas_per_sm: resident CTAs per SM of the persistent kernel (0 = as many as fit;
+ * a larger count is cut to what fits).  No choice changes any result bit.  The mixed batch factors left-looking (tasks per
  * column: the diagonal pair and the updates, then the solves), the FP64 batch
  * right-looking (tasks per panel: F, updates, solves); the segments merged are
  * those. */
@@ -433,6 +433,13 @@ PBG_API int pbg_batch_autotune(pbg_batch *b, int reps, int *best, float *ms, voi
  * fit or nt < 1. */
 PBG_API int pbg_cholesky_task_list(int nt, int precision, int *tasks, int cap, int *seg, int seg_cap,
                                    int *n_tasks, int *n_segs);
+/* The merged list of a batch (host only, no device needed; no counterpart in
+ * the reference): for replicas of nts[q] tile rows, the (replica, segment) pairs in
+ * the order in which merge_order strings their segments together (segments of
+ * pbg_cholesky_task_list; empty ones included).  out: 2 x cap entries; *n_out receives
+ * the count; PBG_ERR_ARG if it does not fit or an argument is out of range. */
+PBG_API int pbg_cholesky_merge_list(int precision, int merge_order, const int *nts, int n_replicas, int *out, int cap,
+                                    int *n_out);
 /* How the start of a step (Ewald build, copy into B, factorisation,
  * deterministic move) -- or with pbg_batch_step the whole step -- runs:
  * 1 = one CUDA graph launch (captured once a step

@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -768,6 +769,63 @@ void drop_graphs(pbg_batch* b) {
   }
 }
 
+// One replica of a merged task list: its segments, tile rows and matrix bytes.
+struct MergeItem {
+  int segments, nt;
+  size_t bytes;
+};
+
+// The order of the replicas' task segments (see cholesky_df.cu) in the one list, as
+// (replica, segment): every replica's spread evenly over the longest one's, so
+// that the smaller ones fill the waits of the longest to its end instead of its
+// first columns only (a serving batch of 24: 3277 -> 3201 us; FP64, 40 replicas:
+// 161 -> 150), at one place with larger matrices first (default), in the order the
+// replicas were added, or smaller first; replica after replica (all of one
+// replica's segments, larger replicas first); or larger first in chunks of
+// replicas whose matrices fit a byte budget, chunk after chunk.  Each replica's own
+// segments keep their order in every policy, so every task still depends
+// only on earlier tasks.
+std::vector<std::pair<int, int>> merge_segments(int merge_order, const std::vector<MergeItem>& r) {
+  const int R = (int)r.size();
+  int longest = 0;
+  std::vector<int> order(R);
+  for (int q = 0; q < R; ++q) {
+    order[q] = q;
+    longest = std::max(longest, r[q].segments);
+  }
+  if (merge_order != PBG_MERGE_ADDED) {
+    const bool larger = merge_order != PBG_MERGE_SMALLER_FIRST;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return larger ? r[x].nt > r[y].nt : r[x].nt < r[y].nt; });
+  }
+  std::vector<std::pair<int, int>> out;
+  auto push = [&](int q, int sg) {
+    if (sg < r[q].segments) out.emplace_back(q, sg);
+  };
+  if (merge_order == PBG_MERGE_REPLICA_MAJOR) {
+    for (int q : order)
+      for (int sg = 0; sg < longest; ++sg) push(q, sg);
+  } else if (merge_order >= PBG_MERGE_CHUNK_32M) {
+    // chunks of consecutive (larger-first) replicas within the byte budget
+    const size_t budget = (size_t)32 << (20 + (merge_order - PBG_MERGE_CHUNK_32M));
+    for (size_t c0 = 0; c0 < order.size();) {
+      size_t c1 = c0, bytes = 0;
+      do bytes += r[order[c1++]].bytes;
+      while (c1 < order.size() && bytes + r[order[c1]].bytes <= budget);
+      for (int sg = 0; sg < longest; ++sg)
+        for (size_t q = c0; q < c1; ++q) push(order[q], sg);
+      c0 = c1;
+    }
+  } else {
+    std::vector<int> next(R, 0);
+    for (int tick = 0; tick < longest; ++tick)
+      for (int q : order)
+        for (; next[q] < r[q].segments && next[q] * (long long)longest / r[q].segments == tick; ++next[q])
+          push(q, next[q]);
+  }
+  return out;
+}
+
 // Rebuilds the device descriptors and work lists of the current membership:
 // small per-replica descriptors from the host, the task and tile work lists
 // assembled on the device from each replica's cached list.
@@ -827,7 +885,6 @@ int rebuild(pbg_batch* b, cudaStream_t st) {
   std::vector<int4> eparts(R);
   size_t flag_ints = 4, n_ework = 0, ntasks = 0;
   std::vector<size_t> flag_off(R);
-  int max_seg = 0;
   for (int q = 0; q < R; ++q) {
     const BatchReplica* r = b->slots[b->active[q]];
     flag_off[q] = flag_ints;
@@ -837,7 +894,6 @@ int rebuild(pbg_batch* b, cudaStream_t st) {
     eparts[q] = make_int4(T, (int)n_ework, 0, 0);
     n_ework += (size_t)T * (T + 1) / 2;
     ntasks += r->seg_start.empty() ? 0 : r->seg_start.back();
-    max_seg = std::max(max_seg, (int)r->seg_start.size() - 1);
   }
   // after the per-replica flags: the infos, the attempt counts and the step
   // words, contiguous so that one copy reports a step
@@ -883,62 +939,19 @@ int rebuild(pbg_batch* b, cudaStream_t st) {
     c.nt = r->nt;
     c.pad = 0;
   }
-  // Merge order of the replicas' task segments (see cholesky_df.cu): every
-  // replica's spread evenly over the longest one's, so that the smaller ones fill
-  // the waits of the longest to its end instead of its first columns only (a
-  // serving batch of 24: 3277 -> 3201 us; FP64, 40 replicas: 161 -> 150), at one
-  // place with larger matrices first (default), in the order the
-  // replicas were added, or smaller first; replica after replica (all of one
-  // replica's segments, larger replicas first); or larger first in chunks of
-  // replicas whose matrices fit a byte budget, chunk after chunk.  Each replica's own
-  // segments keep their order in every policy, so every task still depends
-  // only on earlier tasks.
-  std::vector<int> order(R);
-  for (int q = 0; q < R; ++q) order[q] = q;
-  if (b->merge_order != PBG_MERGE_ADDED) {
-    const bool larger = b->merge_order != PBG_MERGE_SMALLER_FIRST;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-      const int nx = b->slots[b->active[x]]->nt, ny = b->slots[b->active[y]]->nt;
-      return larger ? nx > ny : nx < ny;
-    });
+  std::vector<MergeItem> items(R);
+  for (int q = 0; q < R; ++q) {
+    const BatchReplica* r = b->slots[b->active[q]];
+    items[q] = MergeItem{(int)r->seg_start.size() - 1, r->nt, (size_t)r->ld * r->ld * elem_size(b->precision)};
   }
   std::vector<GatherSeg> segs;
   long long dst = 0;
-  auto push_seg = [&](int q, int sg) {
-    const BatchReplica* r = b->slots[b->active[q]];
-    if (sg + 1 >= (int)r->seg_start.size()) return;
-    const int count = r->seg_start[sg + 1] - r->seg_start[sg];
-    if (count <= 0) return;
-    segs.push_back(GatherSeg{r->tasks + r->seg_start[sg], dst, count, q});
+  for (const auto& e : merge_segments(b->merge_order, items)) {
+    const BatchReplica* r = b->slots[b->active[e.first]];
+    const int start = r->seg_start[e.second], count = r->seg_start[e.second + 1] - start;
+    if (count <= 0) continue;
+    segs.push_back(GatherSeg{r->tasks + start, dst, count, e.first});
     dst += count;
-  };
-  if (b->merge_order == PBG_MERGE_REPLICA_MAJOR) {
-    for (int q : order)
-      for (int sg = 0; sg < max_seg; ++sg) push_seg(q, sg);
-  } else if (b->merge_order >= PBG_MERGE_CHUNK_32M) {
-    // chunks of consecutive (larger-first) replicas within the byte budget
-    const size_t budget = (size_t)32 << (20 + (b->merge_order - PBG_MERGE_CHUNK_32M));
-    const size_t es = b->precision == PBG_PREC_FP64 ? 8 : 4;
-    for (size_t c0 = 0; c0 < order.size();) {
-      size_t c1 = c0, bytes = 0;
-      do {
-        const BatchReplica* r = b->slots[b->active[order[c1]]];
-        bytes += (size_t)r->ld * r->ld * es;
-        ++c1;
-      } while (c1 < order.size() && bytes + (size_t)b->slots[b->active[order[c1]]]->ld *
-                                                b->slots[b->active[order[c1]]]->ld * es <= budget);
-      for (int sg = 0; sg < max_seg; ++sg)
-        for (size_t q = c0; q < c1; ++q) push_seg(order[q], sg);
-      c0 = c1;
-    }
-  } else {
-    // every replica's segments spread evenly over the longest one's
-    std::vector<int> next(R, 0);
-    for (int tick = 0; tick < max_seg; ++tick)
-      for (int q : order) {
-        const long long n = (long long)b->slots[b->active[q]]->seg_start.size() - 1;
-        for (; next[q] < n && next[q] * (long long)max_seg / n == tick; ++next[q]) push_seg(q, next[q]);
-      }
   }
   if ((rc = ensure(b->d_reps, b->cap_reps, R * sizeof(BatchDev))) ||
       (rc = ensure(b->d_rpy, b->cap_rpy, rpy.size())) ||
@@ -1076,6 +1089,29 @@ PBG_API int pbg_cholesky_task_list(int nt, int precision, int* tasks, int cap, i
     tasks[4 * t + 3] = list[t].w;
   }
   for (size_t q = 0; q < starts.size(); ++q) seg[q] = starts[q];
+  return PBG_OK;
+}
+
+PBG_API int pbg_cholesky_merge_list(int precision, int merge_order, const int* nts, int n_replicas, int* out, int cap,
+                                    int* n_out) {
+  if (!nts || !out || !n_out || n_replicas < 1 || merge_order < 0 || merge_order >= PBG_MERGE_ORDERS)
+    return PBG_ERR_ARG;
+  std::vector<MergeItem> items;
+  for (int q = 0; q < n_replicas; ++q) {
+    if (nts[q] < 1) return PBG_ERR_ARG;
+    std::vector<int4> list;
+    std::vector<int> starts;
+    cholesky_replica_tasks(nts[q], precision, list, starts);
+    const size_t ld = (size_t)nts[q] * PBG_TILE;
+    items.push_back(MergeItem{(int)starts.size() - 1, nts[q], ld * ld * elem_size(precision)});
+  }
+  const auto merged = merge_segments(merge_order, items);
+  *n_out = (int)merged.size();
+  if ((int)merged.size() > cap) return PBG_ERR_ARG;
+  for (size_t e = 0; e < merged.size(); ++e) {
+    out[2 * e] = merged[e].first;
+    out[2 * e + 1] = merged[e].second;
+  }
   return PBG_OK;
 }
 

@@ -2728,9 +2728,10 @@ int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* i
 // F(0), S(i, 0); then for each k three segments F(k+1) | U(i, j, k) (j >= k+2)
 // | S(i, k+1) (i >= k+2).  F(k+1) and S(., k+1) apply their update with panel
 // k themselves.  seg_start holds 1 + 3(nt-1) segment starts and the end.
-// A batch merges the replicas' lists segment number by segment number (all
-// replicas' segment s, larger matrices first, then segment s+1): every
-// replica's F(k+1), then every replica's U(., ., k), then every replica's
+// A batch merges the replicas' lists segment by segment in one of several orders
+// (merge_segments in batch.cu) that all keep each replica's own; the default
+// spreads every replica's evenly over the longest one's.  With replicas of one size that
+// is every replica's F(k+1), then every replica's U(., ., k), then every replica's
 // S(., k+1), so the solves are fetched after their factorisations had the
 // whole update phase to finish.  F(k+1) and U(., ., k) depend only on block
 // k-1; S(., k+1) on F(k+1) and block k-1: every task depends only on earlier
@@ -2739,9 +2740,9 @@ int launch_cholesky_df(void* A, int n, int ld, int precision, int* info, void* i
 // The mixed-precision lists are left-looking (chol_batch_ll_kernel), two
 // segments per column j: LL_DIAG for rows (j, j + 1) and LL_UPDATE for the
 // row pairs (j + 2, j + 3), (j + 4, j + 5), ...; then LL_SOLVE for the same
-// pairs.  Merged by segment number, every replica's solves of column j come
-// after every replica's updates of column j, so F(j) has had that phase to
-// finish; column j + 1's tasks need column j's solves and come after them.
+// pairs.  Column j + 1's tasks need column j's solves and come after them; among
+// replicas of one size, every one's solves of column j come after every one's
+// updates of it, so F(j) has had that phase to finish.
 void cholesky_replica_tasks(int nt, int precision, std::vector<int4>& tasks, std::vector<int>& seg_start) {
   tasks.clear();
   seg_start.clear();
