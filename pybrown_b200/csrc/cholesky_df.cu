@@ -227,13 +227,6 @@ __device__ __forceinline__ void stage_async(const T* g, int ld, T* s, int lds) {
   }
 }
 
-// Asynchronous copy of `count` contiguous T (count * sizeof(T) a multiple of 16).
-template <typename T>
-__device__ __forceinline__ void copy_async(const T* g, T* s, int count) {
-  constexpr int elems = 16 / (int)sizeof(T);
-  for (int t = threadIdx.x; t < count / elems; t += THREADS) cp_async16(s + t * elems, g + t * elems);
-}
-
 // Row-major copy of a 64 x 64 smem tile (rows of `lds`) to global, 16 bytes per store.
 template <typename T>
 __device__ __forceinline__ void store_tile(const T* s, int lds, T* g, int ld) {
@@ -1266,8 +1259,9 @@ __device__ void run_chain(const DFArgs& a, unsigned char* smem, int* s_ok) {
 // staged into sC with cp.async together with L_ik, L_jk (instead of per-thread
 // 4-byte loads), updated in registers, and written back through sC with
 // 16-byte stores.  sC: a third [64][LDA] tile.
-template <typename T>
-__device__ __forceinline__ void update_tile(const DFArgs& a, int i, int j, int k, T acc[16], T* sA, T* sB, T* sC) {
+__device__ __forceinline__ void update_tile(const DFArgs& a, int i, int j, int k, double acc[16], double* sA, double* sB,
+                                            double* sC) {
+  using T = double;
   stage_async(tile<T>(a, i, k), a.ld, sA, LDA);
   if (i != j) stage_async(tile<T>(a, j, k), a.ld, sB, LDA);
   stage_async(tile<T>(a, i, j), a.ld, sC, LDA);
@@ -1283,9 +1277,9 @@ __device__ __forceinline__ void update_tile(const DFArgs& a, int i, int j, int k
 // U(i, j, k) and U(i+1, j, k) together: five tiles (L_ik, L_jk, L_{i+1,k} and
 // both targets) staged with 16-byte copies in one round, two accumulators
 // against the shared L_jk, one round of 16-byte stores.  s: five [64][LDA]
-// T tiles.
-template <typename T>
-__device__ __forceinline__ void update_tile_pair(const DFArgs& a, int i, int j, int k, T acc[16], T* s) {
+// FP64 tiles.
+__device__ __forceinline__ void update_tile_pair(const DFArgs& a, int i, int j, int k, double acc[16], double* s) {
+  using T = double;
   T* sA1 = s;
   T* sB = sA1 + NB * LDA;
   T* sC1 = sB + NB * LDA;
@@ -1790,28 +1784,32 @@ __device__ void df_worker_loop(const DFArgs& a, unsigned char* smem, int* s_task
       publish(a.fin + k * nt + k, 2);
       TRACE(2, t);
     } else if (type == TASK_U) {
-      // U(i, j, k): needs L_ik, L_jk final and the k previous updates of (i, j)
-      const int* fl[3] = {a.fin + i * nt + k, a.fin + j * nt + k, a.upd + i * nt + j};
-      const int tg[3] = {1, 1, k};
-      if (!wait_all(a, fl, tg, 3, &s_ok)) return;
-      TRACE(1, t);
-      update_tile(a, i, j, k, acc, sA, sB, sB + NB * LDA);
-      publish(a.upd + i * nt + j, k + 1);
-      TRACE(2, t);
-    } else if (type == TASK_U2) {
-      // U(i, j, k) and U(i+1, j, k): L_ik, L_{i+1,k}, L_jk final, k previous updates of both
-      const int* fl[5] = {a.fin + i * nt + k, a.fin + (i + 1) * nt + k, a.fin + j * nt + k, a.upd + i * nt + j,
-                          a.upd + (i + 1) * nt + j};
-      const int tg[5] = {1, 1, 1, k, k};
-      if (!wait_all(a, fl, tg, 5, &s_ok)) return;
-      TRACE(1, t);
-      update_tile_pair(a, i, j, k, acc, sA);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        st_release(a.upd + i * nt + j, k + 1);
-        st_release(a.upd + (i + 1) * nt + j, k + 1);
+      if constexpr (sizeof(T) == 8) {  // FP32: on the tensor cores, above
+        // U(i, j, k): needs L_ik, L_jk final and the k previous updates of (i, j)
+        const int* fl[3] = {a.fin + i * nt + k, a.fin + j * nt + k, a.upd + i * nt + j};
+        const int tg[3] = {1, 1, k};
+        if (!wait_all(a, fl, tg, 3, &s_ok)) return;
+        TRACE(1, t);
+        update_tile(a, i, j, k, acc, sA, sB, sB + NB * LDA);
+        publish(a.upd + i * nt + j, k + 1);
+        TRACE(2, t);
       }
-      TRACE(2, t);
+    } else if (type == TASK_U2) {
+      if constexpr (sizeof(T) == 8) {  // FP32: on the tensor cores, above
+        // U(i, j, k) and U(i+1, j, k): L_ik, L_{i+1,k}, L_jk final, k previous updates of both
+        const int* fl[5] = {a.fin + i * nt + k, a.fin + (i + 1) * nt + k, a.fin + j * nt + k, a.upd + i * nt + j,
+                            a.upd + (i + 1) * nt + j};
+        const int tg[5] = {1, 1, 1, k, k};
+        if (!wait_all(a, fl, tg, 5, &s_ok)) return;
+        TRACE(1, t);
+        update_tile_pair(a, i, j, k, acc, sA);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          st_release(a.upd + i * nt + j, k + 1);
+          st_release(a.upd + (i + 1) * nt + j, k + 1);
+        }
+        TRACE(2, t);
+      }
     } else if (type == TASK_LEAD) {
       if (!lead_task<T>(a, k, i, sA, &s_ok)) return;
       TRACE(2, t);
@@ -1860,7 +1858,7 @@ __global__ void __launch_bounds__(THREADS, 1) chol_df_kernel(DFArgs a) {
 // left-looking chol_batch_ll_kernel below): every task comes from the shared
 // list (there is no chain CTA); F(k) applies its last update itself.  Shared
 // memory: two tiles (sA, sB) for the updates and solves; F uses two tiles
-// (L_kk, inverse) over the same bytes and the factor scratch after them.
+// (L_kk, its solve blocks) over the same bytes and the factor scratch after them.
 constexpr size_t batch_smem_bytes() {
   // an F task's tile, solve blocks and factor scratch, or a paired update's five tiles
   return std::max(sizeof(double) * (2 * NB * ChainLd<double>::LT + FACTOR_SCRATCH),
@@ -2853,23 +2851,17 @@ int launch_cholesky_batch(int precision, const CholRep* reps, const int4* tasks,
 
 // ---------------------------------------------------------------- SPD inverse on the tensor cores
 // inv(A) = X^T X with A = L L^T and X = inv(L): the data-flow factorisation
-// forms X's off-diagonal tiles in the same launch (XG / XZ tasks), then X's
-// diagonal tiles are copied from invdiag and X^T X runs with one CTA per lower
-// tile.  Every tile product is
-// TileMMA: FP64 DMMA for FP64 matrices, 3xTF32 split products with FP32
-// accumulation for FP32 ones.  Used by the SPD inverse of the FP64
-// lubrication path (cholesky.cu) and by the mixed lubricated path, which also
-// reads the factor of kBT inv(R) off X (tc_reversed_factor).
+// forms X's off-diagonal tiles in the same launch (XG / XZ tasks, on TileMMA: FP64
+// DMMA, or 3xTF32 split products with FP32 accumulation), then X^T X is formed.
+// FP64 (lauum_kernel): one CTA per lower tile, X's diagonal tiles read from invdiag.
+// FP32 (sym_tc_kernel, tcgen05): pairs of tiles, the diagonal ones copied into X
+// first.  Used by the SPD inverse (cholesky.cu) and by the lubricated steps, which
+// also read the factor of kBT inv(R) off X (launch_reversed_factor_tiles).
 //
 // Mixed workspace (tc_inverse_work_bytes): [inv(L_kk) tiles][data-flow
 // scratch][X: ld x ld][F: ld x ld], F the matrix to factor (in place).
 
 namespace {
-
-template <typename T>
-constexpr size_t tc_smem_bytes() {
-  return 2 * NB * LDA * sizeof(T);
-}
 
 // X_kk = inv(L_kk), upper triangle zero (one CTA per diagonal tile).
 template <typename T>

@@ -46,11 +46,16 @@ constexpr int THREADS = TB * TB;
 
 // Constants of the pair terms, cO = 1/(8 pi L), cQ = (ai^2+aj^2)/(24 pi L^3).
 template <typename T>
-struct PairConst {
+struct PairSums {
   T cO, cQ, alpha, alpha2;
   T o;       // 2 alpha / sqrt(pi)
   T q2;      // 4 alpha^3 / sqrt(pi)
-  T k1, k4;  // exp(-alpha^2), exp(-4 alpha^2)
+};
+template <typename T>
+struct PairConst : PairSums<T> {};
+template <>
+struct PairConst<double> : PairSums<double> {
+  double k1, k4;  // exp(-alpha^2), exp(-4 alpha^2)
 };
 
 struct RpyArgs {
@@ -118,8 +123,8 @@ __device__ __forceinline__ double erfcx_poly(double x) {
   for (int i = 1; i < 23; ++i) p = fma(p, t, c_erfcx[i]);
   return p * r;
 }
-// 1 / sqrt(x) for normal x > 0: the PTX estimate and one third-order step
-// y <- y + y h (1/2 + 3/8 h), h = 1 - x y^2.
+// 1 / sqrt(x) for normal x > 0: the PTX estimate and one third-order step (Householder's
+// method) y <- y + y h (1/2 + 3/8 h), h = 1 - x y^2.
 __device__ __forceinline__ double rsqrt_step(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -838,10 +843,9 @@ static void fill_args(RpyArgs& a, const PairSource& src, const double* pos, cons
   if (smith && t) {
     a.alpha = t->alpha;
     const double al = t->alpha, sqrt_pi = std::sqrt(PBG_PI);
-    a.kd = PairConst<double>{1.0 / (8 * PBG_PI * src.L), 0.0, al, al * al, 2 * al / sqrt_pi, 4 * al * al * al / sqrt_pi,
+    a.kd = PairConst<double>{{1.0 / (8 * PBG_PI * src.L), 0.0, al, al * al, 2 * al / sqrt_pi, 4 * al * al * al / sqrt_pi},
                              std::exp(-al * al), std::exp(-4 * al * al)};
-    a.kf = PairConst<float>{(float)a.kd.cO, 0.0f, (float)al, (float)a.kd.alpha2, (float)a.kd.o, (float)a.kd.q2,
-                            (float)a.kd.k1, (float)a.kd.k4};
+    a.kf = PairConst<float>{{(float)a.kd.cO, 0.0f, (float)al, (float)a.kd.alpha2, (float)a.kd.o, (float)a.kd.q2}};
     a.w = t->d_w;
     a.w_f = t->d_w_f;
     a.m_max = t->m_max;

@@ -35,13 +35,6 @@ __global__ void copy_lower_pad_kernel(const T* __restrict__ src, T* __restrict__
 }
 
 template <typename T>
-__global__ void cast_matrix_kernel(const double* __restrict__ src, T* __restrict__ dst, long long total) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x)
-    dst[t] = (T)src[t];
-}
-
-template <typename T>
 __global__ void export_matrix_kernel(const T* __restrict__ src, int n, int ld, int lower_only,
                                      double* __restrict__ dst) {
   const long long total = (long long)n * n;
