@@ -23,9 +23,11 @@
 //    cos and sin of 2 pi s by angle addition: no per-vector phase tables.
 // The minimum image does not enter the reciprocal part (the phase is
 // periodic), only the real-space images.
-// Measured (one B200, m_max = 2, n_max = 4): 1024 beads FP64 110 us (225 before
-// these forms; FP64 pipe 68% busy), FP32 42 us (107; 77% of the issue slots);
-// 1999 beads FP32 132 us (374).
+// Measured (one B200, m_max = 2, n_max = 4), before these forms -> now: 1000 beads
+// FP64 217 -> 100 us (FP64 pipe 67% busy), FP32 107 -> 53 us (75% of the issue
+// slots; a quarter of it the compensated image sum); 1999 beads FP32 374 -> 192 us.
+// Larger lattices (the rolled sums), 1000 beads, alpha = sqrt(pi), m_max = 3, n_max
+// = 5: FP64 494 -> 275 us, FP32 193 -> 148 us.
 #include <cmath>
 #include <cstring>
 #include <map>
