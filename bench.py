@@ -321,11 +321,12 @@ def mixed_vs_oracle(pos, radii, seed, steps=5):
 
 # DRAM bytes (read + write) of one mixed factorisation of the N=1024 matrix,
 # from one ncu capture of the same kernel on the same order
-# (profiles/chol_df_mixed_order3072_full.md):
-#   ncu --set full --clock-control none -k regex:chol_df -s 1 -c 1 \
+# (profiles/tile_kernels_counters.md):
+#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none \
+#       -k regex:chol_df -s 1 -c 1 \
 #       python -m pybrown_b200.profile_cases cholesky --order 3072 --precision mixed --reps 1
-# (19,468,544 + 1,830,912 B); re-measure when the factorisation changes.
-CHOL_MIXED_TRAFFIC_BYTES = 19468544 + 1830912
+# (19,848,960 + 1,235,456 B); re-measure when the factorisation changes.
+CHOL_MIXED_TRAFFIC_BYTES = 19848960 + 1235456
 
 
 def replica_seed(rank):
@@ -572,7 +573,7 @@ def run_batch_section(args, torch):
             "steps": args.steps, "ms_per_step": ms / args.steps,
             "bead_steps_per_s": beads * args.steps / (ms * 1e-3),
             "replica_steps_per_s": 256 * args.steps / (ms * 1e-3), "gpu_launches_per_step": launches,
-            "host_launch_calls_per_step": calls, "attempt_rounds_per_step": attempts / args.steps,
+            "host_launch_calls_per_step": calls, "max_attempts_per_step": attempts / args.steps,
             "step_graph": {1: "one CUDA graph launch per step (attempt rounds under a device-side WHILE node)",
                            0: "direct launches", -1: "capture refused"}[graph],
             "schedule": {"merge_order": tune["merge_order"], "ctas_per_sm": tune["ctas_per_sm"],
